@@ -46,17 +46,11 @@ typedef enum mk_device_status {
 
 enum { MK_ROPE_HF = 0, MK_ROPE_HALF_SWAP = 1 };
 /* TCGEN05: tensor-core projections (tcgen05.mma, TMEM accumulators) for every launch.
- * FMA: decode launches of at most 4 tokens run the small-launch kernel, which consumes its
- *      TMA-fed weight ring without tcgen05 (a matrix-vector product cannot fill a 128-row
- *      MMA): CUDA-core FMAs for one token (the row table: one grid barrier per launch),
- *      warp-level mma.sync for two to four; every other launch uses tcgen05.  Falls back to
- *      tcgen05 when the shape does not fit the small kernel (hidden > 2048 or a K slice
- *      longer than 2048).
+ * FMA: decode launches of up to 32 sequences run the streaming decode kernel (weights and cache tiles through one TMA ring,
+ *      warp-level mma.sync, no grid barrier between phases); every other launch uses tcgen05, and so do shapes
+ *      the streaming kernel does not cover (hidden > 2048, tensor parallel).
  * AUTO: the faster of the two per launch; today the same choice as FMA.
- * (Value 1 named a bring-up engine without TMA or tensor cores; it is gone and rejected.)
- * Process-wide tunables of the small-launch kernel, read by mk_create: MEGABAKE_SMALL_RING_KB
- * (weight ring of the one-token kernel, 64..152, default 120) and MEGABAKE_SMALL_COPY_KB
- * (its largest weight copy, default 36). */
+ * (Value 1 named a bring-up engine without TMA or tensor cores; it is gone and rejected.) */
 enum { MK_ENGINE_TCGEN05 = 0, MK_ENGINE_FMA = 2, MK_ENGINE_AUTO = 3 };
 
 /* Decoder shape.  Mirrors the facts the reference reads off the captured graph
@@ -138,8 +132,8 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
  * src/megabake/bodies/gemm.py:1809-1843. */
 int mk_bind_weights(mk_handle handle, const mk_weights* weights, void* stream);
 
-/* One decode step for `batch` sequences, no sync: one cooperative launch (the small-launch kernel for
- * up to 4 sequences under MK_ENGINE_AUTO / MK_ENGINE_FMA when the shape allows, else the tensor engine).
+/* One decode step for `batch` sequences, no sync: one cooperative launch (the streaming kernel for
+ * up to 32 sequences under MK_ENGINE_AUTO / MK_ENGINE_FMA when the shape allows, else the tensor engine).
  * ids/positions: int64 [batch].  key_caches/value_caches: host arrays of
  * config.layers device pointers, each bf16 [batch, capacity, kv_heads,
  * head_dim] contiguous.  valid_lengths: host array of config.layers device

@@ -14,17 +14,17 @@ from pathlib import Path
 PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libmegabake_b200.so"
-SOURCES = [CSRC / "api.cu", CSRC / "reference_mma_baseline.cu"]
+SOURCES = sorted(CSRC.glob("*.cu"))
 
 
 def headers() -> list[Path]:
     """Every header the library is built from: a new .cuh cannot be forgotten."""
-    return sorted(CSRC.glob("*.cuh")) + sorted((PACKAGE.parent / "include").glob("*.h"))
+    return sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + sorted((PACKAGE.parent / "include").glob("*.h"))
 
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
+    "--threads", "0", "-shared", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
 ]
 
 

@@ -15,7 +15,8 @@
 #include <algorithm>
 #include <vector>
 
-#include "decode_small.cuh"
+#include "decoder_kernel.cuh"
+#include "stream_plan.h"
 
 using namespace mk;
 
@@ -40,7 +41,10 @@ int fail(int code, const char* fmt, ...) {
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct Carve {
-  size_t ctrl, tmaps, kvmaps, phases, hidden, hidden2, xnorm, qkv, qkv_ll, act_ll, att_ll, attn_ll, res_a, res_b, attn, act, partial, partial2, att_xch, att_part, host_io, total;
+  size_t ctrl, tmaps, kvmaps, phases, hidden, hidden2, xnorm, qkv, attn, act, partial, att_xch, att_part, host_io;
+  size_t splan, smaps, slayers, sunits, srec;          // streaming decode kernel
+  size_t handover, handover_bytes, shalf[5][3], spart[2][3];       // its hand-over buffers, filled with the unset word
+  size_t total;
 };
 
 int qkv_width(const mk_config& c) { return (c.q_heads + 2 * c.kv_heads) * c.head_dim; }
@@ -54,7 +58,7 @@ int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 :
 size_t maps_per_table(const mk_config& c) { return 7 * static_cast<size_t>(c.layers) + 1; }
 size_t phases_per_table(const mk_config& c) { return 4 * static_cast<size_t>(c.layers) + 1; }
 
-Carve carve(const mk_config& c) {
+Carve carve(const mk_config& c, int grid) {
   Carve v{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -64,26 +68,47 @@ Carve carve(const mk_config& c) {
   };
   const size_t m = static_cast<size_t>(c.max_tokens);
   v.ctrl = take(sizeof(Control));
-  v.tmaps = take(sizeof(CUtensorMap) * (4 * maps_per_table(c) + 1 + kOperandMaps));  // split, plain and small-launch tables, mk_linear, token operands, row table
+  v.tmaps = take(sizeof(CUtensorMap) * (2 * maps_per_table(c) + kOperandMaps));  // split and plain tables, token operands
   v.kvmaps = take(sizeof(CUtensorMap) * 2 * static_cast<size_t>(c.layers) * kCacheMapSets);  // decode attention: per set, key caches then value caches
-  v.phases = take(sizeof(GemmPhase) * (4 * phases_per_table(c) + 1));  // + the one-token row table
+  v.phases = take(sizeof(GemmPhase) * 2 * phases_per_table(c));
   v.hidden = take(m * c.hidden * 2);
   v.hidden2 = take(m * c.hidden * 2);
   v.xnorm = take(m * c.hidden * 2);
   v.qkv = take(m * qkv_width(c) * 2);
-  v.qkv_ll = take(static_cast<size_t>(kSplitTokens) * qkv_width(c) * 4);
-  v.act_ll = take(static_cast<size_t>(kSplitTokens) * c.intermediate * 4);
-  v.att_ll = take(static_cast<size_t>(kSplitTokens) * c.q_heads * kMaxChunks * c.head_dim * 8);
-  v.attn_ll = take(static_cast<size_t>(kSplitTokens) * c.q_heads * c.head_dim * 4);
-  v.res_a = take(static_cast<size_t>(kSplitTokens) * c.hidden * 4);  // stamped residual stream after the MLP
-  v.res_b = take(static_cast<size_t>(kSplitTokens) * c.hidden * 4);  // ... and after attention
   v.attn = take(m * c.q_heads * c.head_dim * 2);
   v.act = take(m * c.intermediate * 2);
-  v.partial = take(static_cast<size_t>(kMaxSplit) * std::max<size_t>(m, kSplitTokens) * c.hidden * 4);
-  v.partial2 = take(static_cast<size_t>(kMaxSplit) * kSplitTokens * c.hidden * 4);  // down-proj partials of the small-launch table
+  v.partial = take(static_cast<size_t>(kMaxSplit) * m * c.hidden * 4);
   v.att_xch = take(m * c.kv_heads * kMaxChunks * kExchangeFloats * 4);
   v.att_part = take(m * c.q_heads * kMaxChunks * c.head_dim * 4);
   v.host_io = take(3 * m * sizeof(int64_t));  // mk_decode_step_host: ids, positions, sampled tokens
+  if (stream_shape_ok(c)) {
+    const size_t tokens = std::min<size_t>(m, kStreamTokens);
+    v.splan = take(sizeof(StreamPlan) * kStreamPlans);
+    v.smaps = take(sizeof(CUtensorMap) * kStreamPlans * maps_per_table(c));
+    v.slayers = take(sizeof(StreamLayer) * c.layers);
+    v.sunits = take(sizeof(int) * kStreamPlans * kStreamPhases * (kStreamMaxGrid + 1));
+    v.srec = take(tokens * c.q_heads * kStreamMaxSegments * (c.head_dim + 2) * 8);
+    size_t part[2] = {0, 0};
+    for (int i = 0; i < kStreamPlans && stream_plan_used(c, i); ++i) {
+      StreamPhase ph[kStreamPhases];
+      stream_phases(c, i, grid, ph);
+      const size_t t = std::min<size_t>(tokens, 8u << i);
+      for (int k = 0; k < kStreamPhases; ++k) {
+        const size_t sums = static_cast<size_t>(ph[k].ntiles) * t * kStreamRows * sizeof(float);
+        if (ph[k].nslice > 1) part[k == SP_O ? 0 : 1] = std::max(part[k == SP_O ? 0 : 1], sums * ph[k].nslice);
+      }
+    }
+    v.handover = off;
+    size_t copied = 0;
+    for (int i = 0; i <= stream_class_of(static_cast<int>(tokens)); ++i) copied = std::max<size_t>(copied, kStreamClassTokens[i] * stream_copies(kStreamClassTokens[i]));
+    const size_t widths[5] = {static_cast<size_t>(qkv_width(c)), static_cast<size_t>(c.q_heads) * c.head_dim, static_cast<size_t>(c.hidden),
+                              static_cast<size_t>(c.hidden), static_cast<size_t>(c.intermediate)};
+    for (int b = 0; b < 5; ++b)
+      for (int h = 0; h < 3; ++h) v.shalf[b][h] = take(copied * widths[b] * 2);
+    for (int b = 0; b < 2; ++b)
+      for (int h = 0; h < 3; ++h) v.spart[b][h] = take(part[b]);
+    v.handover_bytes = off - v.handover;
+  }
   v.total = off;
   return v;
 }
@@ -109,9 +134,35 @@ int check_config(const mk_config& c) {
   return MK_OK;
 }
 
+// What this library needs to know of a device, asked for once: the clock-rate query goes to the driver's control path and
+// took 2 to 170 ms per handle on a busy host.
+struct DeviceFacts {
+  int known = 0, sms = 0, major = 0, coop = 0, khz = 0;
+};
+int device_facts(int device, DeviceFacts* out) {
+  constexpr int kDevices = 64;
+  static std::mutex lock;
+  static DeviceFacts all[kDevices];
+  std::lock_guard<std::mutex> guard(lock);
+  if (device < 0 || device >= kDevices) return fail(MK_ERR_INVALID, "device %d outside [0, %d)", device, kDevices);
+  DeviceFacts& f = all[device];
+  if (!f.known) {
+    MK_CUDA(cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, device));
+    MK_CUDA(cudaDeviceGetAttribute(&f.major, cudaDevAttrComputeCapabilityMajor, device));
+    MK_CUDA(cudaDeviceGetAttribute(&f.coop, cudaDevAttrCooperativeLaunch, device));
+    MK_CUDA(cudaDeviceGetAttribute(&f.khz, cudaDevAttrClockRate, device));
+    f.known = 1;
+  }
+  *out = f;
+  if (f.major != 10) return fail(MK_ERR_UNSUPPORTED, "device %d is sm_%d0; this library is built for sm_100a only", device, f.major);
+  if (!f.coop) return fail(MK_ERR_UNSUPPORTED, "device %d does not support cooperative launch", device);
+  return MK_OK;
+}
+
 int device_grid(const mk_config& c, int device, int* grid) {
-  int sms = 0;
-  MK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  DeviceFacts facts;
+  if (int e = device_facts(device, &facts)) return e;
+  const int sms = facts.sms;
   *grid = (c.sm_limit > 0 && c.sm_limit < sms) ? c.sm_limit : sms;
   return MK_OK;
 }
@@ -231,20 +282,17 @@ struct mk_handle_s {
   int64_t launches;
   long long timeout_cycles;
   float att_scale;
-  bool fma_ok;  // the small-launch kernel can run the split-K table: every K slice fits its fp32 operand buffer
-  bool row_ok;    // the one-token row table (no K split, no per-layer grid barrier) is available
-  bool small_ll;  // its q/k/v phases hand their outputs to attention as stamped words (one grid barrier fewer per layer)
   unsigned long long* trace;
   int trace_cap;
-  int small_ring;       // weight ring of the small-launch kernel, 1 KiB granules
-  int fat_copy;         // largest weight copy of the small-launch tables, bytes (three to four fit the ring)
   struct CacheMapSet {
     std::vector<const void*> seen;  // cache pointers the set's descriptors were encoded for (keys, then values)
-    int capacity = 0, batch = 0;
+    int capacity = 0, batch = 0, heads = 0, keys = 0;  // geometry the boxes were encoded for
     uint64_t used = 0;              // launch counter at the last use (least recently used is replaced)
   };
   CacheMapSet kv_sets[kCacheMapSets];
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
+  bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
+  StreamPhase stream_ph[kStreamPlans][kStreamPhases];
   bool use3d;           // weight descriptors of the tensor engine are three-dimensional (several K chunks per copy)
   uint32_t tp_epoch;    // all-reduces launched so far (tensor parallel)
   uint8_t* tp_peer[kMaxTp];
@@ -335,16 +383,8 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
 }
 
 // The split-K table (o_proj and down_proj cut along K so that every SM streams, fp32 partial sums added by
-// the next norm phase) serves every launch of a single-GPU handle.  The small-launch kernel further needs a
-// reduction length of at most 2048 per K slice (its fp32 operand buffer).
+// the next norm phase) serves every launch of a single-GPU handle.
 bool split_table_ok(const mk_config& c) { return c.tp_size <= 1; }
-bool small_shape_ok(const mk_config& c) { return c.hidden / kChunkK <= kBSlots && c.tp_size <= 1; }
-
-// One-token launches run the row table with the handle's ring; the split-K table of two to four tokens
-// measured best with a 92 KiB ring and copies of at most 30 KiB.
-constexpr int kSplitTableRing = 92;
-constexpr int kBoxCopyBytes = 30 * 1024;
-int small_ring_for(mk_handle h, int tokens) { return tokens == 1 ? h->small_ring : std::min(h->small_ring, kSplitTableRing); }
 
 void base_params(mk_handle h, KParams& p) {
   memset(&p, 0, sizeof(p));
@@ -367,7 +407,6 @@ void base_params(mk_handle h, KParams& p) {
   p.trace = h->trace;
   p.trace_cap = h->trace ? h->trace_cap : 0;
   p.status_mirror = h->mirror;
-  p.small_ring = small_ring_for(h, 1);  // launches of two to four tokens overwrite it
   p.ctrl = at<Control>(h, h->cv.ctrl);
   p.att_xch = at<float>(h, h->cv.att_xch);
   p.att_part = at<float>(h, h->cv.att_part);
@@ -378,45 +417,40 @@ void base_params(mk_handle h, KParams& p) {
   p.qkv = at<bf16>(h, h->cv.qkv);
   p.attn = at<bf16>(h, h->cv.attn);
   p.act = at<bf16>(h, h->cv.act);
-  p.qkv_ll = at<unsigned long long>(h, h->cv.qkv_ll);
-  p.att_ll = at<unsigned long long>(h, h->cv.att_ll);
-  p.attn_ll = at<unsigned long long>(h, h->cv.attn_ll);
   p.embed = static_cast<const bf16*>(h->weights.embed);
   p.cos_t = static_cast<const bf16*>(h->weights.rope_cos);
   p.sin_t = static_cast<const bf16*>(h->weights.rope_sin);
 }
 
-// The small-launch kernel is instantiated per token count (1..kSplitTokens).
-// One kernel per token count, and one more for the one-token row table (`row`): code that is compiled in
-// but never runs still costs instruction-cache reach.
-const void* small_kernel(int tokens, bool row) {
-  if (row) return reinterpret_cast<const void*>(&megakernel_small<1, true>);
-  switch (tokens) {
-    case 1: return reinterpret_cast<const void*>(&megakernel_small<1, false>);
-    case 2: return reinterpret_cast<const void*>(&megakernel_small<2, false>);
-    case 3: return reinterpret_cast<const void*>(&megakernel_small<3, false>);
-    default: return reinterpret_cast<const void*>(&megakernel_small<4, false>);
-  }
-}
-
-int prepare_small_kernels(int device, int ring_granules) {
-  for (int t = 0; t <= kSplitTokens; ++t) {  // 0: the row-table kernel
-    const void* fn = small_kernel(t, t == 0);
-    const int bytes = small_smem_bytes(t == 0 ? ring_granules : std::min(ring_granules, kSplitTableRing));
-    MK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    MK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (bytes * 100 + 233471) / 233472));
+// Shared-memory attributes belong to the function: set once per device and process (each call costs milliseconds once
+// kernels have run).  head_dim 0: the tensor engine only.
+int prepare_kernels(int device, int head_dim) {
+  constexpr int kDevices = 64;
+  static std::mutex lock;
+  static bool tensor_done[kDevices], stream_done[kDevices][2];
+  std::lock_guard<std::mutex> guard(lock);
+  if (device < 0 || device >= kDevices) return fail(MK_ERR_INVALID, "device %d outside [0, %d)", device, kDevices);
+  if (!tensor_done[device]) {
+    MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
     int per_sm = 0;
-    MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSmallThreads, bytes));
-    if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the small-launch megakernel does not fit on an SM of device %d", device);
+    MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, megakernel, kThreads, kSmemBytes));
+    if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the megakernel does not fit on an SM of device %d", device);
+    tensor_done[device] = true;
+  }
+  if (head_dim && !stream_done[device][head_dim == 128]) {
+    for (int i = 0; i < kStreamClasses; ++i)
+      MK_CUDA(cudaFuncSetAttribute(stream_kernel(i, head_dim), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmemLimit));
+    stream_done[device][head_dim == 128] = true;
   }
   return MK_OK;
 }
 
-int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0, bool small = false) {
+int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
   void* args[] = {&p};
-  if (small)
-    MK_CUDA(cudaLaunchCooperativeKernel(small_kernel(p.m, p.rowmode != 0), dim3(h->grid), dim3(kSmallThreads), args, small_smem_bytes(p.small_ring),
-                                        static_cast<cudaStream_t>(stream)));
+  if (p.splan)
+    MK_CUDA(cudaLaunchCooperativeKernel(stream_kernel(stream_class_of(p.m), p.head_dim), dim3(h->grid), dim3(kStreamThreads), args,
+                                        stream_smem_bytes(p), static_cast<cudaStream_t>(stream)));
   else
     MK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&megakernel), dim3(h->grid), dim3(kThreads), args,
                                         kSmemBytes, static_cast<cudaStream_t>(stream)));
@@ -424,6 +458,12 @@ int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0, bool
   h->att_epoch += static_cast<uint32_t>(attention_phases);
   h->launches += 1;
   return MK_OK;
+}
+
+// The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.
+bool stream_usable(mk_handle h, int batch, bool ragged) {
+  return h->cfg.engine != MK_ENGINE_TCGEN05 && batch <= kStreamTokens && h->stream_ok[stream_plan_of(batch)] &&
+         h->kv_maps_ok && stream_parts_ok(h->cfg, batch, h->grid) && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
 }
 
 int token_tiles(int m) { return (m + token_tile_of(m) - 1) / token_tile_of(m); }
@@ -440,6 +480,67 @@ int attention_fits(mk_handle h, int keys, const char* what) {
 
 }  // namespace
 
+namespace {
+// The streaming decode kernel's plans: descriptors (boxes of 16 rows x the phase's chunks), the per-layer vectors,
+// and every CTA's units of each phase.
+int bind_stream(mk_handle h, const mk_weights& w, std::vector<CUtensorMap>& maps, std::vector<StreamLayer>& layers,
+                std::vector<int>& units, StreamPlan* plans) {
+  const mk_config& c = h->cfg;
+  const int L = c.layers, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const size_t nmaps = maps_per_table(c);
+  maps.resize(kStreamPlans * nmaps);
+  units.assign(static_cast<size_t>(kStreamPlans) * kStreamPhases * (kStreamMaxGrid + 1), 0);
+  for (int l = 0; l < L; ++l) {
+    const mk_layer_weights& lw = w.layers[l];
+    StreamLayer& sl = layers[l];
+    sl.input_norm = static_cast<const bf16*>(lw.input_norm);
+    sl.post_norm = static_cast<const bf16*>(lw.post_norm);
+    const void* biases[3] = {lw.q_bias, lw.k_bias, lw.v_bias};
+    for (int i = 0; i < 3; ++i) sl.bias[i] = c.qkv_bias ? static_cast<const bf16*>(biases[i]) : nullptr;
+  }
+  for (int i = 0; i < kStreamPlans; ++i) {
+    h->stream_ok[i] = false;
+    if (!stream_plan_used(c, i)) continue;
+    StreamPlan& plan = plans[i];
+    stream_phases(c, i, h->grid, plan.ph);
+    memcpy(h->stream_ph[i], plan.ph, sizeof(plan.ph));
+    for (int l = 0; l < L; ++l) {
+      const mk_layer_weights& lw = w.layers[l];
+      const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
+      const int rows[7] = {q_size, kv_size, kv_size, c.hidden, c.intermediate, c.intermediate, c.hidden};
+      const int which[7] = {SP_QKV, SP_QKV, SP_QKV, SP_O, SP_GU, SP_GU, SP_DOWN};
+      for (int m = 0; m < 7; ++m)
+        if (int e = encode_weight_map3(&maps[i * nmaps + 7 * l + m], mats[m], rows[m], plan.ph[which[m]].k, plan.ph[which[m]].rows, kStreamKb)) return e;
+    }
+    if (int e = encode_weight_map3(&maps[i * nmaps + 7 * L], w.lm_head, c.vocab, c.hidden, plan.ph[SP_HEAD].rows, kStreamKb)) return e;
+    int* table = units.data() + static_cast<size_t>(i) * kStreamPhases * (kStreamMaxGrid + 1);
+    stream_deal_units(plan.ph, h->grid, table);
+    plan.maps = at<CUtensorMap>(h, h->cv.smaps) + i * nmaps;
+    plan.layers = at<StreamLayer>(h, h->cv.slayers);
+    plan.final_norm = static_cast<const bf16*>(w.final_norm);
+    plan.units = at<int>(h, h->cv.sunits) + static_cast<size_t>(i) * kStreamPhases * (kStreamMaxGrid + 1);
+    for (int half = 0; half < 3; ++half) {
+      const int next = (half + 1) % 3;
+      bf16 *qkv = at<bf16>(h, h->cv.shalf[0][half]), *attn = at<bf16>(h, h->cv.shalf[1][half]), *res_in = at<bf16>(h, h->cv.shalf[2][half]);
+      bf16 *res_next = at<bf16>(h, h->cv.shalf[2][next]), *res_mid = at<bf16>(h, h->cv.shalf[3][half]), *act = at<bf16>(h, h->cv.shalf[4][half]);
+      const bf16* src[kStreamPhases] = {res_in, attn, res_mid, act, res_in};
+      bf16* dst[kStreamPhases] = {qkv, res_mid, act, res_next, nullptr};
+      const bf16* res[kStreamPhases] = {nullptr, res_in, nullptr, res_mid, nullptr};
+      for (int k = 0; k < kStreamPhases; ++k) {
+        plan.src[k][half] = src[k];
+        plan.dst[k][half] = dst[k];
+        plan.res[k][half] = res[k];
+        plan.part[k][half] = at<float>(h, h->cv.spart[k == SP_O ? 0 : 1][half]);
+      }
+      plan.attn[half] = attn;
+    }
+    plan.rec = at<unsigned long long>(h, h->cv.srec);
+    h->stream_ok[i] = h->grid <= kStreamMaxGrid;
+  }
+  return MK_OK;
+}
+}  // namespace
+
 extern "C" {
 
 const char* mk_last_error(void) { return g_error; }
@@ -448,7 +549,7 @@ size_t mk_workspace_bytes(const mk_config* config, int device) {
   if (!config || check_config(*config) != MK_OK) return 0;
   int grid = 0;
   if (device_grid(*config, device, &grid) != MK_OK) return 0;
-  return carve(*config).total;
+  return carve(*config, grid).total;
 }
 
 int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, int device, void* stream,
@@ -459,29 +560,14 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
   MK_CUDA(cudaSetDevice(device));
   int grid = 0;
   if (int e = device_grid(*config, device, &grid)) return e;
-  const Carve cv = carve(*config);
+  const Carve cv = carve(*config, grid);
   if (workspace_bytes < cv.total)
     return fail(MK_ERR_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, cv.total);
-  int major = 0, coop = 0, khz = 0;
-  MK_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
-  MK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-  MK_CUDA(cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, device));
-  if (major != 10) return fail(MK_ERR_UNSUPPORTED, "device %d is sm_%d0; this library is built for sm_100a only", device, major);
-  if (!coop) return fail(MK_ERR_UNSUPPORTED, "device %d does not support cooperative launch", device);
-  MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-  MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
-  int per_sm = 0;
-  MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, megakernel, kThreads, kSmemBytes));
-  if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the megakernel does not fit on an SM of device %d", device);
-  // Tunables of the small-launch kernel (process-wide: shared-memory attributes belong to the function).
-  int small_ring = kSmallRingGranules, fat_copy = 36 * 1024;
-  if (const char* env = getenv("MEGABAKE_SMALL_RING_KB")) small_ring = std::max(64, std::min(kSmallRingMax, atoi(env)));
-  if (const char* env = getenv("MEGABAKE_SMALL_COPY_KB")) fat_copy = std::max(16, std::min(small_ring / 2, atoi(env))) * 1024;
-  if (int e = prepare_small_kernels(device, small_ring)) return e;
+  DeviceFacts facts;
+  if (int e = device_facts(device, &facts)) return e;
+  if (int e = prepare_kernels(device, config->head_dim)) return e;
   mk_handle h = new (std::nothrow) mk_handle_s();
   if (!h) return fail(MK_ERR_INVALID, "out of host memory");
-  h->small_ring = small_ring;
-  h->fat_copy = fat_copy;
   h->cfg = *config;
   h->device = device;
   h->grid = grid;
@@ -499,19 +585,27 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
     h->use3d = getenv("MEGABAKE_NO_3D_MAPS") == nullptr &&
                encode_weight_map3(&probe, workspace, 128, 256, 64, 2) == MK_OK;
   }
+  for (int i = 0; i < kStreamPlans; ++i) h->stream_ok[i] = false;
   h->kv_maps_ok = getenv("MEGABAKE_NO_CACHE_MAPS") == nullptr;
   h->tp_epoch = 0;
   h->tp_bound = false;
   for (int r = 0; r < kMaxTp; ++r) h->tp_peer[r] = nullptr;
   double ms = 2000.0;
   if (const char* env = getenv("MEGABAKE_WAIT_LIMIT_MS")) ms = atof(env) > 0 ? atof(env) : ms;
-  h->timeout_cycles = static_cast<long long>(ms * static_cast<double>(khz));
+  h->timeout_cycles = static_cast<long long>(ms * static_cast<double>(facts.khz));
   h->att_scale = static_cast<float>(std::pow(static_cast<double>(config->head_dim), -0.5));
   memset(&h->weights, 0, sizeof(h->weights));
   cudaError_t e = cudaMemsetAsync(workspace, 0, cv.total, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) {
     delete h;
     return fail(MK_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+  }
+  if (cv.handover_bytes > 0) {
+    e = cudaMemsetAsync(h->ws + cv.handover, 0xFF, cv.handover_bytes, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) {
+      delete h;
+      return fail(MK_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+    }
   }
   *out = h;
   return MK_OK;
@@ -531,12 +625,10 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   const int L = c.layers;
   const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
   const size_t nmaps = maps_per_table(c), nphases = phases_per_table(c);
-  std::vector<CUtensorMap> maps(3 * nmaps);
-  std::vector<GemmPhase> phases(4 * nphases);
+  std::vector<CUtensorMap> maps(2 * nmaps);
+  std::vector<GemmPhase> phases(2 * nphases);
   CUtensorMap* dmaps = at<CUtensorMap>(h, h->cv.tmaps);
-  CUtensorMap* operand_maps = dmaps + 3 * nmaps + 1;
-  CUtensorMap* row_dmaps = operand_maps + kOperandMaps;  // the one-token row table's own (plain-row) descriptors
-  std::vector<CUtensorMap> row_maps(nmaps);
+  CUtensorMap* operand_maps = dmaps + 2 * nmaps;
   bf16* hidden_a = at<bf16>(h, h->cv.hidden);
   bf16* hidden_b = at<bf16>(h, h->cv.hidden2);
   bf16* qkv = at<bf16>(h, h->cv.qkv);
@@ -550,7 +642,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     if (c.qkv_bias && (!lw.q_bias || !lw.k_bias || !lw.v_bias))
       return fail(MK_ERR_INVALID, "mk_bind_weights: layer %d lacks a q/k/v bias", l);
   }
-  // Table 0: split-K (small launches): o and down store K-slice partials; the next
+  // Table 0: split-K: o and down store K-slice partials; the next
   // normalising phase adds them to the residual stream, which ping-pongs between
   // hidden_b (after attention) and hidden_a (after the MLP).  Table 1: plain.
   bool use3d = h->use3d;
@@ -644,131 +736,6 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_maps + OPERAND_XNORM * kOperandTiles + t;
     if (int e = encode_phase_weight_map(&tmaps_host[7 * L], w->lm_head, c.vocab, c.hidden, head, use3d)) return e;
   }
-  // Table 2: the split-K table again for the small-launch kernel, whose mma.sync consumer takes tiles of
-  // at most 64 rows (four 16-row fragments) of any height below that.
-  h->fma_ok = small_shape_ok(c) && h->use3d;
-  for (size_t i = 0; i < nphases && h->fma_ok; ++i)
-    if (phases[i].kslice > kBSlots || phases[i].rows > kTileRows) h->fma_ok = false;
-  if (h->fma_ok) {
-    for (size_t i = 0; i < nphases; ++i) {
-      GemmPhase& ph = phases[2 * nphases + i];
-      ph = phases[i];
-      finish_phase(ph, h->grid, ph.epi == EPI_PARTIAL);  // any tile height: no rounding to 8
-      if (ph.rows > kSmallTileRows) {
-        if (ph.ksplit != 1) return fail(MK_ERR_UNSUPPORTED, "small-launch table: a split phase with more than 64 rows");
-        finish_phase(ph, h->grid, false, kSmallTileRows);
-      }
-      if (ph.nseg == 3 || ph.nacc == 2) {  // q/k/v and gate/up: outputs leave in pairs of rows: even tile height
-        if (ph.rows & 1) {
-          ph.rows += 1;
-          const int nsg = ph.nacc == 2 ? 1 : ph.nseg;
-          int tile = 0;
-          for (int sg = 0; sg < nsg; ++sg) {
-            ph.tile_start[sg] = tile;
-            tile += (ph.n[sg] + ph.rows - 1) / ph.rows;
-          }
-          ph.tile_start[nsg] = tile;
-          ph.ntiles = tile;
-          ph.nunits = tile * ph.ksplit;
-        }
-        const bool even = ph.n[0] % 2 == 0 && (ph.nacc == 2 || (ph.n[1] % 2 == 0 && ph.n[2] % 2 == 0));
-        ph.ll = (ph.rows <= kSmallTileRows && even && ph.ksplit == 1) ? 1 : 0;
-      }
-      // One copy = one three-dimensional box: the tile's rows x kb K chunks, each chunk 128-byte swizzled
-      // for ldmatrix; as many chunks as fit the copy size (a copy of less than ~16 KB cannot keep an
-      // SM's share of HBM busy: the copy engine retires about three per microsecond).
-      int kb = 1;
-      for (int cand = 2; cand <= std::min(ph.kslice, 256); ++cand)
-        if (ph.kslice % cand == 0 && ph.rows * cand * 128 <= kBoxCopyBytes) kb = cand;
-      ph.kb = kb;
-      ph.map3d = 1;
-      ph.gran = (ph.rows * kb * 128 + kGranule - 1) / kGranule;
-      const int nseg = ph.nacc == 2 ? 2 : ph.nseg;
-      for (int sg = 0; sg < nseg; ++sg) {
-        const size_t index = static_cast<size_t>(ph.tmap[sg] - dmaps);  // same matrix, same slot in the third set
-        ph.tmap[sg] = dmaps + 2 * nmaps + index;
-        if (encode_weight_map3(&maps[2 * nmaps + index], ph.w[sg], ph.n[sg], ph.k, ph.rows, kb) != MK_OK) h->fma_ok = false;
-      }
-    }
-  }
-  // Stamped hand-offs of the small-launch table (q/k/v -> attention -> o_proj, gate/up -> down): all or none.
-  h->small_ll = h->fma_ok;
-  for (int l = 0; l < L && h->small_ll; ++l)
-    if (!phases[2 * nphases + 4 * l].ll || !phases[2 * nphases + 4 * l + 2].ll) h->small_ll = false;
-  for (int l = 0; l < L && h->fma_ok; ++l) {
-    GemmPhase* ph = phases.data() + 2 * nphases + 4 * l;
-    for (int i = 0; i < 4; ++i) {
-      ph[i].ll = 0; ph[i].ll_dst = nullptr; ph[i].ll_src = nullptr; ph[i].ll_ld = 0; ph[i].ll_src_ld = 0;
-    }
-    if (!h->small_ll) continue;
-    ph[0].ll = 1; ph[0].ll_dst = at<unsigned long long>(h, h->cv.qkv_ll); ph[0].ll_ld = qkv_width(c) / 2;
-    // o_proj reads the attention output that the first chunk's CTA of every head combined and stamped as bf16 pairs
-    ph[1].ll_src = at<unsigned long long>(h, h->cv.attn_ll); ph[1].ll_src_ld = q_size / 2; ph[1].bmode = B_PLAIN;
-    ph[2].ll = 1; ph[2].ll_dst = at<unsigned long long>(h, h->cv.act_ll); ph[2].ll_ld = c.intermediate / 2;
-    ph[3].ll_src = at<unsigned long long>(h, h->cv.act_ll); ph[3].ll_src_ld = c.intermediate / 2;
-    // with no barrier between attention and o_proj, nor gate/up and down, their partials need buffers of their own
-    ph[3].partial = at<float>(h, h->cv.partial2);
-    if (l + 1 < L) ph[4].partial = at<float>(h, h->cv.partial2);
-  }
-  if (h->fma_ok && h->small_ll) phases[2 * nphases + 4 * L].partial = at<float>(h, h->cv.partial2);  // lm_head adds the last down-proj
-  // Table 3, one-token launches: o_proj and down_proj are not cut along K.  A CTA takes whole weight rows
-  // (contiguous in memory, fetched by one-dimensional bulk copies of up to 28 KB), adds the residual in its
-  // epilogue and stamps the new residual stream, which the next normalising phase polls: no fp32 partials,
-  // no grid barrier inside a layer.  The residual stream alternates between res_a (after the MLP) and res_b.
-  h->row_ok = h->small_ll && c.hidden % 2 == 0 && q_size * 2 <= h->fat_copy - 2048 && c.intermediate * 2 <= h->fat_copy - 2048 &&
-              c.intermediate <= kSplitTokens * kBSlots * kChunkK && q_size <= kSplitTokens * kBSlots * kChunkK;
-  if (h->row_ok) {
-    unsigned long long* res_a = at<unsigned long long>(h, h->cv.res_a);
-    unsigned long long* res_b = at<unsigned long long>(h, h->cv.res_b);
-    // The row table's consumer runs on CUDA cores over plain rows: its box phases (q/k/v, gate/up, lm_head)
-    // get descriptors of their own, boxes of kb * 64 elements x the tile's rows without swizzle.
-    for (size_t i = 0; i < nphases && h->row_ok; ++i) {
-      GemmPhase& ph = phases[3 * nphases + i];
-      ph = phases[2 * nphases + i];
-      ph.map3d = 0;
-      int kb = 1;
-      for (int cand = 2; cand <= 4; cand += 2)
-        if (ph.kslice % cand == 0 && ph.rows * cand * 128 <= kBoxCopyBytes) kb = cand;
-      ph.kb = kb;
-      ph.gran = (ph.rows * kb * 128 + kGranule - 1) / kGranule;
-      const int nseg = ph.nacc == 2 ? 2 : ph.nseg;
-      for (int sg = 0; sg < nseg; ++sg) {
-        const size_t index = static_cast<size_t>(ph.tmap[sg] - (dmaps + 2 * nmaps));
-        ph.tmap[sg] = row_dmaps + index;
-        if (encode_weight_map(&row_maps[index], ph.w[sg], ph.n[sg], ph.k, ph.rows, kb, false) != MK_OK) h->row_ok = false;
-      }
-    }
-    for (int l = 0; l <= L; ++l) {
-      GemmPhase* ph = phases.data() + 3 * nphases + 4 * l;
-      // normalising phases read the stamped residual stream (layer 0 still gathers embedding rows)
-      ph[0].add_parts = 0; ph[0].h_out = nullptr; ph[0].partial = nullptr;
-      ph[0].ll_src = ph[0].gather ? nullptr : res_a; ph[0].ll_src_ld = c.hidden / 2;
-      if (l == L) break;  // the lm_head phase
-      ph[2].add_parts = 0; ph[2].h_out = nullptr; ph[2].partial = nullptr;
-      ph[2].ll_src = res_b; ph[2].ll_src_ld = c.hidden / 2;
-      for (int which = 1; which <= 3; which += 2) {
-        GemmPhase& rp = ph[which];
-        rp.ksplit = 1; rp.kslice = rp.kc;
-        rp.rows = choose_rows(rp, h->grid, kSmallTileRows);
-        if (rp.rows & 1) rp.rows += 1;
-        rp.tile_start[0] = 0;
-        rp.ntiles = (rp.n[0] + rp.rows - 1) / rp.rows;
-        rp.tile_start[1] = rp.ntiles;
-        rp.nunits = rp.ntiles;
-        rp.bulk = 1;
-        const int row_bytes = rp.k * 2;
-        rp.rpc = std::max(1, std::min(8, (h->fat_copy - 2048) / row_bytes));
-        if (rp.rpc > rp.rows) rp.rpc = rp.rows;
-        rp.kb = 1;
-        rp.gran = (rp.rpc * row_bytes + kGranule - 1) / kGranule;
-        rp.epi = EPI_ROWRES; rp.partial = nullptr;
-        rp.ll = 1; rp.ll_ld = c.hidden / 2;
-        rp.res_src = (which == 1) ? res_a : res_b;   // layer 0's o_proj adds the embedding row (rp.gather below)
-        rp.ll_dst = (which == 1) ? res_b : res_a;
-        rp.gather = (which == 1 && l == 0) ? 1 : 0;
-      }
-    }
-  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   {
     CUtensorMap operand_host[kOperandMaps];
@@ -783,9 +750,20 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     MK_CUDA(cudaStreamSynchronize(s));
   }
   MK_CUDA(cudaMemcpyAsync(dmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
-  MK_CUDA(cudaMemcpyAsync(row_dmaps, row_maps.data(), row_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
   MK_CUDA(cudaMemcpyAsync(at<GemmPhase>(h, h->cv.phases), phases.data(), phases.size() * sizeof(GemmPhase),
                           cudaMemcpyHostToDevice, s));
+  std::vector<CUtensorMap> stream_maps;
+  std::vector<StreamLayer> stream_layers(L);
+  std::vector<int> stream_units;
+  StreamPlan stream_plans[kStreamPlans];
+  memset(stream_plans, 0, sizeof(stream_plans));
+  if (stream_shape_ok(c) && h->use3d) {
+    if (int e = bind_stream(h, *w, stream_maps, stream_layers, stream_units, stream_plans)) return e;
+    MK_CUDA(cudaMemcpyAsync(at<CUtensorMap>(h, h->cv.smaps), stream_maps.data(), stream_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
+    MK_CUDA(cudaMemcpyAsync(at<StreamLayer>(h, h->cv.slayers), stream_layers.data(), stream_layers.size() * sizeof(StreamLayer), cudaMemcpyHostToDevice, s));
+    MK_CUDA(cudaMemcpyAsync(at<int>(h, h->cv.sunits), stream_units.data(), stream_units.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    MK_CUDA(cudaMemcpyAsync(at<StreamPlan>(h, h->cv.splan), stream_plans, sizeof(stream_plans), cudaMemcpyHostToDevice, s));
+  }
   // The source vectors die at return: make sure the copies have read them.
   MK_CUDA(cudaStreamSynchronize(s));
   h->layers.assign(w->layers, w->layers + L);
@@ -796,14 +774,6 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
 }
 
 namespace {
-// Keys the small-launch kernel's 16 KB score buffer covers: at most 16 context chunks of 4096 / group keys.
-int small_launch_keys(const mk_config& c) { return kMaxChunks * ((kAttScoreBytes / 4 / (c.q_heads / c.kv_heads)) & ~7); }
-
-bool small_launch_ok(mk_handle h, int capacity) {
-  return (h->cfg.engine == MK_ENGINE_FMA || h->cfg.engine == MK_ENGINE_AUTO) && small_shape_ok(h->cfg) && h->fma_ok &&
-         capacity <= small_launch_keys(h->cfg);
-}
-
 int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int batch, void* const* key_caches,
                 void* const* value_caches, int32_t* const* valid_lengths, int capacity, void* logits, void* stream,
                 int64_t* tokens_out = nullptr, bool sample = false, bool ragged = false);
@@ -912,22 +882,23 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
   p.mode = MODE_DECODE; p.m = batch; p.batch = batch; p.seq = 1; p.capacity = capacity;
   p.split = split_table_ok(h->cfg) ? 1 : 0;
   p.phases = at<GemmPhase>(h, h->cv.phases) + (p.split ? 0 : phases_per_table(h->cfg));
-  const bool small = !ragged && batch <= kSplitTokens && small_launch_ok(h, capacity);
+  const bool streamed = stream_usable(h, batch, ragged);
   p.ragged = ragged ? 1 : 0;
-  if (!small && h->kv_maps_ok) {
+  if (h->kv_maps_ok) {
     // Tiled descriptors of the caches for the tensor engine's decode attention, encoded again only when a
     // cache pointer or the geometry differs from the last call's (the copy is ordered on `stream`
     // before the launch; its pageable source is staged before cudaMemcpyAsync returns).
     const mk_config& c = h->cfg;
     const int gs = c.q_heads / c.kv_heads, row_elems = c.kv_heads * c.head_dim;
-    const int hpu = decode_heads_per_unit(c.kv_heads, gs, c.head_dim);
-    const int tile_keys = kDecTileBytes / (c.head_dim * 2 * hpu);
+    const int hpu = streamed ? stream_heads_per_tile(c, batch) : decode_heads_per_unit(c.kv_heads, gs, c.head_dim);
+    const int tile_keys = (streamed ? kStreamSlotBytes : kDecTileBytes) / (c.head_dim * 2 * hpu);
     const bool shape_ok = (hpu & (hpu - 1)) == 0 && tile_keys % 16 == 0 && tile_keys <= 256 && c.head_dim % kChunkK == 0;
     int slot = -1, oldest = 0;
     for (int i = 0; i < kCacheMapSets && shape_ok && slot < 0; ++i) {
       const auto& set = h->kv_sets[i];
       if (set.used < h->kv_sets[oldest].used) oldest = i;
-      bool same = static_cast<int>(set.seen.size()) == 2 * L && set.capacity == capacity && set.batch == batch;
+      bool same = static_cast<int>(set.seen.size()) == 2 * L && set.capacity == capacity && set.batch == batch &&
+                  set.heads == hpu && set.keys == tile_keys;
       for (int l = 0; l < L && same; ++l) same = set.seen[l] == key_caches[l] && set.seen[L + l] == value_caches[l];
       if (same) slot = i;
     }
@@ -951,6 +922,8 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
         }
         set.capacity = capacity;
         set.batch = batch;
+        set.heads = hpu;
+        set.keys = tile_keys;
       } else {
         h->kv_maps_ok = false;  // this driver refuses the view: plain copies from here on
       }
@@ -960,17 +933,18 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
       p.kv_maps = device_sets + static_cast<size_t>(slot) * 2 * L;
     }
   }
-  if (small) p.phases = at<GemmPhase>(h, h->cv.phases) + 2 * phases_per_table(h->cfg);
   p.n_gemm = 4 * L + 1;
   p.nbar = 7 * L + 1;  // tensor engine: five per layer and one behind each norm phase (two per layer, one for the lm_head)
-  if (small) p.nbar = 5 * L;
-  if (small && h->small_ll) p.nbar = 2 * L;  // stamped hand-offs: only o_proj -> gate/up and down -> next layer keep a grid barrier
-  if (small && h->row_ok && batch == 1) {     // one token: the row table, a single grid barrier at the very end
-    p.phases = at<GemmPhase>(h, h->cv.phases) + 3 * phases_per_table(h->cfg);
+  if (streamed) {
+    if (!p.kv_maps) return fail(MK_ERR_CUDA, "mk_decode: the driver refuses the cache descriptors");
+    const mk_config& c = h->cfg;
+    const int plan = stream_plan_of(batch);
+    p.splan = at<StreamPlan>(h, h->cv.splan) + plan;
     p.nbar = 1;
-    p.rowmode = 1;
+    p.stream_hpu = stream_heads_per_tile(c, batch);
+    p.stream_tile_keys = kStreamSlotBytes / (c.head_dim * 2 * p.stream_hpu);
+    stream_divide(p, stream_scratch_bytes(c, batch), batch);
   }
-  p.small_ring = small_ring_for(h, p.rowmode ? 1 : 2);
   p.stream_once = (ntt == 1);
   p.ids = reinterpret_cast<long long*>(const_cast<int64_t*>(ids));
   p.pos = reinterpret_cast<long long*>(const_cast<int64_t*>(positions));
@@ -983,9 +957,9 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
   if (sample) {
     p.sample = 1;
     p.tokens_out = reinterpret_cast<long long*>(tokens_out);
-    if (!p.rowmode) p.nbar += 1;  // the sampler runs behind one more grid barrier (the row table already ends with one)
+    if (!streamed) p.nbar += 1;  // the sampler runs behind one more grid barrier (the streaming kernel already ends with one)
   }
-  if (int e = launch(h, p, stream, L, small)) return e;
+  if (int e = launch(h, p, stream, L)) return e;
   if (p.tp_size > 1) h->tp_epoch += 2u * static_cast<uint32_t>(L);
   return MK_OK;
 }
@@ -1111,6 +1085,8 @@ int mk_status(mk_handle h, void* stream, mk_status_info* out) {
   if (c.status != MK_STATUS_OK || c.abort) {
     // Counters are in an unknown state after an aborted launch: start over.
     MK_CUDA(cudaMemset(at<Control>(h, h->cv.ctrl), 0, sizeof(Control)));
+    if (h->cv.handover_bytes > 0)  // hand-over words of the aborted launch
+      MK_CUDA(cudaMemset(h->ws + h->cv.handover, 0xFF, h->cv.handover_bytes));
     h->epoch = 0;
     if (h->mirror) *h->mirror = 0;
     return fail(MK_ERR_DEVICE_STATUS, "device status %d at site %d (cta %d, detail %d)", c.status, c.where, c.cta, c.detail);
@@ -1207,18 +1183,16 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
     va_end(ap);
     if (n > 0) used += static_cast<size_t>(n);
   };
-  add("ctas %d, weight copies %s, small-launch tables %s/%s/%s, tp %d/%d\n", h->grid,
-      h->use3d ? "3-D (several K chunks per copy)" : "2-D (one K chunk per copy)", h->fma_ok ? "split-K" : "-",
-      h->small_ll ? "stamped" : "-", h->row_ok ? "rows" : "-", h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
+  add("ctas %d, weight copies %s, streaming decode %s, tp %d/%d\n", h->grid,
+      h->use3d ? "3-D (several K chunks per copy)" : "2-D (one K chunk per copy)", h->stream_ok[0] ? "yes" : "no",
+      h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
       h->cfg.tp_size > 1 ? h->cfg.tp_size : 1);
   if (h->bound) {
-    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * 4);
+    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * 2);
     MK_CUDA(cudaMemcpy(phases.data(), at<GemmPhase>(h, h->cv.phases), phases.size() * sizeof(GemmPhase), cudaMemcpyDeviceToHost));
     static const char* names[5] = {"qkv", "o", "gate/up", "down", "lm_head"};
-    for (int table = 0; table < 4; ++table) {
+    for (int table = 0; table < 2; ++table) {
       if (table == 0 && !split_table_ok(h->cfg)) continue;
-      if (table == 2 && !h->fma_ok) continue;
-      if (table == 3 && !h->row_ok) continue;
       add("table %d:", table);
       for (int i = 0; i < 5; ++i) {
         const GemmPhase& ph = phases[table * phases_per_table(h->cfg) + (i < 4 ? i : 4 * h->cfg.layers)];
@@ -1300,29 +1274,20 @@ StaticLayout static_layout(int batch, int q_heads, int kv_heads, int head_dim) {
 
 // One-time set-up per device: symbol address, launch attributes, zeroed scratch.
 int static_setup(StaticSlot& slot, int device, cudaStream_t stream) {
-  int major = 0, coop = 0, khz = 0, sms = 0;
-  MK_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
-  MK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-  MK_CUDA(cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, device));
-  MK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  if (major != 10) return fail(MK_ERR_UNSUPPORTED, "device %d is sm_%d0; this library is built for sm_100a only", device, major);
-  if (!coop) return fail(MK_ERR_UNSUPPORTED, "device %d does not support cooperative launch", device);
+  DeviceFacts facts;
+  if (int e = device_facts(device, &facts)) return e;
   void* address = nullptr;
   const cudaError_t found = cudaGetSymbolAddress(&address, g_static_scratch);
   if (found != cudaSuccess || !address)
     return fail(MK_ERR_CUDA, "cudaGetSymbolAddress(static scratch) on device %d: %s", device, cudaGetErrorString(found));
-  MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-  MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
-  int per_sm = 0;
-  MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, megakernel, kThreads, kSmemBytes));
-  if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the megakernel does not fit on an SM of device %d", device);
+  if (int e = prepare_kernels(device, 0)) return e;
   // Barrier counter, abort flag, status word and every exchange stamp must start at zero.
   MK_CUDA(cudaMemsetAsync(address, 0, kStaticScratchBytes, stream));
   double ms = 2000.0;
   if (const char* env = getenv("MEGABAKE_WAIT_LIMIT_MS")) ms = atof(env) > 0 ? atof(env) : ms;
   slot.base = static_cast<uint8_t*>(address);
-  slot.grid = sms;
-  slot.timeout_cycles = static_cast<long long>(ms * static_cast<double>(khz));
+  slot.grid = facts.sms;
+  slot.timeout_cycles = static_cast<long long>(ms * static_cast<double>(facts.khz));
   slot.epoch = slot.att_epoch = 0;
   slot.launches = 0;
   slot.ready = true;
@@ -1412,7 +1377,8 @@ int mk_kv_attention_static(int q_heads, int kv_heads, int head_dim, const void* 
   view.epoch = slot.epoch; view.att_epoch = slot.att_epoch; view.launches = slot.launches;
   view.timeout_cycles = slot.timeout_cycles;
   view.att_scale = static_cast<float>(std::pow(static_cast<double>(head_dim), -0.5));
-  view.fma_ok = false; view.small_ll = false; view.row_ok = false; view.trace = nullptr; view.trace_cap = 0;
+  for (int i = 0; i < kStreamPlans; ++i) view.stream_ok[i] = false;
+  view.trace = nullptr; view.trace_cap = 0;
   view.mirror = nullptr; view.use3d = false;
   view.tp_epoch = 0; view.tp_bound = false;
   for (int r = 0; r < kMaxTp; ++r) view.tp_peer[r] = nullptr;

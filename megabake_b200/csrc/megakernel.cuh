@@ -36,11 +36,10 @@ constexpr int kExchangeFloats = 48;      // per (row group, chunk), 192 bytes: m
 constexpr int kXchStatsFlag = 32;        // float index of "the statistics are out" (flag protocol)
 constexpr int kXchPartsFlag = 33;        // float index of "the chunk's partial sums are out"
 constexpr int kMaxSplit = 4;             // K slices a projection may be cut into
-constexpr int kSplitTokens = 4;          // launches with at most this many tokens use the split-K table
 
 static_assert(kSmemBytes <= 200704, "dynamic shared memory exceeds the 196 KiB carve-out");
 
-enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SILU = 2, EPI_PARTIAL = 3, EPI_ROWRES = 4, EPI_TP = 5 };
+enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SILU = 2, EPI_PARTIAL = 3, EPI_TP = 4 };
 enum { B_PLAIN = 0, B_NORM = 1, B_ATTN = 2 };
 enum { MODE_DECODE = 0, MODE_PREFILL = 1, MODE_LINEAR = 2, MODE_KVATT = 3, MODE_ATT = 4 };
 enum { EV_PHASE_ENTER = 1, EV_B_STAGED = 2, EV_FIRST_ACC = 3, EV_PHASE_DONE = 4, EV_BARRIER_DONE = 5, EV_ATTENTION_DONE = 6,
@@ -73,8 +72,7 @@ struct GemmPhase {
   int nseg, nacc;
   int k, kc;                   // reduction length, in elements and in 64-element chunks
   int rows;                    // weight rows per tile
-  int kb;                      // K chunks one weight copy brings (tensor engine: kb swizzled chunks of rows x 128 B per matrix;
-                               // small-launch kernel: unswizzled boxes of kb * 64 elements x rows)
+  int kb;                      // K chunks one weight copy brings (kb swizzled chunks of rows x 128 B per matrix)
   int gran;                    // ring granules one entry occupies (tensor engine: nacc * kb * rows / 8)
   int gate;                    // tensor engine: 1 = this phase follows decode attention, whose cache tiles stream through the weight
                                // ring: its weights may be fetched only once the workers have released the ring (a_ready)
@@ -85,14 +83,6 @@ struct GemmPhase {
   int epi, bmode;
   int gather;                  // 1: activation rows are embedding rows selected by the token ids
   int to_logits;               // 1: output goes to the caller's logits buffer
-  int ll;                      // small-launch table: 1 = the bf16 outputs of this phase leave as 64-bit words
-                               // {stamp, bf16 pair} in ll_dst, which the consumer polls instead of waiting at a grid barrier
-  int ll_ld, ll_src_ld;        // words per token in ll_dst / ll_src
-  unsigned long long* ll_dst;
-  const unsigned long long* ll_src;  // B_PLAIN / B_NORM: the operand as stamped bf16 pairs; B_ATTN: attention partials as {stamp, fp32}
-  int bulk;                    // one-token row table: 1 = a tile is `rows` whole weight rows, contiguous in memory, fetched by
-  int rpc;                     // one-dimensional bulk copies of `rpc` rows; the epilogue (EPI_ROWRES) adds the residual it
-  const unsigned long long* res_src;  // reads as stamped pairs from res_src (or the embedding row when `gather`) and stamps the sum into ll_dst
   int tp_buf;                  // EPI_TP: which half of the exchange buffers this projection's partial sums go to
   int add_parts;               // B_NORM: fp32 partial slices of the previous projection to add to the residual
   const bf16* normw;
@@ -130,7 +120,6 @@ struct KParams {
   int max_positions;
   int stream_once;    // 1: weights are read once per launch (L2 evict-first)
   int split;          // 1: this launch runs the split-K phase table (residual updates applied by the consumer)
-  int rowmode;        // 1: one-token row table: stamped hand-offs everywhere, one grid barrier at the end of the launch
   int ragged;         // 1: len[l] points to one valid length per sequence (int32 [batch]) instead of one shared by the batch
   int sample;         // 1: after the logits, pick each sequence's greedy token on the device, store it in tokens_out and as the
                       //    next id, and advance the position: the next launch needs no host round trip
@@ -142,9 +131,6 @@ struct KParams {
   const GemmPhase* phases;
   bf16 *hidden_buf, *qkv, *attn, *act;
   bf16* xnorm;        // [m][hidden]: the normalised rows a norm phase leaves for the projections that follow
-  unsigned long long* qkv_ll;  // [kSplitTokens][qkv width / 2]: stamped q/k/v outputs of the small-launch kernel
-  unsigned long long* att_ll;  // [kSplitTokens * q_heads][kMaxChunks][head_dim]: stamped attention partials {stamp, fp32}
-  unsigned long long* attn_ll; // [kSplitTokens][q_heads * head_dim / 2]: the combined attention output as stamped bf16 pairs
   float* att_xch;     // [row groups][kMaxChunks][kExchangeFloats]
   float* att_part;    // [batch * q_heads][kMaxChunks][head_dim]
   Control* ctrl;
@@ -167,9 +153,12 @@ struct KParams {
   // stand-alone projection (MODE_LINEAR): its phase and its two descriptors travel in the parameter block,
   // so the call needs no upload and no synchronisation
   GemmPhase linear_phase;
-  int small_ring;  // weight ring of the small-launch kernel, in 1 KiB granules
   const CUtensorMap* kv_maps;  // decode on the tensor engine: 4-D descriptors of the key caches [layers], then of the value caches [layers]; null = plain copies
   CUtensorMap linear_wmap, linear_xmap;
+  // streaming decode kernel (stream_kernel.cuh)
+  const struct StreamPlan* splan;
+  int stream_slots, stream_scratch_bytes;      // ring slots, bytes of the attention area
+  int stream_hpu, stream_tile_keys;            // adjacent KV heads and positions of a cache tile
   void* kc[MK_MAX_LAYERS];
   void* vc[MK_MAX_LAYERS];
   int* len[MK_MAX_LAYERS];

@@ -1,0 +1,150 @@
+// Host side of the streaming decode kernel: how projections are cut, how their units are dealt to the CTAs, and how
+// shared memory is divided.  Pure functions of the configuration and the batch.
+#pragma once
+#include <algorithm>
+#include <numeric>
+#include <vector>
+
+#include "stream_common.cuh"
+
+namespace mk {
+
+constexpr int kStreamPlans = 3;           // 8, 16 and 32 tokens (one, two and four MMA tiles)
+constexpr int kStreamMaxGrid = 512;
+constexpr int kStreamSmemLimit = 232448;  // 227 KiB
+
+inline int stream_plan_of(int tokens) { return tokens <= 8 ? 0 : (tokens <= 16 ? 1 : 2); }
+inline bool stream_plan_used(const mk_config& c, int plan) { return plan == 0 || c.max_tokens > (4 << plan); }
+
+// The kernel for a token class (up to 1, 4, 8, 16, 32 tokens); one translation unit per head size.
+constexpr int kStreamClasses = 5;
+constexpr int kStreamClassTokens[kStreamClasses] = {1, 4, 8, 16, 32};
+const void* stream_kernel_64(int token_class);
+const void* stream_kernel_128(int token_class);
+inline int stream_class_of(int tokens) { return tokens <= 1 ? 0 : (tokens <= 4 ? 1 : (tokens <= 8 ? 2 : (tokens <= 16 ? 3 : 4))); }
+inline const void* stream_kernel(int token_class, int head_dim) {
+  return head_dim == 64 ? stream_kernel_64(token_class) : stream_kernel_128(token_class);
+}
+
+// Cut a reduction of `k` into the fewest slices of at most `copies` copies each.  (A slice that does not end at the row's end
+// should be a multiple of four chunks: windows are dealt to eight warps.)
+inline bool stream_cut(StreamPhase& ph, int copies) {
+  const int chunks = ph.k / kChunkK;
+  for (int nslice = 1; nslice <= chunks; ++nslice) {
+    if (chunks % nslice) continue;
+    ph.nslice = nslice;
+    ph.cs = chunks / nslice;
+    ph.ncopy = (ph.cs + kStreamKb - 1) / kStreamKb;
+    if (ph.ncopy <= copies) return true;
+  }
+  return false;
+}
+
+// Rows per tile: what leaves the busiest CTA the fewest rows.  2048 rows in tiles of 16 are 128 tiles for 148 CTAs, 14 % of
+// which would stand idle; in tiles of 14 they are 147.  A tile costs about two rows' time besides its rows.
+inline void stream_rows(StreamPhase& ph, const int* matrices, int count, int grid) {
+  int best_cost = 1 << 30;
+  for (int rows = kStreamRows; rows >= 8; rows -= 2) {
+    int tiles = 0;
+    for (int i = 0; i < count; ++i) tiles += (matrices[i] + rows - 1) / rows;
+    const int units = tiles * ph.nslice;
+    const int cost = (units + grid - 1) / grid * (rows + 2);
+    if (cost < best_cost) {
+      best_cost = cost;
+      ph.rows = rows;
+      ph.ntiles = tiles;
+    }
+  }
+}
+
+inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* ph) {
+  const int nt = 1 << plan, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const int ks[kStreamPhases] = {c.hidden, q_size, c.hidden, c.intermediate, c.hidden};
+  const int ns[kStreamPhases] = {q_size + 2 * kv_size, c.hidden, c.intermediate, c.hidden, c.vocab};
+  const int fit = nt == 4 ? 2 : 4;  // copies whose operand fits a warp's registers
+  bool ok = true;
+  for (int i = 0; i < kStreamPhases; ++i) {
+    StreamPhase& p = ph[i];
+    p = StreamPhase{};
+    p.k = ks[i];
+    p.n = ns[i];
+    // Up to eight tokens a long reduction is not cut: its operand is small enough to be read in parts by every CTA, which
+    // saves a hand-over of partial sums.
+    const bool cross = i == SP_O || i == SP_DOWN;
+    ok = stream_cut(p, cross && nt == 1 ? 8 : fit) && (cross || p.nslice == 1) && ok;
+    p.parts = (p.ncopy + fit - 1) / fit;
+    const int qkv[3] = {q_size, kv_size, kv_size};
+    stream_rows(p, i == SP_QKV ? qkv : &ns[i], i == SP_QKV ? 3 : 1, grid);
+  }
+  StreamPhase& qkv = ph[SP_QKV];
+  qkv.row1 = q_size;
+  qkv.row2 = q_size + kv_size;
+  qkv.tile1 = (q_size + qkv.rows - 1) / qkv.rows;
+  qkv.tile2 = qkv.tile1 + (kv_size + qkv.rows - 1) / qkv.rows;
+  return ok;
+}
+
+// Hidden sizes up to 2048.  Wider shapes would fit batches of up to 16 too, but they come with 32 layers and more, where two
+// correct bf16 evaluations are 2.0 to 2.2 % apart (measured on the 8B shape: this kernel, the tensor engine and an eager
+// evaluation, each against each): they stay on the tensor engine, whose results their users have.
+inline bool stream_shape_ok(const mk_config& c) {
+  if (c.tp_size > 1 || c.hidden > 2048) return false;
+  StreamPhase ph[kStreamPhases];
+  for (int i = 0; i < kStreamPlans; ++i)
+    if (stream_plan_used(c, i) && !stream_phases(c, i, 148, ph)) return false;
+  return true;
+}
+
+// Every CTA's units of each phase, as ranges: table[phase][cta], table[phase][grid] = count.  Every phase is dealt evenly
+// (an SM takes in at most about 60 GB/s, so a CTA with more units than the rest ends a phase late); the units that
+// are left over go to the CTAs with the fewest bytes so far.
+inline void stream_deal_units(const StreamPhase* ph, int grid, int* table) {
+  std::vector<long long> load(grid, 0);
+  std::vector<int> order(grid), extra(grid);
+  for (int kind = 0; kind < kStreamPhases; ++kind) {
+    const int units = ph[kind].ntiles * ph[kind].nslice;
+    const long long cost = static_cast<long long>(ph[kind].rows) * ph[kind].cs * (kind == SP_GU ? 2 : 1);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return load[a] < load[b]; });
+    std::fill(extra.begin(), extra.end(), 0);
+    for (int i = 0; i < units % grid; ++i) extra[order[i]] = 1;
+    int* row = table + kind * (grid + 1);
+    row[0] = 0;
+    for (int i = 0; i < grid; ++i) {
+      row[i + 1] = row[i] + units / grid + extra[i];
+      load[i] += cost * (units / grid + extra[i]);
+    }
+  }
+}
+
+// Adjacent KV heads of a cache tile: as many as leave about one (sequence, head group) per two CTAs.  Wider tiles read
+// longer runs of a cache row (DRAM pages) and leave a warp to itself; fewer groups mean more parts to add up.
+inline int stream_heads_per_tile(const mk_config& c, int batch) {
+  const int gs = c.q_heads / c.kv_heads;
+  int hpu = 1;
+  while (2 * hpu * gs <= 8 && c.kv_heads % (2 * hpu) == 0 && batch * (c.kv_heads / (2 * hpu)) >= 64) hpu *= 2;
+  return hpu;
+}
+
+// Attention: one row per warp and query head of its KV head (and 64 pairs of statistics per KV head of a tile).
+// Up to four tokens: the normalised operand on its way to the fragments (16 windows of 64 bytes per warp and token).
+inline int stream_scratch_bytes(const mk_config& c, int batch) {
+  return std::max(batch <= 4 ? kStreamClassTokens[stream_class_of(batch)] * 8192 : 4096, (8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 15) / 16 * 16);
+}
+inline int stream_psum_bytes(int batch) {
+  return std::max(1024, (batch <= 16 ? 2 : 1) * kStreamWarps * 2 * kStreamClassTokens[stream_class_of(batch)] * kStreamPartPitch * 4);
+}
+// The ring takes as many slots as fit.
+inline void stream_divide(KParams& p, int scratch, int batch) {
+  p.stream_scratch_bytes = scratch;
+  p.stream_slots = std::min(kStreamMaxSlots, (kStreamSmemLimit - 1024 - kStreamMiscBytes - scratch - stream_psum_bytes(batch)) / kStreamSlotBytes);
+}
+inline int stream_smem_bytes(const KParams& p) {
+  return 1024 + p.stream_slots * kStreamSlotBytes + kStreamMiscBytes + p.stream_scratch_bytes + stream_psum_bytes(p.m);
+}
+// A CTA's run must not touch more head groups than it has room for.
+inline bool stream_parts_ok(const mk_config& c, int batch, int grid) {
+  return batch * (c.kv_heads / stream_heads_per_tile(c, batch)) / grid + 3 <= kStreamSegments;
+}
+
+}  // namespace mk
