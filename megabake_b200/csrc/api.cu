@@ -52,8 +52,12 @@ int qkv_width(const mk_config& c) { return (c.q_heads + 2 * c.kv_heads) * c.head
 // source) x (token tiles of 16, 32, 64), behind the weight descriptors.
 constexpr int kCacheMapSets = 8;  // cache-descriptor sets a handle remembers (one per KV state it is called with in turn)
 constexpr int kOperandTiles = 4;  // token tiles of 16, 32, 64, 128
-constexpr int kOperandKinds = 4, kOperandMaps = kOperandKinds * kOperandTiles;
-enum { OPERAND_XNORM = 0, OPERAND_ATTN = 1, OPERAND_ACT = 2, OPERAND_LINEAR = 3 };
+constexpr int kOperandChunks = 4; // K chunks per copy: 1 .. 4
+constexpr int kOperandKinds = 3, kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;
+enum { OPERAND_XNORM = 0, OPERAND_ATTN = 1, OPERAND_ACT = 2 };
+// Phase tables: split-K, plain, and for prompts of more than one token tile one each for two, three and four or more.
+constexpr int kSpreadTables = 3;
+int phase_tables(const mk_config& c) { return 2 + (c.max_tokens > 128 && c.tp_size <= 1 ? kSpreadTables : 0); }
 int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128)); }
 size_t maps_per_table(const mk_config& c) { return 7 * static_cast<size_t>(c.layers) + 1; }
 size_t phases_per_table(const mk_config& c) { return 4 * static_cast<size_t>(c.layers) + 1; }
@@ -68,9 +72,9 @@ Carve carve(const mk_config& c, int grid) {
   };
   const size_t m = static_cast<size_t>(c.max_tokens);
   v.ctrl = take(sizeof(Control));
-  v.tmaps = take(sizeof(CUtensorMap) * (2 * maps_per_table(c) + kOperandMaps));  // split and plain tables, token operands
+  v.tmaps = take(sizeof(CUtensorMap) * (phase_tables(c) * maps_per_table(c) + kOperandMaps));
   v.kvmaps = take(sizeof(CUtensorMap) * 2 * static_cast<size_t>(c.layers) * kCacheMapSets);  // decode attention: per set, key caches then value caches
-  v.phases = take(sizeof(GemmPhase) * 2 * phases_per_table(c));
+  v.phases = take(sizeof(GemmPhase) * phase_tables(c) * phases_per_table(c));
   v.hidden = take(m * c.hidden * 2);
   v.hidden2 = take(m * c.hidden * 2);
   v.xnorm = take(m * c.hidden * 2);
@@ -231,17 +235,18 @@ int encode_phase_weight_map(CUtensorMap* out, const void* base, int rows, int k,
   return encode_weight_map(out, base, rows, k, ph.rows);
 }
 
-// Tensor engine, token operand: bf16 [tokens, k] row-major, box = 64 elements x `tile` tokens, 128-byte
-// swizzle; token rows past `tokens` read as zeros.
-int encode_operand_map(CUtensorMap* out, const void* base, int tokens, int k, int tile) {
+// Tensor engine, token operand: bf16 [tokens, k] row-major seen as (64 elements, tokens, k / 64 chunks), box = 64 elements x
+// `tile` tokens x `chunks` chunks, each 128-byte swizzled; token rows past `tokens` read as zeros.
+int encode_operand_map(CUtensorMap* out, const void* base, int tokens, int k, int tile, int chunks, bool use3d) {
   if (reinterpret_cast<uintptr_t>(base) % 16) return fail(MK_ERR_ALIGNMENT, "operand base %p is not 16-byte aligned", base);
   auto fn = encode_fn();
   if (!fn) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(tokens)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kChunkK), static_cast<cuuint32_t>(tile)};
-  const cuuint32_t elem[2] = {1, 1};
-  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+  const cuuint64_t dims3[3] = {static_cast<cuuint64_t>(kChunkK), static_cast<cuuint64_t>(tokens), static_cast<cuuint64_t>(k / kChunkK)};
+  const cuuint64_t dims2[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(tokens)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(k) * 2, static_cast<cuuint64_t>(kChunkK) * 2};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(kChunkK), static_cast<cuuint32_t>(tile), static_cast<cuuint32_t>(chunks)};
+  const cuuint32_t elem[3] = {1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, use3d ? 3 : 2, const_cast<void*>(base), use3d ? dims3 : dims2, strides, box, elem,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled (operand) failed with %d (tokens %d, k %d)", (int)r, tokens, k);
@@ -362,7 +367,7 @@ void finish_phase(GemmPhase& ph, int grid, bool allow_split, int max_rows = kTil
 // Tensor engine: tile heights are multiples of 8 (a swizzled chunk of a tile must start on a 1 KiB boundary
 // inside a ring entry), and an entry carries `kb` K chunks per matrix: as many as divide the K range and keep
 // the entry under ~36 KB (three entries of the 120 KB ring in flight); two at most when launches can have
-// token tiles of 64 (the activation ring holds 64 KB).
+// token tiles of 128 (the activation ring holds 64 KB, two entries of 32).
 void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) {
   finish_phase(ph, grid, allow_split);
   ph.rows = std::min(kTileRows, (ph.rows + 7) / 8 * 8);
@@ -376,10 +381,52 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
   ph.ntiles = tile;
   ph.nunits = tile * ph.ksplit;
   int kb = 1;
-  for (int cand = 2; cand <= (max_tokens > 32 ? 2 : 4); ++cand)
+  for (int cand = 2; cand <= (max_tokens > 64 ? 2 : kOperandChunks); ++cand)
     if (ph.kslice % cand == 0 && ph.nacc * cand * ph.rows * 128 <= 36 * 1024) kb = cand;
   ph.kb = kb;
   ph.gran = ph.nacc * kb * ph.rows / 8;
+}
+
+// Tensor engine, prompts of several token tiles of 128: every (row tile, K slice, token tile) is a unit.  With the decode
+// tables, whose tiles are as low as it takes to give every CTA one, an MMA of 48 or 56 rows takes the time of 128, and
+// every CTA walks all token tiles (500 tokens of the 1.7B shape: 318 TFLOP/s in the projections).  Here the tile height
+// and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs (64 cycles per 128 x 128 x
+// 16) and of its copies (48 bytes per cycle and SM from L2), plus what a unit costs besides.
+void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_tiles) {
+  const int nseg = ph.nacc == 2 ? 1 : ph.nseg;
+  ph.kc = ph.k / kChunkK;
+  long long best = -1;
+  auto shape = [&](int rows, int split) {
+    ph.rows = rows;
+    ph.ksplit = split;
+    ph.kslice = ph.kc / split;
+    int tile = 0;
+    for (int s = 0; s < nseg; ++s) {
+      ph.tile_start[s] = tile;
+      tile += (ph.n[s] + rows - 1) / rows;
+    }
+    ph.tile_start[nseg] = tile;
+    ph.ntiles = tile;
+    ph.nunits = tile * split;
+  };
+  int best_rows = kTileRows, best_split = 1;
+  for (int split = 1; split <= (allow_split ? kMaxSplit : 1); split *= 2) {
+    if (ph.kc % split) continue;
+    for (int rows = kTileRows; rows >= 64; rows -= 8) {
+      shape(rows, split);
+      const long long units = static_cast<long long>(ph.nunits) * token_tiles, rounds = (units + grid - 1) / grid;
+      const long long chunk = std::max(256 * ph.nacc, (ph.nacc * rows + 128) * 128 / 48);
+      const long long cost = rounds * (ph.kslice * chunk + 3000) + split * 600;
+      if (best < 0 || cost < best) {
+        best = cost;
+        best_rows = rows;
+        best_split = split;
+      }
+    }
+  }
+  shape(best_rows, best_split);
+  ph.kb = 1;
+  ph.gran = ph.nacc * ph.rows / 8;
 }
 
 // The split-K table (o_proj and down_proj cut along K so that every SM streams, fp32 partial sums added by
@@ -625,10 +672,12 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   const int L = c.layers;
   const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
   const size_t nmaps = maps_per_table(c), nphases = phases_per_table(c);
-  std::vector<CUtensorMap> maps(2 * nmaps);
-  std::vector<GemmPhase> phases(2 * nphases);
+  const int ntables = phase_tables(c);
+  std::vector<CUtensorMap> maps(ntables * nmaps);
+  std::vector<GemmPhase> phases(ntables * nphases);
   CUtensorMap* dmaps = at<CUtensorMap>(h, h->cv.tmaps);
-  CUtensorMap* operand_maps = dmaps + 2 * nmaps;
+  CUtensorMap* operand_maps = dmaps + ntables * nmaps;
+  auto operand_map = [&](int kind, int tile, int chunks) { return operand_maps + (kind * kOperandTiles + tile) * kOperandChunks + chunks - 1; };
   bf16* hidden_a = at<bf16>(h, h->cv.hidden);
   bf16* hidden_b = at<bf16>(h, h->cv.hidden2);
   bf16* qkv = at<bf16>(h, h->cv.qkv);
@@ -644,10 +693,11 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   }
   // Table 0: split-K: o and down store K-slice partials; the next
   // normalising phase adds them to the residual stream, which ping-pongs between
-  // hidden_b (after attention) and hidden_a (after the MLP).  Table 1: plain.
+  // hidden_b (after attention) and hidden_a (after the MLP).  Table 1: plain.  From table 2 on: split-K for prompts
+  // of that many token tiles (the last one: and more).
   bool use3d = h->use3d;
-  for (int table = 0; table < 2; ++table) {
-    const bool split = (table == 0);
+  for (int table = 0; table < ntables; ++table) {
+    const bool split = table != 1;
     if (split && !split_table_ok(c)) continue;
     GemmPhase* tp = phases.data() + table * nphases;
     CUtensorMap* tmaps_host = maps.data() + table * nmaps;
@@ -703,16 +753,20 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
         ph[3].epi = EPI_TP; ph[3].tp_buf = 1;
       }
       ph[1].gate = 1;  // decode attention streams cache tiles through the weight ring just before this phase
-      for (int i = 0; i < 4; ++i) finish_phase_tc(ph[i], h->grid, split && ph[i].epi == EPI_PARTIAL, c.max_tokens);
+      for (int i = 0; i < 4; ++i) {
+        const bool may_split = split && ph[i].epi == EPI_PARTIAL;
+        if (table < 2) finish_phase_tc(ph[i], h->grid, may_split, c.max_tokens);
+        else finish_phase_spread(ph[i], h->grid, may_split, table);
+      }
       if (split) {
         ph[2].add_parts = ph[1].ksplit; ph[2].partial = partial; ph[2].h_out = hidden_a;
         prev_parts = ph[3].ksplit;
       }
       for (int t = 0; t < kOperandTiles; ++t) {  // token operands: normalised rows, attention output, SiLU*up
-        ph[0].bmap[t] = operand_maps + OPERAND_XNORM * kOperandTiles + t;
-        ph[1].bmap[t] = operand_maps + OPERAND_ATTN * kOperandTiles + t;
-        ph[2].bmap[t] = operand_maps + OPERAND_XNORM * kOperandTiles + t;
-        ph[3].bmap[t] = operand_maps + OPERAND_ACT * kOperandTiles + t;
+        ph[0].bmap[t] = operand_map(OPERAND_XNORM, t, ph[0].kb);
+        ph[1].bmap[t] = operand_map(OPERAND_ATTN, t, ph[1].kb);
+        ph[2].bmap[t] = operand_map(OPERAND_XNORM, t, ph[2].kb);
+        ph[3].bmap[t] = operand_map(OPERAND_ACT, t, ph[3].kb);
       }
       // One TMA descriptor per matrix, boxed to the tile height and the K chunks per copy its phase chose.
       const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
@@ -732,8 +786,9 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     if (split) {
       head.add_parts = prev_parts; head.partial = partial;
     }
-    finish_phase_tc(head, h->grid, false, c.max_tokens);
-    for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_maps + OPERAND_XNORM * kOperandTiles + t;
+    if (table < 2) finish_phase_tc(head, h->grid, false, c.max_tokens);
+    else finish_phase_spread(head, h->grid, false, table);
+    for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_map(OPERAND_XNORM, t, head.kb);
     if (int e = encode_phase_weight_map(&tmaps_host[7 * L], w->lm_head, c.vocab, c.hidden, head, use3d)) return e;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -745,7 +800,9 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     static const int tiles[kOperandTiles] = {16, 32, 64, 128};
     for (int kind = 0; kind < 3; ++kind)
       for (int t = 0; t < kOperandTiles; ++t)
-        if (int e = encode_operand_map(&operand_host[kind * kOperandTiles + t], bases[kind], c.max_tokens, widths[kind], tiles[t])) return e;
+        for (int chunks = 1; chunks <= kOperandChunks && tiles[t] * chunks * 128 <= kBBytes / 2; ++chunks)
+          if (int e = encode_operand_map(&operand_host[(kind * kOperandTiles + t) * kOperandChunks + chunks - 1], bases[kind], c.max_tokens,
+                                         widths[kind], tiles[t], chunks, use3d)) return e;
     MK_CUDA(cudaMemcpyAsync(operand_maps, operand_host, sizeof(operand_host), cudaMemcpyHostToDevice, s));
     MK_CUDA(cudaStreamSynchronize(s));
   }
@@ -984,6 +1041,10 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
   p.mode = MODE_PREFILL; p.m = static_cast<int>(m); p.batch = batch; p.seq = sequence; p.capacity = 0;
   p.split = split_table_ok(h->cfg) ? 1 : 0;
   p.phases = at<GemmPhase>(h, h->cv.phases) + (p.split ? 0 : phases_per_table(h->cfg));
+  if (p.split && ntt > 1) {
+    p.spread = 1;
+    p.phases = at<GemmPhase>(h, h->cv.phases) + std::min(ntt, kSpreadTables + 1) * phases_per_table(h->cfg);
+  }
   p.n_gemm = 4 * L + 1;
   p.nbar = 8 * L + 1;  // as decode, plus one behind the rotation of q and k
   p.stream_once = (ntt == 1);
@@ -1022,7 +1083,7 @@ int mk_linear(mk_handle h, const void* x, const void* weight, const void* bias, 
   // Phase and descriptors go into the kernel's parameter block: nothing is uploaded, nothing synchronised.
   bool use3d = h->use3d;
   if (int e = encode_phase_weight_map(&p.linear_wmap, weight, n, k, ph, use3d)) return e;
-  if (int e = encode_operand_map(&p.linear_xmap, x, m, k, token_tile_of(m))) return e;
+  if (int e = encode_operand_map(&p.linear_xmap, x, m, k, token_tile_of(m), ph.kb, ph.map3d != 0)) return e;
   p.phases = nullptr;
   p.mode = MODE_LINEAR; p.m = m; p.batch = m; p.seq = 1;
   p.n_gemm = 1;
@@ -1188,10 +1249,11 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
       h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
       h->cfg.tp_size > 1 ? h->cfg.tp_size : 1);
   if (h->bound) {
-    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * 2);
+    const int ntables = phase_tables(h->cfg);
+    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * ntables);
     MK_CUDA(cudaMemcpy(phases.data(), at<GemmPhase>(h, h->cv.phases), phases.size() * sizeof(GemmPhase), cudaMemcpyDeviceToHost));
     static const char* names[5] = {"qkv", "o", "gate/up", "down", "lm_head"};
-    for (int table = 0; table < 2; ++table) {
+    for (int table = 0; table < ntables; ++table) {
       if (table == 0 && !split_table_ok(h->cfg)) continue;
       add("table %d:", table);
       for (int i = 0; i < 5; ++i) {

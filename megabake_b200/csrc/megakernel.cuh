@@ -63,7 +63,7 @@ constexpr int kTpFlagBytes = 256;        // head of a rank's exchange buffer: on
 // phase adds them, in slice order, while it builds its activation operand.
 struct GemmPhase {
   const CUtensorMap* tmap[3];  // device copies of the weights' TMA descriptors (tensor engine: box = 64 x rows x kb chunks)
-  const CUtensorMap* bmap[4];  // tensor engine: descriptors of the token operand for token tiles of 16, 32, 64, 128 (box = 64 x tile)
+  const CUtensorMap* bmap[4];  // descriptors of the token operand for token tiles of 16, 32, 64, 128 (box = 64 x tile x kb chunks)
   const bf16* w[3];            // raw weight pointers [N, K]
   const bf16* bias[3];
   int n[3];                    // rows of each matrix
@@ -119,6 +119,7 @@ struct KParams {
   int qkv_ld;
   int max_positions;
   int stream_once;    // 1: weights are read once per launch (L2 evict-first)
+  int spread;         // 1: prompts of several token tiles: every (row tile, K slice, token tile) is a unit of its own
   int split;          // 1: this launch runs the split-K phase table (residual updates applied by the consumer)
   int ragged;         // 1: len[l] points to one valid length per sequence (int32 [batch]) instead of one shared by the batch
   int sample;         // 1: after the logits, pick each sequence's greedy token on the device, store it in tokens_out and as the
