@@ -425,8 +425,8 @@ void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_ti
     }
   }
   shape(best_rows, best_split);
-  ph.kb = 1;
-  ph.gran = ph.nacc * ph.rows / 8;
+  ph.kb = getenv("XKB") ? atoi(getenv("XKB")) : 2;
+  ph.gran = ph.kb * ph.nacc * ph.rows / 8;
 }
 
 // The split-K table (o_proj and down_proj cut along K so that every SM streams, fp32 partial sums added by
