@@ -480,6 +480,8 @@ int prepare_kernels(int device, int head_dim) {
   if (!tensor_done[device]) {
     MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
+    MK_CUDA(cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem));
+    MK_CUDA(cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem));
     int per_sm = 0;
     MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, megakernel, kThreads, kSmemBytes));
     if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the megakernel does not fit on an SM of device %d", device);
@@ -1121,16 +1123,25 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
     return fail(MK_ERR_UNSUPPORTED, "mk_attention: %d keys exceed the per-row score buffer", k_len);
   if (reinterpret_cast<uintptr_t>(key) % 16 || reinterpret_cast<uintptr_t>(value) % 16)
     return fail(MK_ERR_ALIGNMENT, "mk_attention: key/value must be 16-byte aligned");
-  KParams p;
-  base_params(h, p);
-  p.mode = MODE_ATT; p.m = batch * q_len; p.batch = batch; p.seq = q_len;
-  p.n_gemm = 0; p.nbar = 0;
-  p.att_scale = scale;
-  p.op_q = static_cast<const bf16*>(query); p.op_k = static_cast<const bf16*>(key); p.op_v = static_cast<const bf16*>(value);
-  p.op_out = static_cast<bf16*>(output);
-  p.mask = static_cast<const bf16*>(mask);
-  p.op_qlen = q_len; p.op_klen = k_len;
-  return launch(h, p, stream);
+  const int q_size = h->cfg.q_heads * h->cfg.head_dim, kv_size = h->cfg.kv_heads * h->cfg.head_dim;
+  AttnArgs A{};
+  A.q = static_cast<const bf16*>(query); A.q_bstride = static_cast<long long>(q_len) * q_size; A.q_ld = q_size;
+  A.k = static_cast<bf16*>(const_cast<void*>(key)); A.v = static_cast<bf16*>(const_cast<void*>(value));
+  A.kv_bstride = static_cast<long long>(k_len) * kv_size; A.kv_ld = kv_size;
+  A.out = static_cast<bf16*>(output);  // [batch * heads, q_len, head_dim]
+  A.out_bstride = static_cast<long long>(h->cfg.q_heads) * q_len * h->cfg.head_dim;
+  A.out_tstride = h->cfg.head_dim; A.out_hstride = q_len * h->cfg.head_dim;
+  A.mask = static_cast<const bf16*>(mask); A.sq = q_len; A.klen = k_len; A.scale = scale;
+  const long long units = static_cast<long long>(batch) * h->cfg.q_heads * ((q_len + kPromptQueries - 1) / kPromptQueries);
+  if (units > INT32_MAX) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %lld blocks of queries", units);
+  auto go = [&](auto kernel, int smem) {
+    const int blocks = h->cfg.sm_limit > 0 ? std::min(static_cast<int>(units), h->grid) : static_cast<int>(units);
+    kernel<<<blocks, kWorkers, smem, static_cast<cudaStream_t>(stream)>>>(A, h->cfg.q_heads, h->cfg.kv_heads, batch, static_cast<int>(units));
+    return cudaGetLastError();
+  };
+  MK_CUDA(h->cfg.head_dim == 64 ? go(prompt_attention<64>, PromptLaunch<64>::kSmem) : go(prompt_attention<128>, PromptLaunch<128>::kSmem));
+  h->launches += 1;
+  return MK_OK;
 }
 
 int mk_status(mk_handle h, void* stream, mk_status_info* out) {

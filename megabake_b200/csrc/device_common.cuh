@@ -90,6 +90,14 @@ __device__ __forceinline__ uint4 normalise_vec(const uint4 xu, const uint4 wu, f
                     mul_bf16x2(wu.z, pack2(x[4] * r, x[5] * r)), mul_bf16x2(wu.w, pack2(x[6] * r, x[7] * r)));
 }
 
+// 2^x; softmax weights are 2^(s log2(e) - m log2(e)).
+constexpr float kLog2e = 1.4426950408889634f;
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 
 __device__ __forceinline__ float ldcg_bf16(const bf16* ptr) {

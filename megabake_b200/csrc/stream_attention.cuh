@@ -20,11 +20,6 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
   return d;
 }
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float word_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float word_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
