@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "decoder_kernel.cuh"
+#include "kv_attention.cuh"
 #include "stream_plan.h"
 
 using namespace mk;
@@ -482,6 +483,8 @@ int prepare_kernels(int device, int head_dim) {
     MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
     MK_CUDA(cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem));
     MK_CUDA(cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem));
+    MK_CUDA(cudaFuncSetAttribute(kv_attention_parts<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvLaunch<64>::kSmem));
+    MK_CUDA(cudaFuncSetAttribute(kv_attention_parts<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvLaunch<128>::kSmem));
     int per_sm = 0;
     MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, megakernel, kThreads, kSmemBytes));
     if (per_sm < 1) return fail(MK_ERR_UNSUPPORTED, "the megakernel does not fit on an SM of device %d", device);
@@ -516,6 +519,36 @@ bool stream_usable(mk_handle h, int batch, bool ragged) {
 }
 
 int token_tiles(int m) { return (m + token_tile_of(m) - 1) / token_tile_of(m); }
+
+int launch_kv_attention(mk_handle h, const void* query, const void* key, const void* value, void* key_cache, void* value_cache,
+                        int32_t* valid_length, int batch, int capacity, void* output, cudaStream_t stream) {
+  const mk_config& c = h->cfg;
+  const bool small = c.head_dim == 64;
+  KvAttentionArgs a{};
+  a.q = static_cast<const bf16*>(query); a.knew = static_cast<const bf16*>(key); a.vnew = static_cast<const bf16*>(value);
+  a.k = static_cast<bf16*>(key_cache); a.v = static_cast<bf16*>(value_cache); a.out = static_cast<bf16*>(output);
+  a.length = valid_length;
+  a.stats = at<float>(h, h->cv.att_xch); a.parts = at<float>(h, h->cv.att_part); a.ctrl = at<Control>(h, h->cv.ctrl);
+  a.status_mirror = h->mirror;
+  a.batch = batch; a.q_heads = c.q_heads; a.kv_heads = c.kv_heads; a.capacity = capacity;
+  a.width = std::min(c.kv_heads, 8);
+  while (c.kv_heads % a.width) --a.width;
+  a.shares = 8 / a.width;
+  // as many runs of positions as make one wave of blocks, but no fewer than four tiles of 16 positions to a warp
+  const int blocks_per_run = batch * (c.kv_heads / a.width), wave = h->grid * (small ? KvLaunch<64>::kBlocks : KvLaunch<128>::kBlocks);
+  const int by_length = (capacity + 64 * a.shares - 1) / (64 * a.shares);
+  a.chunks = std::max(1, std::min({wave / blocks_per_run, kMaxChunks / a.shares, by_length}));
+  a.slots = a.chunks * a.shares;
+  a.scale_log2 = h->att_scale * kLog2e;
+  const int units = blocks_per_run * a.chunks, blocks = c.sm_limit > 0 ? std::min(units, wave) : units;
+  if (small) kv_attention_parts<64><<<blocks, 256, KvLaunch<64>::kSmem, stream>>>(a, units);
+  else kv_attention_parts<128><<<blocks, 256, KvLaunch<128>::kSmem, stream>>>(a, units);
+  MK_CUDA(cudaGetLastError());
+  kv_attention_combine<<<(batch * c.q_heads * (c.head_dim / 4) + 127) / 128, 128, 0, stream>>>(a, c.head_dim);
+  MK_CUDA(cudaGetLastError());
+  h->launches += 1;
+  return MK_OK;
+}
 
 int attention_fits(mk_handle h, int keys, const char* what) {
   const int gs = h->cfg.q_heads / h->cfg.kv_heads;
@@ -1103,14 +1136,8 @@ int mk_kv_attention(mk_handle h, const void* query, const void* key, const void*
   if (int e = attention_fits(h, capacity, "mk_kv_attention")) return e;
   if (reinterpret_cast<uintptr_t>(key_cache) % 16 || reinterpret_cast<uintptr_t>(value_cache) % 16)
     return fail(MK_ERR_ALIGNMENT, "mk_kv_attention: caches must be 16-byte aligned");
-  KParams p;
-  base_params(h, p);
-  p.mode = MODE_KVATT; p.m = batch; p.batch = batch; p.seq = 1; p.capacity = capacity;
-  p.n_gemm = 0; p.nbar = 1;
-  p.op_q = static_cast<const bf16*>(query); p.op_k = static_cast<const bf16*>(key); p.op_v = static_cast<const bf16*>(value);
-  p.op_out = static_cast<bf16*>(output);
-  p.kc[0] = key_cache; p.vc[0] = value_cache; p.len[0] = valid_length;
-  return launch(h, p, stream, 1);
+  return launch_kv_attention(h, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output,
+                             static_cast<cudaStream_t>(stream));
 }
 
 int mk_attention(mk_handle h, const void* query, const void* key, const void* value, const void* mask, float scale,
@@ -1456,14 +1483,9 @@ int mk_kv_attention_static(int q_heads, int kv_heads, int head_dim, const void* 
   view.tp_epoch = 0; view.tp_bound = false;
   for (int r = 0; r < kMaxTp; ++r) view.tp_peer[r] = nullptr;
   if (int e = attention_fits(&view, capacity, "mk_kv_attention_static")) return e;
-  KParams p;
-  base_params(&view, p);
-  p.mode = MODE_KVATT; p.m = batch; p.batch = batch; p.seq = 1; p.capacity = capacity;
-  p.n_gemm = 0; p.nbar = 1;
-  p.op_q = static_cast<const bf16*>(query); p.op_k = static_cast<const bf16*>(key); p.op_v = static_cast<const bf16*>(value);
-  p.op_out = static_cast<bf16*>(output);
-  p.kc[0] = key_cache; p.vc[0] = value_cache; p.len[0] = valid_length;
-  if (int e = launch(&view, p, stream, 1)) return e;
+  if (int e = launch_kv_attention(&view, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output,
+                                  static_cast<cudaStream_t>(stream)))
+    return e;
   slot.epoch = view.epoch; slot.att_epoch = view.att_epoch; slot.launches = view.launches;
   return MK_OK;
 }

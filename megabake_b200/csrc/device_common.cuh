@@ -128,9 +128,6 @@ static __device__ __noinline__ void refuse_outputs(const Ctx& cx, int bad, int t
   if (p.mode == MODE_DECODE || p.mode == MODE_PREFILL) {
     out = p.logits;
     count = static_cast<long long>(p.m) * p.vocab;
-  } else if (p.mode == MODE_KVATT) {
-    out = p.op_out;
-    count = static_cast<long long>(p.batch) * p.q_heads * p.head_dim;
   }
   const bf16 nan = __ushort_as_bfloat16(0x7FC0);
   for (long long i = static_cast<long long>(cx.cta) * nthreads + tid; out != nullptr && i < count;

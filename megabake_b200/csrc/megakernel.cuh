@@ -41,7 +41,7 @@ static_assert(kSmemBytes <= 200704, "dynamic shared memory exceeds the 196 KiB c
 
 enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SILU = 2, EPI_PARTIAL = 3, EPI_TP = 4 };
 enum { B_PLAIN = 0, B_NORM = 1, B_ATTN = 2 };
-enum { MODE_DECODE = 0, MODE_PREFILL = 1, MODE_LINEAR = 2, MODE_KVATT = 3 };
+enum { MODE_DECODE = 0, MODE_PREFILL = 1, MODE_LINEAR = 2 };
 enum { EV_PHASE_ENTER = 1, EV_B_STAGED = 2, EV_FIRST_ACC = 3, EV_PHASE_DONE = 4, EV_BARRIER_DONE = 5, EV_ATTENTION_DONE = 6,
        EV_ATT_INPUTS = 7, EV_ATT_SCORES = 8, EV_ATT_STATS = 9, EV_ATT_VALUES = 10, EV_ATT_PARTIAL = 11, EV_FIRST_COPY = 12 };
 enum {
@@ -98,7 +98,7 @@ struct Control {
   int status;         // mk_device_status
   int where, cta, detail;
   int att_nch;        // context chunks the last attention phase used (read by the o projection)
-  uint32_t pad;
+  uint32_t pad;       // the stand-alone decode attention: 1 if its first launch refused the valid length
 };
 
 struct KParams {
@@ -148,8 +148,6 @@ struct KParams {
   const bf16 *embed, *cos_t, *sin_t;
   bf16* logits;
   // stand-alone attention ops
-  const bf16 *op_q, *op_k, *op_v;
-  bf16* op_out;
   // stand-alone projection (MODE_LINEAR): its phase and its two descriptors travel in the parameter block,
   // so the call needs no upload and no synchronisation
   GemmPhase linear_phase;

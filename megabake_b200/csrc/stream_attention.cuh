@@ -15,11 +15,6 @@
 
 namespace mk {
 
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
-  uint32_t d;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
-  return d;
-}
 __device__ __forceinline__ float word_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float word_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 

@@ -69,11 +69,18 @@ def kv_attention(
     source: torch.Tensor, key: torch.Tensor, value: torch.Tensor,
     key_cache: torch.Tensor, value_cache: torch.Tensor, valid_length: torch.Tensor,
 ) -> torch.Tensor:
+    if source.is_cuda:
+        return _kv_attention_cuda(source, key, value, key_cache, value_cache, valid_length)
     if source.shape[1] != 1:
         raise RuntimeError("megabake kv_attention supports one-token decode only")
     _check_layout(source, key)
-    if not source.is_cuda:
-        return _kv_attention_eager(source, key, value, key_cache, value_cache, valid_length)
+    return _kv_attention_eager(source, key, value, key_cache, value_cache, valid_length)
+
+
+def _kv_attention_cuda(source, key, value, key_cache, value_cache, valid_length):
+    if source.shape[1] != 1:
+        raise RuntimeError("megabake kv_attention supports one-token decode only")
+    _check_layout(source, key)
     kernels = _gpu_kernels(source.shape[2], key.shape[2], source.shape[3], source.shape[0], source.device)
     return kernels.kv_attention(source.contiguous(), key.contiguous(), value.contiguous(), key_cache, value_cache,
                                 valid_length)
@@ -91,9 +98,14 @@ def attention(
     """Softmax attention with Hugging Face eager numerics: ``query`` [batch, q, heads, dim],
     ``key``/``value`` [batch, k, kv_heads, dim], additive ``mask`` broadcastable to
     [batch, heads, q, k]; returns [batch * heads, q, dim]."""
+    if query.is_cuda:
+        return _attention_cuda(query, key, value, mask, scale)
     _check_layout(query, key)
-    if not query.is_cuda:
-        return _attention_eager(query, key, value, mask, scale)
+    return _attention_eager(query, key, value, mask, scale)
+
+
+def _attention_cuda(query, key, value, mask, scale):
+    _check_layout(query, key)
     batch, q_len, heads, dim = query.shape
     kernels = _gpu_kernels(heads, key.shape[2], dim, batch * q_len, query.device)
     if mask is not None:
@@ -110,6 +122,12 @@ def attention(
 def _(query, key, value, mask, scale):
     return query.new_empty((query.shape[0] * query.shape[2], query.shape[1], query.shape[3]))
 
+
+# CUDA calls go from the dispatcher straight to the functions above; the wrapper that custom_op puts around a
+# device-generic implementation (it checks that no output aliases an input) costs more than the launch.
+_cuda = torch.library.Library(_NAMESPACE, "FRAGMENT")
+_cuda.impl("kv_attention", _kv_attention_cuda, "CUDA")
+_cuda.impl("attention", _attention_cuda, "CUDA")
 
 KV_ATTENTION_OP = torch.ops.megabake.kv_attention.default
 ATTENTION_OP = torch.ops.megabake.attention.default

@@ -9,6 +9,7 @@ go to the current CUDA stream and return without synchronising.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from typing import Mapping, Sequence
@@ -50,6 +51,9 @@ def decode_trace(buffer: torch.Tensor):
     codes = (raw >> 56) & 0xFF
     times = raw & ((1 << 56) - 1)
     return codes, times
+
+
+_ALREADY = contextlib.nullcontext()
 
 
 class DecoderKernel:
@@ -118,6 +122,10 @@ class DecoderKernel:
     def _stream(self) -> int:
         return torch.cuda.current_stream(self.device).cuda_stream
 
+    def _on_device(self):
+        """The handle's device as the current one; most callers have made it that already."""
+        return _ALREADY if torch.cuda.current_device() == self.device.index else torch.cuda.device(self.device)
+
     def _compiler_error(self, stage: str, error: NativeError) -> CompilerError:
         return CompilerError(CompilerDiagnostic(stage, str(error)), safe_for_fallback=False)
 
@@ -138,12 +146,13 @@ class DecoderKernel:
         (the reference raises: src/megabake/lowering.py:229, src/megabake/compiler.py:2690)."""
         self._host_step_logits = None
         self._mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self._mirror_word = ctypes.c_int32.from_address(self._mirror.data_ptr())  # an indexed tensor read costs 3 us
         with torch.cuda.device(self.device):
             self._call("mk_set_status_mirror", self.lib.mk_set_status_mirror(self._handle, self._mirror.data_ptr()))
 
     def raise_if_failed(self) -> None:
         """Non-blocking: raise what an earlier launch reported, if anything."""
-        if int(self._mirror[0]) != 0:
+        if self._mirror_word.value != 0:
             self.check()
 
     def close(self) -> None:
@@ -205,7 +214,7 @@ class DecoderKernel:
             embed=_ptr(kept["model.embed_tokens.weight"]), final_norm=_ptr(kept["model.norm.weight"]),
             lm_head=_ptr(kept["lm_head.weight"]), rope_cos=_ptr(cosine), rope_sin=_ptr(sine), layers=layers,
         )
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_bind_weights", self.lib.mk_bind_weights(self._handle, ctypes.byref(packed), self._stream()))
         self._weights = kept  # keep the tensors alive while their pointers are bound
         self._bound_ptrs = tuple(t.data_ptr() for t in kept.values())
@@ -240,7 +249,7 @@ class DecoderKernel:
         keys, values, lengths, capacity = self._checked_state(batch, key_caches, value_caches, valid_lengths)
         self.raise_if_failed()
         logits = torch.empty((batch, 1, config.vocab), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_decode", self.lib.mk_decode(
                 self._handle, input_ids.data_ptr(), position_ids.data_ptr(), batch, keys, values, lengths,
                 capacity, logits.data_ptr(), self._stream()), stage="input-binding")
@@ -258,7 +267,7 @@ class DecoderKernel:
         keys, values, lengths, capacity = self._checked_state(batch, key_caches, value_caches, valid_lengths, per_sequence=True)
         self.raise_if_failed()
         logits = torch.empty((batch, 1, config.vocab), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_decode_ragged", self.lib.mk_decode_ragged(
                 self._handle, input_ids.data_ptr(), position_ids.data_ptr(), batch, keys, values, lengths,
                 capacity, logits.data_ptr(), self._stream()), stage="input-binding")
@@ -309,7 +318,7 @@ class DecoderKernel:
         self.raise_if_failed()
         tokens = torch.empty((steps, batch), dtype=torch.int64, device=self.device)
         logits = torch.empty((batch, 1, config.vocab), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_decode_steps", self.lib.mk_decode_steps(
                 self._handle, input_ids.data_ptr(), position_ids.data_ptr(), batch, keys, values, lengths,
                 capacity, int(steps), tokens.data_ptr(), logits.data_ptr(), self._stream()), stage="input-binding")
@@ -339,7 +348,7 @@ class DecoderKernel:
         self.raise_if_failed()
         if self._host_step_logits is None or self._host_step_logits.shape[0] != batch:
             self._host_step_logits = torch.empty((batch, 1, self.config.vocab), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_decode_step_host", self.lib.mk_decode_step_host(
                 self._handle, host_ids.data_ptr(), host_positions.data_ptr(), batch, keys, values, lengths, capacity,
                 self._host_step_logits.data_ptr(), host_tokens.data_ptr(), self._stream()), stage="input-binding")
@@ -359,7 +368,7 @@ class DecoderKernel:
             _require(mask, "attention mask", dtype=torch.bfloat16, device=self.device, shape=(batch, 1, sequence, sequence))
         self.raise_if_failed()
         logits = torch.empty((batch, sequence, self.config.vocab), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_prefill", self.lib.mk_prefill(
                 self._handle, input_ids.data_ptr(), position_ids.data_ptr(), _ptr(mask), batch, sequence,
                 logits.data_ptr(), self._stream()), stage="input-binding")
@@ -374,7 +383,7 @@ class DecoderKernel:
         if bias is not None:
             _require(bias, "bias", dtype=torch.bfloat16, device=self.device, shape=(n,))
         out = torch.empty((rows, n), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_linear", self.lib.mk_linear(
                 self._handle, source.data_ptr(), weight.data_ptr(), _ptr(bias), out.data_ptr(), rows, n, k,
                 self._stream()))
@@ -390,7 +399,7 @@ class DecoderKernel:
         _require(valid_length, "valid_length", dtype=torch.int32, device=self.device, shape=(1,))
         self.raise_if_failed()
         out = torch.empty((batch * heads, 1, dim), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_kv_attention", self.lib.mk_kv_attention(
                 self._handle, source.data_ptr(), key.data_ptr(), value.data_ptr(), key_cache.data_ptr(),
                 value_cache.data_ptr(), valid_length.data_ptr(), batch, key_cache.shape[1], out.data_ptr(),
@@ -404,10 +413,11 @@ class DecoderKernel:
         for name, tensor in (("query", query), ("key", key), ("value", value)):
             _require(tensor, name, dtype=torch.bfloat16, device=self.device)
         if mask is not None:
-            mask = mask.expand(batch, 1, q_len, k_len).contiguous()
+            if mask.shape != (batch, 1, q_len, k_len) or not mask.is_contiguous():
+                mask = mask.expand(batch, 1, q_len, k_len).contiguous()
             _require(mask, "mask", dtype=torch.bfloat16, device=self.device)
         out = torch.empty((batch * heads, q_len, dim), dtype=torch.bfloat16, device=self.device)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             self._call("mk_attention", self.lib.mk_attention(
                 self._handle, query.data_ptr(), key.data_ptr(), value.data_ptr(), _ptr(mask), float(scale),
                 batch, q_len, k_len, out.data_ptr(), self._stream()))
@@ -417,7 +427,7 @@ class DecoderKernel:
     def status(self) -> dict:
         """Synchronise and read the device status word (resets the handle's counters if it is not OK)."""
         info = MkStatusInfo()
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             code = self.lib.mk_status(self._handle, self._stream(), ctypes.byref(info))
         result = dict(status=_native.STATUS_NAMES.get(info.status, str(info.status)), where=info.where,
                       cta=info.cta, detail=info.detail, code=code)
@@ -506,6 +516,7 @@ class AttentionKernels:
 
     # The launches reuse DecoderKernel's methods: same handle layout, same checks.
     _stream = DecoderKernel._stream
+    _on_device = DecoderKernel._on_device
     _call = DecoderKernel._call
     _compiler_error = DecoderKernel._compiler_error
     kv_attention = DecoderKernel.kv_attention
