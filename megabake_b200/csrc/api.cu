@@ -426,7 +426,7 @@ void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_ti
     }
   }
   shape(best_rows, best_split);
-  ph.kb = getenv("XKB") ? atoi(getenv("XKB")) : 2;
+  ph.kb = ph.kslice % 2 == 0 ? 2 : 1;  // two chunks an entry: what the roles do per entry bounds a chunk with one
   ph.gran = ph.kb * ph.nacc * ph.rows / 8;
 }
 

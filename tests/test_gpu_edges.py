@@ -1,0 +1,103 @@
+"""The sizes at which the kernels' own splits have their edges, against the oracle.
+
+Tolerance: the one of the parity tests, 2e-2 absolute + 1e-2 relative.  Both sides round to bf16 (2^-9 relative) at the
+same places or one rounding apart, a few such roundings meet in an output of these one- and two-layer shapes, and the
+values are of order one: half of the bound is what the longest chain here can reach.
+"""
+
+import pytest
+import torch
+
+from conftest import assert_parity
+from megabake_b200.synth import rope_tables, synth_ids, synth_normal, synth_weights, tiny_config
+from test_gpu_parity import make_kernel, oracle_decode_compare
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    return torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,head_dim,context,vocab", [
+    (1, 4, 4, 64, 0, 250), (1, 8, 2, 64, 255, 333), (1, 9, 3, 64, 256, 512), (1, 7, 1, 128, 257, 512),  # one token: its own kernel class
+    (4, 8, 8, 64, 511, 512), (5, 9, 3, 64, 64, 250),    # last size of the second class, first of the third
+    (8, 4, 2, 128, 129, 512), (9, 8, 2, 64, 300, 333),  # one MMA tile of tokens, two
+    (16, 4, 4, 128, 40, 512), (17, 8, 8, 64, 200, 250), (32, 14, 2, 64, 70, 512), (33, 4, 2, 64, 90, 512),  # two, four, past the kernel
+])
+def test_streaming_decode_at_class_and_tile_edges(device, batch, heads, kv_heads, head_dim, context, vocab):
+    config = tiny_config(hidden=512, q_heads=heads, kv_heads=kv_heads, head_dim=head_dim, intermediate=768, vocab=vocab)
+    oracle_decode_compare(config, device, batch=batch, capacity=context + 2, prefill=context, steps=2)
+
+
+@pytest.mark.parametrize("kv_heads,head_dim,context", [(40, 64, 300), (40, 64, 319), (20, 128, 258)])
+def test_tensor_engine_attention_with_two_units_to_a_block(device, kv_heads, head_dim, context):
+    """More (sequence, head group) units than SMs: the second unit's cache stream starts before the first one ends."""
+    config = tiny_config(hidden=256, q_heads=kv_heads, kv_heads=kv_heads, head_dim=head_dim)
+    oracle_decode_compare(config, device, batch=32, capacity=context + 2, prefill=context, steps=2, engine="tcgen05")
+
+
+@pytest.mark.parametrize("tokens", [16, 17, 64, 65, 128, 129, 256, 257, 385, 513])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_prompts_at_token_tile_edges(device, tokens, head_dim):
+    """One token tile (16 to 128), then a unit per token tile with tables for two, three and four or more."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=512, q_heads=6, kv_heads=2, head_dim=head_dim, intermediate=832, rope_style="hf")
+    weights = synth_weights(config, seed=12, norm_std=0.1, device=device)
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=tokens)
+    ids = synth_ids(tokens, config.vocab, seed=12).view(1, tokens).to(device)
+    positions = torch.arange(tokens, device=device).view(1, tokens)
+    with torch.no_grad():
+        expected = oracle.prefill(config, weights, rope_tables(config, tokens, device=device), ids, positions,
+                                  oracle.causal_mask(1, tokens).to(device))
+    logits = kernel.prefill(ids)
+    kernel.check()
+    assert_parity(logits, expected, f"prompt of {tokens}")
+
+
+def _tensors(device, batch, queries, keys, heads, kv_heads, head_dim):
+    return [synth_normal((batch, n, h, head_dim), seed=13, name=name, std=1.0, device=device)
+            for name, n, h in (("q", queries, heads), ("k", keys, kv_heads), ("v", keys, kv_heads))]
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (8, 2, 128)])
+@pytest.mark.parametrize("queries,keys", [(1, 1), (1, 65), (63, 63), (64, 64), (65, 65), (130, 33), (200, 449)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_prompt_attention_op_at_block_and_tile_edges(device, heads, kv_heads, head_dim, queries, keys, masked):
+    """Ragged query blocks and key tiles, odd key counts (mask rows off the 4-byte grid), rows that begin with whole tiles of
+    the lowest finite mask value."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value = _tensors(device, 2, queries, keys, heads, kv_heads, head_dim)
+    mask = None
+    if masked:
+        mask = torch.zeros((2, 1, queries, keys), dtype=torch.bfloat16, device=device)
+        hidden = torch.arange(keys, device=device) < torch.arange(queries, device=device).view(-1, 1).clamp(max=keys - 1)
+        mask[:, 0].masked_fill_(hidden, torch.finfo(torch.bfloat16).min)
+    out = torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5)
+    expected = oracle.attention(query, key, value, mask, head_dim ** -0.5)
+    assert_parity(out, expected, f"attention {queries} x {keys}")
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (14, 2, 64), (11, 11, 64), (32, 32, 64), (32, 8, 128)])
+@pytest.mark.parametrize("batch,context", [(1, 0), (3, 15), (1, 16), (2, 17), (16, 63), (2, 700)])
+def test_decode_attention_op_at_tile_and_run_edges(device, heads, kv_heads, head_dim, batch, context):
+    """The new position first, last and alone in a tile of 16, runs of positions without any; cache rows past the valid
+    length hold NaN, which must not reach the result."""
+    from oracle import decoder_oracle as oracle
+
+    capacity = context + 5
+    query, key, value = _tensors(device, batch, 1, 1, heads, kv_heads, head_dim)
+    caches = [synth_normal((batch, capacity, kv_heads, head_dim), seed=14, name=name, std=1.0, device=device) for name in ("kc", "vc")]
+    for cache in caches:
+        cache[:, context:] = float("nan")
+    mine, ref = [c.clone() for c in caches], [c.clone() for c in caches]
+    length, ref_length = (torch.full((1,), context, dtype=torch.int32, device=device) for _ in range(2))
+    out = torch.ops.megabake.kv_attention(query, key, value, mine[0], mine[1], length)
+    expected = oracle.kv_attention(query, key, value, ref[0], ref[1], ref_length)
+    assert_parity(out, expected, f"kv_attention at {context}")
+    assert int(length) == context + 1
+    for a, b in zip(mine, ref):
+        assert torch.equal(a[:, :context + 1], b[:, :context + 1]) and bool(torch.isnan(a[:, context + 1:].float()).all())
