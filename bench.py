@@ -499,8 +499,8 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "traffic_source": traffic_source, "peak_source": f"of {peak_kind}",
                      "algorithmic_bytes_per_launch": bytes_per_launch,
-                     "kernel": ("mk::megakernel_small<%d, %s>" % (args.batch, "true" if args.batch == 1 else "false")
-                                if args.batch <= 4 and args.engine != "tcgen05" else "mk::megakernel"),
+                     "kernel": ("mk::decode_stream" if args.batch <= 32 and config.hidden <= 2048 and args.engine != "tcgen05"
+                                else "mk::megakernel"),
                      "launch_us": launch_ms * 1e3, "frac_of_8TBps_nominal": achieved / 8000.0},
         "e2e": {"value": e2e_value, "unit": "tokens/s", "h2d_bytes_per_step": 16 * args.batch,
                 "d2h_bytes_per_step": 8 * args.batch, "us_per_call": 1e3 * e2e_ms / e2e_steps,

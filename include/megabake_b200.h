@@ -149,8 +149,7 @@ int mk_decode(mk_handle handle, const int64_t* ids, const int64_t* positions, in
 /* mk_decode for sequences of different lengths in one batch: valid_lengths[layer] points to int32 [batch],
  * one filled-position count per sequence (each is read, used as that sequence's append row and advanced by
  * one); sequence b attends over its own [0, valid_length[b]] and rotates with positions[b].  Everything else
- * as mk_decode.  Runs on the tensor engine (the context split follows the longest sequence; chunks past a
- * shorter sequence's end are empty).
+ * as mk_decode.  The context split follows the longest sequence; parts past a shorter sequence's end are empty.
  * Reference: none; its contract is one length shared by the batch (src/megabake/lowering.py:160-190,
  * README.md:29 lists per-sequence lengths as not supported). */
 int mk_decode_ragged(mk_handle handle, const int64_t* ids, const int64_t* positions, int batch,
