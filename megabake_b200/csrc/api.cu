@@ -52,11 +52,11 @@ int qkv_width(const mk_config& c) { return (c.q_heads + 2 * c.kv_heads) * c.head
 // Token-operand descriptors of the tensor engine: (normalised rows, attention output, SiLU*up, mk_linear's
 // source) x (token tiles of 16, 32, 64), behind the weight descriptors.
 constexpr int kCacheMapSets = 8;  // cache-descriptor sets a handle remembers (one per KV state it is called with in turn)
-constexpr int kOperandTiles = 4;  // token tiles of 16, 32, 64, 128
+constexpr int kOperandTiles = 5;  // token tiles of 16, 32, 64, 128, 256
 constexpr int kOperandChunks = 4; // K chunks per copy: 1 .. 4
 constexpr int kOperandKinds = 3, kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;
 enum { OPERAND_XNORM = 0, OPERAND_ATTN = 1, OPERAND_ACT = 2 };
-// Phase tables: split-K, plain, and for prompts of more than one token tile one each for two, three and four or more.
+// Phase tables: split-K, plain, and for prompts of more than 128 tokens one each for one, two and three or more tiles of 256.
 constexpr int kSpreadTables = 3;
 int phase_tables(const mk_config& c) { return 2 + (c.max_tokens > 128 && c.tp_size <= 1 ? kSpreadTables : 0); }
 int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128)); }
@@ -388,11 +388,12 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
   ph.gran = ph.nacc * kb * ph.rows / 8;
 }
 
-// Tensor engine, prompts of several token tiles of 128: every (row tile, K slice, token tile) is a unit.  With the decode
+// Tensor engine, prompts of more than 128 tokens: every (row tile, K slice, tile of 256 tokens) is a unit.  With the decode
 // tables, whose tiles are as low as it takes to give every CTA one, an MMA of 48 or 56 rows takes the time of 128, and
-// every CTA walks all token tiles (500 tokens of the 1.7B shape: 318 TFLOP/s in the projections).  Here the tile height
-// and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs (64 cycles per 128 x 128 x
-// 16) and of its copies (48 bytes per cycle and SM from L2), plus what a unit costs besides.
+// every CTA walks all token tiles.  Here both operands come from L2, about 44 bytes per cycle and SM when all of them read
+// (128-token tiles: the projections of 500 tokens of the 1.7B shape at 12 TB/s), so the tile is as wide as tensor memory
+// allows, and the tile height and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs
+// and of its copies, plus what a unit costs besides.
 void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_tiles) {
   const int nseg = ph.nacc == 2 ? 1 : ph.nseg;
   ph.kc = ph.k / kChunkK;
@@ -416,7 +417,7 @@ void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_ti
     for (int rows = kTileRows; rows >= 64; rows -= 8) {
       shape(rows, split);
       const long long units = static_cast<long long>(ph.nunits) * token_tiles, rounds = (units + grid - 1) / grid;
-      const long long chunk = std::max(256 * ph.nacc, (ph.nacc * rows + 128) * 128 / 48);
+      const long long chunk = std::max(512 * ph.nacc, (ph.nacc * rows + kSpreadTok) * 128 / 44);
       const long long cost = rounds * (ph.kslice * chunk + 3000) + split * 600;
       if (best < 0 || cost < best) {
         best = cost;
@@ -426,7 +427,7 @@ void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_ti
     }
   }
   shape(best_rows, best_split);
-  ph.kb = ph.kslice % 2 == 0 ? 2 : 1;  // two chunks an entry: what the roles do per entry bounds a chunk with one
+  ph.kb = 1;
   ph.gran = ph.kb * ph.nacc * ph.rows / 8;
 }
 
@@ -791,7 +792,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
       for (int i = 0; i < 4; ++i) {
         const bool may_split = split && ph[i].epi == EPI_PARTIAL;
         if (table < 2) finish_phase_tc(ph[i], h->grid, may_split, c.max_tokens);
-        else finish_phase_spread(ph[i], h->grid, may_split, table);
+        else finish_phase_spread(ph[i], h->grid, may_split, table - 1);
       }
       if (split) {
         ph[2].add_parts = ph[1].ksplit; ph[2].partial = partial; ph[2].h_out = hidden_a;
@@ -822,7 +823,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
       head.add_parts = prev_parts; head.partial = partial;
     }
     if (table < 2) finish_phase_tc(head, h->grid, false, c.max_tokens);
-    else finish_phase_spread(head, h->grid, false, table);
+    else finish_phase_spread(head, h->grid, false, table - 1);
     for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_map(OPERAND_XNORM, t, head.kb);
     if (int e = encode_phase_weight_map(&tmaps_host[7 * L], w->lm_head, c.vocab, c.hidden, head, use3d)) return e;
   }
@@ -832,7 +833,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     memset(operand_host, 0, sizeof(operand_host));
     const void* bases[3] = {at<bf16>(h, h->cv.xnorm), attn, act};
     const int widths[3] = {c.hidden, q_size, c.intermediate};
-    static const int tiles[kOperandTiles] = {16, 32, 64, 128};
+    static const int tiles[kOperandTiles] = {16, 32, 64, 128, 256};
     for (int kind = 0; kind < 3; ++kind)
       for (int t = 0; t < kOperandTiles; ++t)
         for (int chunks = 1; chunks <= kOperandChunks && tiles[t] * chunks * 128 <= kBBytes / 2; ++chunks)
@@ -1077,8 +1078,9 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
   p.split = split_table_ok(h->cfg) ? 1 : 0;
   p.phases = at<GemmPhase>(h, h->cv.phases) + (p.split ? 0 : phases_per_table(h->cfg));
   if (p.split && ntt > 1) {
+    const int tiles = static_cast<int>((m + kSpreadTok - 1) / kSpreadTok);
     p.spread = 1;
-    p.phases = at<GemmPhase>(h, h->cv.phases) + std::min(ntt, kSpreadTables + 1) * phases_per_table(h->cfg);
+    p.phases = at<GemmPhase>(h, h->cv.phases) + (1 + std::min(tiles, kSpreadTables)) * phases_per_table(h->cfg);
   }
   p.n_gemm = 4 * L + 1;
   p.nbar = 8 * L + 1;  // as decode, plus one behind the rotation of q and k

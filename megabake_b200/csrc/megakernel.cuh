@@ -20,7 +20,10 @@ constexpr int kRingGranules = 120;       // keeps the CTA under 196 KiB of share
 constexpr int kRingBytes = kRingGranules * kGranule;
 constexpr int kChunkBars = 128;          // full/empty barrier pairs, indexed by chunk sequence number
 constexpr int kTok = MK_TOKEN_TILE;      // token columns an epilogue step reads from TMEM
-constexpr int kMaxTok = 128;             // largest token tile (UMMA N is 16, 32, 64 or 128)
+constexpr int kMaxTok = 128;             // largest token tile (UMMA N is 16, 32, 64 or 128) ...
+constexpr int kSpreadTok = 256;          // ... but for prompts of more tokens (see spread): operands are read from L2, and fewer bytes per product
+// Those read both operands from L2, several chunks of each in flight: the activation ring takes a part of the weight ring.
+constexpr int kSpreadRingGranules = 88;
 constexpr int kBSlots = 32;              // activation K-chunks resident per CTA (two halves of 16)
 constexpr int kBHalf = kBSlots / 2;
 constexpr int kBSlotBytes = kTok * 128;  // 2 KiB
@@ -63,7 +66,7 @@ constexpr int kTpFlagBytes = 256;        // head of a rank's exchange buffer: on
 // phase adds them, in slice order, while it builds its activation operand.
 struct GemmPhase {
   const CUtensorMap* tmap[3];  // device copies of the weights' TMA descriptors (tensor engine: box = 64 x rows x kb chunks)
-  const CUtensorMap* bmap[4];  // descriptors of the token operand for token tiles of 16, 32, 64, 128 (box = 64 x tile x kb chunks)
+  const CUtensorMap* bmap[5];  // descriptors of the token operand for token tiles of 16, 32, 64, 128, 256 (box = 64 x tile x kb chunks)
   const bf16* w[3];            // raw weight pointers [N, K]
   const bf16* bias[3];
   int n[3];                    // rows of each matrix
