@@ -57,6 +57,27 @@ def test_prompts_at_token_tile_edges(device, tokens, head_dim):
     assert_parity(logits, expected, f"prompt of {tokens}")
 
 
+def test_gates_beyond_the_straight_line_of_the_silu(device):
+    """Gates past +-80 take the epilogue's plain division, their neighbours in a token's column the corrected quotient."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=512, q_heads=6, kv_heads=2, intermediate=832, rope_style="hf")
+    weights = dict(synth_weights(config, seed=15, norm_std=0.1, device=device))
+    for layer in range(config.layers):
+        for name, factor in (("gate", 64.0), ("up", 1 / 64.0)):  # powers of two: the products only change their exponents
+            key = f"model.layers.{layer}.mlp.{name}_proj.weight"
+            weights[key] = (weights[key] * factor).contiguous()
+    tokens = 40
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=tokens)
+    ids = synth_ids(tokens, config.vocab, seed=15).view(1, tokens).to(device)
+    positions = torch.arange(tokens, device=device).view(1, tokens)
+    with torch.no_grad():
+        expected = oracle.prefill(config, weights, rope_tables(config, tokens, device=device), ids, positions,
+                                  oracle.causal_mask(1, tokens).to(device))
+    assert_parity(kernel.prefill(ids), expected, "prompt with large gates")
+    kernel.check()
+
+
 def _tensors(device, batch, queries, keys, heads, kv_heads, head_dim):
     return [synth_normal((batch, n, h, head_dim), seed=13, name=name, std=1.0, device=device)
             for name, n, h in (("q", queries, heads), ("k", keys, kv_heads), ("v", keys, kv_heads))]
