@@ -211,20 +211,28 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
           own[0] += __shfl_xor_sync(0xffffffffu, own[0], x);
           own[1] += __shfl_xor_sync(0xffffffffu, own[1], x);
         }
+        // A warp that holds its heads' whole context alone has nothing to exchange: the others, which it does not wait for,
+        // may have their value sums in the scratch already.
         float2* const stat = reinterpret_cast<float2*>(scratch) + hh * 64;  // [split][query head]
-        if (lg == 0) {
-          stat[split * 8 + 2 * lt] = make_float2(mt[0], own[0]);
-          stat[split * 8 + 2 * lt + 1] = make_float2(mt[1], own[1]);
+        if (nsplit > 1) {
+          if (lg == 0) {
+            stat[split * 8 + 2 * lt] = make_float2(mt[0], own[0]);
+            stat[split * 8 + 2 * lt + 1] = make_float2(mt[1], own[1]);
+          }
+          stream_sync();
         }
-        if (nsplit == 1) __syncwarp();
-        else stream_sync();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float2 all[8];
           float top = -INFINITY, total = 0.f;
 #pragma unroll
           for (int s8 = 0; s8 < 8; ++s8) {
-            all[s8] = s8 < nsplit ? stat[s8 * 8 + 2 * lt + h] : make_float2(-INFINITY, 0.f);
+            all[s8] = make_float2(-INFINITY, 0.f);
+            if (nsplit == 1) {
+              if (s8 == 0) all[s8] = make_float2(mt[h], own[h]);
+            } else if (s8 < nsplit) {
+              all[s8] = stat[s8 * 8 + 2 * lt + h];
+            }
             top = fmaxf(top, all[s8].x);
           }
 #pragma unroll
@@ -238,8 +246,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
             s[bi][h + 2] = bf16_round(ex2(s[bi][h + 2] - top) / total);
           }
         }
-        if (nsplit == 1) __syncwarp();
-        else stream_sync();  // the statistics have been read: the area is free for the sums
+        if (nsplit > 1) stream_sync();  // the statistics have been read: the area is free for the sums
       } else {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

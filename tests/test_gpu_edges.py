@@ -31,6 +31,14 @@ def test_streaming_decode_at_class_and_tile_edges(device, batch, heads, kv_heads
     oracle_decode_compare(config, device, batch=batch, capacity=context + 2, prefill=context, steps=2)
 
 
+@pytest.mark.parametrize("batch,context", [(batch, context) for batch in (16, 32) for context in (0, 15, 16, 30, 31)])
+def test_streaming_decode_with_a_context_of_one_tile_to_a_warp(device, batch, context):
+    """Eight heads to a tile of 32 positions: every warp has its head's whole context, and none waits for another.  From 32
+    positions on there is a second tile."""
+    config = tiny_config(hidden=512, q_heads=32, kv_heads=32, head_dim=64, intermediate=768, vocab=512)
+    oracle_decode_compare(config, device, batch=batch, capacity=context + 3, prefill=context, steps=3)
+
+
 @pytest.mark.parametrize("kv_heads,head_dim,context", [(40, 64, 300), (40, 64, 319), (20, 128, 258)])
 def test_tensor_engine_attention_with_two_units_to_a_block(device, kv_heads, head_dim, context):
     """More (sequence, head group) units than SMs: the second unit's cache stream starts before the first one ends."""
