@@ -516,7 +516,7 @@ int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
 // The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.
 bool stream_usable(mk_handle h, int batch, bool ragged) {
   return h->cfg.engine != MK_ENGINE_TCGEN05 && batch <= kStreamTokens && h->stream_ok[stream_plan_of(batch)] &&
-         h->kv_maps_ok && stream_parts_ok(h->cfg, batch, h->grid) && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
+         h->kv_maps_ok && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
 }
 
 int token_tiles(int m) { return (m + token_tile_of(m) - 1) / token_tile_of(m); }

@@ -62,11 +62,6 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
   StreamMisc* const sm = stream_opaque(th.sm);
   const int wtid = stream_opaque(th.wtid);
   const KParams& p = *sm->p;
-  while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= layer && !stream_aborted(sm)) {
-  }
-  __threadfence_block();
-  const StreamSegment* const segs = sm->seg[layer & 1];
-  const int nparts = stream_aborted(sm) ? 0 : sm->seg_count[layer & 1];
   const bf16* const qkv = sm->plan.dst[SP_QKV][th.turn];  // [sequence][q | k | v], plain order
   const uint32_t stamp = p.att_epoch + static_cast<uint32_t>(layer) + 1u;
   float* const scratch = reinterpret_cast<float*>(stream_scratch(sm));  // [slot of a (warp, head)][HD + 2]
@@ -83,9 +78,26 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
   const int style = p.rope_style;
   constexpr int kRow = HD + 2;
 
+  // Lists of parts, mostly one (every layer has at least one, if empty).
+  while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= th.list && !stream_aborted(sm)) {
+  }
+  __threadfence_block();
+  int count = stream_aborted(sm) ? 0 : sm->seg_count[th.list & 1];
 #pragma unroll 1
-  for (int part = 0; part < nparts; ++part) {
-    const StreamSegment sg = segs[part];
+  for (int part = 0;; ++part) {
+    if (part == (count & (kStreamMoreParts - 1))) {
+      ++th.list;
+      if (!(count & kStreamMoreParts)) break;
+      stream_sync();  // everybody is done with the list: the helper may write the next but one
+      if (wtid == 0) *reinterpret_cast<volatile int*>(&sm->seg_taken) = th.list;
+      while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= th.list && !stream_aborted(sm)) {
+      }
+      __threadfence_block();
+      count = stream_aborted(sm) ? 0 : sm->seg_count[th.list & 1];
+      part = -1;
+      continue;
+    }
+    const StreamSegment sg = sm->seg[th.list & 1][part];
     const int len = sg.len;  // the new position
     const int kvh = sg.group * hpu + hh, pos = sm->pos_s[sg.b];
     const bf16* row = qkv + static_cast<size_t>(sg.b) * qkv_ld;

@@ -87,7 +87,10 @@ struct StreamSegment {
   int seg, nseg;             // this part's number and how many parts there are
   int len;                   // cached positions of the sequence: the new one's place
 };
-constexpr int kStreamSegments = 16;  // parts of a layer a CTA can have (the host checks)
+// A CTA's parts of a layer come in lists of at most this many.  Equal lengths need one list; a long sequence beside many
+// short ones makes the runs long, and a run through the short ones crosses a head group per tile.
+constexpr int kStreamSegments = 16;
+constexpr int kStreamMoreParts = 1 << 16;  // in a list's count: another list of the same layer follows
 
 // Shared memory beside the ring.  What the phases need now and then lives here and not in registers, which the token
 // operand fills.
@@ -107,9 +110,10 @@ struct StreamMisc {
   int psum_offset;  // bytes from the end of this block to the partial sums (the attention area comes first)
   int first_tile[kStreamPhases], first_slice[kStreamPhases], units[kStreamPhases];  // where this CTA's units start, how many
   StreamLayer lw[2];            // this layer's and the next one's vectors
-  StreamSegment seg[2][kStreamSegments];  // this CTA's attention parts of two layers, worked out ahead by a helper thread
-  int seg_count[2];             // ... how many
-  int seg_ready;                // layers whose parts are in place
+  StreamSegment seg[2][kStreamSegments];  // two lists of this CTA's attention parts, worked out ahead by a helper thread
+  int seg_count[2];             // ... how many, and whether the layer has more (kStreamMoreParts)
+  int seg_ready;                // lists put in place so far
+  int seg_taken;                // the list the consumers are at: all of them are done with the ones before
   StreamPlan plan;
   int id_s[kStreamTokens];
   int pos_s[kStreamTokens];
@@ -198,6 +202,7 @@ struct StreamThread {
   int wtid;
   int turn, last_turn;  // layer % 3, and the layer before's
   int pbuf;      // which half of the partial-sum area the next tile uses
+  int list;      // the list of attention parts that comes next
   bool tracing;  // this thread records events
   __device__ __forceinline__ void trace(int code) const {
     if (tracing) stream_trace_record(sm, code);
@@ -240,13 +245,13 @@ struct StreamTiles {
   int runs;        // > 0: every group is cut into this many runs, none of which crosses groups
   int nt;          // tiles per (sequence, group) when all lengths are equal, else 0 (the new position included)
   const int* len;  // valid lengths: one, or one per sequence
-  __device__ __forceinline__ int tiles_of(int b) const {
+  __host__ __device__ __forceinline__ int tiles_of(int b) const {
     return nt > 0 ? nt : len[b] / tile_keys + 1;
   }
-  __device__ __forceinline__ int length_of(int b) const { return nt > 0 ? len[0] : len[b]; }
+  __host__ __device__ __forceinline__ int length_of(int b) const { return nt > 0 ? len[0] : len[b]; }
 };
 
-__device__ __forceinline__ StreamTiles stream_tiles(const KParams& p, const int* len, int cta, int grid) {
+__host__ __device__ __forceinline__ StreamTiles stream_tiles(const KParams& p, const int* len, int cta, int grid) {
   StreamTiles s;
   s.groups = p.kv_heads / p.stream_hpu;
   s.tile_keys = p.stream_tile_keys;
@@ -292,7 +297,7 @@ __device__ __forceinline__ const int* stream_lengths(const KParams& p, const Str
   return sm->len_s + (p.ragged ? layer * p.batch : layer);
 }
 
-__device__ __forceinline__ StreamSegment stream_segment(const StreamTiles& s, int at, int cta) {
+__host__ __device__ __forceinline__ StreamSegment stream_segment(const StreamTiles& s, int at, int cta) {
   StreamSegment g;
   int start;  // first tile of the (sequence, group)
   if (s.nt > 0) {
@@ -326,24 +331,35 @@ __device__ __forceinline__ StreamSegment stream_segment(const StreamTiles& s, in
   return g;
 }
 
-// A helper thread works out the parts of each layer, one layer ahead: the divisions would be on every consumer's path.
+// The parts that follow from tile `at` of this CTA's run on, as many as a list holds; `at` moves past them.
+__host__ __device__ __forceinline__ int stream_next_parts(const StreamTiles& s, int cta, int& at, StreamSegment* list) {
+  int n = 0;
+  while (n < kStreamSegments && at < s.last) {
+    const StreamSegment g = stream_segment(s, at, cta);
+    list[n++] = g;
+    at += g.t1 - g.t0;
+  }
+  return n;
+}
+
+// A helper thread works out the parts of each layer, a list ahead: the divisions would be on every consumer's path.
 __device__ __forceinline__ void stream_plan_parts(StreamMisc* sm) {
   const KParams& p = *sm->p;
+  int list = 0;
   for (int layer = 0; layer < p.layers; ++layer) {
-    while (*reinterpret_cast<volatile int*>(&sm->progress) < layer - 1) {
-      if (stream_aborted(sm)) return;
-      __nanosleep(200);
-    }
     const StreamTiles tiles = stream_tiles(p, stream_lengths(p, sm, layer), sm->cta, sm->grid);
-    int n = 0;
-    for (int at = tiles.first; at < tiles.last; ++n) {
-      const StreamSegment g = stream_segment(tiles, at, sm->cta);
-      if (n < kStreamSegments) sm->seg[layer & 1][n] = g;
-      at += g.t1 - g.t0;
-    }
-    sm->seg_count[layer & 1] = n;
-    __threadfence_block();
-    *reinterpret_cast<volatile int*>(&sm->seg_ready) = layer + 1;
+    int at = tiles.first;
+    do {
+      while (*reinterpret_cast<volatile int*>(&sm->seg_taken) < list - 1) {  // the list before the last is still in use
+        if (stream_aborted(sm)) return;
+        __nanosleep(200);
+      }
+      const int n = stream_next_parts(tiles, sm->cta, at, sm->seg[list & 1]);
+      sm->seg_count[list & 1] = n | (at < tiles.last ? kStreamMoreParts : 0);
+      ++list;
+      __threadfence_block();
+      *reinterpret_cast<volatile int*>(&sm->seg_ready) = list;
+    } while (at < tiles.last);
   }
 }
 

@@ -137,12 +137,16 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
   th.pbuf = 0;
   th.turn = 0;
   th.last_turn = 2;
+  th.list = 0;
   th.tracing = wtid == 0 && sm->trace_on != 0;
   stream_embed<TM>(sm, wtid);
 #pragma unroll 1
   for (int layer = 0;; ++layer) {  // the last round is the output head
     const bool head = layer == layers;
-    if (wtid == 0) *reinterpret_cast<volatile int*>(&sm->progress) = layer;
+    if (wtid == 0) {
+      *reinterpret_cast<volatile int*>(&sm->progress) = layer;
+      *reinterpret_cast<volatile int*>(&sm->seg_taken) = th.list;
+    }
     // the next layer's vectors: requested here, passed on through shared memory at the end of the layer
     uint32_t word = 0u;
     if (wtid < kLayerWords && layer + 1 < layers) word = __ldg(reinterpret_cast<const uint32_t*>(sm->plan.layers + layer + 1) + wtid);
@@ -221,6 +225,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
     sm->wabort = 0;
     sm->progress = 0;
     sm->seg_ready = 0;
+    sm->seg_taken = 0;
     sm->copies = stream_copies(TM);
     sm->bad = 0;
     sm->trace_n = 0;

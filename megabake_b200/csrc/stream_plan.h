@@ -142,9 +142,5 @@ inline void stream_divide(KParams& p, int scratch, int batch) {
 inline int stream_smem_bytes(const KParams& p) {
   return 1024 + p.stream_slots * kStreamSlotBytes + kStreamMiscBytes + p.stream_scratch_bytes + stream_psum_bytes(p.m);
 }
-// A CTA's run must not touch more head groups than it has room for.
-inline bool stream_parts_ok(const mk_config& c, int batch, int grid) {
-  return batch * (c.kv_heads / stream_heads_per_tile(c, batch)) / grid + 3 <= kStreamSegments;
-}
 
 }  // namespace mk

@@ -1,0 +1,70 @@
+// Host build of the streaming decode kernel's dealing of cached positions, for test_stream_dealing.py: walks one layer the
+// way the kernel's producer and its helper thread do and checks what the consumers rely on.
+#include <vector>
+
+#include "../megabake_b200/csrc/stream_plan.h"
+
+using namespace mk;
+
+// Returns 0, or the number of the first rule that is broken; `longest` and `lists`: the most parts and lists of a CTA.
+extern "C" int check_dealing(int grid, int batch, int q_heads, int kv_heads, int head_dim, int ragged, const int* len, int* longest, int* lists) {
+  mk_config c{};
+  c.q_heads = q_heads;
+  c.kv_heads = kv_heads;
+  c.head_dim = head_dim;
+  static KParams p;
+  p = KParams{};
+  p.batch = batch;
+  p.kv_heads = kv_heads;
+  p.ragged = ragged;
+  p.stream_hpu = stream_heads_per_tile(c, batch);
+  p.stream_tile_keys = kStreamSlotBytes / (head_dim * 2 * p.stream_hpu);
+  const int groups = kv_heads / p.stream_hpu;
+  struct Group {
+    int tiles = 0, parts = 0, nseg = 0;
+    std::vector<int> seen;  // by part number
+  };
+  std::vector<Group> all(static_cast<size_t>(batch) * groups);
+  *longest = *lists = 0;
+  for (int cta = 0; cta < grid; ++cta) {
+    const StreamTiles s = stream_tiles(p, len, cta, grid);
+    int at = s.first, streamed = s.first, parts = 0, n_lists = 0;
+    do {
+      StreamSegment list[kStreamSegments + 1];
+      list[kStreamSegments].nt = -12345;
+      const int n = stream_next_parts(s, cta, at, list);
+      if (n > kStreamSegments || list[kStreamSegments].nt != -12345) return 1;
+      if (n == 0 && at < s.last) return 2;
+      for (int i = 0; i < n; ++i) {
+        const StreamSegment& g = list[i];
+        const StreamSegment copied = stream_segment(s, streamed, cta);  // the producer's own walk
+        if (copied.b != g.b || copied.group != g.group || copied.t0 != g.t0 || copied.t1 != g.t1) return 3;
+        streamed += copied.t1 - copied.t0;
+        if (g.b < 0 || g.b >= batch || g.group < 0 || g.group >= groups) return 4;
+        const int length = len[ragged ? g.b : 0];
+        if (g.len != length || g.nt != length / p.stream_tile_keys + 1) return 5;
+        if (g.t0 < 0 || g.t1 <= g.t0 || g.t1 > g.nt) return 6;
+        if (g.seg < 0 || g.seg >= g.nseg || g.nseg > kStreamMaxSegments) return 7;
+        Group& of = all[static_cast<size_t>(g.b) * groups + g.group];
+        if (of.parts > 0 && of.nseg != g.nseg) return 8;
+        of.nseg = g.nseg;
+        of.parts += 1;
+        of.tiles += g.t1 - g.t0;
+        of.seen.resize(g.nseg);
+        if (of.seen[g.seg]++) return 9;
+      }
+      parts += n;
+      n_lists += 1;
+    } while (at < s.last);
+    if (streamed != s.last && s.first < s.last) return 10;
+    if (parts > *longest) *longest = parts;
+    if (n_lists > *lists) *lists = n_lists;
+  }
+  for (int b = 0; b < batch; ++b)
+    for (int g = 0; g < groups; ++g) {
+      const Group& of = all[static_cast<size_t>(b) * groups + g];
+      if (of.tiles != len[ragged ? b : 0] / p.stream_tile_keys + 1) return 11;  // every position exactly once
+      if (of.parts != of.nseg) return 12;                                        // every part is handed in
+    }
+  return 0;
+}

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from conftest import assert_parity
-from megabake_b200.synth import rope_tables, synth_ids, synth_normal, synth_weights, tiny_config
+from megabake_b200.synth import new_kv_state, rope_tables, synth_ids, synth_normal, synth_weights, tiny_config
 from test_gpu_parity import make_kernel, oracle_decode_compare
 
 pytestmark = pytest.mark.gpu
@@ -37,6 +37,42 @@ def test_streaming_decode_with_a_context_of_one_tile_to_a_warp(device, batch, co
     positions on there is a second tile."""
     config = tiny_config(hidden=512, q_heads=32, kv_heads=32, head_dim=64, intermediate=768, vocab=512)
     oracle_decode_compare(config, device, batch=batch, capacity=context + 3, prefill=context, steps=3)
+
+
+@pytest.mark.parametrize("lengths_now,sm_limit", [
+    ([1000] * 28 + [10] * 4, 0), ([10] * 7 + [4000] * 9, 0), ([8000] * 6 + [10] * 6, 0),  # 17, 22 and 42 parts in one CTA
+    ([40] * 32, 4),                                                                       # 32 of equal lengths: few CTAs
+])
+def test_streaming_decode_with_more_parts_than_a_list_holds(device, lengths_now, sm_limit):
+    """Long sequences make the runs long, and a run through short ones crosses a head group per tile.  Every sequence must
+    come out as if it had been decoded alone."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=512, q_heads=32, kv_heads=32, head_dim=64, intermediate=768)
+    batch, capacity = len(lengths_now), max(lengths_now) + 2
+    weights = synth_weights(config, seed=16, norm_std=0.1, device=device)
+    kernel = make_kernel(config, weights, device, max_tokens=batch, max_positions=capacity, sm_limit=sm_limit)
+    tables = rope_tables(config, capacity, device=device)
+    keys, values, _ = new_kv_state(config, batch, capacity, device)
+    for layer in range(config.layers):
+        for name, caches in (("k", keys), ("v", values)):
+            caches[layer].copy_(synth_normal(tuple(caches[layer].shape), seed=16, name=f"{name}{layer}", std=0.5, device=device))
+    lengths = [torch.tensor(lengths_now, dtype=torch.int32, device=device) for _ in range(config.layers)]
+    alone = [([k[row:row + 1].clone() for k in keys], [v[row:row + 1].clone() for v in values],
+              [torch.full((1,), filled, dtype=torch.int32, device=device) for _ in range(config.layers)])
+             for row, filled in enumerate(lengths_now)]
+    ids = synth_ids(batch, config.vocab, seed=16).view(batch, 1).to(device)
+    for step in range(2):
+        positions = torch.tensor([[n + step] for n in lengths_now], dtype=torch.int64, device=device)
+        logits = kernel.decode_ragged(ids, positions, keys, values, lengths)
+        kernel.check()
+        with torch.no_grad():
+            expected = torch.cat([oracle.decode_step(config, weights, tables, ids[row:row + 1], positions[row:row + 1], *alone[row])
+                                  for row in range(batch)])
+        assert_parity(logits, expected, f"logits at step {step}")
+    for row, filled in enumerate(lengths_now):
+        assert_parity(keys[-1][row, :filled + 2], alone[row][0][-1][0, :filled + 2], f"sequence {row} key cache")
+        assert_parity(values[-1][row, :filled + 2], alone[row][1][-1][0, :filled + 2], f"sequence {row} value cache")
 
 
 @pytest.mark.parametrize("kv_heads,head_dim,context", [(40, 64, 300), (40, 64, 319), (20, 128, 258)])
