@@ -79,10 +79,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
   constexpr int kRow = HD + 2;
 
   // Lists of parts, mostly one (every layer has at least one, if empty).
-  while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= th.list && !stream_aborted(sm)) {
-  }
-  __threadfence_block();
-  int count = stream_aborted(sm) ? 0 : sm->seg_count[th.list & 1];
+  int count = stream_next_list(sm, th.list);
 #pragma unroll 1
   for (int part = 0;; ++part) {
     if (part == (count & (kStreamMoreParts - 1))) {
@@ -90,10 +87,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
       if (!(count & kStreamMoreParts)) break;
       stream_sync();  // everybody is done with the list: the helper may write the next but one
       if (wtid == 0) *reinterpret_cast<volatile int*>(&sm->seg_taken) = th.list;
-      while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= th.list && !stream_aborted(sm)) {
-      }
-      __threadfence_block();
-      count = stream_aborted(sm) ? 0 : sm->seg_count[th.list & 1];
+      count = stream_next_list(sm, th.list);
       part = -1;
       continue;
     }

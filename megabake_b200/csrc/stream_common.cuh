@@ -105,6 +105,7 @@ struct StreamMisc {
   int wabort;    // the limit on waits has run out: nobody waits any more
   int progress;  // layer the consumers are in; layers + 1: at the grid barrier; -1: finished
   int bad;       // prologue verdict
+  int complete;  // the grid barrier was reached: one thread's verdict, so that all threads end the launch the same way
   int trace_n, trace_on;
   int copies;       // hand-over buffers exist this often
   int psum_offset;  // bytes from the end of this block to the partial sums (the attention area comes first)
@@ -151,6 +152,8 @@ __device__ __forceinline__ void stream_sync() { named_bar_sync(1, kStreamConsume
 __device__ __forceinline__ bool stream_aborted(StreamMisc* sm) { return *reinterpret_cast<volatile int*>(&sm->wabort) != 0; }
 
 // Waits look at one word of shared memory; the limit on them is kept by a thread with nothing else to do (stream_watch).
+// The word may change between two warps' looks at it: after a wait that it ended every warp goes on through the same
+// phases, parts and block barriers, with whatever it has.
 __device__ __forceinline__ void stream_wait(StreamMisc* sm, uint32_t bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity))
     if (stream_aborted(sm)) return;
@@ -342,7 +345,10 @@ __host__ __device__ __forceinline__ int stream_next_parts(const StreamTiles& s, 
   return n;
 }
 
-// A helper thread works out the parts of each layer, a list ahead: the divisions would be on every consumer's path.
+// A helper thread works out the parts of each layer, a list ahead: the divisions would be on every consumer's path.  It and the
+// consumers wait for each other without a look at `wabort`: consumers that have given up on everything else still come by
+// here, and a warp that skipped its parts because it saw the abort, beside one that did not, would leave that one alone at
+// a block barrier.
 __device__ __forceinline__ void stream_plan_parts(StreamMisc* sm) {
   const KParams& p = *sm->p;
   int list = 0;
@@ -350,10 +356,7 @@ __device__ __forceinline__ void stream_plan_parts(StreamMisc* sm) {
     const StreamTiles tiles = stream_tiles(p, stream_lengths(p, sm, layer), sm->cta, sm->grid);
     int at = tiles.first;
     do {
-      while (*reinterpret_cast<volatile int*>(&sm->seg_taken) < list - 1) {  // the list before the last is still in use
-        if (stream_aborted(sm)) return;
-        __nanosleep(200);
-      }
+      while (*reinterpret_cast<volatile int*>(&sm->seg_taken) < list - 1) __nanosleep(200);  // the list before the last is still in use
       const int n = stream_next_parts(tiles, sm->cta, at, sm->seg[list & 1]);
       sm->seg_count[list & 1] = n | (at < tiles.last ? kStreamMoreParts : 0);
       ++list;
@@ -361,6 +364,14 @@ __device__ __forceinline__ void stream_plan_parts(StreamMisc* sm) {
       *reinterpret_cast<volatile int*>(&sm->seg_ready) = list;
     } while (at < tiles.last);
   }
+}
+
+// Consumers: the count of list `list`, once it is there.
+__device__ __forceinline__ int stream_next_list(StreamMisc* sm, int list) {
+  while (*reinterpret_cast<volatile int*>(&sm->seg_ready) <= list) {
+  }
+  __threadfence_block();
+  return sm->seg_count[list & 1];
 }
 
 }  // namespace mk

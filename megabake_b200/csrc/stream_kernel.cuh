@@ -90,7 +90,7 @@ __device__ __forceinline__ void stream_producer(StreamMisc* sm, StreamPipe pipe)
     weights(SP_HEAD, maps + 7 * layers);
   };
   run();
-  if (stream_aborted(sm)) {  // every copy already issued must land before the CTA exits
+  {  // every copy already issued must land before the CTA exits; consumers that have given up do not wait for it
     const int back = min(issued, pipe.nslots);
     for (int i = 0; i < back; ++i) {
       const int s = (issued - back + i) % pipe.nslots;
@@ -173,11 +173,12 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     while (static_cast<int32_t>(ld_relaxed_u32(&sm->ctrl->barrier) - target) < 0 && !stream_aborted(sm)) {
     }
     __threadfence();
+    sm->complete = !stream_aborted(sm);
     *reinterpret_cast<volatile int*>(&sm->progress) = -1;
   }
   stream_sync();
   th.trace(EV_BARRIER_DONE);
-  if (stream_aborted(sm)) return;
+  if (!sm->complete) return;
   if (sm->cta == 0)
     for (int i = wtid; i < layers * (p.ragged ? p.batch : 1); i += kStreamConsumers) {
       const int per = p.ragged ? p.batch : 1;

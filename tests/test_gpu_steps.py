@@ -168,6 +168,39 @@ def test_a_grid_barrier_that_cannot_be_reached_times_out_and_the_handle_recovers
     assert torch.equal(logits, expected) and all(int(length) == 1 for length in state[2])
 
 
+@pytest.mark.parametrize("batch", [1, 4, 8, 16, 32])
+def test_a_limit_that_runs_out_inside_a_launch_ends_it_and_the_handle_recovers(batch, monkeypatch):
+    """Limits shorter than the launch: the streaming kernel gives up wherever it is, every CTA leaves, the status says
+    TIMEOUT and the lengths have not moved (or the launch was through in time).  Then the handle's state is as new: a
+    second handle's logits come out of a launch that is not cut short."""
+    config = tiny_config(q_heads=8, kv_heads=8, hidden=512, layers=24)
+    weights = synth_weights(config, seed=17, norm_std=0.1, device=DEVICE)
+    reference = make_kernel(config, weights, max_tokens=batch, max_positions=512)
+    ids = synth_ids(batch, config.vocab, seed=17).view(batch, 1).to(DEVICE)
+    positions = torch.full((batch, 1), 300, dtype=torch.int64, device=DEVICE)
+    state = new_kv_state(config, batch, 512, DEVICE)
+
+    def step(kernel):
+        for length in state[2]:
+            length.fill_(300)
+        return kernel.decode(ids, positions, *state), kernel.status()["status"]
+
+    expected, verdict = step(reference)
+    assert verdict == "OK"
+    verdicts = []
+    for limit in (0.005, 0.01, 0.02, 0.03, 0.05, 0.07, 0.1, 0.13, 0.16, 0.2, 0.25, 0.3, 0.4, 100.0):
+        monkeypatch.setenv("MEGABAKE_WAIT_LIMIT_MS", str(limit))
+        kernel = make_kernel(config, weights, max_tokens=batch, max_positions=512)
+        for _ in range(4):
+            logits, verdict = step(kernel)
+            verdicts.append(verdict)
+            assert verdict in ("OK", "TIMEOUT")
+            assert {int(length) for length in state[2]} <= ({301} if verdict == "OK" else {300, 301})
+            assert verdict == "TIMEOUT" or torch.equal(logits, expected)
+    assert verdicts[:4] == ["TIMEOUT"] * 4 and verdicts[-4:] == ["OK"] * 4
+    assert torch.equal(step(reference)[0], expected)
+
+
 def test_static_scratch_status_recovers_from_a_refused_launch():
     """The allocation-free attention entry point has no handle: its status word lives in the static
     array and is read and cleared through mk_kv_attention_static_status."""
