@@ -203,11 +203,22 @@ int mk_linear(mk_handle handle, const void* x, const void* weight, const void* b
 /* megabake::kv_attention on caller tensors (shapes as in mk_decode, one layer):
  * query bf16 [batch, 1, q_heads, head_dim], key/value bf16 [batch, 1, kv_heads,
  * head_dim] (already rotated), output bf16 [batch*q_heads, 1, head_dim].
- * Appends, attends, advances valid_length.
+ * Appends, attends, advances valid_length.  Two launches that share an area of the handle's workspace: a
+ * call waits, on the device, for the one before it on this handle, whatever its stream (but not inside a
+ * stream capture, where the order is the graph's).  Other calls on the handle use that workspace too:
+ * order them.
  * Reference: src/megabake/lowering.py:211-247. */
 int mk_kv_attention(mk_handle handle, const void* query, const void* key, const void* value,
                     void* key_cache, void* value_cache, int32_t* valid_length, int batch,
                     int capacity, void* output, void* stream);
+
+/* mk_kv_attention with that area from the caller: `scratch` is device memory of at least
+ * mk_kv_attention_scratch_bytes, 16-byte aligned, in any state, used until the call's work on `stream` is
+ * done.  Calls with scratch of their own may run side by side on several streams. */
+size_t mk_kv_attention_scratch_bytes(int batch, int q_heads, int head_dim);
+int mk_kv_attention_scratch(mk_handle handle, const void* query, const void* key, const void* value,
+                            void* key_cache, void* value_cache, int32_t* valid_length, int batch,
+                            int capacity, void* output, void* scratch, size_t scratch_bytes, void* stream);
 
 /* megabake::attention: query bf16 [batch, q_len, q_heads, head_dim], key/value
  * bf16 [batch, k_len, kv_heads, head_dim], mask bf16 additive [batch, 1, q_len,

@@ -30,6 +30,7 @@ EXPORTS = (
     "mk_kv_attention", "mk_kv_attention_static", "mk_kv_attention_static_status", "mk_attention", "mk_status", "mk_set_trace",
     "mk_launch_info", "mk_last_error", "mk_destroy", "mk_decode_steps", "mk_decode_step_host", "mk_set_status_mirror", "mk_debug_skew_barrier",
     "mk_describe", "mk_decode_ragged", "mk_baseline_mma_gemm", "mk_tp_exchange_bytes", "mk_tp_bind", "mk_ipc_export", "mk_ipc_open", "mk_ipc_close",
+    "mk_kv_attention_scratch", "mk_kv_attention_scratch_bytes",
 )
 
 
@@ -106,6 +107,12 @@ def load() -> ctypes.CDLL:
     lib.mk_kv_attention.argtypes = [
         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
     ]
+    lib.mk_kv_attention_scratch.restype = c_int
+    lib.mk_kv_attention_scratch.argtypes = [
+        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_size_t, c_void_p,
+    ]
+    lib.mk_kv_attention_scratch_bytes.restype = c_size_t
+    lib.mk_kv_attention_scratch_bytes.argtypes = [c_int, c_int, c_int]
     lib.mk_attention.restype = c_int
     lib.mk_attention.argtypes = [
         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_int, c_void_p, c_void_p,

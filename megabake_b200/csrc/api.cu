@@ -296,6 +296,7 @@ struct mk_handle_s {
     uint64_t used = 0;              // launch counter at the last use (least recently used is replaced)
   };
   CacheMapSet kv_sets[kCacheMapSets];
+  cudaEvent_t kv_done;  // behind the last mk_kv_attention, once there was one
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
   StreamPhase stream_ph[kStreamPlans][kStreamPhases];
@@ -521,15 +522,24 @@ bool stream_usable(mk_handle h, int batch, bool ragged) {
 
 int token_tiles(int m) { return (m + token_tile_of(m) - 1) / token_tile_of(m); }
 
+// What the two launches of a decode attention share.  The workspace has one such area: its users order their calls.
+struct KvScratch {
+  uint32_t* verdict;
+  float *stats, *parts;
+};
+KvScratch workspace_kv_scratch(mk_handle h) {
+  return {&at<Control>(h, h->cv.ctrl)->pad, at<float>(h, h->cv.att_xch), at<float>(h, h->cv.att_part)};
+}
+
 int launch_kv_attention(mk_handle h, const void* query, const void* key, const void* value, void* key_cache, void* value_cache,
-                        int32_t* valid_length, int batch, int capacity, void* output, cudaStream_t stream) {
+                        int32_t* valid_length, int batch, int capacity, void* output, const KvScratch& scratch, cudaStream_t stream) {
   const mk_config& c = h->cfg;
   const bool small = c.head_dim == 64;
   KvAttentionArgs a{};
   a.q = static_cast<const bf16*>(query); a.knew = static_cast<const bf16*>(key); a.vnew = static_cast<const bf16*>(value);
   a.k = static_cast<bf16*>(key_cache); a.v = static_cast<bf16*>(value_cache); a.out = static_cast<bf16*>(output);
   a.length = valid_length;
-  a.stats = at<float>(h, h->cv.att_xch); a.parts = at<float>(h, h->cv.att_part); a.ctrl = at<Control>(h, h->cv.ctrl);
+  a.verdict = scratch.verdict; a.stats = scratch.stats; a.parts = scratch.parts; a.ctrl = at<Control>(h, h->cv.ctrl);
   a.status_mirror = h->mirror;
   a.batch = batch; a.q_heads = c.q_heads; a.kv_heads = c.kv_heads; a.capacity = capacity;
   a.width = std::min(c.kv_heads, 8);
@@ -672,6 +682,7 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
   h->kv_maps_ok = getenv("MEGABAKE_NO_CACHE_MAPS") == nullptr;
   h->tp_epoch = 0;
   h->tp_bound = false;
+  h->kv_done = nullptr;
   for (int r = 0; r < kMaxTp; ++r) h->tp_peer[r] = nullptr;
   double ms = 2000.0;
   if (const char* env = getenv("MEGABAKE_WAIT_LIMIT_MS")) ms = atof(env) > 0 ? atof(env) : ms;
@@ -695,6 +706,7 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
 }
 
 int mk_destroy(mk_handle h) {
+  if (h && h->kv_done) cudaEventDestroy(h->kv_done);
   delete h;
   return MK_OK;
 }
@@ -1129,17 +1141,57 @@ int mk_linear(mk_handle h, const void* x, const void* weight, const void* bias, 
   return launch(h, p, stream);
 }
 
+namespace {
+int check_kv_attention(mk_handle h, const void* key_cache, const void* value_cache, int batch, int capacity, const char* what) {
+  if (batch < 1 || batch > h->cfg.max_tokens) return fail(MK_ERR_INVALID, "%s: batch %d outside [1, %d]", what, batch, h->cfg.max_tokens);
+  if (int e = attention_fits(h, capacity, what)) return e;
+  if (reinterpret_cast<uintptr_t>(key_cache) % 16 || reinterpret_cast<uintptr_t>(value_cache) % 16)
+    return fail(MK_ERR_ALIGNMENT, "%s: caches must be 16-byte aligned", what);
+  return MK_OK;
+}
+}  // namespace
+
 int mk_kv_attention(mk_handle h, const void* query, const void* key, const void* value, void* key_cache,
                     void* value_cache, int32_t* valid_length, int batch, int capacity, void* output, void* stream) {
   if (!h || !query || !key || !value || !key_cache || !value_cache || !valid_length || !output)
     return fail(MK_ERR_INVALID, "mk_kv_attention: null argument");
   std::lock_guard<std::mutex> guard(h->lock);
-  if (batch < 1 || batch > h->cfg.max_tokens) return fail(MK_ERR_INVALID, "mk_kv_attention: batch %d outside [1, %d]", batch, h->cfg.max_tokens);
-  if (int e = attention_fits(h, capacity, "mk_kv_attention")) return e;
-  if (reinterpret_cast<uintptr_t>(key_cache) % 16 || reinterpret_cast<uintptr_t>(value_cache) % 16)
-    return fail(MK_ERR_ALIGNMENT, "mk_kv_attention: caches must be 16-byte aligned");
-  return launch_kv_attention(h, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output,
+  if (int e = check_kv_attention(h, key_cache, value_cache, batch, capacity, "mk_kv_attention")) return e;
+  // The scratch is the handle's: a call waits for the one before it, on whatever stream that was.  (A captured call is
+  // ordered by whoever launches the graph: an event from outside would end the capture.)
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  MK_CUDA(cudaStreamIsCapturing(s, &capturing));
+  const bool ordered = capturing == cudaStreamCaptureStatusNone;
+  if (ordered) {
+    if (!h->kv_done) MK_CUDA(cudaEventCreateWithFlags(&h->kv_done, cudaEventDisableTiming));
+    else MK_CUDA(cudaStreamWaitEvent(s, h->kv_done, 0));
+  }
+  if (int e = launch_kv_attention(h, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output, workspace_kv_scratch(h), s))
+    return e;
+  if (ordered) MK_CUDA(cudaEventRecord(h->kv_done, s));
+  return MK_OK;
+}
+
+int mk_kv_attention_scratch(mk_handle h, const void* query, const void* key, const void* value, void* key_cache,
+                            void* value_cache, int32_t* valid_length, int batch, int capacity, void* output, void* scratch,
+                            size_t scratch_bytes, void* stream) {
+  if (!h || !query || !key || !value || !key_cache || !value_cache || !valid_length || !output || !scratch)
+    return fail(MK_ERR_INVALID, "mk_kv_attention_scratch: null argument");
+  std::lock_guard<std::mutex> guard(h->lock);
+  if (int e = check_kv_attention(h, key_cache, value_cache, batch, capacity, "mk_kv_attention_scratch")) return e;
+  if (reinterpret_cast<uintptr_t>(scratch) % 16) return fail(MK_ERR_ALIGNMENT, "mk_kv_attention_scratch: scratch must be 16-byte aligned");
+  const size_t need = kv_scratch_bytes(batch, h->cfg.q_heads, h->cfg.head_dim);
+  if (scratch_bytes < need) return fail(MK_ERR_WORKSPACE, "mk_kv_attention_scratch: scratch has %zu bytes, %zu needed", scratch_bytes, need);
+  uint8_t* const base = static_cast<uint8_t*>(scratch);
+  const KvScratch own{reinterpret_cast<uint32_t*>(base), reinterpret_cast<float*>(base + 256),
+                      reinterpret_cast<float*>(base + 256 + kv_scratch_stats(batch, h->cfg.q_heads))};
+  return launch_kv_attention(h, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output, own,
                              static_cast<cudaStream_t>(stream));
+}
+
+size_t mk_kv_attention_scratch_bytes(int batch, int q_heads, int head_dim) {
+  return batch < 1 || q_heads < 1 || head_dim < 1 ? 0 : kv_scratch_bytes(batch, q_heads, head_dim);
 }
 
 int mk_attention(mk_handle h, const void* query, const void* key, const void* value, const void* mask, float scale,
@@ -1481,12 +1533,12 @@ int mk_kv_attention_static(int q_heads, int kv_heads, int head_dim, const void* 
   view.att_scale = static_cast<float>(std::pow(static_cast<double>(head_dim), -0.5));
   for (int i = 0; i < kStreamPlans; ++i) view.stream_ok[i] = false;
   view.trace = nullptr; view.trace_cap = 0;
-  view.mirror = nullptr; view.use3d = false;
+  view.mirror = nullptr; view.use3d = false; view.kv_done = nullptr;
   view.tp_epoch = 0; view.tp_bound = false;
   for (int r = 0; r < kMaxTp; ++r) view.tp_peer[r] = nullptr;
   if (int e = attention_fits(&view, capacity, "mk_kv_attention_static")) return e;
   if (int e = launch_kv_attention(&view, query, key, value, key_cache, value_cache, valid_length, batch, capacity, output,
-                                  static_cast<cudaStream_t>(stream)))
+                                  workspace_kv_scratch(&view), static_cast<cudaStream_t>(stream)))
     return e;
   slot.epoch = view.epoch; slot.att_epoch = view.att_epoch; slot.launches = view.launches;
   return MK_OK;

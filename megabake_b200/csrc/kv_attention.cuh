@@ -8,7 +8,8 @@
 // (cp.async, three stages) without a block barrier.  Blocks of 8 warps, two per SM with head size 64, keep 128 KB of
 // copies in flight per SM.  Scores are bf16(q.k) times the scale, the softmax a running one in fp32, the weights rounded
 // to bf16 for the value product; every warp leaves its maximum, sum and value sums, and a second launch, which the
-// stream orders behind the first, adds them up, divides and rounds once.  16 sequences of 1024 positions, 32 heads of 64:
+// stream orders behind the first, adds them up, divides and rounds once.  What the first launch leaves for the second is the
+// call's own: two streams' launches may run side by side.  16 sequences of 1024 positions, 32 heads of 64:
 // as a phase of the persistent kernel, whose blocks waited for one another's partial sums, 74 us.
 #include "device_common.cuh"
 #include "prompt_attention.cuh"
@@ -19,15 +20,22 @@ struct KvAttentionArgs {
   const bf16 *q, *knew, *vnew;
   bf16 *k, *v, *out;
   int* length;
+  uint32_t* verdict;  // 1: the first launch refused the length
   float* stats;   // [batch * q_heads][slots][maximum, sum]
   float* parts;   // [batch * q_heads][slots][head_dim]
-  Control* ctrl;  // its pad word carries the first launch's verdict on the length to the second
+  Control* ctrl;
   volatile int* status_mirror;
   int batch, q_heads, kv_heads, capacity;
   int width, shares;   // KV heads per block, warps per head
   int chunks, slots;   // runs of positions; slots = chunks * shares
   float scale_log2;
 };
+
+// Scratch of a call: [verdict, 256 bytes][stats][parts], sized for the most slots.
+inline size_t kv_scratch_stats(int batch, int q_heads) { return (static_cast<size_t>(batch) * q_heads * kMaxChunks * 8 + 255) / 256 * 256; }
+inline size_t kv_scratch_bytes(int batch, int q_heads, int head_dim) {
+  return 256 + kv_scratch_stats(batch, q_heads) + static_cast<size_t>(batch) * q_heads * kMaxChunks * head_dim * 4;
+}
 
 template <int HD>
 struct KvLaunch {
@@ -42,7 +50,7 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
   extern __shared__ __align__(128) uint8_t kv_smem[];
   const int len = *a.length, n = len + 1;
   const bool bad = len < 0 || n > a.capacity;
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.ctrl->pad = bad ? 1u : 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.verdict = bad ? 1u : 0u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int hw = warp % a.width, share = warp / a.width;
   if (bad || share >= a.shares) return;
@@ -182,7 +190,7 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
 __global__ void __launch_bounds__(128) kv_attention_combine(const __grid_constant__ KvAttentionArgs a, int head_dim) {
   const int quads = head_dim / 4, at = blockIdx.x * 128 + threadIdx.x;
   const int row = at / quads, d = (at - row * quads) * 4;
-  const bool bad = a.ctrl->pad != 0;
+  const bool bad = *a.verdict != 0;
   if (at == 0) {
     if (!bad) {
       *a.length += 1;

@@ -101,7 +101,7 @@ struct Control {
   int status;         // mk_device_status
   int where, cta, detail;
   int att_nch;        // context chunks the last attention phase used (read by the o projection)
-  uint32_t pad;       // the stand-alone decode attention: 1 if its first launch refused the valid length
+  uint32_t pad;       // mk_kv_attention, mk_kv_attention_static: 1 if the first launch refused the valid length
 };
 
 struct KParams {

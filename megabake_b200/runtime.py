@@ -54,6 +54,7 @@ def decode_trace(buffer: torch.Tensor):
 
 
 _ALREADY = contextlib.nullcontext()
+_KV_STREAMS = 8  # streams whose decode-attention scratch an object keeps
 
 
 class DecoderKernel:
@@ -145,6 +146,7 @@ class DecoderKernel:
         wait is reported at the caller's next call instead of handing out NaN silently
         (the reference raises: src/megabake/lowering.py:229, src/megabake/compiler.py:2690)."""
         self._host_step_logits = None
+        self._kv_streams: dict[int, tuple] = {}
         self._mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._mirror_word = ctypes.c_int32.from_address(self._mirror.data_ptr())  # an indexed tensor read costs 3 us
         with torch.cuda.device(self.device):
@@ -400,11 +402,30 @@ class DecoderKernel:
         self.raise_if_failed()
         out = torch.empty((batch * heads, 1, dim), dtype=torch.bfloat16, device=self.device)
         with self._lock, self._on_device():
-            self._call("mk_kv_attention", self.lib.mk_kv_attention(
+            stream = self._stream()
+            scratch = self._kv_streams.get(stream)
+            if scratch is None or scratch[2] < batch or torch.cuda.is_current_stream_capturing():
+                scratch = self._new_kv_scratch(stream, batch, heads, dim)
+            self._call("mk_kv_attention_scratch", self.lib.mk_kv_attention_scratch(
                 self._handle, source.data_ptr(), key.data_ptr(), value.data_ptr(), key_cache.data_ptr(),
                 value_cache.data_ptr(), valid_length.data_ptr(), batch, key_cache.shape[1], out.data_ptr(),
-                self._stream()))
+                scratch[0], scratch[1], stream))
         return out
+
+    def _new_kv_scratch(self, stream: int, batch: int, heads: int, dim: int) -> tuple:
+        """What the two launches of a decode attention share: (address, bytes, batch, tensor).  One object serves every stream
+        of the process, so a stream has its own, from its own memory (it may be freed or replaced while launches that use it
+        are still queued there), kept for a few streams.  A captured call's belongs to the graph, which may be launched on
+        any stream."""
+        size = self.lib.mk_kv_attention_scratch_bytes(batch, heads, dim)
+        tensor = torch.empty(size, dtype=torch.uint8, device=self.device)
+        scratch = (tensor.data_ptr(), size, batch, tensor)
+        if not torch.cuda.is_current_stream_capturing():
+            self._kv_streams.pop(stream, None)
+            while len(self._kv_streams) >= _KV_STREAMS:
+                self._kv_streams.pop(next(iter(self._kv_streams)))
+            self._kv_streams[stream] = scratch
+        return scratch
 
     def attention(self, query, key, value, mask, scale: float) -> torch.Tensor:
         """``megabake::attention`` (reference src/megabake/lowering.py:273-300) on the GPU."""
@@ -520,6 +541,7 @@ class AttentionKernels:
     _call = DecoderKernel._call
     _compiler_error = DecoderKernel._compiler_error
     kv_attention = DecoderKernel.kv_attention
+    _new_kv_scratch = DecoderKernel._new_kv_scratch
     attention = DecoderKernel.attention
     status = DecoderKernel.status
     check = DecoderKernel.check

@@ -166,3 +166,98 @@ def test_decode_attention_op_at_tile_and_run_edges(device, heads, kv_heads, head
     assert int(length) == context + 1
     for a, b in zip(mine, ref):
         assert torch.equal(a[:, :context + 1], b[:, :context + 1]) and bool(torch.isnan(a[:, context + 1:].float()).all())
+
+
+def _interleaved(device, call, rounds=40):
+    """Decode attention calls of one head shape on two streams, whose launches may run in any order and side by side: small
+    ones that leave room for the others."""
+    from oracle import decoder_oracle as oracle
+
+    heads, kv_heads, head_dim, capacity = 8, 8, 64, 1200
+    streams, sides = [torch.cuda.Stream(device) for _ in range(2)], []
+    for index, (batch, context) in enumerate(((1, 1100), (2, 37))):
+        query, key, value = _tensors(device, batch, 1, 1, heads, kv_heads, head_dim)
+        query, key, value = (t * (index + 1) for t in (query, key, value))
+        caches = [synth_normal((batch, capacity, kv_heads, head_dim), seed=18 + index, name=name, std=1.0, device=device) for name in ("kc", "vc")]
+        ref = [c.clone() for c in caches]
+        expected = oracle.kv_attention(query, key, value, *ref, torch.full((1,), context, dtype=torch.int32, device=device))
+        lengths = [torch.full((1,), context, dtype=torch.int32, device=device) for _ in range(rounds)]
+        sides.append((query, key, value, caches, lengths, expected, context, []))
+    torch.cuda.synchronize(device)
+    for i in range(rounds):
+        for stream, (query, key, value, caches, lengths, _, _, outs) in zip(streams, sides):
+            with torch.cuda.stream(stream):
+                outs.append(call(query, key, value, *caches, lengths[i]))
+    torch.cuda.synchronize(device)
+    for query, key, value, caches, lengths, expected, context, outs in sides:
+        assert [int(n) for n in lengths] == [context + 1] * rounds
+        for out in outs:
+            assert_parity(out.view(expected.shape), expected, f"decode attention at {context} beside another stream's")
+
+
+def test_decode_attention_op_on_two_streams(device):
+    _interleaved(device, torch.ops.megabake.kv_attention)
+
+
+def test_decode_attention_op_in_a_graph_beside_calls_on_the_capturing_stream(device):
+    """A captured call's scratch is the graph's: replays beside eager calls on the stream that captured it."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value = _tensors(device, 1, 1, 1, 8, 8, 64)
+    caches = [synth_normal((1, 1200, 8, 64), seed=21, name=name, std=1.0, device=device) for name in ("kc", "vc")]
+    eager_caches = [c.clone() * 2 for c in caches]
+    expected = oracle.kv_attention(query, key, value, *[c.clone() for c in caches], torch.full((1,), 1100, dtype=torch.int32, device=device))
+    eager = oracle.kv_attention(query, key, value, *[c.clone() for c in eager_caches], torch.full((1,), 900, dtype=torch.int32, device=device))
+    lengths, side, graph = [torch.zeros(1, dtype=torch.int32, device=device) for _ in range(2)], torch.cuda.Stream(device), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize(device)
+    with torch.cuda.stream(side):
+        lengths[1].fill_(900)
+        torch.ops.megabake.kv_attention(query, key, value, *eager_caches, lengths[1])
+    torch.cuda.synchronize(device)
+    with torch.cuda.graph(graph, stream=side):
+        lengths[0].fill_(1100)
+        out = torch.ops.megabake.kv_attention(query, key, value, *caches, lengths[0])
+    outs = []
+    for _ in range(40):
+        graph.replay()
+        with torch.cuda.stream(side):
+            lengths[1].fill_(900)
+            outs.append(torch.ops.megabake.kv_attention(query, key, value, *eager_caches, lengths[1]))
+    torch.cuda.synchronize(device)
+    assert_parity(out.view(expected.shape), expected, "replayed decode attention")
+    for each in outs:
+        assert_parity(each.view(eager.shape), eager, "decode attention beside a replay")
+
+
+def test_decode_attention_entry_point_with_the_handles_scratch_on_two_streams(device):
+    from megabake_b200 import _native
+
+    config = tiny_config(hidden=512, q_heads=8, kv_heads=8, head_dim=64)
+    kernel = make_kernel(config, synth_weights(config, device=device), device, max_tokens=2, max_positions=16)
+
+    def call(query, key, value, key_cache, value_cache, length):
+        out = torch.empty((query.shape[0] * 8, 1, 64), dtype=torch.bfloat16, device=device)
+        _native.check("mk_kv_attention", kernel.lib.mk_kv_attention(
+            kernel._handle, query.data_ptr(), key.data_ptr(), value.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(),
+            length.data_ptr(), query.shape[0], key_cache.shape[1], out.data_ptr(), torch.cuda.current_stream(device).cuda_stream))
+        return out
+
+    _interleaved(device, call)
+
+
+def test_decode_attention_entry_point_refuses_scratch_that_is_too_small_or_misaligned(device):
+    from megabake_b200 import _native
+
+    config = tiny_config(hidden=512, q_heads=8, kv_heads=8, head_dim=64)
+    kernel = make_kernel(config, synth_weights(config, device=device), device, max_tokens=2, max_positions=16)
+    size = kernel.lib.mk_kv_attention_scratch_bytes(2, 8, 64)
+    scratch = torch.empty(size + 16, dtype=torch.uint8, device=device)
+    one = torch.zeros(2 * 16 * 512, dtype=torch.bfloat16, device=device)
+    length = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def call(at, count):
+        return kernel.lib.mk_kv_attention_scratch(kernel._handle, *[one.data_ptr()] * 5, length.data_ptr(), 2, 16, one.data_ptr(),
+                                                  scratch.data_ptr() + at, count, None)
+
+    assert call(0, size - 1) == _native.MK_ERR_WORKSPACE and call(8, size) == _native.MK_ERR_ALIGNMENT
+    assert call(0, 0) == _native.MK_ERR_WORKSPACE and int(length) == 0
