@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128) kv_attention_combine(const __grid_constan
   for (int s = 0; s < kMaxChunks; ++s) top = fmaxf(top, st[s].x);
 #pragma unroll
   for (int s = 0; s < kMaxChunks; ++s) {
-    if (st[s].y > 0.f) {
+    if (st[s].y != 0.f) {  // 0: no position, and no value sums; not a number where a score was not: so is the result
       const float w = ex2(st[s].x - top);
       total += w * st[s].y;
       acc[0] += w * pt[s].x; acc[1] += w * pt[s].y;

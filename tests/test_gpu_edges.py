@@ -168,6 +168,24 @@ def test_decode_attention_op_at_tile_and_run_edges(device, heads, kv_heads, head
         assert torch.equal(a[:, :context + 1], b[:, :context + 1]) and bool(torch.isnan(a[:, context + 1:].float()).all())
 
 
+def _filled_decode(device, batch, context, heads=8, kv_heads=8, head_dim=64):
+    """Query, key, value and the two caches of a decode attention call."""
+    caches = [synth_normal((batch, context + 2, kv_heads, head_dim), seed=20, name=name, std=1.0, device=device) for name in ("kc", "vc")]
+    return (*_tensors(device, batch, 1, 1, heads, kv_heads, head_dim), *caches)
+
+
+@pytest.mark.parametrize("where", [0, 40, 700, 1023])
+@pytest.mark.parametrize("spoilt", [float("nan"), float("inf")])
+def test_decode_attention_op_shows_a_key_that_is_not_a_number(device, where, spoilt):
+    """One spoilt key in a context of several parts: its heads' results are not numbers, wherever the context was cut."""
+    query, key, value, key_cache, value_cache = _filled_decode(device, 2, 1024)
+    query[:, 0, 3, 0] = 1.0
+    key_cache[1, where, 3, 0] = spoilt
+    out = torch.ops.megabake.kv_attention(query, key, value, key_cache, value_cache, torch.full((1,), 1024, dtype=torch.int32, device=device))
+    bad = torch.isnan(out.float()).view(2, 8, 64)
+    assert bool(bad[1, 3].all()) and int(bad.sum()) == 64
+
+
 def _interleaved(device, call, rounds=40):
     """Decode attention calls of one head shape on two streams, whose launches may run in any order and side by side: small
     ones that leave room for the others."""
