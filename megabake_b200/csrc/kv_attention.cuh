@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
       }
       n0 = fmaxf(n0, m0);
       n1 = fmaxf(n1, m1);
+      const float s0 = n0 > -INFINITY ? n0 : 0.f, s1 = n1 > -INFINITY ? n1 : 0.f;  // every score so far -inf: weights of zero
       if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
-        const float a0 = ex2(m0 - n0), a1 = ex2(m1 - n1);
+        const float a0 = ex2(m0 - s0), a1 = ex2(m1 - s1);
         l0 *= a0;
         l1 *= a1;
 #pragma unroll
@@ -150,8 +151,8 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
         m0 = n0;
         m1 = n1;
       }
-      s[0] = ex2(s[0] - n0); s[1] = ex2(s[1] - n1);
-      s[2] = ex2(s[2] - n0); s[3] = ex2(s[3] - n1);
+      s[0] = ex2(s[0] - s0); s[1] = ex2(s[1] - s1);
+      s[2] = ex2(s[2] - s0); s[3] = ex2(s[3] - s1);
       l0 += s[0] + s[2];
       l1 += s[1] + s[3];
       const uint32_t p0 = movmatrix_trans(pack2(s[0], s[1])), p1 = movmatrix_trans(pack2(s[2], s[3]));

@@ -357,7 +357,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
 #pragma unroll
       for (int x = 1; x < 8; x <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, x));
       mm = __shfl_sync(0xffffffffu, mm, 0);
-      weight = ex2(weight - mm);
+      weight = ex2(weight - (mm > -INFINITY ? mm : 0.f));  // (a part may hold nothing but scores of -inf: its weights are zero)
       ll *= weight;
 #pragma unroll
       for (int x = 1; x < 8; x <<= 1) ll += __shfl_xor_sync(0xffffffffu, ll, x);
@@ -415,7 +415,8 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
           if (s0 + s4 < sg.nseg) {
             const float om = __uint_as_float(static_cast<uint32_t>(w[s4][DPL])), pl = __uint_as_float(static_cast<uint32_t>(w[s4][DPL + 1]));
             const float mn = fmaxf(mm, om);
-            const float wa = ex2(mm - mn), wb = ex2(om - mn);
+            const float safe = mn > -INFINITY ? mn : 0.f;
+            const float wa = ex2(mm - safe), wb = ex2(om - safe);
             mm = mn;
             ll = ll * wa + pl * wb;
 #pragma unroll

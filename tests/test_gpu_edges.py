@@ -186,6 +186,47 @@ def test_decode_attention_op_shows_a_key_that_is_not_a_number(device, where, spo
     assert bool(bad[1, 3].all()) and int(bad.sum()) == 64
 
 
+@pytest.mark.parametrize("hidden", [1, 16, 300, 1023])
+def test_decode_attention_op_with_scores_of_minus_infinity(device, hidden):
+    """Positions with a score of -inf weigh nothing, also where a warp, or a whole run of positions, has no others."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value, key_cache, value_cache = _filled_decode(device, 2, 1024, heads=14, kv_heads=2)
+    query[..., 0] = 1.0
+    key_cache[:, :hidden, :, 0] = float("-inf")
+    caches = [key_cache.clone(), value_cache.clone()]
+    length, ref_length = (torch.full((1,), 1024, dtype=torch.int32, device=device) for _ in range(2))
+    out = torch.ops.megabake.kv_attention(query, key, value, key_cache, value_cache, length)
+    assert_parity(out, oracle.kv_attention(query, key, value, *caches, ref_length), f"{hidden} positions of -inf")
+
+
+@pytest.mark.parametrize("batch,context,hidden", [(1, 700, 400), (1, 700, 699), (16, 1100, 1000), (32, 70, 30), (2, 20, 17)])
+def test_streaming_decode_with_scores_of_minus_infinity(device, batch, context, hidden):
+    """The same in the streaming kernel: q is its bias (1 in every place, position 0 does not rotate), so that the cached keys
+    decide which scores are -inf."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=512, q_heads=16, kv_heads=16, intermediate=768, layers=1, qkv_bias=True)
+    weights = dict(synth_weights(config, seed=19, norm_std=0.1, device=device))
+    prefix = "model.layers.0.self_attn."
+    weights[prefix + "q_proj.weight"] = torch.zeros_like(weights[prefix + "q_proj.weight"])
+    weights[prefix + "q_proj.bias"] = torch.ones_like(weights[prefix + "q_proj.bias"])
+    kernel = make_kernel(config, weights, device, max_tokens=batch, max_positions=16)
+    keys, values, lengths = new_kv_state(config, batch, context + 2, device)
+    keys[0].copy_(synth_normal(tuple(keys[0].shape), seed=19, name="k", std=0.3, device=device))
+    values[0].copy_(synth_normal(tuple(values[0].shape), seed=19, name="v", std=1.0, device=device))
+    keys[0][:, :hidden, :, 0] = float("-inf")
+    lengths[0].fill_(context)
+    ref = ([keys[0].clone()], [values[0].clone()], [lengths[0].clone()])
+    ids = synth_ids(batch, config.vocab, seed=19).view(batch, 1).to(device)
+    positions = torch.zeros((batch, 1), dtype=torch.int64, device=device)
+    with torch.no_grad():
+        expected = oracle.decode_step(config, weights, rope_tables(config, 16, device=device), ids, positions, *ref)
+    assert bool(torch.isfinite(expected.float()).all())
+    assert_parity(kernel.decode(ids, positions, keys, values, lengths), expected, f"{hidden} of {context} positions of -inf")
+    kernel.check()
+
+
 def _interleaved(device, call, rounds=40):
     """Decode attention calls of one head shape on two streams, whose launches may run in any order and side by side: small
     ones that leave room for the others."""
