@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
       cp_async_wait_group<kStages - 2>();
       __syncwarp();  // every lane's copies are in, and every lane has left the stage that is filled next
       issue(i + kStages - 1);
-      if (j0 + 16 > len) {  // the new position: into the cache and into its row of the tile; value rows past it, finite
+      if (j0 + 16 > len) {  // the new position: into the cache and into its row of the tile; value rows past it, zero
         unsigned short* const ktile = reinterpret_cast<unsigned short*>(mine + (i % kStages) * kStage);
         unsigned short* const vtile = ktile + 16 * pitch / 2;
         for (int d = lane; d < HD; d += 32) {
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256, KvLaunch<HD>::kBlocks) kv_attention_parts
           reinterpret_cast<unsigned short*>(kbase + static_cast<size_t>(len) * kv_size)[d] = kv;
           reinterpret_cast<unsigned short*>(vbase + static_cast<size_t>(len) * kv_size)[d] = vv;
           ktile[(len - j0) * (pitch / 2) + d] = kv;
-          for (int r = len - j0; r < 16; ++r) vtile[r * (pitch / 2) + d] = vv;
+          for (int r = len - j0; r < 16; ++r) vtile[r * (pitch / 2) + d] = r == len - j0 ? vv : 0;
         }
         __syncwarp();
       }

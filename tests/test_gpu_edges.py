@@ -200,6 +200,22 @@ def test_decode_attention_op_with_scores_of_minus_infinity(device, hidden):
     assert_parity(out, oracle.kv_attention(query, key, value, *caches, ref_length), f"{hidden} positions of -inf")
 
 
+@pytest.mark.parametrize("context", [0, 3, 15, 1000])
+def test_decode_attention_op_with_an_infinite_new_value(device, context):
+    """The positions that pad the last tile must not turn it into something that is not a number."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value, key_cache, value_cache = _filled_decode(device, 2, context)
+    value[0, 0, 5, 7] = float("inf")
+    caches = [key_cache.clone(), value_cache.clone()]
+    length, ref_length = (torch.full((1,), context, dtype=torch.int32, device=device) for _ in range(2))
+    out = torch.ops.megabake.kv_attention(query, key, value, key_cache, value_cache, length)
+    expected = oracle.kv_attention(query, key, value, *caches, ref_length)
+    infinite = torch.isinf(expected.float())
+    assert int(infinite.sum()) == 1 and torch.equal(out[infinite], expected[infinite])
+    assert_parity(out.masked_fill(infinite, 0.0), expected.masked_fill(infinite, 0.0), "the finite results")
+
+
 @pytest.mark.parametrize("batch,context,hidden", [(1, 700, 400), (1, 700, 699), (16, 1100, 1000), (32, 70, 30), (2, 20, 17)])
 def test_streaming_decode_with_scores_of_minus_infinity(device, batch, context, hidden):
     """The same in the streaming kernel: q is its bias (1 in every place, position 0 does not rotate), so that the cached keys
