@@ -297,6 +297,7 @@ struct mk_handle_s {
   };
   CacheMapSet kv_sets[kCacheMapSets];
   cudaEvent_t kv_done;  // behind the last mk_kv_attention, once there was one
+  bool kv_maps_refused; // tests: the first encoding counts as refused by the driver
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
   StreamPhase stream_ph[kStreamPlans][kStreamPhases];
@@ -680,6 +681,7 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
   }
   for (int i = 0; i < kStreamPlans; ++i) h->stream_ok[i] = false;
   h->kv_maps_ok = getenv("MEGABAKE_NO_CACHE_MAPS") == nullptr;
+  h->kv_maps_refused = getenv("MEGABAKE_REFUSE_CACHE_MAPS") != nullptr;
   h->tp_epoch = 0;
   h->tp_bound = false;
   h->kv_done = nullptr;
@@ -987,7 +989,7 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
   p.mode = MODE_DECODE; p.m = batch; p.batch = batch; p.seq = 1; p.capacity = capacity;
   p.split = split_table_ok(h->cfg) ? 1 : 0;
   p.phases = at<GemmPhase>(h, h->cv.phases) + (p.split ? 0 : phases_per_table(h->cfg));
-  const bool streamed = stream_usable(h, batch, ragged);
+  bool streamed = stream_usable(h, batch, ragged);
   p.ragged = ragged ? 1 : 0;
   if (h->kv_maps_ok) {
     // Tiled descriptors of the caches for the tensor engine's decode attention, encoded again only when a
@@ -1010,7 +1012,7 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
     CUtensorMap* const device_sets = at<CUtensorMap>(h, h->cv.kvmaps);
     if (shape_ok && slot < 0) {
       std::vector<CUtensorMap> fresh(2 * static_cast<size_t>(L));
-      bool encoded = true;
+      bool encoded = !h->kv_maps_refused;
       for (int l = 0; l < L && encoded; ++l) {
         encoded = encode_cache_map(&fresh[l], key_caches[l], batch, capacity, row_elems, tile_keys, hpu * (c.head_dim / kChunkK)) == MK_OK &&
                   encode_cache_map(&fresh[L + l], value_caches[l], batch, capacity, row_elems, tile_keys, hpu * (c.head_dim / kChunkK)) == MK_OK;
@@ -1030,9 +1032,10 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
         set.heads = hpu;
         set.keys = tile_keys;
       } else {
-        h->kv_maps_ok = false;  // this driver refuses the view: plain copies from here on
+        h->kv_maps_ok = false;  // this driver refuses the view: the tensor engine with plain copies from here on
       }
     }
+    if (slot < 0) streamed = false;
     if (slot >= 0) {
       h->kv_sets[slot].used = static_cast<uint64_t>(h->launches) + 1;
       p.kv_maps = device_sets + static_cast<size_t>(slot) * 2 * L;
@@ -1041,7 +1044,6 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
   p.n_gemm = 4 * L + 1;
   p.nbar = 7 * L + 1;  // tensor engine: five per layer and one behind each norm phase (two per layer, one for the lm_head)
   if (streamed) {
-    if (!p.kv_maps) return fail(MK_ERR_CUDA, "mk_decode: the driver refuses the cache descriptors");
     const mk_config& c = h->cfg;
     const int plan = stream_plan_of(batch);
     p.splan = at<StreamPlan>(h, h->cv.splan) + plan;

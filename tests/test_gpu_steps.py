@@ -201,6 +201,28 @@ def test_a_limit_that_runs_out_inside_a_launch_ends_it_and_the_handle_recovers(b
     assert torch.equal(step(reference)[0], expected)
 
 
+@pytest.mark.parametrize("batch", [1, 6])
+def test_a_driver_that_refuses_the_cache_descriptors_leaves_the_tensor_engine(batch, monkeypatch):
+    """From the first call on (the streaming kernel cannot do without the descriptors, the tensor engine can)."""
+    monkeypatch.setenv("MEGABAKE_REFUSE_CACHE_MAPS", "1")
+    config = tiny_config(q_heads=4, kv_heads=2, hidden=256)
+    weights = synth_weights(config, seed=6, norm_std=0.1, device=DEVICE)
+    refused = make_kernel(config, weights, max_tokens=batch, max_positions=400)
+    monkeypatch.delenv("MEGABAKE_REFUSE_CACHE_MAPS")
+    monkeypatch.setenv("MEGABAKE_NO_CACHE_MAPS", "1")
+    without = make_kernel(config, weights, max_tokens=batch, max_positions=400, engine="tcgen05")
+    ids = synth_ids(batch, config.vocab, seed=6).view(batch, 1).to(DEVICE)
+    states = [new_kv_state(config, batch, 400, DEVICE) for _ in range(2)]
+    for position in (0, 1, 330):
+        positions = torch.full((batch, 1), position, dtype=torch.int64, device=DEVICE)
+        for state in states:
+            for length in state[2]:
+                length.fill_(position)
+        logits, expected = (kernel.decode(ids, positions, *state) for kernel, state in zip((refused, without), states))
+        refused.check()
+        assert torch.isfinite(logits.float()).all() and torch.equal(logits, expected)
+
+
 def test_static_scratch_status_recovers_from_a_refused_launch():
     """The allocation-free attention entry point has no handle: its status word lives in the static
     array and is read and cleared through mk_kv_attention_static_status."""
