@@ -439,7 +439,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
           store(col, pack2(sum[0].x + b0, sum[0].y + b1));
         } else {
           bf16* out = sm->p->logits + static_cast<size_t>(tok) * n_cols + col;
-          if (col < n_cols && (n_cols & 1) == 0) {
+          if ((n_cols & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0) {  // logits may begin at any element
             *reinterpret_cast<uint32_t*>(out) = pack2(sum[0].x, sum[0].y);
           } else {
             if (col < n_cols) out[0] = __float2bfloat16_rn(sum[0].x);

@@ -223,6 +223,24 @@ def test_a_driver_that_refuses_the_cache_descriptors_leaves_the_tensor_engine(ba
         assert torch.isfinite(logits.float()).all() and torch.equal(logits, expected)
 
 
+@pytest.mark.parametrize("batch", [1, 5, 17])
+def test_logits_may_begin_at_any_element(batch):
+    """A C caller's logits buffer on a 2-byte boundary gets what an aligned one gets, and nothing beside it is written."""
+    config = tiny_config(q_heads=4, kv_heads=2, hidden=256)
+    kernel = make_kernel(config, synth_weights(config, seed=6, norm_std=0.1, device=DEVICE), max_tokens=batch, max_positions=16)
+    ids = synth_ids(batch, config.vocab, seed=6).view(batch, 1).to(DEVICE)
+    positions = torch.zeros((batch, 1), dtype=torch.int64, device=DEVICE)
+    expected = kernel.decode(ids, positions, *new_kv_state(config, batch, 16, DEVICE))
+    keys, values, lengths = new_kv_state(config, batch, 16, DEVICE)
+    pointers = [(ctypes.c_void_p * config.layers)(*[t.data_ptr() for t in tensors]) for tensors in (keys, values, lengths)]
+    buffer = torch.full((batch * config.vocab + 2,), -3.0, dtype=torch.bfloat16, device=DEVICE)
+    _native.check("mk_decode", kernel.lib.mk_decode(kernel._handle, ids.data_ptr(), positions.data_ptr(), batch, *pointers, 16,
+                                                    buffer.data_ptr() + 2, torch.cuda.current_stream(DEVICE).cuda_stream))
+    kernel.check()
+    assert torch.equal(buffer[1:-1].view(expected.shape), expected)
+    assert float(buffer[0]) == -3.0 and float(buffer[-1]) == -3.0
+
+
 def test_static_scratch_status_recovers_from_a_refused_launch():
     """The allocation-free attention entry point has no handle: its status word lives in the static
     array and is read and cleared through mk_kv_attention_static_status."""
