@@ -4,9 +4,10 @@ mutation annotations (reference src/megabake/lowering.py:211-309):
     torch.ops.megabake.kv_attention(source, key, value, key_cache, value_cache, valid_length)
     torch.ops.megabake.attention(query, key, value, mask, scale)
 
-For CUDA tensors they launch the sm_100a attention phase of the megakernel through the
-C ABI (and raise if the library is missing).  For CPU tensors they run the eager
-definition of the op, which is what ``compile_kernel=False`` graphs execute.
+For CUDA tensors they launch the library's sm_100a attention kernels through the C ABI
+(and raise if the library is missing): the registrations at the end of this file.  For CPU
+tensors they run the eager definition of the op, which is what ``compile_kernel=False``
+graphs execute.
 """
 
 from __future__ import annotations
@@ -69,8 +70,6 @@ def kv_attention(
     source: torch.Tensor, key: torch.Tensor, value: torch.Tensor,
     key_cache: torch.Tensor, value_cache: torch.Tensor, valid_length: torch.Tensor,
 ) -> torch.Tensor:
-    if source.is_cuda:
-        return _kv_attention_cuda(source, key, value, key_cache, value_cache, valid_length)
     if source.shape[1] != 1:
         raise RuntimeError("megabake kv_attention supports one-token decode only")
     _check_layout(source, key)
@@ -81,6 +80,8 @@ def _kv_attention_cuda(source, key, value, key_cache, value_cache, valid_length)
     if source.shape[1] != 1:
         raise RuntimeError("megabake kv_attention supports one-token decode only")
     _check_layout(source, key)
+    if not source.is_cuda:  # some other argument is on the GPU: a length there is fine beside tensors on the CPU
+        return _kv_attention_eager(source, key, value, key_cache, value_cache, valid_length)
     kernels = _gpu_kernels(source.shape[2], key.shape[2], source.shape[3], source.shape[0], source.device)
     return kernels.kv_attention(source.contiguous(), key.contiguous(), value.contiguous(), key_cache, value_cache,
                                 valid_length)
@@ -98,14 +99,14 @@ def attention(
     """Softmax attention with Hugging Face eager numerics: ``query`` [batch, q, heads, dim],
     ``key``/``value`` [batch, k, kv_heads, dim], additive ``mask`` broadcastable to
     [batch, heads, q, k]; returns [batch * heads, q, dim]."""
-    if query.is_cuda:
-        return _attention_cuda(query, key, value, mask, scale)
     _check_layout(query, key)
     return _attention_eager(query, key, value, mask, scale)
 
 
 def _attention_cuda(query, key, value, mask, scale):
     _check_layout(query, key)
+    if not query.is_cuda:
+        return _attention_eager(query, key, value, mask, scale)
     batch, q_len, heads, dim = query.shape
     kernels = _gpu_kernels(heads, key.shape[2], dim, batch * q_len, query.device)
     if mask is not None:

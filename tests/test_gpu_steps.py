@@ -129,6 +129,21 @@ def test_cuda_op_reports_a_full_cache_on_its_next_call():
     assert torch.isfinite(ok.float()).all() and int(length) == 1
 
 
+def test_ops_on_the_cpu_with_an_argument_on_the_gpu():
+    """The dispatcher goes by any argument, the ops by their first one: tensors on the CPU with the length on the GPU run the
+    eager definition, and a mask on another device is torch's error."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value = (torch.randn(1, 1, heads, 64).bfloat16() for heads in (4, 2, 2))
+    caches, ref = ([torch.zeros(1, 8, 2, 64, dtype=torch.bfloat16) for _ in range(2)] for _ in range(2))
+    length, ref_length = torch.full((1,), 3, dtype=torch.int32, device=DEVICE), torch.full((1,), 3, dtype=torch.int32)
+    out = torch.ops.megabake.kv_attention(query, key, value, *caches, length)
+    assert torch.equal(out, oracle.kv_attention(query, key, value, *ref, ref_length))
+    assert int(length) == 4 and all(torch.equal(a, b) for a, b in zip(caches, ref))
+    with pytest.raises(RuntimeError, match="same device"):
+        torch.ops.megabake.attention(query, key, value, torch.zeros(1, 1, 1, 1, dtype=torch.bfloat16, device=DEVICE), 0.125)
+
+
 def test_a_bad_id_refuses_the_whole_step():
     """One out-of-range id among six sequences: nothing is appended, no length moves, the logits are NaN."""
     config = tiny_config(q_heads=4, kv_heads=1, hidden=256)
