@@ -63,6 +63,9 @@ int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 :
 size_t maps_per_table(const mk_config& c) { return 7 * static_cast<size_t>(c.layers) + 1; }
 size_t phases_per_table(const mk_config& c) { return 4 * static_cast<size_t>(c.layers) + 1; }
 
+// Handles that ask for the tensor engine (the attention ops' among them) have no streaming plans and buffers.
+bool stream_wanted(const mk_config& c) { return c.engine != MK_ENGINE_TCGEN05 && stream_shape_ok(c); }
+
 Carve carve(const mk_config& c, int grid) {
   Carve v{};
   size_t off = 0;
@@ -86,7 +89,7 @@ Carve carve(const mk_config& c, int grid) {
   v.att_xch = take(m * c.kv_heads * kMaxChunks * kExchangeFloats * 4);
   v.att_part = take(m * c.q_heads * kMaxChunks * c.head_dim * 4);
   v.host_io = take(3 * m * sizeof(int64_t));  // mk_decode_step_host: ids, positions, sampled tokens
-  if (stream_shape_ok(c)) {
+  if (stream_wanted(c)) {
     const size_t tokens = std::min<size_t>(m, kStreamTokens);
     v.splan = take(sizeof(StreamPlan) * kStreamPlans);
     v.smaps = take(sizeof(CUtensorMap) * kStreamPlans * maps_per_table(c));
@@ -300,7 +303,6 @@ struct mk_handle_s {
   bool kv_maps_refused; // tests: the first encoding counts as refused by the driver
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
-  StreamPhase stream_ph[kStreamPlans][kStreamPhases];
   bool use3d;           // weight descriptors of the tensor engine are three-dimensional (several K chunks per copy)
   uint32_t tp_epoch;    // all-reduces launched so far (tensor parallel)
   uint8_t* tp_peer[kMaxTp];
@@ -392,9 +394,8 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
 
 // Tensor engine, prompts of more than 128 tokens: every (row tile, K slice, tile of 256 tokens) is a unit.  With the decode
 // tables, whose tiles are as low as it takes to give every CTA one, an MMA of 48 or 56 rows takes the time of 128, and
-// every CTA walks all token tiles.  Here both operands come from L2, about 44 bytes per cycle and SM when all of them read
-// (128-token tiles: the projections of 500 tokens of the 1.7B shape at 12 TB/s), so the tile is as wide as tensor memory
-// allows, and the tile height and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs
+// every CTA walks all token tiles.  Here both operands come from L2 (the model below takes 44 bytes per cycle and SM), so the
+// tile is as wide as tensor memory allows, and the tile height and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs
 // and of its copies, plus what a unit costs besides.
 void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_tiles) {
   const int nseg = ph.nacc == 2 ? 1 : ph.nseg;
@@ -517,7 +518,7 @@ int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
 
 // The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.
 bool stream_usable(mk_handle h, int batch, bool ragged) {
-  return h->cfg.engine != MK_ENGINE_TCGEN05 && batch <= kStreamTokens && h->stream_ok[stream_plan_of(batch)] &&
+  return batch <= kStreamTokens && h->stream_ok[stream_plan_of(batch)] &&
          h->kv_maps_ok && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
 }
 
@@ -562,6 +563,9 @@ int launch_kv_attention(mk_handle h, const void* query, const void* key, const v
   return MK_OK;
 }
 
+// Keys of a prompt: the limit of the interface, 10240 per query head of a KV head.  The kernel, one pass over the keys, has none.
+int prompt_keys(mk_handle h) { return (kScoreBytes / 4 / (h->cfg.q_heads / h->cfg.kv_heads)) & ~7; }
+
 int attention_fits(mk_handle h, int keys, const char* what) {
   const int gs = h->cfg.q_heads / h->cfg.kv_heads;
   const int heads = gs * decode_heads_per_unit(h->cfg.kv_heads, gs, h->cfg.head_dim);  // query heads of one attention unit
@@ -597,7 +601,6 @@ int bind_stream(mk_handle h, const mk_weights& w, std::vector<CUtensorMap>& maps
     if (!stream_plan_used(c, i)) continue;
     StreamPlan& plan = plans[i];
     stream_phases(c, i, h->grid, plan.ph);
-    memcpy(h->stream_ph[i], plan.ph, sizeof(plan.ph));
     for (int l = 0; l < L; ++l) {
       const mk_layer_weights& lw = w.layers[l];
       const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
@@ -771,7 +774,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
         ph[0].out_col[s] = col;
         col += seg_rows[s];
       }
-      ph[0].epi = EPI_STORE; ph[0].bmode = B_NORM; ph[0].gather = (l == 0);
+      ph[0].epi = EPI_STORE; ph[0].gather = (l == 0);
       ph[0].normw = static_cast<const bf16*>(lw.input_norm);
       ph[0].src = hidden_a; ph[0].src_ld = c.hidden; ph[0].dst = qkv; ph[0].dst_ld = qkv_width(c);
       if (split) {
@@ -781,7 +784,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
       ph[1].nseg = 1; ph[1].nacc = 1; ph[1].k = q_size;
       ph[1].tmap[0] = tmaps_dev + 7 * l + 3; ph[1].w[0] = static_cast<const bf16*>(lw.o);
       ph[1].n[0] = c.hidden;
-      ph[1].epi = split ? EPI_PARTIAL : EPI_RESIDUAL; ph[1].bmode = B_ATTN;
+      ph[1].epi = split ? EPI_PARTIAL : EPI_RESIDUAL;
       ph[1].src = attn; ph[1].src_ld = q_size; ph[1].dst = hidden_a; ph[1].dst_ld = c.hidden;
       ph[1].partial = partial;
       // gate, up -> silu(gate) * up
@@ -789,13 +792,13 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
       ph[2].tmap[0] = tmaps_dev + 7 * l + 4; ph[2].tmap[1] = tmaps_dev + 7 * l + 5;
       ph[2].w[0] = static_cast<const bf16*>(lw.gate); ph[2].w[1] = static_cast<const bf16*>(lw.up);
       ph[2].n[0] = c.intermediate; ph[2].n[1] = c.intermediate;
-      ph[2].epi = EPI_SILU; ph[2].bmode = B_NORM; ph[2].normw = static_cast<const bf16*>(lw.post_norm);
+      ph[2].epi = EPI_SILU; ph[2].normw = static_cast<const bf16*>(lw.post_norm);
       ph[2].src = split ? hidden_b : hidden_a; ph[2].src_ld = c.hidden; ph[2].dst = act; ph[2].dst_ld = c.intermediate;
       // down
       ph[3].nseg = 1; ph[3].nacc = 1; ph[3].k = c.intermediate;
       ph[3].tmap[0] = tmaps_dev + 7 * l + 6; ph[3].w[0] = static_cast<const bf16*>(lw.down);
       ph[3].n[0] = c.hidden;
-      ph[3].epi = split ? EPI_PARTIAL : EPI_RESIDUAL; ph[3].bmode = B_PLAIN;
+      ph[3].epi = split ? EPI_PARTIAL : EPI_RESIDUAL;
       ph[3].src = act; ph[3].src_ld = c.intermediate; ph[3].dst = hidden_a; ph[3].dst_ld = c.hidden;
       ph[3].partial = partial;
       if (c.tp_size > 1) {  // tensor parallel: the residual add moves behind the all-reduce (tp_allreduce)
@@ -831,7 +834,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     head.nseg = 1; head.nacc = 1; head.k = c.hidden;
     head.tmap[0] = tmaps_dev + 7 * L; head.w[0] = static_cast<const bf16*>(w->lm_head);
     head.n[0] = c.vocab;
-    head.epi = EPI_STORE; head.bmode = B_NORM; head.normw = static_cast<const bf16*>(w->final_norm);
+    head.epi = EPI_STORE; head.normw = static_cast<const bf16*>(w->final_norm);
     head.src = hidden_a; head.src_ld = c.hidden; head.to_logits = 1; head.dst_ld = c.vocab;
     if (split) {
       head.add_parts = prev_parts; head.partial = partial;
@@ -864,7 +867,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   std::vector<int> stream_units;
   StreamPlan stream_plans[kStreamPlans];
   memset(stream_plans, 0, sizeof(stream_plans));
-  if (stream_shape_ok(c) && h->use3d) {
+  if (stream_wanted(c) && h->use3d) {
     if (int e = bind_stream(h, *w, stream_maps, stream_layers, stream_units, stream_plans)) return e;
     MK_CUDA(cudaMemcpyAsync(at<CUtensorMap>(h, h->cv.smaps), stream_maps.data(), stream_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
     MK_CUDA(cudaMemcpyAsync(at<StreamLayer>(h, h->cv.slayers), stream_layers.data(), stream_layers.size() * sizeof(StreamLayer), cudaMemcpyHostToDevice, s));
@@ -1081,9 +1084,7 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
   if (batch < 1 || sequence < 1 || m > h->cfg.max_tokens)
     return fail(MK_ERR_INVALID, "mk_prefill: %d x %d tokens outside [1, %d]", batch, sequence, h->cfg.max_tokens);
   if (int e = attention_fits(h, sequence, "mk_prefill")) return e;
-  const int gs = h->cfg.q_heads / h->cfg.kv_heads;
-  if (sequence > ((kScoreBytes / 4 / gs) & ~7))
-    return fail(MK_ERR_UNSUPPORTED, "mk_prefill: sequence %d exceeds the per-row score buffer", sequence);
+  if (sequence > prompt_keys(h)) return fail(MK_ERR_UNSUPPORTED, "mk_prefill: sequence %d exceeds %d keys", sequence, prompt_keys(h));
   KParams p;
   base_params(h, p);
   const int L = h->cfg.layers;
@@ -1127,7 +1128,7 @@ int mk_linear(mk_handle h, const void* x, const void* weight, const void* bias, 
   ph.nseg = 1; ph.nacc = 1; ph.k = k;
   ph.w[0] = static_cast<const bf16*>(weight); ph.bias[0] = static_cast<const bf16*>(bias);
   ph.n[0] = n;
-  ph.epi = EPI_STORE; ph.bmode = B_PLAIN;
+  ph.epi = EPI_STORE;
   ph.src = static_cast<const bf16*>(x); ph.src_ld = k;
   ph.dst = static_cast<bf16*>(y); ph.dst_ld = n;
   finish_phase_tc(ph, h->grid, false, h->cfg.max_tokens);
@@ -1201,9 +1202,7 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   if (!h || !query || !key || !value || !output) return fail(MK_ERR_INVALID, "mk_attention: null argument");
   std::lock_guard<std::mutex> guard(h->lock);
   if (batch < 1 || q_len < 1 || k_len < 1) return fail(MK_ERR_INVALID, "mk_attention: sizes must be positive");
-  const int gs = h->cfg.q_heads / h->cfg.kv_heads;
-  if (k_len > ((kScoreBytes / 4 / gs) & ~7))
-    return fail(MK_ERR_UNSUPPORTED, "mk_attention: %d keys exceed the per-row score buffer", k_len);
+  if (k_len > prompt_keys(h)) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %d keys exceed %d", k_len, prompt_keys(h));
   if (reinterpret_cast<uintptr_t>(key) % 16 || reinterpret_cast<uintptr_t>(value) % 16)
     return fail(MK_ERR_ALIGNMENT, "mk_attention: key/value must be 16-byte aligned");
   const int q_size = h->cfg.q_heads * h->cfg.head_dim, kv_size = h->cfg.kv_heads * h->cfg.head_dim;

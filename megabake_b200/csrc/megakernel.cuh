@@ -43,7 +43,6 @@ constexpr int kMaxSplit = 4;             // K slices a projection may be cut int
 static_assert(kSmemBytes <= 200704, "dynamic shared memory exceeds the 196 KiB carve-out");
 
 enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SILU = 2, EPI_PARTIAL = 3, EPI_TP = 4 };
-enum { B_PLAIN = 0, B_NORM = 1, B_ATTN = 2 };
 enum { MODE_DECODE = 0, MODE_PREFILL = 1, MODE_LINEAR = 2 };
 enum { EV_PHASE_ENTER = 1, EV_B_STAGED = 2, EV_FIRST_ACC = 3, EV_PHASE_DONE = 4, EV_BARRIER_DONE = 5, EV_ATTENTION_DONE = 6,
        EV_ATT_INPUTS = 7, EV_ATT_SCORES = 8, EV_ATT_STATS = 9, EV_ATT_VALUES = 10, EV_ATT_PARTIAL = 11, EV_FIRST_COPY = 12 };
@@ -83,16 +82,16 @@ struct GemmPhase {
   int ntiles;                  // row tiles
   int ksplit, kslice;          // K slices and chunks per slice (kc == ksplit * kslice)
   int nunits;                  // ntiles * ksplit
-  int epi, bmode;
+  int epi;
   int gather;                  // 1: activation rows are embedding rows selected by the token ids
   int to_logits;               // 1: output goes to the caller's logits buffer
   int tp_buf;                  // EPI_TP: which half of the exchange buffers this projection's partial sums go to
-  int add_parts;               // B_NORM: fp32 partial slices of the previous projection to add to the residual
+  int add_parts;               // norm phases: fp32 partial slices of the previous projection to add to the residual
   const bf16* normw;
-  const bf16* src; int src_ld; // activation source (B_NORM: the residual stream before this phase)
+  const bf16* src; int src_ld; // activation source (norm phases: the residual stream before this phase)
   bf16* dst; int dst_ld;
-  float* partial;              // EPI_PARTIAL output / B_NORM add_parts input: [slice][token][hidden]
-  bf16* h_out;                 // B_NORM with add_parts or gather: where the updated residual stream goes
+  float* partial;              // EPI_PARTIAL output / add_parts input: [slice][token][hidden]
+  bf16* h_out;                 // norm phases with add_parts or gather: where the updated residual stream goes
 };
 
 struct Control {
@@ -100,7 +99,6 @@ struct Control {
   uint32_t abort;     // set once by whoever gives up a wait; every wait polls it
   int status;         // mk_device_status
   int where, cta, detail;
-  int att_nch;        // context chunks the last attention phase used (read by the o projection)
   uint32_t pad;       // mk_kv_attention, mk_kv_attention_static: 1 if the first launch refused the valid length
 };
 

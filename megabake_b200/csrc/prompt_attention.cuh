@@ -19,9 +19,7 @@ struct AttnArgs {
   int len;            // decode: filled positions before this call (the longest sequence's when lengths are per sequence)
   const int* lens;    // decode with per-sequence valid lengths: filled positions of each sequence; null = `len` for all
   int decode;         // 1: append the new key/value at `len` and attend over [0, len]
-  int rope;           // 1: rotate q and the new key while loading (decode)
   int causal;         // prefill without a mask tensor: key j <= query qi
-  int combine;        // 1: a split context is summed here into `out`; 0: the consumer sums att_part
   uint32_t stamp;     // value the chunks of this phase publish with their softmax statistics
   float scale;
   const CUtensorMap *kmap, *vmap;  // decode: tiled descriptors of the two caches (see attention_decode), or null

@@ -84,9 +84,10 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
   return ok;
 }
 
-// Hidden sizes up to 2048.  Wider shapes would fit batches of up to 16 too, but they come with 32 layers and more, where two
-// correct bf16 evaluations are 2.0 to 2.2 % apart (measured on the 8B shape: this kernel, the tensor engine and an eager
-// evaluation, each against each): they stay on the tensor engine, whose results their users have.
+// Hidden sizes up to 2048: an operand of 2048 columns fits a warp's registers at 32 tokens (two copies of a slice), and only
+// such shapes have been measured and tested here.  Wider ones would fit up to 16 tokens and are left on the tensor engine;
+// that is not a limit of the hardware.  What to expect of a change: on the 8B shape's 32 layers this kernel, the tensor
+// engine and an eager evaluation are 2.0 to 2.2 % apart, each from each, as correct bf16 evaluations of that depth are.
 inline bool stream_shape_ok(const mk_config& c) {
   if (c.tp_size > 1 || c.hidden > 2048) return false;
   StreamPhase ph[kStreamPhases];
