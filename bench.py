@@ -254,7 +254,7 @@ def run_c4(args, config, weights, group: Group, rank: int, peak: float):
         "value": n_streams * batch * steps / (elapsed_ms / 1e3), "unit": "tokens/s", "n_gpus": group.world,
         "ms_total": elapsed_ms, "us_per_stream_step": 1e3 * elapsed_ms / (steps * streams_per_gpu),
         "per_gpu_roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                             "kernel": "mk::megakernel (one launch per step of 8 sequences)"},
+                             "kernel": "mk::decode_stream (one launch per step of 8 sequences)"},
         "gpu_launches_per_gpu": launches,
         "tokens_checked": None if tokens is None else int(sum(t.numel() for t in tokens)),
     }

@@ -1,0 +1,20 @@
+// The epilogues' SiLU against the division it stands for, for test_gpu_steps.py: every bf16 pattern once.
+#include "../megabake_b200/csrc/device_common.cuh"
+
+__global__ void sweep(unsigned* same, unsigned* differ) {
+  const unsigned bits = blockIdx.x * blockDim.x + threadIdx.x;  // 65536 threads
+  const float x = __uint_as_float(bits << 16);
+  if (!(fabsf(x) < 80.f)) return;
+  const float mine = mk::silu_inner(x), exact = mk::silu(x);
+  const bool equal = __float_as_uint(mine) == __float_as_uint(exact) || (mine == 0.f && exact == 0.f);
+  atomicAdd(equal ? same : differ, 1u);
+}
+
+extern "C" int silu_sweep(unsigned* counts) {
+  unsigned* device = nullptr;
+  if (cudaMalloc(&device, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(device, 0, 2 * sizeof(unsigned)) != cudaSuccess) return 1;
+  sweep<<<256, 256>>>(device, device + 1);
+  const cudaError_t done = cudaMemcpy(counts, device, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost);
+  cudaFree(device);
+  return done == cudaSuccess ? 0 : 2;
+}

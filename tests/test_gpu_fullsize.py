@@ -79,15 +79,16 @@ def three_way_decode(name, config, batch, capacity, context, steps, engine="auto
     return per_step
 
 
-def test_smollm_1_7b_batch_16_context_1024():
-    """Benchmark configuration 3 at batch 16: the tensor engine, one launch per step."""
-    assert three_way_decode("c3_batch16_ctx1024", CONFIGS["smollm-1.7b"], 16, 2048, 1024, steps=3) == 1
+@pytest.mark.parametrize("engine", ["auto", "tcgen05"])
+def test_smollm_1_7b_batch_16_context_1024(engine):
+    """Benchmark configuration 3 at batch 16, one launch per step: the streaming kernel and the tensor engine."""
+    assert three_way_decode(f"c3_batch16_ctx1024_{engine}", CONFIGS["smollm-1.7b"], 16, 2048, 1024, steps=3, engine=engine) == 1
 
 
-def test_smollm_1_7b_batch_8_context_512():
-    """The per-GPU workload of the data-parallel sweep: 8 sequences from a 512-token prefix (tensor engine,
-    one launch per step)."""
-    assert three_way_decode("c4_batch8_ctx512", CONFIGS["smollm-1.7b"], 8, 1024, 512, steps=3) == 1
+@pytest.mark.parametrize("engine", ["auto", "tcgen05"])
+def test_smollm_1_7b_batch_8_context_512(engine):
+    """The per-GPU workload of the data-parallel sweep: 8 sequences from a 512-token prefix, one launch per step."""
+    assert three_way_decode(f"c4_batch8_ctx512_{engine}", CONFIGS["smollm-1.7b"], 8, 1024, 512, steps=3, engine=engine) == 1
 
 
 def llama3_two_layers() -> DecoderConfig:

@@ -108,7 +108,7 @@ def test_decode_tiny_matches_reference(device, name, engine):
 @pytest.mark.parametrize("engine", ["tcgen05", "fma"])
 def test_decode_smollm_135m_64_steps(device, engine):
     ties, run = run_golden_decode("c1", device, engine, deep=True)
-    # measured on a B200: 5 (tensor engine) and 4 (small-launch kernel) of 64 greedy tokens differ from the
+    # measured on a B200: 5 (tensor engine) and 3 (streaming kernel) of 64 greedy tokens differ from the
     # CPU-made golden ones, each at a position where the reference's own top two logits tie in bf16
     # (token_agrees checks that)
     assert run == 67 and ties <= 5
@@ -117,8 +117,8 @@ def test_decode_smollm_135m_64_steps(device, engine):
 @pytest.mark.parametrize("engine", ["auto", "tcgen05"])
 def test_decode_qwen2_half_b_64_steps(device, engine):
     ties, run = run_golden_decode("c2", device, engine, deep=True)
-    # measured on a B200: 1 of 64 (tensor engine) and 2 of 64 (small-launch kernel, whose attention sums in
-    # tensor-core order for grouped heads), each a bf16 tie of the reference's own top two logits
+    # measured on a B200: 1 of 64 on the tensor engine and on the streaming kernel, a bf16 tie of the reference's own top
+    # two logits
     assert run == 67 and ties <= 2
 
 
@@ -260,8 +260,8 @@ def test_decode_error_no_worse_than_eager_bf16(device):
 @pytest.mark.parametrize("engine", ["auto", "tcgen05"])
 @pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 8, 16, 21])
 def test_decode_batches_match_oracle(device, batch, engine):
-    """Batches 1-4 run the small-launch kernel under "auto" (one instantiation per token count),
-    larger ones the tensor engine (token tiles of 16 and 32)."""
+    """Under "auto" the streaming kernel's token classes (up to 1, 4, 8, 16, 32), else the tensor engine (token tiles of 16
+    and 32)."""
     oracle_decode_compare(tiny_config(q_heads=4, kv_heads=1, hidden=256), device, batch, capacity=24, prefill=0, steps=4,
                           engine=engine)
 
@@ -511,8 +511,8 @@ def test_event_trace_reports_every_phase(device, engine):
     codes, times = decode_trace(buffer)
     barriers = int((codes[0] == 5).sum())
     # seven grid barriers per layer on the tensor engine (five between phases, two behind the norm phases) and one
-    # behind the final norm; the small-launch kernel at one token hands every phase's outputs to the next as
-    # stamped words and keeps a single barrier at the end of the launch
+    # behind the final norm; the streaming kernel's phases wait for words to be set, and it keeps a single barrier at the
+    # end of the launch
     assert barriers == (7 * config.layers + 1 if engine == "tcgen05" else 1)
     stamps = times[0][codes[0] > 0][:barriers]
     assert bool((stamps[1:] >= stamps[:-1]).all())

@@ -36,9 +36,10 @@ def greedy_on_host(kernel, config, ids, start, steps, state):
     return torch.stack(tokens, dim=1)
 
 
-@pytest.mark.parametrize("batch,engine", [(1, "auto"), (3, "auto"), (6, "auto"), (9, "auto"), (2, "tcgen05")])
+@pytest.mark.parametrize("batch,engine", [(1, "auto"), (3, "auto"), (6, "auto"), (9, "auto"), (20, "auto"), (33, "auto"), (2, "tcgen05"),
+                                          (6, "tcgen05"), (9, "tcgen05")])
 def test_decode_steps_equals_the_step_by_step_path(batch, engine):
-    """Row table (1 token), split-K table (3) and the tensor engine (6, 9, forced 2)."""
+    """Every token class of the streaming kernel, and the tensor engine (33 sequences, or asked for)."""
     config = tiny_config(q_heads=4, kv_heads=2, hidden=256)
     weights = synth_weights(config, seed=4, norm_std=0.1, device=DEVICE)
     kernel = make_kernel(config, weights, max_tokens=batch, max_positions=32, engine=engine)
@@ -157,17 +158,17 @@ def test_a_bad_id_refuses_the_whole_step():
     assert all(not bool(cache.any()) for cache in keys)
 
 
-@pytest.mark.parametrize("batch", [1, 3, 9])
-def test_a_grid_barrier_that_cannot_be_reached_times_out_and_the_handle_recovers(batch, monkeypatch):
+@pytest.mark.parametrize("batch,engine", [(1, "auto"), (3, "auto"), (9, "auto"), (32, "auto"), (1, "tcgen05"), (9, "tcgen05"), (33, "auto")])
+def test_a_grid_barrier_that_cannot_be_reached_times_out_and_the_handle_recovers(batch, engine, monkeypatch):
     """Failure detection without a hang: the host skews the barrier count it expects, the kernel's
     bounded wait (40 ms here) runs out, the status word says TIMEOUT, the valid lengths have not
-    moved, and after the reset the same handle decodes correctly.  One token count per kernel:
-    row table, split-K table, tensor engine."""
+    moved, and after the reset the same handle decodes correctly.  The streaming kernel (one barrier, at
+    the end) and the tensor engine (33 sequences, or asked for: several barriers a layer)."""
     monkeypatch.setenv("MEGABAKE_WAIT_LIMIT_MS", "40")
     config = tiny_config(q_heads=4, kv_heads=2, hidden=256)
     weights = synth_weights(config, seed=6, norm_std=0.1, device=DEVICE)
-    kernel = make_kernel(config, weights, max_tokens=batch, max_positions=16)
-    reference = make_kernel(config, weights, max_tokens=batch, max_positions=16)
+    kernel = make_kernel(config, weights, max_tokens=batch, max_positions=16, engine=engine)
+    reference = make_kernel(config, weights, max_tokens=batch, max_positions=16, engine=engine)
     ids = synth_ids(batch, config.vocab, seed=6).view(batch, 1).to(DEVICE)
     positions = torch.zeros((batch, 1), dtype=torch.int64, device=DEVICE)
     expected = reference.decode(ids, positions, *new_kv_state(config, batch, 16, DEVICE))
@@ -254,6 +255,22 @@ def test_logits_may_begin_at_any_element(batch):
     kernel.check()
     assert torch.equal(buffer[1:-1].view(expected.shape), expected)
     assert float(buffer[0]) == -3.0 and float(buffer[-1]) == -3.0
+
+
+def test_silu_of_the_epilogues_has_the_bits_of_the_division(tmp_path):
+    """``silu_inner`` over every bf16 below 80 (the sign of zero aside), built as the library is."""
+    import subprocess
+    from pathlib import Path
+
+    from megabake_b200.build import NVCC_FLAGS, find_nvcc
+
+    library = tmp_path / "silu_sweep.so"
+    subprocess.run([find_nvcc(), *NVCC_FLAGS, "-o", str(library), str(Path(__file__).resolve().parent / "silu_sweep.cu"), "-lcudart"],
+                   check=True, capture_output=True, text=True)
+    counts = (ctypes.c_uint32 * 2)()
+    assert ctypes.CDLL(str(library)).silu_sweep(counts) == 0
+    below = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float().abs() < 80
+    assert list(counts) == [int(below.sum()), 0]
 
 
 def test_static_scratch_status_recovers_from_a_refused_launch():
