@@ -395,8 +395,8 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
 // Tensor engine, prompts of more than 128 tokens: every (row tile, K slice, tile of 256 tokens) is a unit.  With the decode
 // tables, whose tiles are as low as it takes to give every CTA one, an MMA of 48 or 56 rows takes the time of 128, and
 // every CTA walks all token tiles.  Here both operands come from L2 (the model below takes 44 bytes per cycle and SM), so the
-// tile is as wide as tensor memory allows, and the tile height and the K split are the cheapest by this model of a unit: per K chunk the longer of its MMAs
-// and of its copies, plus what a unit costs besides.
+// tile is as wide as tensor memory allows, and the tile height and the K split are the cheapest by this model of a unit: per
+// K chunk the longer of its MMAs and of its copies, plus what a unit costs besides.
 void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_tiles) {
   const int nseg = ph.nacc == 2 ? 1 : ph.nseg;
   ph.kc = ph.k / kChunkK;
