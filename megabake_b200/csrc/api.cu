@@ -17,6 +17,7 @@
 
 #include "decoder_kernel.cuh"
 #include "kv_attention.cuh"
+#include "prompt_plan.h"
 #include "stream_plan.h"
 
 using namespace mk;
@@ -43,6 +44,7 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct Carve {
   size_t ctrl, tmaps, kvmaps, phases, hidden, hidden2, xnorm, qkv, attn, act, partial, att_xch, att_part, host_io;
+  size_t pmaps;                                        // prompt kernels: weight descriptors per class
   size_t splan, smaps, slayers, sunits, srec;          // streaming decode kernel
   size_t handover, handover_bytes, shalf[5][3], spart[2][3];       // its hand-over buffers, filled with the unset word
   size_t total;
@@ -52,19 +54,17 @@ int qkv_width(const mk_config& c) { return (c.q_heads + 2 * c.kv_heads) * c.head
 // Token-operand descriptors of the tensor engine: (normalised rows, attention output, SiLU*up, mk_linear's
 // source) x (token tiles of 16, 32, 64), behind the weight descriptors.
 constexpr int kCacheMapSets = 8;  // cache-descriptor sets a handle remembers (one per KV state it is called with in turn)
-constexpr int kOperandTiles = 5;  // token tiles of 16, 32, 64, 128, 256
-constexpr int kOperandChunks = 4; // K chunks per copy: 1 .. 4
-constexpr int kOperandKinds = 3, kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;
-enum { OPERAND_XNORM = 0, OPERAND_ATTN = 1, OPERAND_ACT = 2 };
-// Phase tables: split-K, plain, and for prompts of more than 128 tokens one each for one, two and three or more tiles of 256.
-constexpr int kSpreadTables = 3;
-int phase_tables(const mk_config& c) { return 2 + (c.max_tokens > 128 && c.tp_size <= 1 ? kSpreadTables : 0); }
+constexpr int kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;
+constexpr int kPhaseTables = 2;   // split-K, plain
 int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128)); }
 size_t maps_per_table(const mk_config& c) { return 7 * static_cast<size_t>(c.layers) + 1; }
 size_t phases_per_table(const mk_config& c) { return 4 * static_cast<size_t>(c.layers) + 1; }
 
 // Handles that ask for the tensor engine (the attention ops' among them) have no streaming plans and buffers.
 bool stream_wanted(const mk_config& c) { return c.engine != MK_ENGINE_TCGEN05 && stream_shape_ok(c); }
+
+// Prompt passes of a single-GPU handle run on kernels of their own, in classes by token count.
+int prompt_classes(const mk_config& c, int grid) { return c.tp_size > 1 ? 0 : 1 + prompt_class(c.max_tokens, grid); }
 
 Carve carve(const mk_config& c, int grid) {
   Carve v{};
@@ -76,9 +76,10 @@ Carve carve(const mk_config& c, int grid) {
   };
   const size_t m = static_cast<size_t>(c.max_tokens);
   v.ctrl = take(sizeof(Control));
-  v.tmaps = take(sizeof(CUtensorMap) * (phase_tables(c) * maps_per_table(c) + kOperandMaps));
+  v.tmaps = take(sizeof(CUtensorMap) * (kPhaseTables * maps_per_table(c) + kOperandMaps));
+  v.pmaps = take(sizeof(CUtensorMap) * prompt_classes(c, grid) * maps_per_table(c));
   v.kvmaps = take(sizeof(CUtensorMap) * 2 * static_cast<size_t>(c.layers) * kCacheMapSets);  // decode attention: per set, key caches then value caches
-  v.phases = take(sizeof(GemmPhase) * phase_tables(c) * phases_per_table(c));
+  v.phases = take(sizeof(GemmPhase) * kPhaseTables * phases_per_table(c));
   v.hidden = take(m * c.hidden * 2);
   v.hidden2 = take(m * c.hidden * 2);
   v.xnorm = take(m * c.hidden * 2);
@@ -303,6 +304,7 @@ struct mk_handle_s {
   bool kv_maps_refused; // tests: the first encoding counts as refused by the driver
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
+  PromptPhase prompt[kPromptClasses][kPromptPhases];
   bool use3d;           // weight descriptors of the tensor engine are three-dimensional (several K chunks per copy)
   uint32_t tp_epoch;    // all-reduces launched so far (tensor parallel)
   uint8_t* tp_peer[kMaxTp];
@@ -392,48 +394,6 @@ void finish_phase_tc(GemmPhase& ph, int grid, bool allow_split, int max_tokens) 
   ph.gran = ph.nacc * kb * ph.rows / 8;
 }
 
-// Tensor engine, prompts of more than 128 tokens: every (row tile, K slice, tile of 256 tokens) is a unit.  With the decode
-// tables, whose tiles are as low as it takes to give every CTA one, an MMA of 48 or 56 rows takes the time of 128, and
-// every CTA walks all token tiles.  Here both operands come from L2 (the model below takes 44 bytes per cycle and SM), so the
-// tile is as wide as tensor memory allows, and the tile height and the K split are the cheapest by this model of a unit: per
-// K chunk the longer of its MMAs and of its copies, plus what a unit costs besides.
-void finish_phase_spread(GemmPhase& ph, int grid, bool allow_split, int token_tiles) {
-  const int nseg = ph.nacc == 2 ? 1 : ph.nseg;
-  ph.kc = ph.k / kChunkK;
-  long long best = -1;
-  auto shape = [&](int rows, int split) {
-    ph.rows = rows;
-    ph.ksplit = split;
-    ph.kslice = ph.kc / split;
-    int tile = 0;
-    for (int s = 0; s < nseg; ++s) {
-      ph.tile_start[s] = tile;
-      tile += (ph.n[s] + rows - 1) / rows;
-    }
-    ph.tile_start[nseg] = tile;
-    ph.ntiles = tile;
-    ph.nunits = tile * split;
-  };
-  int best_rows = kTileRows, best_split = 1;
-  for (int split = 1; split <= (allow_split ? kMaxSplit : 1); split *= 2) {
-    if (ph.kc % split) continue;
-    for (int rows = kTileRows; rows >= 64; rows -= 8) {
-      shape(rows, split);
-      const long long units = static_cast<long long>(ph.nunits) * token_tiles, rounds = (units + grid - 1) / grid;
-      const long long chunk = std::max(512 * ph.nacc, (ph.nacc * rows + kSpreadTok) * 128 / 44);
-      const long long cost = rounds * (ph.kslice * chunk + 3000) + split * 600;
-      if (best < 0 || cost < best) {
-        best = cost;
-        best_rows = rows;
-        best_split = split;
-      }
-    }
-  }
-  shape(best_rows, best_split);
-  ph.kb = 1;
-  ph.gran = ph.kb * ph.nacc * ph.rows / 8;
-}
-
 // The split-K table (o_proj and down_proj cut along K so that every SM streams, fp32 partial sums added by
 // the next norm phase) serves every launch of a single-GPU handle.
 bool split_table_ok(const mk_config& c) { return c.tp_size <= 1; }
@@ -485,8 +445,7 @@ int prepare_kernels(int device, int head_dim) {
   if (!tensor_done[device]) {
     MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     MK_CUDA(cudaFuncSetAttribute(megakernel, cudaFuncAttributePreferredSharedMemoryCarveout, (kSmemBytes * 100 + 233471) / 233472));
-    MK_CUDA(cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem));
-    MK_CUDA(cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem));
+    MK_CUDA(prompt_prepare());
     MK_CUDA(cudaFuncSetAttribute(kv_attention_parts<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvLaunch<64>::kSmem));
     MK_CUDA(cudaFuncSetAttribute(kv_attention_parts<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, KvLaunch<128>::kSmem));
     int per_sm = 0;
@@ -725,11 +684,10 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   const int L = c.layers;
   const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
   const size_t nmaps = maps_per_table(c), nphases = phases_per_table(c);
-  const int ntables = phase_tables(c);
-  std::vector<CUtensorMap> maps(ntables * nmaps);
-  std::vector<GemmPhase> phases(ntables * nphases);
+  std::vector<CUtensorMap> maps(kPhaseTables * nmaps);
+  std::vector<GemmPhase> phases(kPhaseTables * nphases);
   CUtensorMap* dmaps = at<CUtensorMap>(h, h->cv.tmaps);
-  CUtensorMap* operand_maps = dmaps + ntables * nmaps;
+  CUtensorMap* operand_maps = dmaps + kPhaseTables * nmaps;
   auto operand_map = [&](int kind, int tile, int chunks) { return operand_maps + (kind * kOperandTiles + tile) * kOperandChunks + chunks - 1; };
   bf16* hidden_a = at<bf16>(h, h->cv.hidden);
   bf16* hidden_b = at<bf16>(h, h->cv.hidden2);
@@ -746,10 +704,9 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
   }
   // Table 0: split-K: o and down store K-slice partials; the next
   // normalising phase adds them to the residual stream, which ping-pongs between
-  // hidden_b (after attention) and hidden_a (after the MLP).  Table 1: plain.  From table 2 on: split-K for prompts
-  // of that many token tiles (the last one: and more).
+  // hidden_b (after attention) and hidden_a (after the MLP).  Table 1: plain.
   bool use3d = h->use3d;
-  for (int table = 0; table < ntables; ++table) {
+  for (int table = 0; table < kPhaseTables; ++table) {
     const bool split = table != 1;
     if (split && !split_table_ok(c)) continue;
     GemmPhase* tp = phases.data() + table * nphases;
@@ -808,18 +765,17 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
       ph[1].gate = 1;  // decode attention streams cache tiles through the weight ring just before this phase
       for (int i = 0; i < 4; ++i) {
         const bool may_split = split && ph[i].epi == EPI_PARTIAL;
-        if (table < 2) finish_phase_tc(ph[i], h->grid, may_split, c.max_tokens);
-        else finish_phase_spread(ph[i], h->grid, may_split, table - 1);
+        finish_phase_tc(ph[i], h->grid, may_split, c.max_tokens);
       }
       if (split) {
         ph[2].add_parts = ph[1].ksplit; ph[2].partial = partial; ph[2].h_out = hidden_a;
         prev_parts = ph[3].ksplit;
       }
       for (int t = 0; t < kOperandTiles; ++t) {  // token operands: normalised rows, attention output, SiLU*up
-        ph[0].bmap[t] = operand_map(OPERAND_XNORM, t, ph[0].kb);
-        ph[1].bmap[t] = operand_map(OPERAND_ATTN, t, ph[1].kb);
-        ph[2].bmap[t] = operand_map(OPERAND_XNORM, t, ph[2].kb);
-        ph[3].bmap[t] = operand_map(OPERAND_ACT, t, ph[3].kb);
+        ph[0].bmap[t] = operand_map(kOperandXnorm, t, ph[0].kb);
+        ph[1].bmap[t] = operand_map(kOperandAttn, t, ph[1].kb);
+        ph[2].bmap[t] = operand_map(kOperandXnorm, t, ph[2].kb);
+        ph[3].bmap[t] = operand_map(kOperandAct, t, ph[3].kb);
       }
       // One TMA descriptor per matrix, boxed to the tile height and the K chunks per copy its phase chose.
       const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
@@ -839,9 +795,8 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     if (split) {
       head.add_parts = prev_parts; head.partial = partial;
     }
-    if (table < 2) finish_phase_tc(head, h->grid, false, c.max_tokens);
-    else finish_phase_spread(head, h->grid, false, table - 1);
-    for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_map(OPERAND_XNORM, t, head.kb);
+    finish_phase_tc(head, h->grid, false, c.max_tokens);
+    for (int t = 0; t < kOperandTiles; ++t) head.bmap[t] = operand_map(kOperandXnorm, t, head.kb);
     if (int e = encode_phase_weight_map(&tmaps_host[7 * L], w->lm_head, c.vocab, c.hidden, head, use3d)) return e;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -850,7 +805,7 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     memset(operand_host, 0, sizeof(operand_host));
     const void* bases[3] = {at<bf16>(h, h->cv.xnorm), attn, act};
     const int widths[3] = {c.hidden, q_size, c.intermediate};
-    static const int tiles[kOperandTiles] = {16, 32, 64, 128, 256};
+    static const int tiles[kOperandTiles] = {16, 32, 64, 128};
     for (int kind = 0; kind < 3; ++kind)
       for (int t = 0; t < kOperandTiles; ++t)
         for (int chunks = 1; chunks <= kOperandChunks && tiles[t] * chunks * 128 <= kBBytes / 2; ++chunks)
@@ -873,6 +828,24 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
     MK_CUDA(cudaMemcpyAsync(at<StreamLayer>(h, h->cv.slayers), stream_layers.data(), stream_layers.size() * sizeof(StreamLayer), cudaMemcpyHostToDevice, s));
     MK_CUDA(cudaMemcpyAsync(at<int>(h, h->cv.sunits), stream_units.data(), stream_units.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     MK_CUDA(cudaMemcpyAsync(at<StreamPlan>(h, h->cv.splan), stream_plans, sizeof(stream_plans), cudaMemcpyHostToDevice, s));
+  }
+  std::vector<CUtensorMap> prompt_maps(prompt_classes(c, h->grid) * nmaps);
+  if (h->use3d && !prompt_maps.empty()) {
+    for (int cls = 0; cls < prompt_classes(c, h->grid); ++cls) {
+      PromptPhase* const pp = h->prompt[cls];
+      prompt_phases(c, cls, h->grid, pp);
+      CUtensorMap* const to = prompt_maps.data() + cls * nmaps;
+      for (int l = 0; l < L; ++l) {
+        const mk_layer_weights& lw = w->layers[l];
+        const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
+        const int rows[7] = {q_size, kv_size, kv_size, c.hidden, c.intermediate, c.intermediate, c.hidden};
+        const int which[7] = {PP_QKV, PP_QKV, PP_QKV, PP_O, PP_GU, PP_GU, PP_DOWN};
+        for (int i = 0; i < 7; ++i)
+          if (int e = encode_weight_map3(&to[7 * l + i], mats[i], rows[i], pp[which[i]].k, prompt_box_rows(pp[which[i]], cls), 1)) return e;
+      }
+      if (int e = encode_weight_map3(&to[7 * L], w->lm_head, c.vocab, c.hidden, prompt_box_rows(pp[PP_HEAD], cls), 1)) return e;
+    }
+    MK_CUDA(cudaMemcpyAsync(at<CUtensorMap>(h, h->cv.pmaps), prompt_maps.data(), prompt_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
   }
   // The source vectors die at return: make sure the copies have read them.
   MK_CUDA(cudaStreamSynchronize(s));
@@ -1085,18 +1058,38 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
     return fail(MK_ERR_INVALID, "mk_prefill: %d x %d tokens outside [1, %d]", batch, sequence, h->cfg.max_tokens);
   if (int e = attention_fits(h, sequence, "mk_prefill")) return e;
   if (sequence > prompt_keys(h)) return fail(MK_ERR_UNSUPPORTED, "mk_prefill: sequence %d exceeds %d keys", sequence, prompt_keys(h));
+  const int L = h->cfg.layers;
+  if (h->cfg.tp_size <= 1 && h->use3d) {
+    const size_t nmaps = maps_per_table(h->cfg);
+    PromptPass pass{};
+    pass.config = &h->cfg;
+    pass.weights = &h->weights;
+    pass.cls = prompt_class(static_cast<int>(m), h->grid);
+    pass.grid = h->grid;
+    pass.phases = h->prompt[pass.cls];
+    pass.maps = at<CUtensorMap>(h, h->cv.pmaps) + pass.cls * nmaps;
+    pass.operands = at<CUtensorMap>(h, h->cv.tmaps) + kPhaseTables * nmaps;
+    pass.hidden_a = at<bf16>(h, h->cv.hidden); pass.hidden_b = at<bf16>(h, h->cv.hidden2);
+    pass.xnorm = at<bf16>(h, h->cv.xnorm); pass.qkv = at<bf16>(h, h->cv.qkv);
+    pass.attn = at<bf16>(h, h->cv.attn); pass.act = at<bf16>(h, h->cv.act);
+    pass.partial = at<float>(h, h->cv.partial);
+    pass.ids = reinterpret_cast<const long long*>(ids);
+    pass.pos = reinterpret_cast<const long long*>(positions);
+    pass.mask = static_cast<const bf16*>(mask);
+    pass.logits = static_cast<bf16*>(logits);
+    pass.m = static_cast<int>(m); pass.batch = batch; pass.seq = sequence;
+    pass.att_scale = h->att_scale;
+    pass.guard = {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles};
+    MK_CUDA(prompt_forward(pass, static_cast<cudaStream_t>(stream)));
+    h->launches += 7 * L + 2;
+    return MK_OK;
+  }
   KParams p;
   base_params(h, p);
-  const int L = h->cfg.layers;
   const int ntt = token_tiles(static_cast<int>(m));
   p.mode = MODE_PREFILL; p.m = static_cast<int>(m); p.batch = batch; p.seq = sequence; p.capacity = 0;
   p.split = split_table_ok(h->cfg) ? 1 : 0;
   p.phases = at<GemmPhase>(h, h->cv.phases) + (p.split ? 0 : phases_per_table(h->cfg));
-  if (p.split && ntt > 1) {
-    const int tiles = static_cast<int>((m + kSpreadTok - 1) / kSpreadTok);
-    p.spread = 1;
-    p.phases = at<GemmPhase>(h, h->cv.phases) + (1 + std::min(tiles, kSpreadTables)) * phases_per_table(h->cfg);
-  }
   p.n_gemm = 4 * L + 1;
   p.nbar = 8 * L + 1;  // as decode, plus one behind the rotation of q and k
   p.stream_once = (ntt == 1);
@@ -1216,12 +1209,9 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   A.mask = static_cast<const bf16*>(mask); A.sq = q_len; A.klen = k_len; A.scale = scale;
   const long long units = static_cast<long long>(batch) * h->cfg.q_heads * ((q_len + kPromptQueries - 1) / kPromptQueries);
   if (units > INT32_MAX) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %lld blocks of queries", units);
-  auto go = [&](auto kernel, int smem) {
-    const int blocks = h->cfg.sm_limit > 0 ? std::min(static_cast<int>(units), h->grid) : static_cast<int>(units);
-    kernel<<<blocks, kWorkers, smem, static_cast<cudaStream_t>(stream)>>>(A, h->cfg.q_heads, h->cfg.kv_heads, batch, static_cast<int>(units));
-    return cudaGetLastError();
-  };
-  MK_CUDA(h->cfg.head_dim == 64 ? go(prompt_attention<64>, PromptLaunch<64>::kSmem) : go(prompt_attention<128>, PromptLaunch<128>::kSmem));
+  const int blocks = h->cfg.sm_limit > 0 ? std::min(static_cast<int>(units), h->grid) : static_cast<int>(units);
+  MK_CUDA(prompt_attention_launch(A, h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads, batch, static_cast<int>(units), blocks, false,
+                                  static_cast<cudaStream_t>(stream)));
   h->launches += 1;
   return MK_OK;
 }
@@ -1342,16 +1332,23 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
       h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
       h->cfg.tp_size > 1 ? h->cfg.tp_size : 1);
   if (h->bound) {
-    const int ntables = phase_tables(h->cfg);
-    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * ntables);
+      std::vector<GemmPhase> phases(phases_per_table(h->cfg) * kPhaseTables);
     MK_CUDA(cudaMemcpy(phases.data(), at<GemmPhase>(h, h->cv.phases), phases.size() * sizeof(GemmPhase), cudaMemcpyDeviceToHost));
     static const char* names[5] = {"qkv", "o", "gate/up", "down", "lm_head"};
-    for (int table = 0; table < ntables; ++table) {
+    for (int table = 0; table < kPhaseTables; ++table) {
       if (table == 0 && !split_table_ok(h->cfg)) continue;
       add("table %d:", table);
       for (int i = 0; i < 5; ++i) {
         const GemmPhase& ph = phases[table * phases_per_table(h->cfg) + (i < 4 ? i : 4 * h->cfg.layers)];
         add(" %s rows %d ksplit %d kb %d units %d;", names[i], ph.rows, ph.ksplit, ph.kb, ph.nunits);
+      }
+      add("\n");
+    }
+    for (int cls = 0; h->use3d && cls < prompt_classes(h->cfg, h->grid); ++cls) {
+      add("prompt class %d:", cls);
+      for (int i = 0; i < kPromptPhases; ++i) {
+        const PromptPhase& ph = h->prompt[cls][i];
+        add(" %s rows %d ksplit %d tiles %d;", names[i], ph.rows, ph.ksplit, ph.tile_start[3]);
       }
       add("\n");
     }

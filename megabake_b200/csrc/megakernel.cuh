@@ -20,10 +20,7 @@ constexpr int kRingGranules = 120;       // keeps the CTA under 196 KiB of share
 constexpr int kRingBytes = kRingGranules * kGranule;
 constexpr int kChunkBars = 128;          // full/empty barrier pairs, indexed by chunk sequence number
 constexpr int kTok = MK_TOKEN_TILE;      // token columns an epilogue step reads from TMEM
-constexpr int kMaxTok = 128;             // largest token tile (UMMA N is 16, 32, 64 or 128) ...
-constexpr int kSpreadTok = 256;          // ... but for prompts of more tokens (see spread): operands are read from L2, and fewer bytes per product
-// Those read both operands from L2, several chunks of each in flight: the activation ring takes a part of the weight ring.
-constexpr int kSpreadRingGranules = 88;
+constexpr int kMaxTok = 128;             // largest token tile (UMMA N is 16, 32, 64 or 128)
 constexpr int kBSlots = 32;              // activation K-chunks resident per CTA (two halves of 16)
 constexpr int kBHalf = kBSlots / 2;
 constexpr int kBSlotBytes = kTok * 128;  // 2 KiB
@@ -65,7 +62,7 @@ constexpr int kTpFlagBytes = 256;        // head of a rank's exchange buffer: on
 // phase adds them, in slice order, while it builds its activation operand.
 struct GemmPhase {
   const CUtensorMap* tmap[3];  // device copies of the weights' TMA descriptors (tensor engine: box = 64 x rows x kb chunks)
-  const CUtensorMap* bmap[5];  // descriptors of the token operand for token tiles of 16, 32, 64, 128, 256 (box = 64 x tile x kb chunks)
+  const CUtensorMap* bmap[4];  // descriptors of the token operand for token tiles of 16, 32, 64, 128 (box = 64 x tile x kb chunks)
   const bf16* w[3];            // raw weight pointers [N, K]
   const bf16* bias[3];
   int n[3];                    // rows of each matrix
@@ -99,6 +96,7 @@ struct Control {
   uint32_t abort;     // set once by whoever gives up a wait; every wait polls it
   int status;         // mk_device_status
   int where, cta, detail;
+  int prompt_refused; // the prompt pass under way met a bad id or position: its logits are NaN
   uint32_t pad;       // mk_kv_attention, mk_kv_attention_static: 1 if the first launch refused the valid length
 };
 
@@ -120,7 +118,6 @@ struct KParams {
   int qkv_ld;
   int max_positions;
   int stream_once;    // 1: weights are read once per launch (L2 evict-first)
-  int spread;         // 1: prompts of several token tiles: every (row tile, K slice, token tile) is a unit of its own
   int split;          // 1: this launch runs the split-K phase table (residual updates applied by the consumer)
   int ragged;         // 1: len[l] points to one valid length per sequence (int32 [batch]) instead of one shared by the batch
   int sample;         // 1: after the logits, pick each sequence's greedy token on the device, store it in tokens_out and as the

@@ -1,0 +1,203 @@
+// Launches of the prompt kernels (prompt_kernels.cuh).
+#include "prompt_kernels.cuh"
+
+namespace mk {
+namespace {
+
+// A launch that may begin while the kernel before it in the stream is still at work (`dependent`), its blocks in clusters of
+// `cluster`.
+template <typename... Params, typename... Args>
+cudaError_t launch(void (*kernel)(Params...), int blocks, int threads, int smem, int cluster, bool dependent, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attributes[2];
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = attributes;
+  if (dependent) {
+    attributes[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attributes[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attributes[config.numAttrs].val.clusterDim.x = cluster;
+    attributes[config.numAttrs].val.clusterDim.y = attributes[config.numAttrs].val.clusterDim.z = 1;
+    ++config.numAttrs;
+  }
+  return cudaLaunchKernelEx(&config, kernel, args...);
+}
+
+template <int EPI>
+cudaError_t launch_gemm(const PromptGemm& g, int cls, int grid, cudaStream_t stream) {
+  if (cls > 0)
+    return launch(prompt_gemm<2, kPromptRow, EPI>, 2 * std::min(g.units, grid / 2), kPromptThreads, kPromptSmem, 2, true, stream, g);
+  const int blocks = std::min(g.units, grid);
+  if (g.m <= 64) return launch(prompt_gemm<1, 64, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);
+  return launch(prompt_gemm<1, kPromptRow, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);
+}
+
+template <int EPI>
+cudaError_t prepare_gemm() {
+  cudaError_t e = cudaFuncSetAttribute(prompt_gemm<2, kPromptRow, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_gemm<1, kPromptRow, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_gemm<1, 64, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
+  return e;
+}
+
+cudaError_t launch_norm(const PromptNorm& n, int blocks, bool dependent, cudaStream_t stream) {
+  const int nvec = n.k / 8, threads = std::min(256, (nvec + 31) / 32 * 32);
+  if (nvec <= threads) return launch(prompt_norm<1>, blocks, threads, 0, 1, dependent, stream, n);
+  if (nvec <= 2 * threads) return launch(prompt_norm<2>, blocks, threads, 0, 1, dependent, stream, n);
+  return launch(prompt_norm<4>, blocks, threads, 0, 1, dependent, stream, n);  // (hidden up to 8192: check_config)
+}
+
+}  // namespace
+
+cudaError_t prompt_prepare() {
+  cudaError_t e = prepare_gemm<PE_QKV>();
+  if (e == cudaSuccess) e = prepare_gemm<PE_PARTIAL>();
+  if (e == cudaSuccess) e = prepare_gemm<PE_SILU>();
+  if (e == cudaSuccess) e = prepare_gemm<PE_LOGITS>();
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem);
+  return e;
+}
+
+cudaError_t prompt_attention_launch(const AttnArgs& args, int head_dim, int q_heads, int kv_heads, int batch, int units, int blocks,
+                                    bool dependent, cudaStream_t stream) {
+  if (head_dim == 64)
+    return launch(prompt_attention<64>, blocks, kWorkers, PromptLaunch<64>::kSmem, 1, dependent, stream, args, q_heads, kv_heads, batch, units);
+  return launch(prompt_attention<128>, blocks, kWorkers, PromptLaunch<128>::kSmem, 1, dependent, stream, args, q_heads, kv_heads, batch, units);
+}
+
+cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
+  const mk_config& c = *pass.config;
+  const int cls = pass.cls, m = pass.m, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const int per_tile = cls > 0 ? 2 * kPromptRow : (m <= 64 ? 64 : kPromptRow), rows_per_cta = cls > 0 ? kPromptRow : per_tile;
+  // the token operand's box: the smallest that holds the launch, a CTA's rows otherwise
+  const int box = m <= 16 ? 0 : (m <= 32 ? 1 : (m <= 64 ? 2 : 3)), box_rows = 16 << box;
+  auto gemm = [&](int kind, int operand) {
+    const PromptPhase& p = pass.phases[kind];
+    PromptGemm g{};
+    g.guard = pass.guard;
+    // Up to 64 tokens a chunk's MMAs take less than a step of the pipeline: two chunks to a stage.
+    g.kb = m <= 64 && p.kslice % 2 == 0 ? 2 : 1;
+    g.a = pass.operands + (operand * kOperandTiles + box) * kOperandChunks + g.kb - 1;
+    for (int s = 0; s < 3; ++s) g.n[s] = p.n[s];
+    for (int s = 0; s < 4; ++s) g.tile_start[s] = p.tile_start[s];
+    g.m = m;
+    g.rows = p.rows;
+    g.nmat = p.nmat;
+    g.ksplit = p.ksplit;
+    g.kslice = p.kslice;
+    g.token_tiles = (m + per_tile - 1) / per_tile;
+    g.units = p.tile_start[3] * p.ksplit * g.token_tiles;
+    g.a_bytes = box_rows * 128;
+    g.b_bytes = prompt_box_rows(p, cls) * 128;
+    g.stage_bytes = g.kb * (g.a_bytes + p.nmat * g.b_bytes);
+    // an MMA reads a CTA's full rows of tokens, past a smaller box whatever lies there: room for that behind the last stage
+    const int room = kPromptSmem - 1024 - rows_per_cta * 128;
+    g.stages = std::min(kPromptStages, room / g.stage_bytes);  // (at least two: a stage is 48 KB at most)
+    const bool joined = p.nmat == 2 && cls == 0;  // gate and up as one MMA of twice the rows
+    g.instr_n = ((joined ? 2 * p.rows : p.rows) + 15) / 16 * 16;  // (a tile may end within an MMA's N: columns nobody reads)
+    g.up_column = joined ? p.rows : 256;
+    g.buffers = p.nmat == 2 && !joined ? 1 : 2;
+    g.head_dim = c.head_dim;
+    g.max_positions = c.max_positions;
+    g.stream_weights = g.token_tiles == 1;
+    return g;
+  };
+  const mk_weights& w = *pass.weights;
+  PromptNorm norm{};
+  norm.guard = pass.guard;
+  norm.embed = static_cast<const bf16*>(w.embed);
+  norm.ids = pass.ids;
+  norm.pos = pass.pos;
+  norm.partial = pass.partial;
+  norm.xnorm = pass.xnorm;
+  norm.m = m;
+  norm.k = c.hidden;
+  norm.embed_rows = c.embed_rows > 0 ? c.embed_rows : c.vocab;
+  norm.max_positions = c.max_positions;
+  norm.eps = c.rms_eps;
+  AttnArgs A{};
+  A.q = pass.qkv;
+  A.q_ld = A.kv_ld = q_size + 2 * kv_size;
+  A.q_bstride = A.kv_bstride = static_cast<long long>(pass.seq) * A.q_ld;
+  A.k = pass.qkv + q_size;
+  A.v = A.k + kv_size;
+  A.out = pass.attn;
+  A.out_bstride = static_cast<long long>(pass.seq) * q_size;
+  A.out_tstride = q_size;
+  A.out_hstride = c.head_dim;
+  A.mask = pass.mask;
+  A.sq = A.klen = pass.seq;
+  A.causal = pass.mask == nullptr;
+  A.scale = pass.att_scale;
+  const int units = pass.batch * c.q_heads * ((pass.seq + kPromptQueries - 1) / kPromptQueries);
+  const int blocks = c.sm_limit > 0 ? std::min(units, pass.grid) : units, rows = c.sm_limit > 0 ? std::min(m, pass.grid) : m;
+  cudaError_t e = cudaSuccess;
+  for (int l = 0; l <= c.layers && e == cudaSuccess; ++l) {
+    const bool head = l == c.layers;
+    const CUtensorMap* maps = pass.maps + 7 * static_cast<size_t>(l);
+    // the residual stream: embedding rows, then down_proj's sums on hidden_a; it goes to hidden_b
+    norm.src = l == 0 ? nullptr : pass.hidden_a;
+    norm.parts = l == 0 ? 0 : pass.phases[PP_DOWN].ksplit;
+    norm.weight = static_cast<const bf16*>(head ? w.final_norm : w.layers[l].input_norm);
+    norm.h_out = head ? nullptr : pass.hidden_b;
+    norm.check = l == 0;
+    e = launch_norm(norm, rows, l > 0, stream);
+    norm.check = 0;
+    if (e != cudaSuccess) return e;
+    if (head) {
+      PromptGemm g = gemm(PP_HEAD, kOperandXnorm);
+      g.b[0] = maps;
+      g.dst = pass.logits;
+      g.ld = c.vocab;
+      return launch_gemm<PE_LOGITS>(g, cls, pass.grid, stream);
+    }
+    const mk_layer_weights& lw = w.layers[l];
+    PromptGemm g = gemm(PP_QKV, kOperandXnorm);
+    const void* biases[3] = {lw.q_bias, lw.k_bias, lw.v_bias};
+    for (int s = 0; s < 3; ++s) {
+      g.b[s] = maps + s;
+      g.bias[s] = c.qkv_bias ? static_cast<const bf16*>(biases[s]) : nullptr;
+    }
+    g.out_col[1] = q_size;
+    g.out_col[2] = q_size + kv_size;
+    g.dst = pass.qkv;
+    g.ld = A.q_ld;
+    g.cos_t = static_cast<const bf16*>(w.rope_cos);
+    g.sin_t = static_cast<const bf16*>(w.rope_sin);
+    g.pos = pass.pos;
+    e = launch_gemm<PE_QKV>(g, cls, pass.grid, stream);
+    if (e == cudaSuccess) e = prompt_attention_launch(A, c.head_dim, c.q_heads, c.kv_heads, pass.batch, units, blocks, true, stream);
+    if (e != cudaSuccess) return e;
+    g = gemm(PP_O, kOperandAttn);
+    g.b[0] = maps + 3;
+    g.partial = pass.partial;
+    e = launch_gemm<PE_PARTIAL>(g, cls, pass.grid, stream);
+    if (e != cudaSuccess) return e;
+    norm.src = pass.hidden_b;
+    norm.parts = pass.phases[PP_O].ksplit;
+    norm.weight = static_cast<const bf16*>(lw.post_norm);
+    norm.h_out = pass.hidden_a;
+    e = launch_norm(norm, rows, true, stream);
+    if (e != cudaSuccess) return e;
+    g = gemm(PP_GU, kOperandXnorm);
+    g.b[0] = maps + 4;
+    g.b[1] = maps + 5;
+    g.dst = pass.act;
+    g.ld = c.intermediate;
+    e = launch_gemm<PE_SILU>(g, cls, pass.grid, stream);
+    if (e != cudaSuccess) return e;
+    g = gemm(PP_DOWN, kOperandAct);
+    g.b[0] = maps + 6;
+    g.partial = pass.partial;
+    e = launch_gemm<PE_PARTIAL>(g, cls, pass.grid, stream);
+  }
+  return e;
+}
+
+}  // namespace mk

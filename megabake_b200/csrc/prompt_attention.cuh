@@ -53,6 +53,16 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
   return r;
 }
 
+__device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+// Programmatic dependent launch: what the kernels before this one have written is there; the kernels behind it may come.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t ldcg_u32(const void* ptr) { return __ldcg(reinterpret_cast<const unsigned int*>(ptr)); }
 
 template <int HD> constexpr int kPromptPitch = HD * 2 + 16;  // bytes per tile row: 16 bytes of padding keep fragment loads conflict-free
@@ -277,6 +287,8 @@ prompt_attention(const __grid_constant__ AttnArgs A, int q_heads, int kv_heads, 
   extern __shared__ __align__(128) uint8_t prompt_smem[];
   constexpr int kStages = PromptLaunch<HD>::kStages;
   float* const sums = reinterpret_cast<float*>(prompt_smem + kStages * kPromptStage<HD>);
+  grid_dependents_go();
+  grid_dependency_wait();
 #pragma unroll 1
   for (int i = blockIdx.x; i < units; i += gridDim.x)  // one, unless the handle limits its SMs
     prompt_unit<HD, kStages>(A, q_heads, kv_heads, batch, i, smem_u32(prompt_smem), sums, threadIdx.x);

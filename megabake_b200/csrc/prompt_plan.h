@@ -1,0 +1,176 @@
+// How a prompt pass cuts its projections (host side, pure functions of the configuration and the token count) and the
+// parameter blocks of its kernels (prompt_kernels.cuh).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "megakernel.cuh"
+
+namespace mk {
+
+enum { PP_QKV = 0, PP_O = 1, PP_GU = 2, PP_DOWN = 3, PP_HEAD = 4, kPromptPhases = 5 };
+
+// Launch classes.  Up to 128 tokens a prompt is bound by reading the weights: one CTA per tile, and tiles that give every SM
+// some.  Beyond, by tensor cores and L2: CTA pairs (256 tokens each), and tiles chosen for one, two, or three and more of
+// those.
+constexpr int kPromptClasses = 4;
+constexpr int kPromptRow = 128;   // token rows per CTA (64 rows are used for up to 64 tokens)
+constexpr int kPromptStages = 16; // most stages of a pipeline
+// Shared memory of a projection's CTA: one per SM, whose first stages travel while the kernels before it end.  (With two to an
+// SM, so that they could travel while another projection is at work, CTAs that start early crowd on the SMs that are free first:
+// 64 tokens of the 1.7B shape 1442 us against 1345.)
+constexpr int kPromptSmem = 225 * 1024;
+
+// Token-operand descriptors, shared with the tensor engine: (normalised rows, attention output, SiLU * up) x (boxes of 16, 32,
+// 64, 128 tokens) x (1 to 4 K chunks).
+constexpr int kOperandTiles = 4, kOperandChunks = 4, kOperandKinds = 3;
+enum { kOperandXnorm = 0, kOperandAttn = 1, kOperandAct = 2 };
+
+inline int prompt_class(int tokens, int grid) {
+  return tokens <= kPromptRow || grid < 2 ? 0 : std::min(3, (tokens + 2 * kPromptRow - 1) / (2 * kPromptRow));
+}
+
+// One projection, the same for every layer of a class.
+struct PromptPhase {
+  int k, kc;             // reduction length, in elements and in 64-element chunks
+  int nseg, nmat;        // matrices side by side along the output (q, k, v); matrices of a tile (gate and up: two)
+  int n[3];              // rows of each
+  int rows;              // weight rows of a tile (of each of its matrices)
+  int tile_start[4];     // first tile of each segment, then the total
+  int ksplit, kslice;    // K slices, and chunks per slice
+};
+
+inline void prompt_tiles(PromptPhase& p, int rows) {
+  p.rows = rows;
+  int tiles = 0;
+  for (int s = 0; s < p.nseg; ++s) {
+    p.tile_start[s] = tiles;
+    tiles += (p.n[s] + rows - 1) / rows;
+  }
+  for (int s = p.nseg; s < 4; ++s) p.tile_start[s] = tiles;
+}
+
+// The five projections of a class.  `grid`: SMs to use.
+inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* out) {
+  const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const int ks[kPromptPhases] = {c.hidden, q_size, c.hidden, c.intermediate, c.hidden};
+  const int ns[kPromptPhases] = {q_size, c.hidden, c.intermediate, c.hidden, c.vocab};
+  for (int i = 0; i < kPromptPhases; ++i) {
+    PromptPhase p{};
+    p.k = ks[i];
+    p.kc = ks[i] / kChunkK;
+    p.nseg = i == PP_QKV ? 3 : 1;
+    p.nmat = i == PP_GU ? 2 : 1;
+    p.n[0] = ns[i];
+    if (i == PP_QKV) p.n[1] = p.n[2] = kv_size;
+    const bool wide = cls > 0, may_split = i == PP_O || i == PP_DOWN;
+    // A tile of q or k rows is whole heads: its epilogue rotates pairs half a head apart.  Elsewhere the MMA's N decides for a
+    // pair (multiples of 32), the logits' 32-byte stores, the swizzle's eight rows otherwise.
+    const int step = i == PP_QKV ? c.head_dim : (wide ? 32 : (i == PP_HEAD ? 16 : 8));
+    const int most = wide ? 256 : 128 / p.nmat;
+    long long best = -1;
+    PromptPhase chosen = p;
+    for (int split = 1; split <= (may_split ? kMaxSplit : 1); ++split) {
+      if (p.kc % split) continue;
+      for (int rows = most / step * step; rows >= step; rows -= step) {
+        PromptPhase t = p;
+        prompt_tiles(t, rows);
+        t.ksplit = split;
+        t.kslice = p.kc / split;
+        long long cost;
+        if (wide) {
+          // per chunk: the MMAs (an N = 256 one of a pair takes 128 cycles) or the operands out of L2 at 44 bytes per cycle
+          // and SM; plus what a unit costs besides, its epilogue included
+          const long long units = static_cast<long long>(t.tile_start[3]) * split * cls, pairs = std::max(1, grid / 2);
+          const long long chunk = std::max<long long>(2 * p.nmat * rows, (kPromptRow + p.nmat * rows / 2) * 128 / 44);
+          cost = (units + pairs - 1) / pairs * (t.kslice * chunk + 2000 + 8 * rows) + split * 600;
+        } else {
+          // per chunk of the busiest SM: its weights at 30 bytes per cycle, weights and (64) tokens at 42, or the pipeline's step
+          const long long units = static_cast<long long>(t.tile_start[3]) * split;
+          const long long chunk = std::max({p.nmat * rows * 128 / 30, (64 + p.nmat * rows) * 128 / 42, 256});
+          cost = (units + grid - 1) / grid * (t.kslice * chunk + 2500) + split * 300;
+        }
+        if (best < 0 || cost < best) {
+          best = cost;
+          chosen = t;
+        }
+      }
+    }
+    out[i] = chosen;
+  }
+}
+
+// Rows of the weight descriptors' boxes: a CTA of a pair brings half a tile.
+inline int prompt_box_rows(const PromptPhase& p, int cls) { return cls > 0 ? p.rows / 2 : p.rows; }
+
+// ---------------------------------------------------------------------------
+// kernel parameters
+
+// What bounds the kernels' waits and where a verdict goes.
+struct PromptGuard {
+  Control* ctrl;
+  volatile int* status_mirror;
+  long long timeout_cycles;
+};
+
+struct PromptGemm {
+  PromptGuard guard;
+  const CUtensorMap* a;     // token operand: box of 64 x tokens x kb
+  const CUtensorMap* b[3];  // weights: q, k, v, or gate, up, or the only one; box of 64 x (rows or rows / 2)
+  const bf16* bias[3];
+  bf16* dst;                // + token * ld + column
+  float* partial;           // cut projections: [slice][token][n]
+  const bf16 *cos_t, *sin_t;
+  const long long* pos;
+  int n[3], tile_start[4], out_col[3];
+  int m, ld, rows, nmat;
+  int ksplit, kslice;
+  int token_tiles, units;
+  int kb;                                     // K chunks per stage
+  int stages, a_bytes, b_bytes, stage_bytes;  // per CTA: a chunk's tokens, a chunk's weights of one matrix, and a whole stage
+  int instr_n;                                // N of an MMA
+  int up_column;                              // gate and up: where the up accumulator begins
+  int buffers;                                // accumulator buffers in tensor memory, 256 columns each
+  int head_dim, max_positions;
+  int stream_weights;                         // weights are read once
+};
+
+struct PromptNorm {
+  PromptGuard guard;
+  const bf16* src;       // residual stream, or null: embedding rows of the token ids
+  const bf16* embed;
+  const long long *ids, *pos;
+  const float* partial;  // [parts][m][k]: the previous projection's K slices
+  const bf16* weight;
+  bf16 *h_out, *xnorm;
+  int m, k, parts;
+  int embed_rows, max_positions, check;  // check: the first kernel of a pass looks at every id and position
+  float eps;
+};
+
+// One prompt pass: everything its launches are made from.
+struct PromptPass {
+  const mk_config* config;
+  const mk_weights* weights;
+  const PromptPhase* phases;    // of the class
+  int cls, grid;
+  const CUtensorMap* maps;      // of the class: 7 per layer, then the output head
+  const CUtensorMap* operands;  // [kind][token tile][chunks - 1], as the tensor engine's
+  bf16 *hidden_a, *hidden_b, *xnorm, *qkv, *attn, *act;
+  float* partial;
+  const long long *ids, *pos;
+  const bf16* mask;
+  bf16* logits;
+  int m, batch, seq;
+  float att_scale;
+  PromptGuard guard;
+};
+
+struct AttnArgs;
+cudaError_t prompt_prepare();  // shared-memory attributes of the kernels, on the current device
+cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream);
+cudaError_t prompt_attention_launch(const AttnArgs& args, int head_dim, int q_heads, int kv_heads, int batch, int units, int blocks,
+                                    bool dependent, cudaStream_t stream);
+
+}  // namespace mk

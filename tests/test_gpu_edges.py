@@ -101,6 +101,75 @@ def test_prompts_at_token_tile_edges(device, tokens, head_dim):
     assert_parity(logits, expected, f"prompt of {tokens}")
 
 
+@pytest.mark.parametrize("batch,sequence", [(1, 1), (3, 7), (2, 33), (5, 25), (3, 61), (4, 129)])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_prompts_with_biases_masks_and_buffers_on_any_element(device, batch, sequence, head_dim):
+    """Every kind of launch (tiles of 64 and 128 tokens, one and more tiles of a CTA pair) with several sequences, a mask,
+    projections with biases that begin at an odd element, a vocabulary that ends inside a tile and logits at an odd element."""
+    from megabake_b200 import _native
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=192, q_heads=6, kv_heads=2, head_dim=head_dim, intermediate=320, vocab=333, rope_style="hf",
+                         qkv_bias=True)
+    weights = dict(synth_weights(config, seed=21, norm_std=0.1, device=device))
+    for name, tensor in weights.items():
+        if name.endswith("proj.bias"):
+            off = torch.empty(tensor.numel() + 1, dtype=tensor.dtype, device=device)[1:]
+            weights[name] = off.copy_(tensor)
+    tokens = batch * sequence
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=max(sequence, 16))
+    ids = synth_ids(tokens, config.vocab, seed=22).view(batch, sequence).to(device)
+    positions = torch.arange(sequence, device=device).expand(batch, sequence).contiguous()
+    mask = oracle.causal_mask(batch, sequence).to(device).contiguous()
+    mask[:, :, :, : sequence // 3] = torch.finfo(torch.bfloat16).min
+    mask[:, :, :, 0] = 0.0  # every row sees something
+    with torch.no_grad():
+        expected = oracle.prefill(config, weights, rope_tables(config, max(sequence, 16), device=device), ids, positions, mask)
+    assert_parity(kernel.prefill(ids, positions, mask), expected, "logits")
+    store = torch.empty(tokens * config.vocab + 2, dtype=torch.bfloat16, device=device).fill_(7.0)
+    _native.check("mk_prefill", kernel.lib.mk_prefill(kernel._handle, ids.data_ptr(), positions.data_ptr(), mask.data_ptr(), batch,
+                                                      sequence, store[1:].data_ptr(), torch.cuda.current_stream().cuda_stream))
+    kernel.check()
+    assert_parity(store[1:-1].view(batch, sequence, -1), expected, "logits at an odd element")
+    assert store[0].item() == 7.0 and store[-1].item() == 7.0
+
+
+@pytest.mark.parametrize("tokens", [40, 200])
+def test_a_refused_prompt_is_all_nan_and_the_next_one_is_not(device, tokens):
+    config = tiny_config(hidden=192, intermediate=320, rope_style="hf")
+    weights = synth_weights(config, seed=23, device=device)
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=tokens)
+    ids = synth_ids(tokens, config.vocab, seed=23).view(1, tokens).to(device)
+    fine = kernel.prefill(ids)
+    kernel.check()
+    for bad_ids, bad_position in ((config.vocab, tokens - 1), (-1, 0), (0, tokens)):
+        wrong, positions = ids.clone(), torch.arange(tokens, device=device).view(1, tokens).clone()
+        wrong[0, tokens // 2] = bad_ids
+        positions[0, -1] = bad_position
+        logits = kernel.prefill(wrong, positions)
+        assert kernel.status()["status"] == "BAD_INDEX" and torch.isnan(logits).all()
+        assert torch.equal(kernel.prefill(ids), fine)
+        kernel.check()
+
+
+@pytest.mark.parametrize("sm_limit", [1, 7])
+@pytest.mark.parametrize("tokens", [50, 300])
+def test_prompts_on_few_sms(device, sm_limit, tokens):
+    """Many units to a CTA: both accumulator buffers and every slot of the pipeline come around several times."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=512, q_heads=6, kv_heads=2, intermediate=832, vocab=1003, rope_style="hf")
+    weights = synth_weights(config, seed=24, norm_std=0.1, device=device)
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=tokens, sm_limit=sm_limit)
+    ids = synth_ids(tokens, config.vocab, seed=24).view(1, tokens).to(device)
+    positions = torch.arange(tokens, device=device).view(1, tokens)
+    with torch.no_grad():
+        expected = oracle.prefill(config, weights, rope_tables(config, tokens, device=device), ids, positions,
+                                  oracle.causal_mask(1, tokens).to(device))
+    assert_parity(kernel.prefill(ids), expected, f"prompt of {tokens} on {sm_limit}")
+    kernel.check()
+
+
 def test_gates_beyond_the_straight_line_of_the_silu(device):
     """Gates past +-80 take the epilogue's plain division, their neighbours in a token's column the corrected quotient."""
     from oracle import decoder_oracle as oracle
