@@ -1,4 +1,5 @@
-"""Build libmegabake_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Build libmegabake_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and beside it the small
+library that puts the two ops' common case under PyTorch's dispatcher.
 
     python -m megabake_b200.build [--force]
 """
@@ -15,6 +16,8 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libmegabake_b200.so"
 SOURCES = sorted(CSRC.glob("*.cu"))
+OPS_LIBRARY = PACKAGE / "libmegabake_b200_ops.so"
+OPS_SOURCE = CSRC / "torch_ops.cpp"
 
 
 def headers() -> list[Path]:
@@ -56,5 +59,26 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIBRARY
 
 
+def build_ops(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the ops' C++ registration against the installed PyTorch if it is missing or older than its sources."""
+    sources = [OPS_SOURCE, PACKAGE.parent / "include" / "megabake_b200.h"]
+    if not force and OPS_LIBRARY.exists() and all(path.stat().st_mtime <= OPS_LIBRARY.stat().st_mtime for path in sources):
+        return OPS_LIBRARY
+    import torch
+    from torch.utils import cpp_extension
+
+    command = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-o", str(OPS_LIBRARY), str(OPS_SOURCE),
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+               *(f"-isystem{path}" for path in cpp_extension.include_paths(device_type="cuda")),
+               *(f"-L{path}" for path in cpp_extension.library_paths(device_type="cuda")), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-lcudart"]
+    result = subprocess.run(command, capture_output=True, text=True)
+    if verbose or result.returncode:
+        sys.stderr.write(result.stdout + result.stderr)
+    if result.returncode:
+        raise RuntimeError(f"{command[0]} failed with exit code {result.returncode}")
+    return OPS_LIBRARY
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose=True))
+    print(build_ops(force="--force" in sys.argv, verbose=True))

@@ -121,7 +121,7 @@ class DecoderKernel:
 
     # ------------------------------------------------------------------ helpers
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return torch._C._cuda_getCurrentRawStream(self.device.index)
 
     def _on_device(self):
         """The handle's device as the current one; most callers have made it that already."""
@@ -532,6 +532,7 @@ class AttentionKernels:
             if found is None or found.max_tokens < tokens:
                 capacity = max(16, 1 << (max(tokens, 1) - 1).bit_length())
                 found = cls(q_heads, kv_heads, head_dim, capacity, device)
+                _native.register_ops(*key, capacity, found._handle, found._mirror.data_ptr())
                 cls._cache[key] = found
         return found
 

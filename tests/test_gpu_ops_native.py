@@ -1,0 +1,99 @@
+"""The two ops through their native registration against the same calls through the Python one, which inference mode takes."""
+
+import pytest
+import torch
+
+from megabake_b200 import CompilerError, ops  # noqa: F401
+from megabake_b200.synth import synth_normal
+
+pytestmark = pytest.mark.gpu
+DEVICE = torch.device("cuda:0")
+
+
+def _tensor(name, *shape):
+    return synth_normal(shape, seed=31, name=name, std=1.0, device=DEVICE)
+
+
+def _kv_case(batch, heads, kv_heads, dim, filled, capacity, strided):
+    def vector(name, n):
+        if strided:  # as a model hands them over: [batch, heads, 1, dim], transposed
+            return _tensor(name, batch, n, 1, dim).transpose(1, 2)
+        return _tensor(name, batch, 1, n, dim)
+    caches = [_tensor(name, batch, capacity, kv_heads, dim) for name in ("kc", "vc")]
+    return [vector("q", heads), vector("k", kv_heads), vector("v", kv_heads), *caches,
+            torch.full((1,), filled, dtype=torch.int32, device=DEVICE)]
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 4, 64, 0, 1), (3, 8, 2, 128, 17, 40), (20, 9, 3, 64, 300, 301)])
+@pytest.mark.parametrize("strided", [False, True])
+def test_decode_op_is_the_same_on_both_routes(shape, strided):
+    for _ in range(2):  # the first call makes the handle, on the Python route in any case
+        mine, theirs = _kv_case(*shape, strided), _kv_case(*shape, strided)
+        versions = [t._version for t in mine]
+        out = torch.ops.megabake.kv_attention(*mine)
+        with torch.inference_mode():
+            expected = torch.ops.megabake.kv_attention(*theirs)
+        assert torch.equal(out, expected) and all(torch.equal(a, b) for a, b in zip(mine, theirs))
+        assert [t._version - v for t, v in zip(mine, versions)] == [0, 0, 0, 1, 1, 1]
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 4, 64, 1, 1), (2, 8, 2, 128, 65, 130), (40, 9, 3, 64, 33, 33)])
+@pytest.mark.parametrize("mask", [None, "plain", "expanded", "float"])
+def test_prompt_op_is_the_same_on_both_routes(shape, mask):
+    batch, heads, kv_heads, dim, queries, keys = shape
+    q, k, v = _tensor("q", batch, queries, heads, dim), _tensor("k", batch, keys, kv_heads, dim), _tensor("v", batch, keys, kv_heads, dim)
+    m = None if mask is None else _tensor("m", 1 if mask == "expanded" else batch, 1, queries, keys)
+    m = m.expand(batch, 1, queries, keys) if mask == "expanded" else (m.float() if mask == "float" else m)
+    for _ in range(2):
+        out = torch.ops.megabake.attention(q, k, v, m, dim ** -0.5)
+        with torch.inference_mode():
+            expected = torch.ops.megabake.attention(q, k, v, m, dim ** -0.5)
+        assert torch.equal(out, expected)
+
+
+def test_what_the_ops_refuse_is_refused_on_both_routes():
+    good = _kv_case(2, 4, 2, 64, 3, 8, False)
+    torch.ops.megabake.kv_attention(*good)
+    for index, wrong in ((0, good[0].half()), (0, good[0].expand(2, 1, 4, 64).repeat(1, 2, 1, 1)), (3, good[3].transpose(0, 1)),
+                         (5, good[5].long())):
+        args = list(good)
+        args[index] = wrong
+        errors = []
+        for mode in (torch.no_grad(), torch.inference_mode()):
+            with mode, pytest.raises(Exception) as caught:
+                torch.ops.megabake.kv_attention(*args)
+            errors.append((type(caught.value), str(caught.value)))
+        assert errors[0] == errors[1]
+    full = _kv_case(2, 4, 2, 64, 8, 8, False)
+    assert torch.isnan(torch.ops.megabake.kv_attention(*full)).all()
+    torch.cuda.synchronize()
+    with pytest.raises(CompilerError, match="state-capacity|exceeds capacity"):
+        torch.ops.megabake.kv_attention(*_kv_case(2, 4, 2, 64, 3, 8, False))
+
+
+def test_a_result_that_wants_a_gradient_says_that_there_is_none():
+    args = _kv_case(2, 4, 2, 64, 3, 8, False)
+    args[0].requires_grad_(True)
+    prompt = [_tensor(name, 1, 8, 4, 64).requires_grad_(True) for name in ("a", "b", "c")]
+    for out in (torch.ops.megabake.kv_attention(*args), torch.ops.megabake.attention(*prompt, None, 0.125)):
+        assert out.requires_grad
+        with pytest.raises(RuntimeError, match="no autograd formula was registered"):
+            out.float().sum().backward()
+
+
+def test_decode_op_in_a_captured_graph_and_on_two_streams():
+    expected = torch.ops.megabake.kv_attention(*_kv_case(3, 8, 2, 128, 17, 40, False))
+    args, start = _kv_case(3, 8, 2, 128, 17, 40, False), torch.full((1,), 17, dtype=torch.int32, device=DEVICE)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert torch.equal(torch.ops.megabake.kv_attention(*args), expected)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        args[5].copy_(start)
+        out = torch.ops.megabake.kv_attention(*args)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, expected)
