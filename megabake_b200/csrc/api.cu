@@ -17,6 +17,7 @@
 
 #include "decoder_kernel.cuh"
 #include "kv_attention.cuh"
+#include "prompt_attention_tc.cuh"
 #include "prompt_plan.h"
 #include "stream_plan.h"
 
@@ -276,6 +277,29 @@ int encode_cache_map(CUtensorMap* out, const void* base, int batch, int capacity
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled (cache) failed with %d", (int)r);
   return MK_OK;
+}
+
+// Prompt attention: rows of `heads` x head_dim elements, `rows` to a sequence, seen as (64 elements, rows, chunks of all heads,
+// sequences); a box is `box_rows` rows of one head.
+int encode_attention_map(CUtensorMap* out, const void* base, int batch, int rows, int heads, int head_dim, long long ld, long long batch_stride, int box_rows) {
+  auto fn = encode_fn();
+  if (!fn) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint32_t chunks = static_cast<cuuint32_t>(head_dim / kChunkK);
+  const cuuint64_t dims[4] = {static_cast<cuuint64_t>(kChunkK), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(heads) * chunks,
+                              static_cast<cuuint64_t>(batch)};
+  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(kChunkK) * 2, static_cast<cuuint64_t>(batch_stride) * 2};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(kChunkK), static_cast<cuuint32_t>(box_rows), chunks, 1};
+  const cuuint32_t elem[4] = {1, 1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled (attention) failed with %d", (int)r);
+  return MK_OK;
+}
+int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, int batch, int q_heads, int kv_heads, int head_dim) {
+  maps->q_ok = (reinterpret_cast<uintptr_t>(A.q) & 15) == 0;
+  if (int e = encode_attention_map(&maps->k, A.k, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
+  if (int e = encode_attention_map(&maps->v, A.v, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
+  return maps->q_ok ? encode_attention_map(&maps->q, A.q, batch, A.sq, q_heads, head_dim, A.q_ld, A.q_bstride, kAttnQueries) : MK_OK;
 }
 
 }  // namespace
@@ -1078,8 +1102,19 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
     pass.mask = static_cast<const bf16*>(mask);
     pass.logits = static_cast<bf16*>(logits);
     pass.m = static_cast<int>(m); pass.batch = batch; pass.seq = sequence;
-    pass.att_scale = h->att_scale;
     pass.guard = {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles};
+    const mk_config& c = h->cfg;
+    const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+    AttnArgs A{};
+    A.q = pass.qkv; A.q_ld = A.kv_ld = q_size + 2 * kv_size;
+    A.q_bstride = A.kv_bstride = static_cast<long long>(sequence) * A.q_ld;
+    A.k = pass.qkv + q_size; A.v = A.k + kv_size;
+    A.out = pass.attn; A.out_bstride = static_cast<long long>(sequence) * q_size; A.out_tstride = q_size; A.out_hstride = c.head_dim;
+    A.mask = pass.mask; A.sq = A.klen = sequence; A.causal = pass.mask == nullptr; A.scale = h->att_scale;
+    AttnTcMaps maps{};
+    if (int e = encode_attention_maps(&maps, A, batch, c.q_heads, c.kv_heads, c.head_dim)) return e;
+    pass.attention = &A;
+    pass.attention_maps = &maps;
     MK_CUDA(prompt_forward(pass, static_cast<cudaStream_t>(stream)));
     h->launches += 7 * L + 2;
     return MK_OK;
@@ -1209,9 +1244,10 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   A.mask = static_cast<const bf16*>(mask); A.sq = q_len; A.klen = k_len; A.scale = scale;
   const long long units = static_cast<long long>(batch) * h->cfg.q_heads * ((q_len + kPromptQueries - 1) / kPromptQueries);
   if (units > INT32_MAX) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %lld blocks of queries", units);
-  const int blocks = h->cfg.sm_limit > 0 ? std::min(static_cast<int>(units), h->grid) : static_cast<int>(units);
-  MK_CUDA(prompt_attention_launch(A, h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads, batch, static_cast<int>(units), blocks, false,
-                                  static_cast<cudaStream_t>(stream)));
+  AttnTcMaps maps{};
+  if (int e = encode_attention_maps(&maps, A, batch, h->cfg.q_heads, h->cfg.kv_heads, h->cfg.head_dim)) return e;
+  MK_CUDA(prompt_attention_launch(A, maps, {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles}, h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads,
+                                  batch, h->cfg.sm_limit > 0 ? h->grid : 0, false, static_cast<cudaStream_t>(stream)));
   h->launches += 1;
   return MK_OK;
 }

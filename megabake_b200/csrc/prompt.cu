@@ -1,11 +1,13 @@
 // Launches of the prompt kernels (prompt_kernels.cuh).
+#include "prompt_attention_tc.cuh"
 #include "prompt_kernels.cuh"
 
 namespace mk {
 namespace {
 
 // A launch that may begin while the kernel before it in the stream is still at work (`dependent`), its blocks in clusters of
-// `cluster`.
+// `cluster`.  The first kernel of a prompt pass is not: it, and through it the ones behind it, read weights ahead of their
+// griddepcontrol.wait, which whatever came before may have written.
 template <typename... Params, typename... Args>
 cudaError_t launch(void (*kernel)(Params...), int blocks, int threads, int smem, int cluster, bool dependent, cudaStream_t stream, const Args&... args) {
   cudaLaunchAttribute attributes[2];
@@ -59,16 +61,35 @@ cudaError_t prompt_prepare() {
   if (e == cudaSuccess) e = prepare_gemm<PE_PARTIAL>();
   if (e == cudaSuccess) e = prepare_gemm<PE_SILU>();
   if (e == cudaSuccess) e = prepare_gemm<PE_LOGITS>();
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnTc<64>::kSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnTc<128>::kSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem);
   return e;
 }
 
-cudaError_t prompt_attention_launch(const AttnArgs& args, int head_dim, int q_heads, int kv_heads, int batch, int units, int blocks,
-                                    bool dependent, cudaStream_t stream) {
+// Where each kernel is the faster one (1.7B shape, us).  On its own, 32 heads with a mask: 64 positions 9.3 with blocks of 64
+// queries on mma.sync, 10.0 with blocks of 128 on tcgen05, half of whose rows are idle then; 128 positions 9.7 and 7.6, 256 13.8 and
+// 9.9, 512 21.6 and 14.3.  In a prompt pass, where the projections' shared memory keeps its tensor memory and barriers from
+// being set up ahead and tiles past the diagonal are not visited: 64 tokens 1266 and 1307 for the whole pass, 200 1774 and 1771,
+// 500 2588 and 2496; 135M shape, 250 tokens 1257 and 1281.
+constexpr int kAttnTcAlone = 65, kAttnTcInPass = 257;
+
+cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps, const PromptGuard& guard, int head_dim, int q_heads, int kv_heads,
+                                    int batch, int limit, bool in_pass, cudaStream_t stream) {
+  const bool tc = args.klen >= (in_pass ? kAttnTcInPass : kAttnTcAlone);
+  const int per = tc ? kAttnQueries : kPromptQueries, units = batch * q_heads * ((args.sq + per - 1) / per);
+  const int blocks = limit > 0 ? std::min(units, limit) : units;
+  // Everything a kernel reads or writes comes behind its griddepcontrol.wait, so that it may be launched as a dependent one behind
+  // any kernel: two to three microseconds less between the two.
+  if (tc) {
+    if (head_dim == 64)
+      return launch(prompt_attention_tc<64>, blocks, kAttnThreads, AttnTc<64>::kSmem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
+    return launch(prompt_attention_tc<128>, blocks, kAttnThreads, AttnTc<128>::kSmem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
+  }
   if (head_dim == 64)
-    return launch(prompt_attention<64>, blocks, kWorkers, PromptLaunch<64>::kSmem, 1, dependent, stream, args, q_heads, kv_heads, batch, units);
-  return launch(prompt_attention<128>, blocks, kWorkers, PromptLaunch<128>::kSmem, 1, dependent, stream, args, q_heads, kv_heads, batch, units);
+    return launch(prompt_attention<64>, blocks, kWorkers, PromptLaunch<64>::kSmem, 1, true, stream, args, q_heads, kv_heads, batch, units);
+  return launch(prompt_attention<128>, blocks, kWorkers, PromptLaunch<128>::kSmem, 1, true, stream, args, q_heads, kv_heads, batch, units);
 }
 
 cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
@@ -121,22 +142,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
   norm.embed_rows = c.embed_rows > 0 ? c.embed_rows : c.vocab;
   norm.max_positions = c.max_positions;
   norm.eps = c.rms_eps;
-  AttnArgs A{};
-  A.q = pass.qkv;
-  A.q_ld = A.kv_ld = q_size + 2 * kv_size;
-  A.q_bstride = A.kv_bstride = static_cast<long long>(pass.seq) * A.q_ld;
-  A.k = pass.qkv + q_size;
-  A.v = A.k + kv_size;
-  A.out = pass.attn;
-  A.out_bstride = static_cast<long long>(pass.seq) * q_size;
-  A.out_tstride = q_size;
-  A.out_hstride = c.head_dim;
-  A.mask = pass.mask;
-  A.sq = A.klen = pass.seq;
-  A.causal = pass.mask == nullptr;
-  A.scale = pass.att_scale;
-  const int units = pass.batch * c.q_heads * ((pass.seq + kPromptQueries - 1) / kPromptQueries);
-  const int blocks = c.sm_limit > 0 ? std::min(units, pass.grid) : units, rows = c.sm_limit > 0 ? std::min(m, pass.grid) : m;
+  const int limit = c.sm_limit > 0 ? pass.grid : 0, rows = c.sm_limit > 0 ? std::min(m, pass.grid) : m;
   cudaError_t e = cudaSuccess;
   for (int l = 0; l <= c.layers && e == cudaSuccess; ++l) {
     const bool head = l == c.layers;
@@ -167,12 +173,12 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     g.out_col[1] = q_size;
     g.out_col[2] = q_size + kv_size;
     g.dst = pass.qkv;
-    g.ld = A.q_ld;
+    g.ld = q_size + 2 * kv_size;
     g.cos_t = static_cast<const bf16*>(w.rope_cos);
     g.sin_t = static_cast<const bf16*>(w.rope_sin);
     g.pos = pass.pos;
     e = launch_gemm<PE_QKV>(g, cls, pass.grid, stream);
-    if (e == cudaSuccess) e = prompt_attention_launch(A, c.head_dim, c.q_heads, c.kv_heads, pass.batch, units, blocks, true, stream);
+    if (e == cudaSuccess) e = prompt_attention_launch(*pass.attention, *pass.attention_maps, pass.guard, c.head_dim, c.q_heads, c.kv_heads, pass.batch, limit, true, stream);
     if (e != cudaSuccess) return e;
     g = gemm(PP_O, kOperandAttn);
     g.b[0] = maps + 3;

@@ -1,0 +1,486 @@
+// Prompt attention on the fifth-generation tensor cores: what megabake::attention and the prompt pass launch.
+//
+// A unit is (sequence, query head, block of 128 query tokens).  Tiles of 64 positions go in turn to two groups of four warps;
+// a thread has one query row and all 64 scores of its group's tile, so maximum and sum of a row need no other thread, and the
+// two groups' statistics and sums meet once, at the end of the unit.  Per tile and group:
+//   scores  D[128 queries, 64 positions] = Q . K^T   (tensor memory, read once into registers)
+//   values  D[128 queries, head_dim]     = P . V     (P from shared memory, V as it lies in the cache: MN-major), added to
+//           sums in registers, which are rescaled where the row's maximum grew
+// One warp issues the MMAs: the next tile's scores while a group is at this one's, which keeps both groups busy.  One thread
+// brings Q and the tiles with tiled TMA copies (with cp.async two warps took 1200 to 2500 cycles a tile, twice the softmax's).
+// Rounding points are those of prompt_unit (prompt_attention.cuh): score = bf16(bf16(q.k) * scale) (+ mask, rounded again),
+// fp32 softmax against the running maximum, exp rounded to bf16 for the value product, division by the fp32 sum at the end.
+// What bounds it: 128 x 64 exponentials are 512 cycles of the SM's special-function units, and about as many issue slots.
+#pragma once
+#include <type_traits>
+
+#include "prompt_attention.cuh"
+#include "prompt_plan.h"
+
+namespace mk {
+
+constexpr int kAttnQueries = 128, kAttnKeys = 64;
+constexpr int kAttnThreads = 384;  // two groups of four warps; of the third the loader and the MMA warp
+
+template <int HD>
+struct AttnTc {
+  static constexpr int kChunks = HD / 64;                         // 64-dimension chunks of a row
+  static constexpr int kStages = HD == 64 ? 6 : 3;
+  static constexpr int kTile = 2 * kChunks * kAttnKeys * 128;     // a K and a V tile
+  static constexpr int kQ = kChunks * kAttnQueries * 128, kP = kAttnQueries * 128;
+  static constexpr int kSmem = 1024 + kQ + 2 * kP + kStages * kTile;
+  static constexpr int kColumns = HD == 64 ? 256 : 512;           // 2 x 64 of scores, 2 x head_dim of values
+  // The groups' exchange at the end of a unit, [head_dim + 2][128] fp32, takes the place of Q, P and (head size 128) a stage.
+  static_assert((HD + 2) * 128 * 4 <= kQ + 2 * kP + kTile, "exchange");
+};
+
+struct AttnTcMisc {
+  uint64_t qfull, kvfull[8], kvempty[8], sfull[2], sfree[2], pfull[2], pvfull[2];
+  uint32_t tmem_base;
+  int abort;
+};
+
+// Descriptors of a launch's operands, rows of 64-element chunks: (64, rows, chunks of all heads, sequences).  Rows past the last
+// one read as zeros.
+struct AttnTcMaps {
+  CUtensorMap q, k, v;
+  int q_ok;  // the queries begin on a 16-byte boundary; otherwise their rows are fetched with plain loads
+};
+
+// B operand stored with its N dimension contiguous: 64-element chunks [8 rows of K][128 B], 128-byte swizzle.  Rows of K in
+// groups of eight are 1024 bytes apart (stride offset), chunks of N `chunk_bytes` (leading offset).
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t chunk_bytes) {
+  return umma_desc_sw128(smem_addr) - (static_cast<uint64_t>(1) << 16) + (static_cast<uint64_t>(chunk_bytes >> 4) << 16);
+}
+constexpr uint32_t kIdescBMajorN = 1u << 16;
+
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+struct AttnTcWait {
+  const PromptGuard* guard;
+  AttnTcMisc* misc;
+  long long deadline;
+};
+static __device__ __noinline__ bool attn_give_up(const AttnTcWait& w) {
+  if (*reinterpret_cast<volatile int*>(&w.misc->abort)) return true;
+  Control* const ctrl = w.guard->ctrl;
+  if (ld_relaxed_u32(&ctrl->abort) == 0) {
+    if (clock64() < w.deadline) return false;
+    if (atomicCAS(&ctrl->status, 0, static_cast<int>(MK_STATUS_TIMEOUT)) == 0) {
+      ctrl->where = SITE_ATT_EXCHANGE;
+      ctrl->cta = blockIdx.x;
+      ctrl->detail = 0;
+      if (w.guard->status_mirror) *w.guard->status_mirror = static_cast<int>(MK_STATUS_TIMEOUT);
+    }
+    atomicExch(&ctrl->abort, 1u);
+    __threadfence();
+  }
+  *reinterpret_cast<volatile int*>(&w.misc->abort) = 1;
+  return true;
+}
+__device__ __forceinline__ bool attn_wait(const AttnTcWait& w, uint64_t* bar, uint32_t parity) {
+  const uint32_t at = smem_u32(bar);
+  uint32_t spins = 0;
+  while (!mbar_try_wait(at, parity))
+    if ((++spins & 63u) == 0 && attn_give_up(w)) return false;
+  return true;
+}
+
+// What every role knows of a unit.
+struct AttnTcUnit {
+  int b, h, kvh, q0, ntiles;
+};
+__device__ __forceinline__ AttnTcUnit attn_unit(const AttnArgs& A, int q_heads, int kv_heads, int batch, int i) {
+  AttnTcUnit u;
+  const int heads = batch * q_heads, qblocks = (A.sq + kAttnQueries - 1) / kAttnQueries;
+  const int qb = qblocks - 1 - i / heads, bh = i % heads;  // causal blocks cost in proportion to their index: heaviest first
+  u.b = bh / q_heads;
+  u.h = bh - u.b * q_heads;
+  u.kvh = u.h / (q_heads / kv_heads);
+  u.q0 = qb * kAttnQueries;
+  const int kend = A.causal ? min(A.klen, u.q0 + kAttnQueries) : A.klen;
+  u.ntiles = (kend + kAttnKeys - 1) / kAttnKeys;
+  return u;
+}
+
+// One thread of warp 8: the queries, then tile t into stage t % kStages (t counts over the launch).
+template <int HD>
+__device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t stages,
+                                          int base) {
+  using T = AttnTc<HD>;
+  const uint64_t policy = l2_policy_evict_normal();
+  if (maps.q_ok) {
+    mbar_expect_tx(smem_u32(&misc->qfull), T::kQ);
+    tma_load_4d(q, &maps.q, 0, u.q0, u.h * T::kChunks, u.b, smem_u32(&misc->qfull), policy);
+  }
+  for (int t = 0; t < u.ntiles; ++t) {
+    const int at = base + t, s = at % T::kStages, use = at / T::kStages;
+    if (use > 0 && !attn_wait(w, &misc->kvempty[s], (use - 1) & 1)) {
+      for (int i = 0; i < 32; ++i) __nanosleep(1000);  // copies under way land within microseconds
+      return;
+    }
+    const uint32_t bar = smem_u32(&misc->kvfull[s]), dst = stages + s * T::kTile;
+    mbar_expect_tx(bar, T::kTile);
+    tma_load_4d(dst, &maps.k, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
+    tma_load_4d(dst + T::kTile / 2, &maps.v, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
+  }
+}
+
+// Warp 10.  `base` and `uses`: tiles of earlier units, all and of each group (uses of the barriers).
+template <int HD>
+__device__ __forceinline__ void attn_mma(const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t p, uint32_t stages, uint32_t tmem,
+                                         int base, const int* uses) {
+  using T = AttnTc<HD>;
+  constexpr uint32_t kScores = umma_idesc_bf16(kAttnQueries, kAttnKeys), kValues = umma_idesc_bf16(kAttnQueries, HD) | kIdescBMajorN;
+  auto scores = [&](int t) -> bool {
+    const int at = base + t, s = at % T::kStages;
+    if (!__all_sync(0xffffffffu, attn_wait(w, &misc->kvfull[s], (at / T::kStages) & 1))) return false;
+    tc_fence_after();
+    const uint64_t a = umma_desc_sw128(q), b = umma_desc_sw128(stages + s * T::kTile);
+    if (elect_one()) {
+#pragma unroll
+      for (int c = 0; c < T::kChunks; ++c)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          umma_bf16(tmem + (t & 1) * kAttnKeys, a + (c * kAttnQueries * 128 + x * 32) / 16, b + (c * kAttnKeys * 128 + x * 32) / 16, kScores,
+                    c + x > 0 ? 1u : 0u);
+      umma_commit(smem_u32(&misc->sfull[t & 1]));
+    }
+    __syncwarp();
+    return true;
+  };
+  for (int t = 0; t < min(2, u.ntiles); ++t)
+    if (!scores(t)) return;
+  for (int t = 0; t < u.ntiles; ++t) {
+    const int g = t & 1, use = uses[g] + (t >> 1);
+    if (t + 2 < u.ntiles) {  // the group has this tile's scores in registers
+      if (!__all_sync(0xffffffffu, attn_wait(w, &misc->sfree[g], use & 1))) return;
+      if (!scores(t + 2)) return;
+    }
+    if (!__all_sync(0xffffffffu, attn_wait(w, &misc->pfull[g], use & 1))) return;
+    tc_fence_after();
+    const int s = (base + t) % T::kStages;
+    const uint64_t a = umma_desc_sw128(p + g * T::kP), b = umma_desc_mn_sw128(stages + s * T::kTile + T::kTile / 2, kAttnKeys * 128);
+    if (elect_one()) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x)  // 16 positions: 32 bytes of a row of P, two groups of eight rows of V
+        umma_bf16(tmem + 2 * kAttnKeys + g * HD, a + x * 2, b + x * (2048 / 16), kValues, x > 0 ? 1u : 0u);
+      umma_commit(smem_u32(&misc->kvempty[s]));
+      umma_commit(smem_u32(&misc->pvfull[g]));
+    }
+    __syncwarp();
+  }
+}
+
+// The mask of a thread's row for 64 positions from j on, as bf16 pairs.  `wide`: rows begin on 16-byte boundaries.  Otherwise the
+// aligned words that hold the elements, shifted into place; past the row's last word it is repeated (those positions are
+// masked below).
+__device__ __forceinline__ void attn_mask(const bf16* row, int j, int klen, bool wide, uint32_t (&m)[32]) {
+  if (wide && j + 64 <= klen) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + j) + i);
+      m[4 * i] = v.x; m[4 * i + 1] = v.y; m[4 * i + 2] = v.z; m[4 * i + 3] = v.w;
+    }
+  } else {
+    const uintptr_t first = reinterpret_cast<uintptr_t>(row + j) & ~static_cast<uintptr_t>(3);
+    const uint32_t shift = (reinterpret_cast<uintptr_t>(row + j) & 2) ? 16u : 0u;
+    const int last = static_cast<int>((reinterpret_cast<uintptr_t>(row + klen - 1) - first) >> 2);  // the word of the last position
+    const unsigned int* const words = reinterpret_cast<const unsigned int*>(first);
+    uint32_t word = __ldg(words);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const uint32_t next = __ldg(words + min(i + 1, last));
+      m[i] = __funnelshift_r(word, next, shift);
+      word = next;
+    }
+  }
+}
+
+// Warps 0 to 7.  A wait that was given up ends the loop; the block barriers behind it are passed all the same.
+template <int HD>
+__device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint8_t* smem, uint32_t p,
+                                             uint32_t tmem, const int* uses, int warp, int lane) {
+  const int g = warp >> 2, quad = warp & 3, row = quad * 32 + lane, r = u.q0 + row;
+  const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
+  const uint32_t s_at = tmem + lanes + g * kAttnKeys, v_at = tmem + lanes + 2 * kAttnKeys + g * HD;
+  const uint32_t p_at = p + g * AttnTc<HD>::kP + row * 128;
+  const bool exact_scale = bf16_round(A.scale) == A.scale;  // head size 64: 1/8; the product is rounded once either way
+  const uint32_t scale2 = pack2(A.scale, A.scale);
+  const bf16* const mrow = A.mask + (static_cast<long long>(u.b) * A.sq + min(r, A.sq - 1)) * A.klen;
+  const bool wide = (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
+  bool ok = true, unseen = false;  // unseen: this warp saw nothing of the tile whose sums come next
+  float m = -INFINITY, l = 0.f, alpha = 1.f, o[HD];
+#pragma unroll
+  for (int d = 0; d < HD; ++d) o[d] = 0.f;
+  auto add_values = [&](int use) {  // the value sums of this group's last tile
+    ok = __all_sync(0xffffffffu, attn_wait(w, &misc->pvfull[g], use & 1));
+    if (!ok || unseen) return;
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < HD; c += 32) {
+      uint32_t v[32];
+      tmem_ld32_async(v_at + c, v);
+      tmem_loaded();
+#pragma unroll
+      for (int d = 0; d < 32; ++d) o[c + d] = fmaf(o[c + d], alpha, __uint_as_float(v[d]));
+    }
+  };
+  uint32_t x[32];  // the mask of a tile's row, its scores, its probabilities
+  if (A.mask && g < u.ntiles) attn_mask(mrow, g * kAttnKeys, A.klen, wide, x);
+#pragma unroll 1
+  for (int t = g; t < u.ntiles && ok; t += 2) {
+    const int use = uses[g] + (t >> 1), j0 = t * kAttnKeys;
+    // (causal: a warp whose rows all come before the tile has nothing to see in it)
+    const bool blind = A.causal && j0 > u.q0 + quad * 32 + 31;
+    ok = __all_sync(0xffffffffu, attn_wait(w, &misc->sfull[g], use & 1));
+    if (!ok) break;
+    tc_fence_after();
+    float grown = 1.f;
+    // With head size 64 there are registers for the next tile's mask: asked for before this tile's exponentials.
+    uint32_t ahead[HD == 64 ? 32 : 1];
+    if (!blind) {
+      // What a pair of scores goes through depends on the launch and the tile: straight lines, not three tests a pair.
+      auto take = [&](auto exact, auto masked) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t s[32];
+          tmem_ld32_async(s_at + c * 32, s);
+          tmem_loaded();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            uint32_t v = pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]));
+            if constexpr (decltype(exact)::value) v = mul_bf16x2(v, scale2);
+            else v = pack2(__uint_as_float(v << 16) * A.scale, __uint_as_float(v & 0xffff0000u) * A.scale);
+            if constexpr (decltype(masked)::value) v = add_bf16x2(v, x[c * 16 + i]);
+            x[c * 16 + i] = v;
+          }
+        }
+      };
+      if (A.mask) {
+        if (exact_scale) take(std::true_type(), std::true_type());
+        else take(std::false_type(), std::true_type());
+      } else {
+        if (exact_scale) take(std::true_type(), std::false_type());
+        else take(std::false_type(), std::false_type());
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&misc->sfree[g]));
+      if constexpr (HD == 64) {
+        if (A.mask && t + 2 < u.ntiles) attn_mask(mrow, j0 + 2 * kAttnKeys, A.klen, wide, ahead);
+      }
+      const int last = (A.causal ? min(A.klen - 1, r) : A.klen - 1) - j0;  // the last position of the tile that the row sees
+      if (__any_sync(0xffffffffu, last < kAttnKeys - 1)) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (2 * i > last) x[i] = (x[i] & 0xffff0000u) | 0xFF80u;
+          if (2 * i + 1 > last) x[i] = (x[i] & 0xffffu) | 0xFF800000u;
+        }
+      }
+      uint32_t top = x[0];
+#pragma unroll
+      for (int i = 1; i < 32; ++i) top = max_bf16x2(top, x[i]);
+      const float n = fmaxf(m, fmaxf(__uint_as_float(top << 16), __uint_as_float(top & 0xffff0000u)));
+      // exp(x - n) = 2^((x - n) log2(e)), the difference first: a mask of the lowest finite value must not overflow; a row
+      // without a visible key so far: 2^(-inf) = 0
+      const float safe = n > -INFINITY ? n : 0.f;
+      grown = ex2((m - safe) * kLog2e);
+      m = n;
+      float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float e0 = ex2((__uint_as_float(x[i] << 16) - safe) * kLog2e), e1 = ex2((__uint_as_float(x[i] & 0xffff0000u) - safe) * kLog2e);
+        sum0 += e0;
+        sum1 += e1;
+        x[i] = pack2(e0, e1);
+      }
+      l = fmaf(l, grown, sum0 + sum1);
+    } else {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&misc->sfree[g]));
+#pragma unroll
+      for (int i = 0; i < 32; ++i) x[i] = 0u;
+    }
+    if (t >= 2) add_values(use - 1);  // and with that the last tile's P has been read
+    alpha = grown;
+    unseen = blind;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(p_at + ((i ^ (row & 7)) << 4)), "r"(x[4 * i]), "r"(x[4 * i + 1]), "r"(x[4 * i + 2]),
+                   "r"(x[4 * i + 3]) : "memory");
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&misc->pfull[g]));
+    if (A.mask && t + 2 < u.ntiles) {
+      if constexpr (HD == 64) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = ahead[i];
+      } else {
+        attn_mask(mrow, j0 + 2 * kAttnKeys, A.klen, wide, x);
+      }
+    }
+  }
+  const int mine = (u.ntiles - g + 1) / 2;  // tiles of this group
+  if (mine > 0 && ok) add_values(uses[g] + mine - 1);
+  // The second group's statistics and sums join the first group's, which divides, rounds once and stores.  Every MMA of the unit
+  // has finished once both groups are here: Q, P and the tiles' stages may be written over.
+  float* const exchange = reinterpret_cast<float*>(smem) + row;
+  named_bar_sync(1, 256);
+  if (g == 1) {
+    exchange[0] = m;
+    exchange[128] = l;
+#pragma unroll
+    for (int d = 0; d < HD; ++d) exchange[(2 + d) * 128] = o[d];
+  }
+  named_bar_sync(1, 256);
+  if (g == 0 && r < A.sq && *reinterpret_cast<volatile int*>(&misc->abort) == 0) {
+    const float om = exchange[0], ol = exchange[128], n = fmaxf(m, om);
+    const float a = m > -INFINITY ? expf(m - n) : 0.f, b = om > -INFINITY ? expf(om - n) : 0.f;
+    const float total = l * a + ol * b, d = total > 0.f ? total : 1.f;  // a row that sees no key: zeros
+    const float inverse = 1.f / d;
+    // a quotient by the reciprocal, corrected by its remainder (Markstein, 1990); what is no finite number stays what it is
+    auto quotient = [&](float first, float second) -> float {
+      const float v = first * a + second * b, by = v * inverse;
+      return fabsf(by) < INFINITY ? fmaf(fmaf(-by, d, v), inverse, by) : by;
+    };
+    bf16* const out = A.out + u.b * A.out_bstride + static_cast<long long>(r) * A.out_tstride + u.h * A.out_hstride;
+    const bool vectors = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+#pragma unroll
+    for (int d0 = 0; d0 < HD; d0 += 8) {
+      uint32_t x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        x[e] = pack2(quotient(o[d0 + 2 * e], exchange[(2 + d0 + 2 * e) * 128]), quotient(o[d0 + 2 * e + 1], exchange[(3 + d0 + 2 * e) * 128]));
+      if (vectors) {
+        *reinterpret_cast<uint4*>(out + d0) = make_uint4(x[0], x[1], x[2], x[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) reinterpret_cast<uint32_t*>(out + d0)[e] = x[e];
+      }
+    }
+  }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kAttnThreads, 1)
+prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ AttnTcMaps maps, const __grid_constant__ PromptGuard guard, int q_heads,
+                    int kv_heads, int batch, int units) {
+  using T = AttnTc<HD>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ AttnTcMisc misc;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_dependents_go();
+  if (tid == 0) {
+    mbar_init(smem_u32(&misc.qfull), 1);
+    for (int s = 0; s < T::kStages; ++s) {
+      mbar_init(smem_u32(&misc.kvfull[s]), 1);
+      mbar_init(smem_u32(&misc.kvempty[s]), 1);
+    }
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(smem_u32(&misc.sfull[g]), 1);
+      mbar_init(smem_u32(&misc.sfree[g]), 4);
+      mbar_init(smem_u32(&misc.pfull[g]), 4);
+      mbar_init(smem_u32(&misc.pvfull[g]), 1);
+    }
+    misc.abort = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&maps.q);
+    tma_prefetch_desc(&maps.k);
+    tma_prefetch_desc(&maps.v);
+  }
+  if (warp == 10) {
+    tmem_alloc(smem_u32(&misc.tmem_base), T::kColumns);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&misc.tmem_base);
+  const uint32_t q = smem_u32(smem), p = q + T::kQ, stages = p + 2 * T::kP;
+  grid_dependency_wait();
+  const AttnTcWait w{&guard, &misc, clock64() + guard.timeout_cycles};
+  int base = 0, uses[2] = {0, 0}, done = 0;  // tiles of earlier units, and their number
+  // The units of this block (one, unless the handle limits its SMs), as one role sees them.
+  auto walk = [&](auto role) {
+#pragma unroll 1
+    for (int i = blockIdx.x; i < units; i += gridDim.x) {
+      const AttnTcUnit u = attn_unit(A, q_heads, kv_heads, batch, i);
+      role(u);
+      named_bar_sync(3, kAttnThreads);
+      if (*reinterpret_cast<volatile int*>(&misc.abort)) {  // MMAs that were issued end within a microsecond
+        __nanosleep(4000);
+        break;
+      }
+      base += u.ntiles;
+      uses[0] += (u.ntiles + 1) / 2;
+      uses[1] += u.ntiles / 2;
+      ++done;
+    }
+  };
+  // 384 threads x 168 registers at launch = 128 x 72 + 256 x 216: with head size 128 a row of value sums is 128 of them
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 10) {
+      walk([&](const AttnTcUnit& u) {
+        if (!maps.q_ok) named_bar_sync(2, 288);  // the queries are there
+        else if (!__all_sync(0xffffffffu, attn_wait(w, &misc.qfull, done & 1))) return;
+        attn_mma<HD>(w, &misc, u, q, p, stages, tmem, base, uses);
+      });
+    } else {
+      walk([&](const AttnTcUnit& u) {
+        if (warp == 8 && lane == 0) {
+          fence_proxy_async_all();  // the operands, and (a later unit) the exchange's plain accesses, before the copies
+          attn_load<HD>(maps, w, &misc, u, q, stages, base);
+        }
+        __syncwarp();
+      });
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    walk([&](const AttnTcUnit& u) {
+      if (!maps.q_ok) {  // [chunk][row][128 B], swizzled; rows past the last one repeat it
+        constexpr int kPieces = HD / 8;
+        const bf16* const from = A.q + u.b * A.q_bstride + u.h * HD;
+#pragma unroll 1
+        for (int x = tid; x < kAttnQueries * kPieces; x += 256) {
+          const int row = x / kPieces, piece = x % kPieces;
+          const bf16* at = from + static_cast<long long>(min(u.q0 + row, A.sq - 1)) * A.q_ld + piece * 8;
+          *reinterpret_cast<uint4*>(smem + (piece >> 3) * kAttnQueries * 128 + row * 128 + (((piece & 7) ^ (row & 7)) << 4)) =
+              make_uint4(ldcg_u32(at), ldcg_u32(at + 2), ldcg_u32(at + 4), ldcg_u32(at + 6));
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(2, 288);
+      }
+      attn_softmax<HD>(A, w, &misc, u, smem, p, tmem, uses, warp, lane);
+      fence_proxy_async_smem();
+    });
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 10) {
+    tc_fence_after();
+    tmem_dealloc(tmem, T::kColumns);
+  }
+}
+
+}  // namespace mk

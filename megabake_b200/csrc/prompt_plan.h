@@ -149,6 +149,9 @@ struct PromptNorm {
   float eps;
 };
 
+struct AttnArgs;
+struct AttnTcMaps;
+
 // One prompt pass: everything its launches are made from.
 struct PromptPass {
   const mk_config* config;
@@ -163,14 +166,15 @@ struct PromptPass {
   const bf16* mask;
   bf16* logits;
   int m, batch, seq;
-  float att_scale;
+  const AttnArgs* attention;
+  const AttnTcMaps* attention_maps;
   PromptGuard guard;
 };
 
-struct AttnArgs;
 cudaError_t prompt_prepare();  // shared-memory attributes of the kernels, on the current device
 cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream);
-cudaError_t prompt_attention_launch(const AttnArgs& args, int head_dim, int q_heads, int kv_heads, int batch, int units, int blocks,
-                                    bool dependent, cudaStream_t stream);
+// limit: blocks of the launch at most, or 0.
+cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps, const PromptGuard& guard, int head_dim, int q_heads, int kv_heads,
+                                    int batch, int limit, bool in_pass, cudaStream_t stream);
 
 }  // namespace mk

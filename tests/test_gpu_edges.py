@@ -152,6 +152,28 @@ def test_a_refused_prompt_is_all_nan_and_the_next_one_is_not(device, tokens):
         kernel.check()
 
 
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("keys", [64, 65, 191, 256, 333])
+@pytest.mark.parametrize("offset", [2, 8])
+def test_prompt_attention_op_with_operands_on_any_word_and_infinite_masks(device, head_dim, keys, offset):
+    """Queries off the 16-byte grid, masks that begin at an odd element, rows whose first tiles are all -inf, rows that see
+    nothing: zeros."""
+    from oracle import decoder_oracle as oracle
+
+    heads, kv_heads, batch = 6, 2, 2
+    query, key, value = _tensors(device, batch, keys, keys, heads, kv_heads, head_dim)
+    moved = torch.empty(query.numel() + offset, dtype=query.dtype, device=device)[offset:].view(query.shape).copy_(query)
+    store = torch.zeros(batch * keys * keys + 1, dtype=torch.bfloat16, device=device)
+    mask = store[1:].view(batch, 1, keys, keys)
+    rows, columns = torch.arange(keys, device=device).view(-1, 1), torch.arange(keys, device=device)
+    mask.masked_fill_((columns > rows) | (columns < rows - 20), -torch.inf)
+    out = torch.ops.megabake.attention(moved, key, value, mask, head_dim ** -0.5)
+    assert_parity(out, oracle.attention(query, key, value, mask, head_dim ** -0.5), f"attention over {keys}")
+    mask[:, :, 5] = -torch.inf
+    again = torch.ops.megabake.attention(moved, key, value, mask, head_dim ** -0.5)
+    assert (again[:, 5] == 0).all() and torch.equal(again[:, 6:], out[:, 6:])
+
+
 @pytest.mark.parametrize("sm_limit", [1, 7])
 @pytest.mark.parametrize("tokens", [50, 300])
 def test_prompts_on_few_sms(device, sm_limit, tokens):
