@@ -39,6 +39,12 @@ enum { SP_QKV = 0, SP_O = 1, SP_GU = 2, SP_DOWN = 3, SP_HEAD = 4, kStreamPhases 
 
 // Token classes: a kernel is compiled for at most 1, 4, 8, 16 or 32 tokens.
 __host__ __device__ constexpr int stream_token_tiles(int tm) { return tm <= 8 ? 1 : tm / 8; }
+// Copies of a slice whose operand a warp's registers hold.
+__host__ __device__ constexpr int stream_fit(int nt) { return nt == 4 ? 2 : 4; }
+// ... of a normalised operand, which is of the hidden size, at most 2048: two.  A phase's length in instructions is its time, so
+// its code holds no more (with four, us a step: 1.7B shape, 3 sequences 957 against 888, 16 sequences 1638 against 1583; 135M, 4
+// sequences 760 against 715) - but for one token, where the shorter code came out 1 to 2 % slower (831 against 848).
+__host__ __device__ constexpr int stream_fit_normalised(int tm) { return tm == 1 ? 4 : 2; }
 
 // Every CTA reads the whole residual stream, and while it waits it reads the same few lines again and again: with few tokens
 // those lines lie in a handful of L2 slices and the readers hold up the writers' stores.  So results are written to

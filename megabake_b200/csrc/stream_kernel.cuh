@@ -128,7 +128,7 @@ template <int TM, int HD>
 __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe, int wtid) {
   const KParams& p = *sm->p;
   constexpr int NT = stream_token_tiles(TM);
-  constexpr int CMAX = NT == 4 ? 2 : 4;  // copies of a slice whose operand fits the registers (stream_phases)
+  constexpr int CNORM = stream_fit_normalised(TM), CPLAIN = stream_fit(NT);
   constexpr int kLayerWords = sizeof(StreamLayer) / 4;
   const int layers = p.layers;
   StreamThread th;
@@ -150,15 +150,15 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     // the next layer's vectors: requested here, passed on through shared memory at the end of the layer
     uint32_t word = 0u;
     if (wtid < kLayerWords && layer + 1 < layers) word = __ldg(reinterpret_cast<const uint32_t*>(sm->plan.layers + layer + 1) + wtid);
-    stream_project<TM, 1, CMAX, SG_NORM>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
+    stream_project<TM, 1, CNORM, SG_NORM>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
     if (head) break;
     stream_attention<HD>(th, pipe, layer);                           // RoPE, append, attention
     th.trace(EV_ATTENTION_DONE);
-    stream_project<TM, 1, CMAX, SG_PLAIN>(th, pipe, SP_O, layer);     // o_proj + residual
-    stream_project<TM, 2, CMAX, SG_MLP>(th, pipe, SP_GU, layer);       // RMSNorm, SiLU(gate) * up
+    stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, SP_O, layer);     // o_proj + residual
+    stream_project<TM, 2, CNORM, SG_MLP>(th, pipe, SP_GU, layer);       // RMSNorm, SiLU(gate) * up
     if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
     __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
-    stream_project<TM, 1, CMAX, SG_PLAIN>(th, pipe, SP_DOWN, layer);  // down_proj + residual
+    stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, SP_DOWN, layer);  // down_proj + residual
     stream_sync();    // the next layer's vectors are in place
     th.last_turn = th.turn;
     th.turn = th.turn == 2 ? 0 : th.turn + 1;

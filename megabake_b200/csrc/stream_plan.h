@@ -61,7 +61,6 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
   const int nt = 1 << plan, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
   const int ks[kStreamPhases] = {c.hidden, q_size, c.hidden, c.intermediate, c.hidden};
   const int ns[kStreamPhases] = {q_size + 2 * kv_size, c.hidden, c.intermediate, c.hidden, c.vocab};
-  const int fit = nt == 4 ? 2 : 4;  // copies whose operand fits a warp's registers
   bool ok = true;
   for (int i = 0; i < kStreamPhases; ++i) {
     StreamPhase& p = ph[i];
@@ -71,6 +70,7 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
     // Up to eight tokens a long reduction is not cut: its operand is small enough to be read in parts by every CTA, which
     // saves a hand-over of partial sums.
     const bool cross = i == SP_O || i == SP_DOWN;
+    const int fit = cross ? stream_fit(nt) : 2;  // (normalised: stream_fit_normalised, or less)
     ok = stream_cut(p, cross && nt == 1 ? 8 : fit) && (cross || p.nslice == 1) && ok;
     p.parts = (p.ncopy + fit - 1) / fit;
     const int qkv[3] = {q_size, kv_size, kv_size};
