@@ -537,11 +537,21 @@ int launch_kv_attention(mk_handle h, const void* query, const void* key, const v
   a.slots = a.chunks * a.shares;
   a.scale_log2 = h->att_scale * kLog2e;
   const int units = blocks_per_run * a.chunks, blocks = c.sm_limit > 0 ? std::min(units, wave) : units;
-  if (small) kv_attention_parts<64><<<blocks, 256, KvLaunch<64>::kSmem, stream>>>(a, units);
-  else kv_attention_parts<128><<<blocks, 256, KvLaunch<128>::kSmem, stream>>>(a, units);
-  MK_CUDA(cudaGetLastError());
-  kv_attention_combine<<<(batch * c.q_heads * (c.head_dim / 4) + 127) / 128, 128, 0, stream>>>(a, c.head_dim);
-  MK_CUDA(cudaGetLastError());
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.stream = stream;
+  config.attrs = &early;
+  config.numAttrs = 1;
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(256);
+  config.dynamicSmemBytes = small ? KvLaunch<64>::kSmem : KvLaunch<128>::kSmem;
+  MK_CUDA(small ? cudaLaunchKernelEx(&config, kv_attention_parts<64>, a, units) : cudaLaunchKernelEx(&config, kv_attention_parts<128>, a, units));
+  config.gridDim = dim3((batch * c.q_heads * (c.head_dim / 4) + 127) / 128);
+  config.blockDim = dim3(128);
+  config.dynamicSmemBytes = 0;
+  MK_CUDA(cudaLaunchKernelEx(&config, kv_attention_combine, a, c.head_dim));
   h->launches += 1;
   return MK_OK;
 }
