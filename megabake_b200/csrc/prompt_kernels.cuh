@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kPromptThreads, 1) prompt_gemm(const __grid_co
   } else if (warp == kPromptMmaWarp) {
     grid_dependency_wait();
     constexpr int kBlocks = CTAS == 2 && EPI == PE_SILU ? 2 : 1;
-    if (TM == 64 && g.kb == 2) prompt_mma_loop<1, 64, 2, 1>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
+    if (CTAS == 1 && g.kb == 2) prompt_mma_loop<1, TM, 2, 1>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
     else if (rank == 0) prompt_mma_loop<CTAS, TM, 1, kBlocks>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
   } else {
     prompt_epilogue<CTAS, TM, EPI>(g, accfull0, accempty0, tmem, rank, first, step, warp - kPromptFirstEpilogue, lane);
