@@ -185,6 +185,8 @@ int mk_decode_step_host(mk_handle handle, const int64_t* host_ids, const int64_t
 /* Stateless prompt pass over [batch, sequence] tokens with causal or additive
  * attention mask (bf16 [batch, 1, sequence, sequence], NULL = causal).
  * logits: bf16 [batch, sequence, vocab].
+ * A chain of 7 * layers + 2 kernels on `stream`, each of which may begin while the one before it
+ * ends; under tensor parallel, one cooperative launch.  No sync.
  * Reference: the mode="prefill" graph whose attention is megabake::attention
  * (src/megabake/lowering.py:273-300, src/megabake/fx_handler/hf_attention.py:28-61). */
 int mk_prefill(mk_handle handle, const int64_t* ids, const int64_t* positions, const void* mask,
@@ -276,7 +278,7 @@ int mk_ipc_close(void* base);
 int mk_baseline_mma_gemm(const void* x, const void* weight, void* y, int m, int n, int k, void* stream);
 
 /* Plain-text summary of what the handle will launch (CTAs, the form of the weight copies, tile height /
- * K split / chunks per copy / unit count of each projection phase per table).  Synchronous (reads the
+ * K split / chunks per copy / unit count of each projection phase per table, and of a prompt pass per launch class).  Synchronous (reads the
  * phase tables back).  Reference: the plan report, src/megabake/plan.py:342-395. */
 int mk_describe(mk_handle handle, char* buffer, size_t bytes);
 
