@@ -245,8 +245,8 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
       copy(base + s * stage_bytes, a_map, p.a_row, chunk, count0 + s * 8u, token_policy);
     }
   }
-  if (CTAS == 2)  // the other CTA's last arrivals here come before this one leaves
-    for (int i = min(n, stages); i > 0 && ok; --i, next()) ok = prompt_wait(w, empty0 + s * 8u, parity ^ 1u, SITE_DRAIN);
+  // the MMA warp's last arrivals here, those of the pair's first CTA among them, come before this one leaves
+  ok = ok && prompt_drain(n, stages, [&](int slot, uint32_t phase) { return prompt_wait(w, empty0 + slot * 8u, phase, SITE_DRAIN); });
   // A pass that is given up: what was asked for lands within microseconds; the CTA stays for thirty.
   if (!ok)
     for (int i = 0; i < 32; ++i) __nanosleep(1000);
@@ -301,6 +301,11 @@ __device__ __noinline__ void prompt_mma_loop(const PromptGemm& g, uint32_t base,
       }
     }
   }
+  // The pair's other CTA hands accumulators back by arrivals on this one's barriers, and the barrier at the end orders no
+  // memory: its last ones are here before this CTA leaves.
+  if constexpr (CTAS == 2)
+    for (int buf = 0; buf < min(kBuffers, q); ++buf)
+      if (!__all_sync(0xffffffffu, prompt_wait(w, accempty0 + buf * 8u, static_cast<uint32_t>((q - 1 - buf) / kBuffers) & 1u, SITE_MMA_ACC))) break;
 }
 
 __device__ __forceinline__ void prompt_pack16(const float* v, uint32_t* w) {

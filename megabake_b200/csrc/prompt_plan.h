@@ -101,6 +101,16 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
   }
 }
 
+// What a CTA still waits for before it leaves: that the last use of every pipeline slot has been consumed, so that no commit
+// is on its way to a barrier of shared memory that is somebody else's by then.  The uses count up over the launch, use u lies in
+// slot u % stages, and a slot's barrier has the parity of its use; wait(slot, parity) returns false to give up.
+template <typename Wait>
+__host__ __device__ inline bool prompt_drain(int uses, int stages, Wait wait) {
+  for (int u = uses < stages ? 0 : uses - stages; u < uses; ++u)
+    if (!wait(u % stages, static_cast<uint32_t>(u / stages) & 1u)) return false;
+  return true;
+}
+
 // Rows of the weight descriptors' boxes: a CTA of a pair brings half a tile.
 inline int prompt_box_rows(const PromptPhase& p, int cls) { return cls > 0 ? p.rows / 2 : p.rows; }
 
