@@ -1243,6 +1243,8 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   if (k_len > prompt_keys(h)) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %d keys exceed %d", k_len, prompt_keys(h));
   if (reinterpret_cast<uintptr_t>(key) % 16 || reinterpret_cast<uintptr_t>(value) % 16)
     return fail(MK_ERR_ALIGNMENT, "mk_attention: key/value must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(query) % 4 || reinterpret_cast<uintptr_t>(output) % 4)  // read and written in pairs of elements
+    return fail(MK_ERR_ALIGNMENT, "mk_attention: query/output must be 4-byte aligned");
   const int q_size = h->cfg.q_heads * h->cfg.head_dim, kv_size = h->cfg.kv_heads * h->cfg.head_dim;
   AttnArgs A{};
   A.q = static_cast<const bf16*>(query); A.q_bstride = static_cast<long long>(q_len) * q_size; A.q_ld = q_size;

@@ -128,7 +128,9 @@ Tensor attention_now(const Tensor& query, const Tensor& key, const Tensor& value
   const c10::cuda::CUDAGuard on(device);
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
-  const Tensor q = query.contiguous(), kk = key.contiguous(), vv = value.contiguous();
+  const Tensor kk = key.contiguous(), vv = value.contiguous();
+  Tensor q = query.contiguous();
+  if (reinterpret_cast<uintptr_t>(q.const_data_ptr()) % 4) q = q.clone();  // begins at an odd element: the kernels read pairs
   Tensor out = at::empty({batch * heads, q_len, dim}, query.options());
   const int code = s.entries.attention(k->handle, q.const_data_ptr(), kk.const_data_ptr(), vv.const_data_ptr(), masked ? mask->const_data_ptr() : nullptr,
                                        static_cast<float>(scale), static_cast<int>(batch), static_cast<int>(q_len), static_cast<int>(k_len),

@@ -437,6 +437,8 @@ class DecoderKernel:
             if mask.shape != (batch, 1, q_len, k_len) or not mask.is_contiguous():
                 mask = mask.expand(batch, 1, q_len, k_len).contiguous()
             _require(mask, "mask", dtype=torch.bfloat16, device=self.device)
+        if query.data_ptr() % 4:  # begins at an odd element: the kernels read pairs
+            query = query.clone()
         out = torch.empty((batch * heads, q_len, dim), dtype=torch.bfloat16, device=self.device)
         with self._lock, self._on_device():
             self._call("mk_attention", self.lib.mk_attention(

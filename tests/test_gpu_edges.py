@@ -174,6 +174,27 @@ def test_prompt_attention_op_with_operands_on_any_word_and_infinite_masks(device
     assert (again[:, 5] == 0).all() and torch.equal(again[:, 6:], out[:, 6:])
 
 
+@pytest.mark.parametrize("keys", [40, 200])
+def test_prompt_attention_with_queries_at_an_odd_element(device, keys):
+    """The ops take them (a copy is attended), the C entry point refuses them and such outputs: the kernels read and write pairs."""
+    from megabake_b200 import _native
+    from megabake_b200.runtime import AttentionKernels
+
+    query, key, value = _tensors(device, 2, keys, keys, 6, 2, 64)
+    odd = torch.empty(query.numel() + 1, dtype=query.dtype, device=device)[1:].view(query.shape).copy_(query)
+    expected = torch.ops.megabake.attention(query, key, value, None, 0.125)
+    assert torch.equal(torch.ops.megabake.attention(odd, key, value, None, 0.125), expected)
+    with torch.inference_mode():
+        assert torch.equal(torch.ops.megabake.attention(odd, key, value, None, 0.125), expected)
+    kernels = AttentionKernels.for_shape(6, 2, 64, 2 * keys, device)
+    out = torch.full((expected.numel() + 1,), 7.0, dtype=torch.bfloat16, device=device)
+    for q, result in ((odd, out), (query, out[1:])):
+        code = kernels.lib.mk_attention(kernels._handle, q.data_ptr(), key.data_ptr(), value.data_ptr(), None, 0.125, 2, keys, keys,
+                                        result.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert code == _native.MK_ERR_ALIGNMENT
+    assert (out == 7.0).all()
+
+
 @pytest.mark.parametrize("sm_limit", [1, 7])
 @pytest.mark.parametrize("tokens", [50, 300])
 def test_prompts_on_few_sms(device, sm_limit, tokens):
