@@ -108,7 +108,7 @@ def _attention_cuda(query, key, value, mask, scale):
     if not query.is_cuda:
         return _attention_eager(query, key, value, mask, scale)
     batch, q_len, heads, dim = query.shape
-    kernels = _gpu_kernels(heads, key.shape[2], dim, batch * q_len, query.device)
+    kernels = _gpu_kernels(heads, key.shape[2], dim, 1, query.device)
     if mask is not None:
         if mask.dim() != 4 or mask.shape[1] != 1:
             mask = mask.expand(batch, heads, q_len, key.shape[1])

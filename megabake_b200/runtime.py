@@ -498,6 +498,10 @@ class AttentionKernels:
 
     _cache: dict = {}
     _cache_lock = threading.Lock()
+    # Objects that a larger one has replaced.  Captured graphs and launches in flight keep the addresses of their status word and
+    # control block, so they stay for the life of the process: one per doubling of the largest decode batch, together no
+    # larger than the one that is in use.
+    _superseded: list = []
 
     def __init__(self, q_heads: int, kv_heads: int, head_dim: int, max_tokens: int, device: torch.device):
         self.device = torch.device(device)
@@ -525,6 +529,7 @@ class AttentionKernels:
 
     @classmethod
     def for_shape(cls, q_heads: int, kv_heads: int, head_dim: int, tokens: int, device: torch.device) -> "AttentionKernels":
+        """``tokens``: sequences of a decode attention; prompt attention needs no room of its own (1)."""
         device = torch.device(device)
         if device.index is None:
             device = torch.device("cuda", torch.cuda.current_device())
@@ -535,6 +540,8 @@ class AttentionKernels:
                 capacity = max(16, 1 << (max(tokens, 1) - 1).bit_length())
                 found = cls(q_heads, kv_heads, head_dim, capacity, device)
                 _native.register_ops(*key, capacity, found._handle, found._mirror.data_ptr())
+                if key in cls._cache:
+                    cls._superseded.append(cls._cache[key])
                 cls._cache[key] = found
         return found
 

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from megabake_b200 import CompilerError, ops  # noqa: F401
+from megabake_b200.runtime import AttentionKernels
 from megabake_b200.synth import synth_normal
 
 pytestmark = pytest.mark.gpu
@@ -79,6 +80,27 @@ def test_a_result_that_wants_a_gradient_says_that_there_is_none():
         assert out.requires_grad
         with pytest.raises(RuntimeError, match="no autograd formula was registered"):
             out.float().sum().backward()
+
+
+def test_a_captured_prompt_op_outlives_longer_prompts_and_larger_batches():
+    """What a graph's launches point to stays where it is: memory that was free for others is written over before the replay."""
+    shape = (5, 5, 64)
+    args = [_tensor(name, 1, 200, 5, 64) for name in ("a", "b", "c")]
+    expected = torch.ops.megabake.attention(*args, None, 0.125)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = torch.ops.megabake.attention(*args, None, 0.125)
+    first = AttentionKernels.for_shape(*shape, 1, DEVICE)
+    torch.ops.megabake.attention(*[_tensor(name, 4, 900, 5, 64) for name in ("a", "b", "c")], None, 0.125)
+    assert AttentionKernels.for_shape(*shape, 1, DEVICE) is first  # a prompt of any length has room
+    torch.ops.megabake.kv_attention(*_kv_case(70, *shape, 17, 40, False))
+    assert AttentionKernels.for_shape(*shape, 1, DEVICE) is not first and first in AttentionKernels._superseded
+    torch.cuda.synchronize()
+    blocks = [torch.full((1 << 20,), -1, dtype=torch.int32, device=DEVICE) for _ in range(64)]
+    out.zero_()
+    graph.replay()
+    assert torch.equal(out, expected) and (first.workspace[:16] != 255).any()
+    del blocks
 
 
 def test_decode_op_in_a_captured_graph_and_on_two_streams():

@@ -24,6 +24,27 @@ def test_library_exports_every_declared_symbol():
         assert hasattr(lib, name), name
 
 
+def test_a_replaced_attention_object_stays_alive(monkeypatch):
+    """Captured graphs and launches in flight hold addresses of its workspace and status word."""
+    import gc
+    import weakref
+
+    from megabake_b200.runtime import AttentionKernels
+
+    def fake(self, q_heads, kv_heads, head_dim, max_tokens, device):
+        self.max_tokens, self._handle, self._mirror = max_tokens, None, torch.zeros(1, dtype=torch.int32)
+
+    monkeypatch.setattr(AttentionKernels, "__init__", fake)
+    monkeypatch.setattr(AttentionKernels, "_cache", {})
+    monkeypatch.setattr(AttentionKernels, "_superseded", [], raising=False)
+    monkeypatch.setattr(_native, "register_ops", lambda *args: None)
+    device = torch.device("cuda", 0)
+    replaced = [weakref.ref(AttentionKernels.for_shape(8, 2, 64, tokens, device)) for tokens in (1, 16, 17, 300)]
+    gc.collect()
+    assert all(ref() is not None for ref in replaced)
+    assert [ref().max_tokens for ref in replaced] == [16, 16, 32, 512] and replaced[0]() is replaced[1]()
+
+
 def test_option_validation_messages():
     with pytest.raises(ValueError, match="Unsupported mode"):
         megabake.make_backend(mode="train")
