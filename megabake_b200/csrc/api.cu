@@ -305,6 +305,7 @@ int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, int batch, int q_
 }  // namespace
 
 struct mk_handle_s {
+  bool quick_limit;     // tests: limits shorter than a launch
   mk_config cfg;
   int device, grid;
   uint8_t* ws;
@@ -507,6 +508,11 @@ bool stream_usable(mk_handle h, int batch, bool ragged) {
 
 int token_tiles(int m) { return (m + token_tile_of(m) - 1) / token_tile_of(m); }
 
+// No wait of the prompt kernels takes 64 tries while work goes on; a limit of less than a millisecond is looked at after each.
+PromptGuard prompt_guard(mk_handle h) {
+  return {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles, h->quick_limit ? 0u : 63u};
+}
+
 // What the two launches of a decode attention share.  The workspace has one such area: its users order their calls.
 struct KvScratch {
   uint32_t* verdict;
@@ -685,6 +691,7 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
   double ms = 2000.0;
   if (const char* env = getenv("MEGABAKE_WAIT_LIMIT_MS")) ms = atof(env) > 0 ? atof(env) : ms;
   h->timeout_cycles = static_cast<long long>(ms * static_cast<double>(facts.khz));
+  h->quick_limit = ms < 1.0;
   h->att_scale = static_cast<float>(std::pow(static_cast<double>(config->head_dim), -0.5));
   memset(&h->weights, 0, sizeof(h->weights));
   cudaError_t e = cudaMemsetAsync(workspace, 0, cv.total, static_cast<cudaStream_t>(stream));
@@ -1112,7 +1119,7 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
     pass.mask = static_cast<const bf16*>(mask);
     pass.logits = static_cast<bf16*>(logits);
     pass.m = static_cast<int>(m); pass.batch = batch; pass.seq = sequence;
-    pass.guard = {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles};
+    pass.guard = prompt_guard(h);
     const mk_config& c = h->cfg;
     const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
     AttnArgs A{};
@@ -1258,7 +1265,7 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   if (units > INT32_MAX) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %lld blocks of queries", units);
   AttnTcMaps maps{};
   if (int e = encode_attention_maps(&maps, A, batch, h->cfg.q_heads, h->cfg.kv_heads, h->cfg.head_dim)) return e;
-  MK_CUDA(prompt_attention_launch(A, maps, {at<Control>(h, h->cv.ctrl), h->mirror, h->timeout_cycles}, h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads,
+  MK_CUDA(prompt_attention_launch(A, maps, prompt_guard(h), h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads,
                                   batch, h->cfg.sm_limit > 0 ? h->grid : 0, false, static_cast<cudaStream_t>(stream)));
   h->launches += 1;
   return MK_OK;

@@ -62,6 +62,18 @@ __device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A launch that is given up: copies and MMAs under way end within microseconds.  A CTA stays for fifty, by the clock (a sleep may
+// be shorter than it was asked to be), before its shared and tensor memory are somebody else's.
+__device__ __forceinline__ void prompt_stay() {
+  unsigned long long begin, now;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(begin));
+  int looks = 0;
+  do {
+    __nanosleep(1000);
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+  } while (now - begin < 50000ull && ++looks < 10000);
+}
+
 __device__ __forceinline__ uint32_t ldcg_u32(const void* ptr) { return __ldcg(reinterpret_cast<const unsigned int*>(ptr)); }
 
 template <int HD> constexpr int kPromptPitch = HD * 2 + 16;  // bytes per tile row: 16 bytes of padding keep fragment loads conflict-free

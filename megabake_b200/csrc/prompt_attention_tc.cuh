@@ -99,7 +99,7 @@ __device__ __forceinline__ bool attn_wait(const AttnTcWait& w, uint64_t* bar, ui
   const uint32_t at = smem_u32(bar);
   uint32_t spins = 0;
   while (!mbar_try_wait(at, parity))
-    if ((++spins & 63u) == 0 && attn_give_up(w)) return false;
+    if ((++spins & w.guard->polls) == 0 && attn_give_up(w)) return false;
   return true;
 }
 
@@ -132,10 +132,7 @@ __device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWa
   }
   for (int t = 0; t < u.ntiles; ++t) {
     const int at = base + t, s = at % T::kStages, use = at / T::kStages;
-    if (use > 0 && !attn_wait(w, &misc->kvempty[s], (use - 1) & 1)) {
-      for (int i = 0; i < 32; ++i) __nanosleep(1000);  // copies under way land within microseconds
-      return;
-    }
+    if (use > 0 && !attn_wait(w, &misc->kvempty[s], (use - 1) & 1)) return;
     const uint32_t bar = smem_u32(&misc->kvfull[s]), dst = stages + s * T::kTile;
     mbar_expect_tx(bar, T::kTile);
     tma_load_4d(dst, &maps.k, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
@@ -427,10 +424,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
       const AttnTcUnit u = attn_unit(A, q_heads, kv_heads, batch, i);
       role(u);
       named_bar_sync(3, kAttnThreads);
-      if (*reinterpret_cast<volatile int*>(&misc.abort)) {  // MMAs that were issued end within a microsecond
-        __nanosleep(4000);
-        break;
-      }
+      if (*reinterpret_cast<volatile int*>(&misc.abort)) break;
       base += u.ntiles;
       uses[0] += (u.ntiles + 1) / 2;
       uses[1] += u.ntiles / 2;
@@ -475,6 +469,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
       fence_proxy_async_smem();
     });
   }
+  if (*reinterpret_cast<volatile int*>(&misc.abort)) prompt_stay();
   tc_fence_before();
   __syncthreads();
   if (warp == 10) {

@@ -140,7 +140,7 @@ __device__ __noinline__ bool prompt_give_up(const PromptWait& w, int site) {
 __device__ __forceinline__ bool prompt_wait(const PromptWait& w, uint32_t bar, uint32_t parity, int site) {
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity))
-    if ((++spins & 63u) == 0 && prompt_give_up(w, site)) return false;
+    if ((++spins & w.guard->polls) == 0 && prompt_give_up(w, site)) return false;
   return true;
 }
 
@@ -247,9 +247,7 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
   }
   // the MMA warp's last arrivals here, those of the pair's first CTA among them, come before this one leaves
   ok = ok && prompt_drain(n, stages, [&](int slot, uint32_t phase) { return prompt_wait(w, empty0 + slot * 8u, phase, SITE_DRAIN); });
-  // A pass that is given up: what was asked for lands within microseconds; the CTA stays for thirty.
-  if (!ok)
-    for (int i = 0; i < 32; ++i) __nanosleep(1000);
+  if (!ok) prompt_stay();
 }
 
 // KB: chunks per stage; BLOCKS: MMAs per K step (gate and up with accumulators of their own).
@@ -305,7 +303,10 @@ __device__ __noinline__ void prompt_mma_loop(const PromptGemm& g, uint32_t base,
   // memory: its last ones are here before this CTA leaves.
   if constexpr (CTAS == 2)
     for (int buf = 0; buf < min(kBuffers, q); ++buf)
-      if (!__all_sync(0xffffffffu, prompt_wait(w, accempty0 + buf * 8u, static_cast<uint32_t>((q - 1 - buf) / kBuffers) & 1u, SITE_MMA_ACC))) break;
+      if (!__all_sync(0xffffffffu, prompt_wait(w, accempty0 + buf * 8u, static_cast<uint32_t>((q - 1 - buf) / kBuffers) & 1u, SITE_MMA_ACC))) {
+        prompt_stay();  // (a give-up before this point leaves slots unread, and the copying warps stay)
+        break;
+      }
 }
 
 __device__ __forceinline__ void prompt_pack16(const float* v, uint32_t* w) {

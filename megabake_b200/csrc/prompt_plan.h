@@ -122,6 +122,7 @@ struct PromptGuard {
   Control* ctrl;
   volatile int* status_mirror;
   long long timeout_cycles;
+  uint32_t polls;  // a wait looks at its limit after every polls + 1 tries (a power of two)
 };
 
 struct PromptGemm {

@@ -217,6 +217,34 @@ def test_a_limit_that_runs_out_inside_a_launch_ends_it_and_the_handle_recovers(b
     assert torch.equal(step(reference)[0], expected)
 
 
+def _run_out(run, make, monkeypatch, limits=(0.0001, 0.001, 0.002, 0.003, 0.005, 0.01, 0.02, 0.03, 0.05, 100.0)):
+    """``run(kernel)`` -> (result, status) under limits shorter and longer than its waits: every launch ends, what is not reported
+    as TIMEOUT is right, and the last limit is never reached."""
+    expected, verdict = run(make())
+    assert verdict == "OK"
+    verdicts = []
+    for limit in limits:
+        monkeypatch.setenv("MEGABAKE_WAIT_LIMIT_MS", str(limit))
+        kernel = make()
+        for _ in range(4):
+            result, verdict = run(kernel)
+            verdicts.append(verdict)
+            assert verdict == "TIMEOUT" or (verdict == "OK" and torch.equal(result, expected))
+    assert "TIMEOUT" in verdicts[:4] and verdicts[-4:] == ["OK"] * 4
+    monkeypatch.delenv("MEGABAKE_WAIT_LIMIT_MS")
+    assert torch.equal(run(make())[0], expected)
+
+
+@pytest.mark.parametrize("tokens", [64, 128, 300])
+def test_a_limit_that_runs_out_inside_a_prompt_ends_it_and_the_handle_recovers(tokens, monkeypatch):
+    """One CTA per tile with 64 and 128 rows of tokens, CTA pairs and the tcgen05 attention."""
+    config = tiny_config(q_heads=8, kv_heads=8, hidden=512, intermediate=2048, layers=6)
+    weights = synth_weights(config, seed=18, norm_std=0.1, device=DEVICE)
+    ids = synth_ids(tokens, config.vocab, seed=18).view(1, tokens).to(DEVICE)
+    _run_out(lambda kernel: (kernel.prefill(ids), kernel.status()["status"]),
+             lambda: make_kernel(config, weights, max_tokens=tokens, max_positions=tokens), monkeypatch)
+
+
 @pytest.mark.parametrize("batch", [1, 6])
 def test_a_driver_that_refuses_the_cache_descriptors_leaves_the_tensor_engine(batch, monkeypatch):
     """From the first call on (the streaming kernel cannot do without the descriptors, the tensor engine can)."""
