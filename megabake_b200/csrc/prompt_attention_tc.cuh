@@ -423,8 +423,9 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
     for (int i = blockIdx.x; i < units; i += gridDim.x) {
       const AttnTcUnit u = attn_unit(A, q_heads, kv_heads, batch, i);
       role(u);
-      named_bar_sync(3, kAttnThreads);
-      if (*reinterpret_cast<volatile int*>(&misc.abort)) break;
+      // Given up or not is one answer for the block: a thread that saw the word set a unit early would not come to this barrier
+      // again, and the others would wait there for good.  (Whoever sets the word sees it set.)
+      if (named_bar_any(3, kAttnThreads, *reinterpret_cast<volatile int*>(&misc.abort) != 0)) break;
       base += u.ntiles;
       uses[0] += (u.ntiles + 1) / 2;
       uses[1] += u.ntiles / 2;

@@ -253,6 +253,18 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, uint32_t addr) {
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+// The same barrier, and whether any of the threads brought `value`: the same answer for all of them.
+__device__ __forceinline__ bool named_bar_any(int id, int threads, bool value) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(static_cast<uint32_t>(value)), "r"(id), "r"(threads)
+      : "memory");
+  return any != 0;
+}
 
 // Read-only 2-byte load.  The toolkit's __ldg overload for bf16 is a non-volatile
 // asm, which the compiler may hoist above a null-pointer guard; this one stays put.

@@ -235,14 +235,26 @@ def _run_out(run, make, monkeypatch, limits=(0.0001, 0.001, 0.002, 0.003, 0.005,
     assert torch.equal(run(make())[0], expected)
 
 
-@pytest.mark.parametrize("tokens", [64, 128, 300])
-def test_a_limit_that_runs_out_inside_a_prompt_ends_it_and_the_handle_recovers(tokens, monkeypatch):
-    """One CTA per tile with 64 and 128 rows of tokens, CTA pairs and the tcgen05 attention."""
+@pytest.mark.parametrize("tokens,sm_limit", [(64, 0), (128, 0), (300, 0), (64, 3), (300, 3)])
+def test_a_limit_that_runs_out_inside_a_prompt_ends_it_and_the_handle_recovers(tokens, sm_limit, monkeypatch):
+    """One CTA per tile with 64 and 128 rows of tokens, CTA pairs and the tcgen05 attention; on three SMs, many units to a CTA."""
     config = tiny_config(q_heads=8, kv_heads=8, hidden=512, intermediate=2048, layers=6)
     weights = synth_weights(config, seed=18, norm_std=0.1, device=DEVICE)
     ids = synth_ids(tokens, config.vocab, seed=18).view(1, tokens).to(DEVICE)
     _run_out(lambda kernel: (kernel.prefill(ids), kernel.status()["status"]),
-             lambda: make_kernel(config, weights, max_tokens=tokens, max_positions=tokens), monkeypatch)
+             lambda: make_kernel(config, weights, max_tokens=tokens, max_positions=tokens, sm_limit=sm_limit), monkeypatch)
+
+
+@pytest.mark.parametrize("head_dim,sm_limit", [(64, 0), (128, 0), (64, 5), (128, 5)])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_a_limit_that_runs_out_inside_prompt_attention_ends_it_and_the_handle_recovers(head_dim, sm_limit, offset, monkeypatch):
+    """Blocks of one unit and, on five SMs, of several; queries by TMA and, off the 16-byte grid, by plain loads."""
+    config = tiny_config(q_heads=6, kv_heads=2, head_dim=head_dim, hidden=512)
+    weights = synth_weights(config, seed=19, device=DEVICE)
+    query, key, value = (torch.randn((2, 700, heads, head_dim), device=DEVICE).bfloat16() for heads in (6, 2, 2))
+    query = torch.empty(query.numel() + offset, dtype=query.dtype, device=DEVICE)[offset:].view(query.shape).copy_(query)
+    _run_out(lambda kernel: (kernel.attention(query, key, value, None, 0.1), kernel.status()["status"]),
+             lambda: make_kernel(config, weights, max_tokens=16, max_positions=16, sm_limit=sm_limit), monkeypatch)
 
 
 @pytest.mark.parametrize("batch", [1, 6])
