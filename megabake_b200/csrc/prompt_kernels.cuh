@@ -299,14 +299,6 @@ __device__ __noinline__ void prompt_mma_loop(const PromptGemm& g, uint32_t base,
       }
     }
   }
-  // The pair's other CTA hands accumulators back by arrivals on this one's barriers, and the barrier at the end orders no
-  // memory: its last ones are here before this CTA leaves.
-  if constexpr (CTAS == 2)
-    for (int buf = 0; buf < min(kBuffers, q); ++buf)
-      if (!__all_sync(0xffffffffu, prompt_wait(w, accempty0 + buf * 8u, static_cast<uint32_t>((q - 1 - buf) / kBuffers) & 1u, SITE_MMA_ACC))) {
-        prompt_stay();  // (a give-up before this point leaves slots unread, and the copying warps stay)
-        break;
-      }
 }
 
 __device__ __forceinline__ void prompt_pack16(const float* v, uint32_t* w) {
@@ -476,7 +468,9 @@ __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t ac
     }
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) {
+    // The accumulator is handed back if another unit of this CTA's will use it: an arrival that nobody waits for could reach the
+    // pair's first CTA after it has left (the barrier at the end orders no memory).
+    if (lane == 0 && unit + g.buffers * step < g.units) {
       if constexpr (CTAS == 2) mbar_arrive_cluster(leader_address(accempty0 + buf * 8u));
       else mbar_arrive(accempty0 + buf * 8u);
     }
