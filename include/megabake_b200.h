@@ -226,6 +226,7 @@ int mk_kv_attention_scratch(mk_handle handle, const void* query, const void* key
  * bf16 [batch, k_len, kv_heads, head_dim], mask bf16 additive [batch, 1, q_len,
  * k_len] or NULL, output bf16 [batch*q_heads, q_len, head_dim].  key and value begin on 16-byte
  * boundaries, query and output on 4-byte ones (else MK_ERR_ALIGNMENT), the mask on any element.
+ * Rows that are given up because a wait ran out (MK_STATUS_TIMEOUT) are NaN.
  * Reference: src/megabake/lowering.py:273-300. */
 int mk_attention(mk_handle handle, const void* query, const void* key, const void* value,
                  const void* mask, float scale, int batch, int q_len, int k_len, void* output,

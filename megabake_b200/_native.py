@@ -23,6 +23,7 @@ ERROR_NAMES = {
 MK_ERR_INVALID, MK_ERR_UNSUPPORTED, MK_ERR_CUDA, MK_ERR_ALIGNMENT = 1, 2, 3, 4
 MK_ERR_WORKSPACE, MK_ERR_UNBOUND, MK_ERR_DEVICE_STATUS = 5, 6, 7
 STATUS_NAMES = {0: "OK", 1: "KV_OVERFLOW", 2: "BAD_INDEX", 3: "TIMEOUT"}
+STATUS_TIMEOUT = 3
 ROPE_STYLES = {"hf": 0, "half_swap": 1}
 ENGINES = {"tcgen05": 0, "fma": 2, "auto": 3}
 

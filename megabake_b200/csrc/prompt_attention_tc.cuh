@@ -87,11 +87,12 @@ static __device__ __noinline__ bool attn_give_up(const AttnTcWait& w) {
       ctrl->where = SITE_ATT_EXCHANGE;
       ctrl->cta = blockIdx.x;
       ctrl->detail = 0;
-      if (w.guard->status_mirror) *w.guard->status_mirror = static_cast<int>(MK_STATUS_TIMEOUT);
     }
     atomicExch(&ctrl->abort, 1u);
     __threadfence();
   }
+  // whatever was reported first, this is what the op looks for before its next call
+  if (w.guard->status_mirror) *w.guard->status_mirror = static_cast<int>(MK_STATUS_TIMEOUT);
   *reinterpret_cast<volatile int*>(&w.misc->abort) = 1;
   return true;
 }
@@ -209,6 +210,16 @@ __device__ __forceinline__ void attn_mask(const bf16* row, int j, int klen, bool
       word = next;
     }
   }
+}
+
+// The row of a unit that was given up: not a number, so that it cannot pass for a result.
+template <int HD>
+__device__ __forceinline__ void attn_store_nan(const AttnArgs& A, const AttnTcUnit& u, int row) {
+  const int r = u.q0 + row;
+  if (r >= A.sq) return;
+  uint32_t* const out = reinterpret_cast<uint32_t*>(A.out + u.b * A.out_bstride + static_cast<long long>(r) * A.out_tstride + u.h * A.out_hstride);
+#pragma unroll 1
+  for (int d = 0; d < HD / 2; ++d) out[d] = 0x7FC07FC0u;
 }
 
 // Warps 0 to 7.  A wait that was given up ends the loop; the block barriers behind it are passed all the same.
@@ -349,7 +360,9 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
     for (int d = 0; d < HD; ++d) exchange[(2 + d) * 128] = o[d];
   }
   named_bar_sync(1, 256);
-  if (g == 0 && r < A.sq && *reinterpret_cast<volatile int*>(&misc->abort) == 0) {
+  if (g == 0 && *reinterpret_cast<volatile int*>(&misc->abort) != 0) {
+    attn_store_nan<HD>(A, u, row);
+  } else if (g == 0 && r < A.sq) {
     const float om = exchange[0], ol = exchange[128], n = fmaxf(m, om);
     const float a = m > -INFINITY ? expf(m - n) : 0.f, b = om > -INFINITY ? expf(om - n) : 0.f;
     const float total = l * a + ol * b, d = total > 0.f ? total : 1.f;  // a row that sees no key: zeros
@@ -469,6 +482,8 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
       attn_softmax<HD>(A, w, &misc, u, smem, p, tmem, uses, warp, lane);
       fence_proxy_async_smem();
     });
+    if (tid < kAttnQueries && *reinterpret_cast<volatile int*>(&misc.abort))  // the units behind the one that was given up
+      for (int i = blockIdx.x + (done + 1) * gridDim.x; i < units; i += gridDim.x) attn_store_nan<HD>(A, attn_unit(A, q_heads, kv_heads, batch, i), tid);
   }
   if (*reinterpret_cast<volatile int*>(&misc.abort)) prompt_stay();
   tc_fence_before();

@@ -124,7 +124,7 @@ Tensor attention_now(const Tensor& query, const Tensor& key, const Tensor& value
   State& s = state();
   std::lock_guard<std::mutex> guard(s.lock);
   Kernels* const k = find(s, heads, kv_heads, dim, device.index());
-  if (k == nullptr) return {};
+  if (k == nullptr || *k->status == MK_STATUS_TIMEOUT) return {};
   const c10::cuda::CUDAGuard on(device);
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();

@@ -157,6 +157,12 @@ class DecoderKernel:
         if self._mirror_word.value != 0:
             self.check()
 
+    def raise_if_timed_out(self) -> None:
+        """The same for an op that only a wait that ran out concerns (``attention``: a full cache is ``kv_attention``'s affair)."""
+        if self._mirror_word.value == _native.STATUS_TIMEOUT:
+            self.check()
+            self._mirror_word.value = 0  # set by a launch on another stream, after the status had been read and put back
+
     def close(self) -> None:
         handle, self._handle = getattr(self, "_handle", None), None
         if handle:
@@ -437,6 +443,7 @@ class DecoderKernel:
             if mask.shape != (batch, 1, q_len, k_len) or not mask.is_contiguous():
                 mask = mask.expand(batch, 1, q_len, k_len).contiguous()
             _require(mask, "mask", dtype=torch.bfloat16, device=self.device)
+        self.raise_if_timed_out()
         if query.data_ptr() % 4:  # begins at an odd element: the kernels read pairs
             query = query.clone()
         out = torch.empty((batch * heads, q_len, dim), dtype=torch.bfloat16, device=self.device)
@@ -556,4 +563,5 @@ class AttentionKernels:
     status = DecoderKernel.status
     check = DecoderKernel.check
     raise_if_failed = DecoderKernel.raise_if_failed
+    raise_if_timed_out = DecoderKernel.raise_if_timed_out
     _install_status_mirror = DecoderKernel._install_status_mirror

@@ -217,7 +217,7 @@ def test_a_limit_that_runs_out_inside_a_launch_ends_it_and_the_handle_recovers(b
     assert torch.equal(step(reference)[0], expected)
 
 
-def _run_out(run, make, monkeypatch, limits=(0.0001, 0.001, 0.002, 0.003, 0.005, 0.01, 0.02, 0.03, 0.05, 100.0)):
+def _run_out(run, make, monkeypatch, limits=(0.0001, 0.001, 0.002, 0.003, 0.005, 0.01, 0.02, 0.03, 0.05, 100.0), rows=False):
     """``run(kernel)`` -> (result, status) under limits shorter and longer than its waits: every launch ends, what is not reported
     as TIMEOUT is right, and the last limit is never reached."""
     expected, verdict = run(make())
@@ -229,6 +229,9 @@ def _run_out(run, make, monkeypatch, limits=(0.0001, 0.001, 0.002, 0.003, 0.005,
         for _ in range(4):
             result, verdict = run(kernel)
             verdicts.append(verdict)
+            if rows:  # of a launch that was cut short: right, or not a number
+                whole, none = (result == expected).all(-1), torch.isnan(result).all(-1)
+                assert (whole | none).all() and (verdict == "TIMEOUT" or whole.all())
             assert verdict == "TIMEOUT" or (verdict == "OK" and torch.equal(result, expected))
     assert "TIMEOUT" in verdicts[:4] and verdicts[-4:] == ["OK"] * 4
     monkeypatch.delenv("MEGABAKE_WAIT_LIMIT_MS")
@@ -254,7 +257,32 @@ def test_a_limit_that_runs_out_inside_prompt_attention_ends_it_and_the_handle_re
     query, key, value = (torch.randn((2, 700, heads, head_dim), device=DEVICE).bfloat16() for heads in (6, 2, 2))
     query = torch.empty(query.numel() + offset, dtype=query.dtype, device=DEVICE)[offset:].view(query.shape).copy_(query)
     _run_out(lambda kernel: (kernel.attention(query, key, value, None, 0.1), kernel.status()["status"]),
-             lambda: make_kernel(config, weights, max_tokens=16, max_positions=16, sm_limit=sm_limit), monkeypatch)
+             lambda: make_kernel(config, weights, max_tokens=16, max_positions=16, sm_limit=sm_limit), monkeypatch, rows=True)
+
+
+def test_the_prompt_op_reports_a_limit_that_ran_out_and_only_that(monkeypatch):
+    """On both routes (inference mode takes the Python one), at the next call; a full cache stays kv_attention's to report."""
+    from megabake_b200 import CompilerError, ops  # noqa: F401
+
+    query, key, value = (torch.randn((1, 4000, 13, 64), device=DEVICE).bfloat16() for _ in range(3))  # heads of no other test
+    monkeypatch.setenv("MEGABAKE_WAIT_LIMIT_MS", "0.0001")
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            assert torch.isnan(torch.ops.megabake.attention(query, key, value, None, 0.125)).any()
+            torch.cuda.synchronize()
+            with pytest.raises(RuntimeError, match="TIMEOUT"):
+                torch.ops.megabake.attention(query, key, value, None, 0.125)
+    monkeypatch.delenv("MEGABAKE_WAIT_LIMIT_MS")  # (read when the handle of a head shape is made)
+    query, key, value = (t[:, :, :7].contiguous() for t in (query, key, value))
+    assert torch.isfinite(torch.ops.megabake.attention(query, key, value, None, 0.125)).all()
+    cache, full = torch.zeros((2, 1, 8, 7, 64), dtype=torch.bfloat16, device=DEVICE), torch.full((1,), 8, dtype=torch.int32, device=DEVICE)
+    torch.ops.megabake.kv_attention(*(t[:, :1] for t in (query, key, value)), cache[0], cache[1], full)
+    torch.cuda.synchronize()
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            assert torch.isfinite(torch.ops.megabake.attention(query, key, value, None, 0.125)).all()
+    with pytest.raises(CompilerError, match="exceeds capacity"):
+        torch.ops.megabake.kv_attention(*(t[:, :1] for t in (query, key, value)), cache[0], cache[1], full)
 
 
 @pytest.mark.parametrize("batch", [1, 6])
