@@ -141,19 +141,21 @@ __device__ __forceinline__ void prompt_unit(const AttnArgs& A, int q_heads, int 
   const bf16* mrow0 = A.mask + (static_cast<long long>(b) * A.sq + r0c) * A.klen;
   const bf16* mrow1 = A.mask + (static_cast<long long>(b) * A.sq + r1c) * A.klen;
   uint32_t mk[4][2];  // mask of this warp's half of the coming tile: [8-key block][row]
-  auto load_mask = [&](int s) {
+  auto load_mask = [&](int s) {  // (plain loads: the kernel that writes the mask may be at work while this one begins)
     if (!A.mask) return;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       const int j = s * kPromptKeys + kh * 32 + nt * 8 + t * 2;
       if (pairs) {
         const int at = min(j, A.klen - 2);
-        mk[nt][0] = __ldg(reinterpret_cast<const unsigned int*>(mrow0 + at));
-        mk[nt][1] = __ldg(reinterpret_cast<const unsigned int*>(mrow1 + at));
+        mk[nt][0] = *reinterpret_cast<const unsigned int*>(mrow0 + at);
+        mk[nt][1] = *reinterpret_cast<const unsigned int*>(mrow1 + at);
       } else {
         const int at = min(j, A.klen - 1), at1 = min(j + 1, A.klen - 1);
-        mk[nt][0] = pack2(ldg_bf16(mrow0 + at), ldg_bf16(mrow0 + at1));
-        mk[nt][1] = pack2(ldg_bf16(mrow1 + at), ldg_bf16(mrow1 + at1));
+        const unsigned short* const row0 = reinterpret_cast<const unsigned short*>(mrow0);
+        const unsigned short* const row1 = reinterpret_cast<const unsigned short*>(mrow1);
+        mk[nt][0] = row0[at] | static_cast<uint32_t>(row0[at1]) << 16;
+        mk[nt][1] = row1[at] | static_cast<uint32_t>(row1[at1]) << 16;
       }
     }
   };

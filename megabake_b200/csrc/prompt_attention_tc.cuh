@@ -189,12 +189,13 @@ __device__ __forceinline__ void attn_mma(const AttnTcWait& w, AttnTcMisc* misc, 
 
 // The mask of a thread's row for 64 positions from j on, as bf16 pairs.  `wide`: rows begin on 16-byte boundaries.  Otherwise the
 // aligned words that hold the elements, shifted into place; past the row's last word it is repeated (those positions are
-// masked below).
+// masked below).  Plain loads: the kernel that writes the mask may be at work while this one begins, which the read-only path
+// does not allow, and no compiler moves them ahead of griddepcontrol.wait.
 __device__ __forceinline__ void attn_mask(const bf16* row, int j, int klen, bool wide, uint32_t (&m)[32]) {
   if (wide && j + 64 <= klen) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + j) + i);
+      const uint4 v = reinterpret_cast<const uint4*>(row + j)[i];
       m[4 * i] = v.x; m[4 * i + 1] = v.y; m[4 * i + 2] = v.z; m[4 * i + 3] = v.w;
     }
   } else {
@@ -202,10 +203,10 @@ __device__ __forceinline__ void attn_mask(const bf16* row, int j, int klen, bool
     const uint32_t shift = (reinterpret_cast<uintptr_t>(row + j) & 2) ? 16u : 0u;
     const int last = static_cast<int>((reinterpret_cast<uintptr_t>(row + klen - 1) - first) >> 2);  // the word of the last position
     const unsigned int* const words = reinterpret_cast<const unsigned int*>(first);
-    uint32_t word = __ldg(words);
+    uint32_t word = words[0];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      const uint32_t next = __ldg(words + min(i + 1, last));
+      const uint32_t next = words[min(i + 1, last)];
       m[i] = __funnelshift_r(word, next, shift);
       word = next;
     }

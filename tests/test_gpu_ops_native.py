@@ -52,6 +52,22 @@ def test_prompt_op_is_the_same_on_both_routes(shape, mask):
         assert torch.equal(out, expected)
 
 
+@pytest.mark.parametrize("keys", [48, 333, 512])
+def test_a_mask_written_by_the_kernel_right_before(keys):
+    """The op's kernel begins while that one is at work: every call sees its own mask."""
+    q, k, v = (_tensor(name, 1, keys, 8, 64) for name in ("a", "b", "c"))
+    masks = [_tensor(f"m{i}", 1, 1, keys, keys) for i in range(4)]
+    expected = [torch.ops.megabake.attention(q, k, v, m, 0.125) for m in masks]
+    mask = torch.empty_like(masks[0])
+    torch.cuda.synchronize()
+    results = []
+    for _ in range(10):
+        for m in masks:
+            mask.copy_(m)
+            results.append(torch.ops.megabake.attention(q, k, v, mask, 0.125))
+    assert all(torch.equal(r, expected[i % 4]) for i, r in enumerate(results))
+
+
 def test_what_the_ops_refuse_is_refused_on_both_routes():
     good = _kv_case(2, 4, 2, 64, 3, 8, False)
     torch.ops.megabake.kv_attention(*good)

@@ -45,6 +45,13 @@ def test_a_replaced_attention_object_stays_alive(monkeypatch):
     assert [ref().max_tokens for ref in replaced] == [16, 16, 32, 512] and replaced[0]() is replaced[1]()
 
 
+def test_dependent_attention_kernels_read_nothing_through_the_read_only_path():
+    """They begin while the kernels before them write their operands; that path is for memory nobody writes meanwhile."""
+    for name in ("prompt_attention.cuh", "prompt_attention_tc.cuh", "kv_attention.cuh"):
+        source = (ROOT / "megabake_b200" / "csrc" / name).read_text()
+        assert not re.findall(r"\b__ldg\b|\bldg_\w+\(|ld\.global\.nc", source), name
+
+
 def test_option_validation_messages():
     with pytest.raises(ValueError, match="Unsupported mode"):
         megabake.make_backend(mode="train")
