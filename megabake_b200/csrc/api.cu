@@ -1266,7 +1266,7 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   AttnTcMaps maps{};
   if (int e = encode_attention_maps(&maps, A, batch, h->cfg.q_heads, h->cfg.kv_heads, h->cfg.head_dim)) return e;
   MK_CUDA(prompt_attention_launch(A, maps, prompt_guard(h), h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads,
-                                  batch, h->cfg.sm_limit > 0 ? h->grid : 0, false, static_cast<cudaStream_t>(stream)));
+                                  batch, h->grid, h->cfg.sm_limit > 0, false, static_cast<cudaStream_t>(stream)));
   h->launches += 1;
   return MK_OK;
 }

@@ -68,18 +68,22 @@ cudaError_t prompt_prepare() {
   return e;
 }
 
-// Where each kernel is the faster one (1.7B shape, us).  On its own, 32 heads with a mask: 64 positions 9.3 with blocks of 64
-// queries on mma.sync, 10.0 with blocks of 128 on tcgen05, half of whose rows are idle then; 128 positions 9.7 and 7.6, 256 13.8 and
-// 9.9, 512 21.6 and 14.3.  In a prompt pass, where the projections' shared memory keeps its tensor memory and barriers from
-// being set up ahead and tiles past the diagonal are not visited: 64 tokens 1266 and 1307 for the whole pass, 200 1774 and 1771,
-// 500 2588 and 2496; 135M shape, 250 tokens 1257 and 1281.
-constexpr int kAttnTcAlone = 65, kAttnTcInPass = 257;
+// In a prompt pass, where the projections' shared memory keeps the tcgen05 kernel's tensor memory and barriers from being set up
+// ahead and tiles past the diagonal are not visited, it is the faster one from here on (1.7B shape, us for the whole pass: 64 tokens
+// 1266 on mma.sync and 1307, 200 1774 and 1771, 500 2588 and 2496; 135M shape, 250 tokens 1257 and 1281).  On its own:
+// attention_on_tcgen05.
+constexpr int kAttnTcInPass = 257;
+
+static bool prompt_attention_tc_wanted(const AttnArgs& args, int head_dim, int q_heads, int batch, int sms, bool limited, bool in_pass) {
+  if (in_pass) return args.klen >= kAttnTcInPass;
+  return attention_on_tcgen05(head_dim, args.sq, args.klen, static_cast<long long>(batch) * q_heads, args.mask != nullptr, sms, limited);
+}
 
 cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps, const PromptGuard& guard, int head_dim, int q_heads, int kv_heads,
-                                    int batch, int limit, bool in_pass, cudaStream_t stream) {
-  const bool tc = args.klen >= (in_pass ? kAttnTcInPass : kAttnTcAlone);
+                                    int batch, int sms, bool limited, bool in_pass, cudaStream_t stream) {
+  const bool tc = prompt_attention_tc_wanted(args, head_dim, q_heads, batch, sms, limited, in_pass);
   const int per = tc ? kAttnQueries : kPromptQueries, units = batch * q_heads * ((args.sq + per - 1) / per);
-  const int blocks = limit > 0 ? std::min(units, limit) : units;
+  const int blocks = limited ? std::min(units, sms) : units;
   // Everything a kernel reads or writes comes behind its griddepcontrol.wait, so that it may be launched as a dependent one behind
   // any kernel: two to three microseconds less between the two.
   if (tc) {
@@ -143,7 +147,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
   norm.embed_rows = c.embed_rows > 0 ? c.embed_rows : c.vocab;
   norm.max_positions = c.max_positions;
   norm.eps = c.rms_eps;
-  const int limit = c.sm_limit > 0 ? pass.grid : 0, rows = c.sm_limit > 0 ? std::min(m, pass.grid) : m;
+  const int rows = c.sm_limit > 0 ? std::min(m, pass.grid) : m;
   cudaError_t e = cudaSuccess;
   for (int l = 0; l <= c.layers && e == cudaSuccess; ++l) {
     const bool head = l == c.layers;
@@ -179,7 +183,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     g.sin_t = static_cast<const bf16*>(w.rope_sin);
     g.pos = pass.pos;
     e = launch_gemm<PE_QKV>(g, cls, pass.grid, stream);
-    if (e == cudaSuccess) e = prompt_attention_launch(*pass.attention, *pass.attention_maps, pass.guard, c.head_dim, c.q_heads, c.kv_heads, pass.batch, limit, true, stream);
+    if (e == cudaSuccess) e = prompt_attention_launch(*pass.attention, *pass.attention_maps, pass.guard, c.head_dim, c.q_heads, c.kv_heads, pass.batch, pass.grid, c.sm_limit > 0, true, stream);
     if (e != cudaSuccess) return e;
     g = gemm(PP_O, kOperandAttn);
     g.b[0] = maps + 3;

@@ -101,6 +101,30 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
   }
 }
 
+// Whether a call of the attention op (not causal; heads: of all sequences) goes to the tcgen05 kernel, with blocks of 128 queries,
+// or to the one on mma.sync, with blocks of 64.  Times in us of a round of blocks as fitted to both kernels over heads 9 to 1024, 1 to
+// 320 queries and 64 to 1400 keys: the first has one block to an SM and half the time per tile of 64 keys; the second has two with head size
+// 64, and half the idle rows where the queries are few.  32 heads of 64 x 32 sequences, one query and 128 keys: 52.6 us on tcgen05, 28.7
+// on mma.sync; 64 x 128 54.8 and 37.4 with a mask; 128 x 512 100 and 146.
+inline bool attention_on_tcgen05(int head_dim, int q_len, int k_len, long long heads, bool masked, int sms, bool limited) {
+  if (k_len < 65) return false;  // one tile: 9.3 us against 10.0 for 32 heads of 64 x 64 with a mask
+  const double tiles = (k_len + 63) / 64;
+  const long long wide = heads * ((q_len + 127) / 128), narrow = heads * ((q_len + 63) / 64);
+  auto rounds = [](long long blocks, int resident) -> double {  // the last one counts whole, but not beside many
+    const double exact = static_cast<double>(blocks) / resident;
+    const long long whole = (blocks + resident - 1) / resident;
+    return whole > 4 ? exact : static_cast<double>(whole);
+  };
+  if (head_dim == 128) {  // one block to an SM either way
+    if (q_len > 8) return true;
+    return rounds(wide, sms) * (6.7 + (2 * wide <= sms ? 1.2 : 1.5) * tiles) <= rounds(narrow, sms) * (5.15 + 1.64 * tiles);
+  }
+  const double first = wide <= sms ? 5.3 + 0.91 * tiles : rounds(wide, sms) * (5.9 + 0.92 * tiles);
+  const double second = narrow <= sms || limited ? rounds(narrow, sms) * ((q_len <= 16 ? 4.2 : 5.2) + (masked ? 1.25 : 1.08) * tiles)
+                                                 : rounds(narrow, 2 * sms) * (6.2 + (masked ? 1.87 : 1.57) * tiles);
+  return first <= second;
+}
+
 // What a CTA still waits for before it leaves: that the last use of every pipeline slot has been consumed, so that no commit
 // is on its way to a barrier of shared memory that is somebody else's by then.  The uses count up over the launch, use u lies in
 // slot u % stages, and a slot's barrier has the parity of its use; wait(slot, parity) returns false to give up.
@@ -184,8 +208,8 @@ struct PromptPass {
 
 cudaError_t prompt_prepare();  // shared-memory attributes of the kernels, on the current device
 cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream);
-// limit: blocks of the launch at most, or 0.
+// sms: the SMs to use; limited: no more blocks than that; in_pass: causal, of a prompt pass.
 cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps, const PromptGuard& guard, int head_dim, int q_heads, int kv_heads,
-                                    int batch, int limit, bool in_pass, cudaStream_t stream);
+                                    int batch, int sms, bool limited, bool in_pass, cudaStream_t stream);
 
 }  // namespace mk
