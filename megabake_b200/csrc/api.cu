@@ -295,7 +295,9 @@ int encode_attention_map(CUtensorMap* out, const void* base, int batch, int rows
   if (r != CUDA_SUCCESS) return fail(MK_ERR_CUDA, "cuTensorMapEncodeTiled (attention) failed with %d", (int)r);
   return MK_OK;
 }
-int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, int batch, int q_heads, int kv_heads, int head_dim) {
+int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, const mk_config& c, int grid, int batch, bool in_pass) {
+  const int q_heads = c.q_heads, kv_heads = c.kv_heads, head_dim = c.head_dim;
+  if (!prompt_attention_tc_wanted(A, head_dim, q_heads, batch, grid, c.sm_limit > 0, in_pass)) return MK_OK;  // nobody reads them
   maps->q_ok = (reinterpret_cast<uintptr_t>(A.q) & 15) == 0;
   if (int e = encode_attention_map(&maps->k, A.k, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
   if (int e = encode_attention_map(&maps->v, A.v, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
@@ -1129,7 +1131,7 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
     A.out = pass.attn; A.out_bstride = static_cast<long long>(sequence) * q_size; A.out_tstride = q_size; A.out_hstride = c.head_dim;
     A.mask = pass.mask; A.sq = A.klen = sequence; A.causal = pass.mask == nullptr; A.scale = h->att_scale;
     AttnTcMaps maps{};
-    if (int e = encode_attention_maps(&maps, A, batch, c.q_heads, c.kv_heads, c.head_dim)) return e;
+    if (int e = encode_attention_maps(&maps, A, c, h->grid, batch, true)) return e;
     pass.attention = &A;
     pass.attention_maps = &maps;
     MK_CUDA(prompt_forward(pass, static_cast<cudaStream_t>(stream)));
@@ -1264,7 +1266,7 @@ int mk_attention(mk_handle h, const void* query, const void* key, const void* va
   const long long units = static_cast<long long>(batch) * h->cfg.q_heads * ((q_len + kPromptQueries - 1) / kPromptQueries);
   if (units > INT32_MAX) return fail(MK_ERR_UNSUPPORTED, "mk_attention: %lld blocks of queries", units);
   AttnTcMaps maps{};
-  if (int e = encode_attention_maps(&maps, A, batch, h->cfg.q_heads, h->cfg.kv_heads, h->cfg.head_dim)) return e;
+  if (int e = encode_attention_maps(&maps, A, h->cfg, h->grid, batch, false)) return e;
   MK_CUDA(prompt_attention_launch(A, maps, prompt_guard(h), h->cfg.head_dim, h->cfg.q_heads, h->cfg.kv_heads,
                                   batch, h->grid, h->cfg.sm_limit > 0, false, static_cast<cudaStream_t>(stream)));
   h->launches += 1;

@@ -74,7 +74,7 @@ cudaError_t prompt_prepare() {
 // attention_on_tcgen05.
 constexpr int kAttnTcInPass = 257;
 
-static bool prompt_attention_tc_wanted(const AttnArgs& args, int head_dim, int q_heads, int batch, int sms, bool limited, bool in_pass) {
+bool prompt_attention_tc_wanted(const AttnArgs& args, int head_dim, int q_heads, int batch, int sms, bool limited, bool in_pass) {
   if (in_pass) return args.klen >= kAttnTcInPass;
   return attention_on_tcgen05(head_dim, args.sq, args.klen, static_cast<long long>(batch) * q_heads, args.mask != nullptr, sms, limited);
 }

@@ -208,6 +208,8 @@ struct PromptPass {
 
 cudaError_t prompt_prepare();  // shared-memory attributes of the kernels, on the current device
 cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream);
+// Whether a launch takes the tcgen05 kernel, the one that reads its operands through `maps`.
+bool prompt_attention_tc_wanted(const AttnArgs& args, int head_dim, int q_heads, int batch, int sms, bool limited, bool in_pass);
 // sms: the SMs to use; limited: no more blocks than that; in_pass: causal, of a prompt pass.
 cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps, const PromptGuard& guard, int head_dim, int q_heads, int kv_heads,
                                     int batch, int sms, bool limited, bool in_pass, cudaStream_t stream);
