@@ -24,7 +24,7 @@ namespace {
 
 using at::Tensor;
 
-// The library's entry points, handed over with the first handle: it is loaded by path, and this file links to nothing of it.
+// The library's entry points, handed over with the handle: it is loaded by path, and this file links to nothing of it.
 struct Entries {
   decltype(&mk_kv_attention_scratch) kv_attention;
   decltype(&mk_kv_attention_scratch_bytes) scratch_bytes;
@@ -39,29 +39,38 @@ struct Scratch {
 };
 constexpr size_t kStreams = 8;
 
+// What serves a head shape on a device.  Made once, never destroyed: its tensors would outlive the allocator.
 struct Kernels {
-  int64_t heads, kv_heads, head_dim;
-  int device;
-  mk_handle handle;
-  int64_t max_tokens;
-  const volatile int32_t* status;  // pinned word a failed launch sets
+  const int64_t heads, kv_heads, head_dim;
+  const int device;
+  std::mutex lock;  // of what follows, held for a call: calls of other shapes and devices go on beside it
+  Entries entries{};
+  mk_handle handle = nullptr;
+  int64_t max_tokens = 0;
+  const volatile int32_t* status = nullptr;  // pinned word a failed launch sets
   std::vector<Scratch> scratch;
+
+  Kernels(int64_t heads, int64_t kv_heads, int64_t head_dim, int device) : heads(heads), kv_heads(kv_heads), head_dim(head_dim), device(device) {}
 };
 
 struct State {
-  std::mutex lock;
-  Entries entries{};
-  std::vector<Kernels> known;  // one per shape and device, a handful
+  std::mutex lock;  // of the list, held for a look at it
+  std::vector<Kernels*> known;  // one per shape and device, a handful
 };
 State& state() {
-  static State* const s = new State;  // not destroyed: its tensors would outlive the allocator
+  static State* const s = new State;
   return *s;
 }
 
 Kernels* find(State& s, int64_t heads, int64_t kv_heads, int64_t head_dim, int device) {
-  for (Kernels& k : s.known)
-    if (k.heads == heads && k.kv_heads == kv_heads && k.head_dim == head_dim && k.device == device) return &k;
+  for (Kernels* k : s.known)
+    if (k->heads == heads && k->kv_heads == kv_heads && k->head_dim == head_dim && k->device == device) return k;
   return nullptr;
+}
+Kernels* find(int64_t heads, int64_t kv_heads, int64_t head_dim, int device) {
+  State& s = state();
+  std::lock_guard<std::mutex> guard(s.lock);
+  return find(s, heads, kv_heads, head_dim, device);
 }
 
 bool plain(const Tensor& t, at::ScalarType type, c10::Device device) {
@@ -84,10 +93,10 @@ Tensor kv_attention_now(const Tensor& source, const Tensor& key, const Tensor& v
       !is_shape(value_cache, batch, capacity, kv_heads, dim) || !key_cache.is_contiguous() || !value_cache.is_contiguous())
     return {};
   if (!plain(valid_length, at::kInt, device) || valid_length.dim() != 1 || valid_length.size(0) != 1 || !valid_length.is_contiguous()) return {};
-  State& s = state();
-  std::lock_guard<std::mutex> guard(s.lock);
-  Kernels* const k = find(s, heads, kv_heads, dim, device.index());
-  if (k == nullptr || batch > k->max_tokens || *k->status != 0) return {};
+  Kernels* const k = find(heads, kv_heads, dim, device.index());
+  if (k == nullptr) return {};
+  std::lock_guard<std::mutex> guard(k->lock);
+  if (k->handle == nullptr || batch > k->max_tokens || *k->status != 0) return {};
   const c10::cuda::CUDAGuard on(device);
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
@@ -99,15 +108,15 @@ Tensor kv_attention_now(const Tensor& source, const Tensor& key, const Tensor& v
       else k->scratch.erase(k->scratch.begin() + i);
     }
   if (!memory.defined()) {
-    memory = at::empty({static_cast<int64_t>(s.entries.scratch_bytes(batch, heads, dim))}, source.options().dtype(at::kByte));
+    memory = at::empty({static_cast<int64_t>(k->entries.scratch_bytes(batch, heads, dim))}, source.options().dtype(at::kByte));
     if (k->scratch.size() >= kStreams) k->scratch.erase(k->scratch.begin());
     k->scratch.push_back({stream, batch, memory});
   }
   Tensor out = at::empty({batch * heads, 1, dim}, source.options());
-  const int code = s.entries.kv_attention(k->handle, q.const_data_ptr(), kn.const_data_ptr(), vn.const_data_ptr(), key_cache.mutable_data_ptr(),
-                                          value_cache.mutable_data_ptr(), static_cast<int32_t*>(valid_length.mutable_data_ptr()), static_cast<int>(batch),
-                                          static_cast<int>(capacity), out.mutable_data_ptr(), memory.mutable_data_ptr(),
-                                          static_cast<size_t>(memory.numel()), stream);
+  const int code = k->entries.kv_attention(k->handle, q.const_data_ptr(), kn.const_data_ptr(), vn.const_data_ptr(), key_cache.mutable_data_ptr(),
+                                           value_cache.mutable_data_ptr(), static_cast<int32_t*>(valid_length.mutable_data_ptr()), static_cast<int>(batch),
+                                           static_cast<int>(capacity), out.mutable_data_ptr(), memory.mutable_data_ptr(),
+                                           static_cast<size_t>(memory.numel()), stream);
   return code == MK_OK ? out : Tensor();
 }
 
@@ -121,10 +130,10 @@ Tensor attention_now(const Tensor& query, const Tensor& key, const Tensor& value
   if (!is_shape(key, batch, k_len, kv_heads, dim) || !is_shape(value, batch, k_len, kv_heads, dim)) return {};
   const bool masked = mask.has_value() && mask->defined();
   if (masked && (!plain(*mask, at::kBFloat16, device) || !is_shape(*mask, batch, 1, q_len, k_len) || !mask->is_contiguous())) return {};
-  State& s = state();
-  std::lock_guard<std::mutex> guard(s.lock);
-  Kernels* const k = find(s, heads, kv_heads, dim, device.index());
-  if (k == nullptr || *k->status == MK_STATUS_TIMEOUT) return {};
+  Kernels* const k = find(heads, kv_heads, dim, device.index());
+  if (k == nullptr) return {};
+  std::lock_guard<std::mutex> guard(k->lock);
+  if (k->handle == nullptr || *k->status == MK_STATUS_TIMEOUT) return {};
   const c10::cuda::CUDAGuard on(device);
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return {};
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
@@ -132,9 +141,9 @@ Tensor attention_now(const Tensor& query, const Tensor& key, const Tensor& value
   Tensor q = query.contiguous();
   if (reinterpret_cast<uintptr_t>(q.const_data_ptr()) % 4) q = q.clone();  // begins at an odd element: the kernels read pairs
   Tensor out = at::empty({batch * heads, q_len, dim}, query.options());
-  const int code = s.entries.attention(k->handle, q.const_data_ptr(), kk.const_data_ptr(), vv.const_data_ptr(), masked ? mask->const_data_ptr() : nullptr,
-                                       static_cast<float>(scale), static_cast<int>(batch), static_cast<int>(q_len), static_cast<int>(k_len),
-                                       out.mutable_data_ptr(), stream);
+  const int code = k->entries.attention(k->handle, q.const_data_ptr(), kk.const_data_ptr(), vv.const_data_ptr(), masked ? mask->const_data_ptr() : nullptr,
+                                        static_cast<float>(scale), static_cast<int>(batch), static_cast<int>(q_len), static_cast<int>(k_len),
+                                        out.mutable_data_ptr(), stream);
   return code == MK_OK ? out : Tensor();
 }
 
@@ -225,15 +234,20 @@ TORCH_LIBRARY_IMPL(megabake, AutogradCUDA, m) {
 extern "C" void megabake_ops_register(int64_t heads, int64_t kv_heads, int64_t head_dim, int device, int64_t max_tokens, void* handle,
                                       const int32_t* status, void* kv_attention_entry, void* scratch_bytes_entry, void* attention_entry) {
   State& s = state();
-  std::lock_guard<std::mutex> guard(s.lock);
-  s.entries.kv_attention = reinterpret_cast<decltype(&mk_kv_attention_scratch)>(kv_attention_entry);
-  s.entries.scratch_bytes = reinterpret_cast<decltype(&mk_kv_attention_scratch_bytes)>(scratch_bytes_entry);
-  s.entries.attention = reinterpret_cast<decltype(&mk_attention)>(attention_entry);
-  Kernels* k = find(s, heads, kv_heads, head_dim, device);
-  if (k == nullptr) {
-    s.known.push_back({heads, kv_heads, head_dim, device, nullptr, 0, nullptr, {}});
-    k = &s.known.back();
+  Kernels* k;
+  {
+    std::lock_guard<std::mutex> guard(s.lock);
+    k = find(s, heads, kv_heads, head_dim, device);
+    if (k == nullptr) {
+      k = new Kernels(heads, kv_heads, head_dim, device);
+      k->status = status;
+      s.known.push_back(k);
+    }
   }
+  std::lock_guard<std::mutex> guard(k->lock);
+  k->entries.kv_attention = reinterpret_cast<decltype(&mk_kv_attention_scratch)>(kv_attention_entry);
+  k->entries.scratch_bytes = reinterpret_cast<decltype(&mk_kv_attention_scratch_bytes)>(scratch_bytes_entry);
+  k->entries.attention = reinterpret_cast<decltype(&mk_attention)>(attention_entry);
   k->handle = static_cast<mk_handle>(handle);
   k->max_tokens = max_tokens;
   k->status = status;

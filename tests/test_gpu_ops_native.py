@@ -1,9 +1,12 @@
 """The two ops through their native registration against the same calls through the Python one, which inference mode takes."""
 
+import ctypes
+import threading
+
 import pytest
 import torch
 
-from megabake_b200 import CompilerError, ops  # noqa: F401
+from megabake_b200 import CompilerError, _native, ops  # noqa: F401
 from megabake_b200.runtime import AttentionKernels
 from megabake_b200.synth import synth_normal
 
@@ -96,6 +99,37 @@ def test_a_result_that_wants_a_gradient_says_that_there_is_none():
         assert out.requires_grad
         with pytest.raises(RuntimeError, match="no autograd formula was registered"):
             out.float().sum().backward()
+
+
+def test_a_call_does_not_wait_for_one_of_another_head_shape():
+    """The library's entry for one shape is replaced by one that waits; meanwhile a call of another shape comes and goes."""
+    slow, quick = ([_tensor(name, 1, 80, heads, 64) for name in ("a", "b", "c")] for heads in (15, 12))
+    expected = [torch.ops.megabake.attention(*args, None, 0.125) for args in (slow, quick)][1]
+    kernels = AttentionKernels.for_shape(15, 15, 64, 1, DEVICE)
+    entered, go_on = threading.Event(), threading.Event()
+
+    @ctypes.CFUNCTYPE(ctypes.c_int, *[ctypes.c_void_p] * 5, ctypes.c_float, *[ctypes.c_int] * 3, ctypes.c_void_p, ctypes.c_void_p)
+    def waits(*args):
+        entered.set()
+        go_on.wait(20)
+        return _native.MK_OK  # (its result is memory as it was allocated, and not looked at)
+
+    def register(entry):
+        lib = _native.load()
+        entries = [ctypes.cast(e, ctypes.c_void_p) for e in (lib.mk_kv_attention_scratch, lib.mk_kv_attention_scratch_bytes, entry)]
+        _native._ops_library.megabake_ops_register(15, 15, 64, 0, kernels.max_tokens, kernels._handle, kernels._mirror.data_ptr(), *entries)
+
+    register(waits)
+    thread = threading.Thread(target=lambda: torch.ops.megabake.attention(*slow, None, 0.125))
+    try:
+        thread.start()
+        assert entered.wait(20)
+        out = torch.ops.megabake.attention(*quick, None, 0.125)
+        assert thread.is_alive() and torch.equal(out, expected)
+    finally:
+        go_on.set()
+        thread.join()
+        register(_native.load().mk_attention)
 
 
 def test_a_captured_prompt_op_outlives_longer_prompts_and_larger_batches():
