@@ -6,11 +6,13 @@ There is no fallback: if the library is missing or a call fails, this raises.
 from __future__ import annotations
 
 import ctypes
+import warnings
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
+from .build import ops_library
+
 LIBRARY_PATH = Path(__file__).resolve().parent / "libmegabake_b200.so"
-OPS_LIBRARY_PATH = LIBRARY_PATH.with_name("libmegabake_b200_ops.so")
 
 MK_MAX_LAYERS = 96
 MK_TOKEN_TILE = 16
@@ -173,19 +175,26 @@ def check(function: str, code: int) -> None:
         raise NativeError(function, code, load().mk_last_error().decode(errors="replace"))
 
 
-_ops_library = None
+_ops_library = None  # False: it is not there, and that has been said
 
 
 def register_ops(heads: int, kv_heads: int, head_dim: int, device: int, max_tokens: int, handle, status_address: int) -> None:
     """Give the ops' C++ registration (csrc/torch_ops.cpp) the handle that serves a head shape on a device; loads the library,
-    and with it the registration, the first time."""
+    and with it the registration, the first time.  Without it (not built, or not for this PyTorch) the same launches are made
+    through Python, 20 to 30 us of host time a call."""
     global _ops_library
     if _ops_library is None:
-        if not OPS_LIBRARY_PATH.exists():
-            raise RuntimeError(f"{OPS_LIBRARY_PATH} is missing: run `python -m megabake_b200.build`")
-        _ops_library = ctypes.CDLL(str(OPS_LIBRARY_PATH))
-        _ops_library.megabake_ops_register.restype = None
-        _ops_library.megabake_ops_register.argtypes = [c_int64, c_int64, c_int64, c_int, c_int64] + [c_void_p] * 5
+        path = ops_library()
+        try:
+            _ops_library = ctypes.CDLL(str(path))
+            _ops_library.megabake_ops_register.restype = None
+            _ops_library.megabake_ops_register.argtypes = [c_int64, c_int64, c_int64, c_int, c_int64] + [c_void_p] * 5
+        except (OSError, AttributeError) as error:
+            _ops_library = False
+            warnings.warn(f"megabake ops go through Python, which is slower: {path.name} cannot be loaded ({error}); "
+                          "run `python -m megabake_b200.build`", RuntimeWarning, stacklevel=2)
+    if _ops_library is False:
+        return
     lib = load()
     entries = [ctypes.cast(entry, c_void_p) for entry in (lib.mk_kv_attention_scratch, lib.mk_kv_attention_scratch_bytes, lib.mk_attention)]
     _ops_library.megabake_ops_register(heads, kv_heads, head_dim, device, max_tokens, handle, status_address, *entries)

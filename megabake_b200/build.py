@@ -16,8 +16,14 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libmegabake_b200.so"
 SOURCES = sorted(CSRC.glob("*.cu"))
-OPS_LIBRARY = PACKAGE / "libmegabake_b200_ops.so"
 OPS_SOURCE = CSRC / "torch_ops.cpp"
+
+
+def ops_library() -> Path:
+    """The ops' C++ registration is built against one PyTorch, and its name says which: another one's is not there."""
+    import torch
+
+    return PACKAGE / f"libmegabake_b200_ops-torch{torch.__version__}.so"
 
 
 def headers() -> list[Path]:
@@ -60,14 +66,15 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def build_ops(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the ops' C++ registration against the installed PyTorch if it is missing or older than its sources."""
+    """Compile the ops' C++ registration against the installed PyTorch if there is none for it or it is older than its sources."""
+    library = ops_library()
     sources = [OPS_SOURCE, PACKAGE.parent / "include" / "megabake_b200.h"]
-    if not force and OPS_LIBRARY.exists() and all(path.stat().st_mtime <= OPS_LIBRARY.stat().st_mtime for path in sources):
-        return OPS_LIBRARY
+    if not force and library.exists() and all(path.stat().st_mtime <= library.stat().st_mtime for path in sources):
+        return library
     import torch
     from torch.utils import cpp_extension
 
-    command = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-o", str(OPS_LIBRARY), str(OPS_SOURCE),
+    command = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-o", str(library), str(OPS_SOURCE),
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
                *(f"-isystem{path}" for path in cpp_extension.include_paths(device_type="cuda")),
                *(f"-L{path}" for path in cpp_extension.library_paths(device_type="cuda")), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-lcudart"]
@@ -76,7 +83,7 @@ def build_ops(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(result.stdout + result.stderr)
     if result.returncode:
         raise RuntimeError(f"{command[0]} failed with exit code {result.returncode}")
-    return OPS_LIBRARY
+    return library
 
 
 if __name__ == "__main__":

@@ -3,6 +3,7 @@ option validation and error formats match the reference's, the ops keep their sc
 backend recognises decoder graphs and keeps the mode contract, ``bucketed`` pads and checks."""
 
 import re
+import warnings
 from pathlib import Path
 
 import pytest
@@ -22,6 +23,31 @@ def test_library_exports_every_declared_symbol():
     assert declared == set(_native.EXPORTS)
     for name in declared:
         assert hasattr(lib, name), name
+
+
+@pytest.mark.parametrize("content", [None, b"", "other"])
+def test_the_ops_go_through_python_without_their_second_library(monkeypatch, tmp_path, content):
+    """Not built, not a library, or a library without the entry: said once, and the CUDA library is all that is needed."""
+    path = tmp_path / "ops.so"
+    if content == "other":
+        path = _native.LIBRARY_PATH
+    elif content is not None:
+        path.write_bytes(content)
+    monkeypatch.setattr(_native, "ops_library", lambda: path)
+    monkeypatch.setattr(_native, "_ops_library", None)
+    with pytest.warns(RuntimeWarning, match="go through Python"):
+        _native.register_ops(4, 4, 64, 0, 16, None, 0)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        _native.register_ops(8, 8, 64, 0, 16, None, 0)
+
+
+def test_the_ops_library_is_built_again_for_another_pytorch(monkeypatch):
+    from megabake_b200 import build
+
+    here = build.ops_library()
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert build.ops_library() != here
 
 
 def test_a_replaced_attention_object_stays_alive(monkeypatch):
