@@ -297,7 +297,10 @@ int mk_debug_skew_barrier(mk_handle handle, uint32_t delta);
  * ctas * events_per_cta * 8 bytes (NULL turns tracing off).  Worker thread 0 of
  * every CTA appends (event code << 56) | globaltimer-ns at phase entry, operand
  * staged, first accumulator ready, phase done, barrier passed, attention done;
- * a launch restarts each CTA's list at 0.
+ * a launch restarts each CTA's list at 0.  A prompt pass of one GPU writes the same list for every CTA:
+ * phase entry at its beginning, then per layer phase done, phase done, attention done and four times
+ * phase done, as norm, QKV, attention, O, norm, gate/up and down end, then the same of the last norm
+ * and the output head.  The attention ops write none.
  * Reference: MEGABAKE_PHASE_TIMER stamps, src/megabake/runtime.py:27-46 and
  * src/megabake/codegen.py:1723-1751. */
 int mk_set_trace(mk_handle handle, void* buffer, int events_per_cta);

@@ -1122,6 +1122,8 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
     pass.logits = static_cast<bf16*>(logits);
     pass.m = static_cast<int>(m); pass.batch = batch; pass.seq = sequence;
     pass.guard = prompt_guard(h);
+    pass.trace = {h->trace, h->trace_cap, h->grid};
+    if (h->trace) MK_CUDA(cudaMemsetAsync(h->trace, 0, sizeof(*h->trace) * h->trace_cap * h->grid, static_cast<cudaStream_t>(stream)));
     const mk_config& c = h->cfg;
     const int q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
     AttnArgs A{};

@@ -149,6 +149,12 @@ struct PromptGuard {
   uint32_t polls;  // a wait looks at its limit after every polls + 1 tries (a power of two)
 };
 
+// The event trace (mk_set_trace).  list: null, or [ctas][cap].
+struct PromptTrace {
+  unsigned long long* list;
+  int cap, ctas;
+};
+
 struct PromptGemm {
   PromptGuard guard;
   const CUtensorMap* a;     // token operand: box of 64 x tokens x kb
@@ -204,6 +210,7 @@ struct PromptPass {
   const AttnArgs* attention;
   const AttnTcMaps* attention_maps;
   PromptGuard guard;
+  PromptTrace trace;
 };
 
 cudaError_t prompt_prepare();  // shared-memory attributes of the kernels, on the current device

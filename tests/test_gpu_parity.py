@@ -497,6 +497,29 @@ def test_rebinding_a_replaced_weight_is_visible(device):
     assert not torch.equal(before, after)
 
 
+@pytest.mark.parametrize("tokens", [40, 300])
+def test_event_trace_of_a_prompt(device, tokens):
+    from megabake_b200.runtime import decode_trace
+
+    config = tiny_config()
+    kernel = make_kernel(config, synth_weights(config, device=device), device, max_tokens=tokens, max_positions=tokens)
+    ids = torch.arange(tokens, device=device).view(1, tokens) % config.vocab
+    untraced = kernel.prefill(ids)
+    expected = [1] + [4, 4, 6, 4, 4, 4, 4] * config.layers + [4, 4]
+    buffer = kernel.set_trace(len(expected) + 3)
+    for _ in range(2):  # the second pass starts its lists again
+        assert torch.equal(kernel.prefill(ids), untraced)
+        kernel.check()
+        codes, times = decode_trace(buffer)
+        assert codes[0].tolist() == expected + [0, 0, 0] and torch.equal(codes, codes[:1].expand_as(codes))
+        assert bool((times[0][1:len(expected)] >= times[0][:len(expected) - 1]).all())
+    short = kernel.set_trace(5)
+    kernel.prefill(ids)
+    kernel.check()
+    assert decode_trace(short)[0][0].tolist() == expected[:5]
+    kernel.set_trace(0)
+
+
 @pytest.mark.parametrize("engine", ["tcgen05", "auto"])
 def test_event_trace_reports_every_phase(device, engine):
     from megabake_b200.runtime import decode_trace
