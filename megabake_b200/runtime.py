@@ -397,6 +397,14 @@ class DecoderKernel:
                 self._stream()))
         return out
 
+    def _require_room(self, **tensors) -> None:
+        """``name=(tensor, rows, heads)``: the launch will go through that many rows of heads, and the tensor has to have them."""
+        for name, (tensor, rows, heads) in tensors.items():
+            needed = rows * heads * self._cfg.head_dim
+            if tensor.numel() < needed:
+                raise CompilerError(CompilerDiagnostic(
+                    "input-binding", f"{name} has shape {tuple(tensor.shape)}: {tensor.numel()} elements, {needed} are needed"))
+
     def kv_attention(self, source, key, value, key_cache, value_cache, valid_length) -> torch.Tensor:
         """``megabake::kv_attention`` (reference src/megabake/lowering.py:211-247) on the GPU."""
         batch, length, heads, dim = source.shape
@@ -405,6 +413,9 @@ class DecoderKernel:
         for name, tensor in (("source", source), ("key", key), ("value", value), ("key_cache", key_cache), ("value_cache", value_cache)):
             _require(tensor, name, dtype=torch.bfloat16, device=self.device)
         _require(valid_length, "valid_length", dtype=torch.int32, device=self.device, shape=(1,))
+        q_heads, kv_heads, cached = self._cfg.q_heads, self._cfg.kv_heads, batch * key_cache.shape[1]
+        self._require_room(source=(source, batch, q_heads), key=(key, batch, kv_heads), value=(value, batch, kv_heads),
+                           key_cache=(key_cache, cached, kv_heads), value_cache=(value_cache, cached, kv_heads))
         self.raise_if_failed()
         out = torch.empty((batch * heads, 1, dim), dtype=torch.bfloat16, device=self.device)
         with self._lock, self._on_device():
@@ -439,6 +450,8 @@ class DecoderKernel:
         k_len = key.shape[1]
         for name, tensor in (("query", query), ("key", key), ("value", value)):
             _require(tensor, name, dtype=torch.bfloat16, device=self.device)
+        self._require_room(query=(query, batch * q_len, self._cfg.q_heads), key=(key, batch * k_len, self._cfg.kv_heads),
+                           value=(value, batch * k_len, self._cfg.kv_heads))
         if mask is not None:
             if mask.shape != (batch, 1, q_len, k_len) or not mask.is_contiguous():
                 mask = mask.expand(batch, 1, q_len, k_len).contiguous()
@@ -557,6 +570,7 @@ class AttentionKernels:
     _on_device = DecoderKernel._on_device
     _call = DecoderKernel._call
     _compiler_error = DecoderKernel._compiler_error
+    _require_room = DecoderKernel._require_room
     kv_attention = DecoderKernel.kv_attention
     _new_kv_scratch = DecoderKernel._new_kv_scratch
     attention = DecoderKernel.attention

@@ -71,6 +71,39 @@ def test_a_replaced_attention_object_stays_alive(monkeypatch):
     assert [ref().max_tokens for ref in replaced] == [16, 16, 32, 512] and replaced[0]() is replaced[1]()
 
 
+def test_attention_refuses_tensors_smaller_than_what_its_kernels_go_through():
+    """Before any launch, on a stand-in whose library must not be reached."""
+    from types import SimpleNamespace
+
+    from megabake_b200.runtime import DecoderKernel
+
+    def never(*args):
+        raise AssertionError("reached the library")
+
+    this = SimpleNamespace(device=torch.device("cpu"), _cfg=SimpleNamespace(q_heads=4, kv_heads=2, head_dim=64), raise_if_failed=never,
+                           raise_if_timed_out=never)
+    this._require_room = lambda **tensors: DecoderKernel._require_room(this, **tensors)
+
+    def zeros(*shape):
+        return torch.zeros(shape, dtype=torch.bfloat16)
+
+    prompt = [zeros(2, 8, 4, 64), zeros(2, 9, 2, 64), zeros(2, 9, 2, 64)]
+    decode = [zeros(2, 1, 4, 64), zeros(2, 1, 2, 64), zeros(2, 1, 2, 64), zeros(2, 16, 2, 64), zeros(2, 16, 2, 64)]
+    length = torch.zeros(1, dtype=torch.int32)
+    for good, call in ((prompt, lambda args: DecoderKernel.attention(this, *args, None, 1.0)),
+                       (decode, lambda args: DecoderKernel.kv_attention(this, *args, length))):
+        with pytest.raises(AssertionError, match="reached"):
+            call(good)
+        for index in range(len(good)):
+            for small in (good[index][:1], good[index][:, :, :1], good[index][..., :32]):
+                args = list(good)
+                args[index] = small.contiguous()
+                if index == 0 and small.shape[0] == 1:
+                    continue  # a smaller batch: the others have more than it needs
+                with pytest.raises(megabake.CompilerError, match="are needed"):
+                    call(args)
+
+
 def test_dependent_attention_kernels_read_nothing_through_the_read_only_path():
     """They begin while the kernels before them write their operands; that path is for memory nobody writes meanwhile."""
     for name in ("prompt_attention.cuh", "prompt_attention_tc.cuh", "kv_attention.cuh"):
