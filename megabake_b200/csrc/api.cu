@@ -52,10 +52,8 @@ struct Carve {
 };
 
 int qkv_width(const mk_config& c) { return (c.q_heads + 2 * c.kv_heads) * c.head_dim; }
-// Token-operand descriptors of the tensor engine: (normalised rows, attention output, SiLU*up, mk_linear's
-// source) x (token tiles of 16, 32, 64), behind the weight descriptors.
 constexpr int kCacheMapSets = 8;  // cache-descriptor sets a handle remembers (one per KV state it is called with in turn)
-constexpr int kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;
+constexpr int kOperandMaps = kOperandKinds * kOperandTiles * kOperandChunks;  // token operands (prompt_plan.h), behind the weight descriptors
 constexpr int kPhaseTables = 2;   // split-K, plain
 int token_tile_of(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128)); }
 size_t maps_per_table(const mk_config& c) { return 7 * static_cast<size_t>(c.layers) + 1; }
@@ -560,7 +558,7 @@ int launch_kv_attention(mk_handle h, const void* query, const void* key, const v
   config.blockDim = dim3(128);
   config.dynamicSmemBytes = 0;
   MK_CUDA(cudaLaunchKernelEx(&config, kv_attention_combine, a, c.head_dim));
-  h->launches += 1;
+  h->launches += 2;
   return MK_OK;
 }
 
@@ -1391,7 +1389,7 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
       h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
       h->cfg.tp_size > 1 ? h->cfg.tp_size : 1);
   if (h->bound) {
-      std::vector<GemmPhase> phases(phases_per_table(h->cfg) * kPhaseTables);
+    std::vector<GemmPhase> phases(phases_per_table(h->cfg) * kPhaseTables);
     MK_CUDA(cudaMemcpy(phases.data(), at<GemmPhase>(h, h->cv.phases), phases.size() * sizeof(GemmPhase), cudaMemcpyDeviceToHost));
     static const char* names[5] = {"qkv", "o", "gate/up", "down", "lm_head"};
     for (int table = 0; table < kPhaseTables; ++table) {

@@ -101,6 +101,26 @@ def test_a_result_that_wants_a_gradient_says_that_there_is_none():
             out.float().sum().backward()
 
 
+def test_standard_calls_do_not_reach_python(monkeypatch):
+    """Once a head shape has its handle: without this the equality of the two routes above could be that of one route."""
+    cases = [_kv_case(3, 8, 2, 128, 17, 40, strided) for strided in (False, True)]
+    prompt = [_tensor("q", 2, 65, 8, 128), _tensor("k", 2, 130, 2, 128), _tensor("v", 2, 130, 2, 128)]
+    mask = _tensor("m", 2, 1, 65, 130)
+    torch.ops.megabake.kv_attention(*_kv_case(3, 8, 2, 128, 17, 40, False))
+
+    def never(*args):
+        raise AssertionError("the Python route")
+
+    monkeypatch.setattr(AttentionKernels, "kv_attention", never)
+    monkeypatch.setattr(AttentionKernels, "attention", never)
+    for args in cases:
+        torch.ops.megabake.kv_attention(*args)
+    for m in (None, mask):
+        torch.ops.megabake.attention(*prompt, m, 0.1)
+    with torch.inference_mode(), pytest.raises(AssertionError, match="the Python route"):
+        torch.ops.megabake.attention(*prompt, None, 0.1)
+
+
 def test_a_call_does_not_wait_for_one_of_another_head_shape():
     """The library's entry for one shape is replaced by one that waits; meanwhile a call of another shape comes and goes."""
     slow, quick = ([_tensor(name, 1, 80, heads, 64) for name in ("a", "b", "c")] for heads in (15, 12))
