@@ -1,5 +1,6 @@
 #pragma once
-// Prompt attention on warp-level tensor cores: short prompts (prompt.cu has the line to the tcgen05 kernel), and the prompt
+// Prompt attention on warp-level tensor cores: short prompts and few queries (attention_on_tcgen05 and
+// prompt.cu have the lines to the tcgen05 kernel), and the prompt
 // phase of the persistent kernel, which tensor parallel runs.
 #include "device_common.cuh"
 

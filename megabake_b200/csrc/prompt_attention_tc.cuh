@@ -10,7 +10,9 @@
 // brings Q and the tiles with tiled TMA copies (with cp.async two warps took 1200 to 2500 cycles a tile, twice the softmax's).
 // Rounding points are those of prompt_unit (prompt_attention.cuh): score = bf16(bf16(q.k) * scale) (+ mask, rounded again),
 // fp32 softmax against the running maximum, exp rounded to bf16 for the value product, division by the fp32 sum at the end.
-// What bounds it: 128 x 64 exponentials are 512 cycles of the SM's special-function units, and about as many issue slots.
+// What bounds it: the chain of a group's tile, one block of eight such warps to an SM (32 heads of 64 x 512 with a mask 14.0 us; issue
+// slots used 0.31, tensor pipe 6.5 %).  The exponentials, 512 cycles a tile of 128 x 64, are 2.1 us of it; the rest is the sums
+// fetched and added in registers for every tile, eight waits, and what surrounds them.
 #pragma once
 #include <type_traits>
 
