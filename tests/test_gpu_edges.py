@@ -448,3 +448,11 @@ def test_decode_attention_entry_point_refuses_scratch_that_is_too_small_or_misal
 
     assert call(0, size - 1) == _native.MK_ERR_WORKSPACE and call(8, size) == _native.MK_ERR_ALIGNMENT
     assert call(0, 0) == _native.MK_ERR_WORKSPACE and int(length) == 0
+
+
+@pytest.mark.parametrize("batch", [1, 3, 4, 7, 12, 16, 29])
+def test_streaming_decode_with_tiles_that_end_early(device, batch):
+    """Rows that no tile height divides, a vocabulary that ends within a tile, and CTAs with several tiles: every warp of the
+    epilogue has tokens, rows or copies that are not there."""
+    config = tiny_config(hidden=320, q_heads=5, kv_heads=5, head_dim=64, intermediate=4992, vocab=5003)
+    oracle_decode_compare(config, device, batch=batch, capacity=40, prefill=21, steps=3)
