@@ -60,13 +60,20 @@ __device__ __forceinline__ void stream_producer(StreamMisc* sm, StreamPipe pipe)
   };
   auto run = [&]() {
 #pragma unroll 1
-    for (int layer = 0; layer < layers; ++layer) {
+    for (int step = 0; step <= 4 * layers; ++step) {  // q k v, o, gate up, down of every layer, then the output head: one copy of the code
+      const int layer = step >> 2, kind = step == 4 * layers ? SP_HEAD : step & 3;
       const CUtensorMap* m = maps + 7 * layer;
       // descriptors are fetched like data: ask for the next ones before they are needed
-      for (int i = 3; i < 7; ++i) tma_prefetch_desc(m + i);
-      tma_prefetch_desc(kv_maps + layer);
-      tma_prefetch_desc(kv_maps + layers + layer);
-      if (!weights(SP_QKV, m)) return;
+      if (kind == SP_QKV) {
+        for (int i = 3; i < 7; ++i) tma_prefetch_desc(m + i);
+        tma_prefetch_desc(kv_maps + layer);
+        tma_prefetch_desc(kv_maps + layers + layer);
+      } else if (kind == SP_GU) {
+        for (int i = 7; i < 10; ++i)
+          if (layer + 1 < layers || i == 7) tma_prefetch_desc(m + i);  // the next layer's q, k, v, or the output head's
+      }
+      if (!weights(kind, m + (kind == SP_O ? 3 : kind == SP_GU ? 4 : kind == SP_DOWN ? 6 : 0))) return;
+      if (kind != SP_QKV) continue;
       const StreamTiles tiles = stream_tiles(p, stream_lengths(p, sm, layer), my_cta, grid);
 #pragma unroll 1
       for (int at = tiles.first; at < tiles.last;) {
@@ -81,13 +88,7 @@ __device__ __forceinline__ void stream_producer(StreamMisc* sm, StreamPipe pipe)
           }
         at += sg.t1 - sg.t0;
       }
-      if (!weights(SP_O, m + 3)) return;
-      for (int i = 7; i < 10; ++i)
-        if (layer + 1 < layers || i == 7) tma_prefetch_desc(m + i);  // the next layer's q, k, v, or the output head's
-      if (!weights(SP_GU, m + 4)) return;
-      if (!weights(SP_DOWN, m + 6)) return;
     }
-    weights(SP_HEAD, maps + 7 * layers);
   };
   run();
   {  // every copy already issued must land before the CTA exits; consumers that have given up do not wait for it
@@ -154,11 +155,14 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     if (head) break;
     stream_attention<HD>(th, pipe, layer);                           // RoPE, append, attention
     th.trace(EV_ATTENTION_DONE);
-    stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, SP_O, layer);     // o_proj + residual
-    stream_project<TM, 2, CNORM, SG_MLP>(th, pipe, SP_GU, layer);       // RMSNorm, SiLU(gate) * up
-    if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
-    __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
-    stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, SP_DOWN, layer);  // down_proj + residual
+#pragma unroll 1
+    for (int kind = SP_O;; kind = SP_DOWN) {  // one copy of the code for both (1.7B shape, 16 sequences 1551 -> 1465 us, 32 2334 -> 2268)
+      stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, kind, layer);  // o_proj, down_proj + residual
+      if (kind == SP_DOWN) break;
+      stream_project<TM, 2, CNORM, SG_MLP>(th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
+      if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
+      __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
+    }
     stream_sync();    // the next layer's vectors are in place
     th.last_turn = th.turn;
     th.turn = th.turn == 2 ? 0 : th.turn + 1;
