@@ -256,7 +256,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
   int slice = CUT ? sm->first_slice[kind] : 0;
   constexpr int COPIES = stream_copies(TM);
   const size_t copy_elems = static_cast<size_t>(TM) * n_cols;
-  const bf16* const src = sm->plan.src[kind][turn] + static_cast<size_t>(sm->cta % COPIES) * TM * k;
+  const bf16* const src = sm->plan.src[kind][turn] + static_cast<size_t>(sm->copy) * TM * k;
   bf16* const dst = sm->plan.dst[kind][turn];
   bf16* const clear = sm->plan.dst[kind][last_turn];
   const bf16* const normw = !NORM ? nullptr : (GROUP == SG_MLP ? sm->lw[half].post_norm : (kind == SP_HEAD ? sm->plan.final_norm : sm->lw[half].input_norm));
@@ -276,7 +276,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
 
   // The two results of one item, columns col and col + 1 of token `tok`.
   auto residual_at = [&](int col) -> const uint32_t* {
-    return reinterpret_cast<const uint32_t*>(sm->plan.res[kind][turn] + (sm->cta % COPIES) * copy_elems + stream_place(TM, tok, col));
+    return reinterpret_cast<const uint32_t*>(sm->plan.res[kind][turn] + sm->copy * copy_elems + stream_place(TM, tok, col));
   };
   auto settled = [&](const uint32_t* at, uint32_t word) -> uint32_t {  // a residual word that was asked for earlier
     while (word == kUnset && !stream_aborted(sm)) word = ld_relaxed_u32(at);

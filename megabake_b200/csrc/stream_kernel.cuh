@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
     sm->ctrl = p.ctrl;
     sm->deadline = clock64() + p.timeout_cycles;
     sm->cta = blockIdx.x;
+    sm->copy = stream_copy_of_sm(stream_copies(TM));
     sm->grid = gridDim.x;
     sm->tokens = p.m;
     sm->token_class = TM;
