@@ -72,8 +72,13 @@ cudaError_t prompt_prepare() {
   if (e == cudaSuccess) e = prepare_gemm<PE_PARTIAL>();
   if (e == cudaSuccess) e = prepare_gemm<PE_SILU>();
   if (e == cudaSuccess) e = prepare_gemm<PE_LOGITS>();
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnTc<64>::kSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnTc<128>::kSmem);
+  const auto attention = [&](auto kernel, int smem) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  };
+  attention(prompt_attention_tc<64, false>, AttnTc<64, false>::kSmem);
+  attention(prompt_attention_tc<64, true>, AttnTc<64, true>::kSmem);
+  attention(prompt_attention_tc<128, false>, AttnTc<128, false>::kSmem);
+  attention(prompt_attention_tc<128, true>, AttnTc<128, true>::kSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem);
   return e;
@@ -98,9 +103,11 @@ cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps
   // Everything a kernel reads or writes comes behind its griddepcontrol.wait, so that it may be launched as a dependent one behind
   // any kernel: two to three microseconds less between the two.
   if (tc) {
-    if (head_dim == 64)
-      return launch(prompt_attention_tc<64>, blocks, kAttnThreads, AttnTc<64>::kSmem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
-    return launch(prompt_attention_tc<128>, blocks, kAttnThreads, AttnTc<128>::kSmem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
+    const auto go = [&](auto kernel, int smem) {
+      return launch(kernel, blocks, kAttnThreads, smem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
+    };
+    if (head_dim == 64) return maps.mask_ok ? go(prompt_attention_tc<64, true>, AttnTc<64, true>::kSmem) : go(prompt_attention_tc<64, false>, AttnTc<64, false>::kSmem);
+    return maps.mask_ok ? go(prompt_attention_tc<128, true>, AttnTc<128, true>::kSmem) : go(prompt_attention_tc<128, false>, AttnTc<128, false>::kSmem);
   }
   if (head_dim == 64)
     return launch(prompt_attention<64>, blocks, kWorkers, PromptLaunch<64>::kSmem, 1, true, stream, args, q_heads, kv_heads, batch, units);

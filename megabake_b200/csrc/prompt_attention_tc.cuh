@@ -10,9 +10,14 @@
 // brings Q and the tiles with tiled TMA copies (with cp.async two warps took 1200 to 2500 cycles a tile, twice the softmax's).
 // Rounding points are those of prompt_unit (prompt_attention.cuh): score = bf16(bf16(q.k) * scale) (+ mask, rounded again),
 // fp32 softmax against the running maximum, exp rounded to bf16 for the value product, division by the fp32 sum at the end.
-// What bounds it: the chain of a group's tile, one block of eight such warps to an SM (32 heads of 64 x 512 with a mask 14.0 us; issue
-// slots used 0.31, tensor pipe 6.5 %).  The exponentials, 512 cycles a tile of 128 x 64, are 2.1 us of it; the rest is the sums
-// fetched and added in registers for every tile, eight waits, and what surrounds them.
+// What bounds it: the chain of a group's tile, one block of eight such warps to an SM (32 heads of 64 x 512 with a mask 12.9 us on
+// the device).  From the first look at memory: scores after 1.9 us, then 1.75 a tile of a group (0.45 scores and mask, 0.65
+// exponentials, of which 0.27 are the unit's rate, 0.3 sums, 0.35 P and waits), 1.2 exchange, 1.3 quotients and stores.
+// A mask with rows on 16-byte boundaries comes by TMA beside the keys and values: a thread reading its own row touched 32 lines a
+// request, 2000 cycles of the load unit for a pair of tiles (512: 13.7 -> 12.9 us, 1024 41.5 -> 38.2, head size 128 20.5 -> 17.7,
+// a third of it the columns that both groups now finish).  Others keep those loads: fetched a row at a time through shared memory
+// they were faster with an even number of positions (500: 17.7 -> 15.8) and slower with an odd one (501: 17.7 -> 20.4); by two warps of
+// their own 27.8.
 #pragma once
 #include <type_traits>
 
@@ -24,16 +29,19 @@ namespace mk {
 constexpr int kAttnQueries = 128, kAttnKeys = 64;
 constexpr int kAttnThreads = 384;  // two groups of four warps; of the third the loader and the MMA warp
 
-template <int HD>
+// MT: the mask's tiles come by TMA beside the keys' and values'.
+template <int HD, bool MT = false>
 struct AttnTc {
   static constexpr int kChunks = HD / 64;                         // 64-dimension chunks of a row
-  static constexpr int kStages = HD == 64 ? 6 : 3;
-  static constexpr int kTile = 2 * kChunks * kAttnKeys * 128;     // a K and a V tile
+  static constexpr int kStages = HD == 64 ? (MT ? 5 : 6) : 3;
+  static constexpr int kKeys = 2 * kChunks * kAttnKeys * 128;     // a K and a V tile
+  static constexpr int kTile = kKeys + (MT ? kAttnQueries * 128 : 0);
   static constexpr int kQ = kChunks * kAttnQueries * 128, kP = kAttnQueries * 128;
   static constexpr int kSmem = 1024 + kQ + 2 * kP + kStages * kTile;
   static constexpr int kColumns = HD == 64 ? 256 : 512;           // 2 x 64 of scores, 2 x head_dim of values
-  // The groups' exchange at the end of a unit, [head_dim + 2][128] fp32, takes the place of Q, P and (head size 128) a stage.
-  static_assert((HD + 2) * 128 * 4 <= kQ + 2 * kP + kTile, "exchange");
+  // The groups' exchange at the end of a unit, 2 x [head_dim / 2 + 2][128] fp32, takes the place of Q, P and (head size 128) a stage.
+  static_assert((HD + 4) * 128 * 4 <= kQ + 2 * kP + kTile, "exchange");
+  static_assert(kSmem <= 232448, "shared memory");
 };
 
 struct AttnTcMisc {
@@ -45,8 +53,9 @@ struct AttnTcMisc {
 // Descriptors of a launch's operands, rows of 64-element chunks: (64, rows, chunks of all heads, sequences).  Rows past the last
 // one read as zeros.
 struct AttnTcMaps {
-  CUtensorMap q, k, v;
-  int q_ok;  // the queries begin on a 16-byte boundary; otherwise their rows are fetched with plain loads
+  CUtensorMap q, k, v, mask;  // (mask: (positions, queries, sequences))
+  int q_ok;     // the queries begin on a 16-byte boundary; otherwise their rows are fetched with plain loads
+  int mask_ok;  // there is a mask, and its rows begin on 16-byte boundaries
 };
 
 // B operand stored with its N dimension contiguous: 64-element chunks [8 rows of K][128 B], 128-byte swizzle.  Rows of K in
@@ -124,10 +133,10 @@ __device__ __forceinline__ AttnTcUnit attn_unit(const AttnArgs& A, int q_heads, 
 }
 
 // One thread of warp 8: the queries, then tile t into stage t % kStages (t counts over the launch).
-template <int HD>
+template <int HD, bool MT>
 __device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t stages,
                                           int base) {
-  using T = AttnTc<HD>;
+  using T = AttnTc<HD, MT>;
   const uint64_t policy = l2_policy_evict_normal();
   if (maps.q_ok) {
     mbar_expect_tx(smem_u32(&misc->qfull), T::kQ);
@@ -139,15 +148,16 @@ __device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWa
     const uint32_t bar = smem_u32(&misc->kvfull[s]), dst = stages + s * T::kTile;
     mbar_expect_tx(bar, T::kTile);
     tma_load_4d(dst, &maps.k, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
-    tma_load_4d(dst + T::kTile / 2, &maps.v, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
+    tma_load_4d(dst + T::kKeys / 2, &maps.v, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
+    if constexpr (MT) tma_load_3d(dst + T::kKeys, &maps.mask, t * kAttnKeys, u.q0, u.b, bar, policy);
   }
 }
 
 // Warp 10.  `base` and `uses`: tiles of earlier units, all and of each group (uses of the barriers).
-template <int HD>
+template <int HD, bool MT>
 __device__ __forceinline__ void attn_mma(const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t p, uint32_t stages, uint32_t tmem,
                                          int base, const int* uses) {
-  using T = AttnTc<HD>;
+  using T = AttnTc<HD, MT>;
   constexpr uint32_t kScores = umma_idesc_bf16(kAttnQueries, kAttnKeys), kValues = umma_idesc_bf16(kAttnQueries, HD) | kIdescBMajorN;
   auto scores = [&](int t) -> bool {
     const int at = base + t, s = at % T::kStages;
@@ -177,7 +187,7 @@ __device__ __forceinline__ void attn_mma(const AttnTcWait& w, AttnTcMisc* misc, 
     if (!__all_sync(0xffffffffu, attn_wait(w, &misc->pfull[g], use & 1))) return;
     tc_fence_after();
     const int s = (base + t) % T::kStages;
-    const uint64_t a = umma_desc_sw128(p + g * T::kP), b = umma_desc_mn_sw128(stages + s * T::kTile + T::kTile / 2, kAttnKeys * 128);
+    const uint64_t a = umma_desc_sw128(p + g * T::kP), b = umma_desc_mn_sw128(stages + s * T::kTile + T::kKeys / 2, kAttnKeys * 128);
     if (elect_one()) {
 #pragma unroll
       for (int x = 0; x < 4; ++x)  // 16 positions: 32 bytes of a row of P, two groups of eight rows of V
@@ -226,17 +236,19 @@ __device__ __forceinline__ void attn_store_nan(const AttnArgs& A, const AttnTcUn
 }
 
 // Warps 0 to 7.  A wait that was given up ends the loop; the block barriers behind it are passed all the same.
-template <int HD>
+template <int HD, bool MT>
 __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint8_t* smem, uint32_t p,
-                                             uint32_t tmem, const int* uses, int warp, int lane) {
+                                             uint32_t stages, uint32_t tmem, int base, const int* uses, int warp, int lane) {
+  using T = AttnTc<HD, MT>;
   const int g = warp >> 2, quad = warp & 3, row = quad * 32 + lane, r = u.q0 + row;
   const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
   const uint32_t s_at = tmem + lanes + g * kAttnKeys, v_at = tmem + lanes + 2 * kAttnKeys + g * HD;
-  const uint32_t p_at = p + g * AttnTc<HD>::kP + row * 128;
+  const uint32_t p_at = p + g * T::kP + row * 128;
   const bool exact_scale = bf16_round(A.scale) == A.scale;  // head size 64: 1/8; the product is rounded once either way
   const uint32_t scale2 = pack2(A.scale, A.scale);
   const bf16* const mrow = A.mask + (static_cast<long long>(u.b) * A.sq + min(r, A.sq - 1)) * A.klen;
   const bool wide = (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
+  const bool fetched = !MT && A.mask;  // the mask comes with plain loads
   bool ok = true, unseen = false;  // unseen: this warp saw nothing of the tile whose sums come next
   float m = -INFINITY, l = 0.f, alpha = 1.f, o[HD];
 #pragma unroll
@@ -255,7 +267,7 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
     }
   };
   uint32_t x[32];  // the mask of a tile's row, its scores, its probabilities
-  if (A.mask && g < u.ntiles) attn_mask(mrow, g * kAttnKeys, A.klen, wide, x);
+  if (fetched && g < u.ntiles) attn_mask(mrow, g * kAttnKeys, A.klen, wide, x);
 #pragma unroll 1
   for (int t = g; t < u.ntiles && ok; t += 2) {
     const int use = uses[g] + (t >> 1), j0 = t * kAttnKeys;
@@ -266,14 +278,26 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
     tc_fence_after();
     float grown = 1.f;
     // With head size 64 there are registers for the next tile's mask: asked for before this tile's exponentials.
-    uint32_t ahead[HD == 64 ? 32 : 1];
+    uint32_t ahead[HD == 64 && !MT ? 32 : 1];
     if (!blind) {
+      uint32_t mask_at = 0u;
+      if constexpr (MT) {  // (the scores came behind the same copies; this thread's own look makes them visible to it)
+        const int at = base + t, s = at % T::kStages;
+        ok = __all_sync(0xffffffffu, attn_wait(w, &misc->kvfull[s], (at / T::kStages) & 1));
+        mask_at = stages + s * T::kTile + T::kKeys + row * 128;
+      }
       // What a pair of scores goes through depends on the launch and the tile: straight lines, not three tests a pair.
       auto take = [&](auto exact, auto masked) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t s[32];
           tmem_ld32_async(s_at + c * 32, s);
+          if constexpr (MT) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x[c * 16 + 4 * i]), "=r"(x[c * 16 + 4 * i + 1]), "=r"(x[c * 16 + 4 * i + 2]),
+                           "=r"(x[c * 16 + 4 * i + 3]) : "r"(mask_at + (((c * 4 + i) ^ (row & 7)) << 4)) : "memory");
+          }
           tmem_loaded();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -285,7 +309,7 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
           }
         }
       };
-      if (A.mask) {
+      if (MT || A.mask) {
         if (exact_scale) take(std::true_type(), std::true_type());
         else take(std::false_type(), std::true_type());
       } else {
@@ -295,8 +319,8 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&misc->sfree[g]));
-      if constexpr (HD == 64) {
-        if (A.mask && t + 2 < u.ntiles) attn_mask(mrow, j0 + 2 * kAttnKeys, A.klen, wide, ahead);
+      if constexpr (HD == 64 && !MT) {
+        if (fetched && t + 2 < u.ntiles) attn_mask(mrow, j0 + 2 * kAttnKeys, A.klen, wide, ahead);
       }
       const int last = (A.causal ? min(A.klen - 1, r) : A.klen - 1) - j0;  // the last position of the tile that the row sees
       if (__any_sync(0xffffffffu, last < kAttnKeys - 1)) {
@@ -341,8 +365,8 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&misc->pfull[g]));
-    if (A.mask && t + 2 < u.ntiles) {
-      if constexpr (HD == 64) {
+    if (fetched && t + 2 < u.ntiles) {
+      if constexpr (HD == 64 && !MT) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = ahead[i];
       } else {
@@ -352,37 +376,48 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
   }
   const int mine = (u.ntiles - g + 1) / 2;  // tiles of this group
   if (mine > 0 && ok) add_values(uses[g] + mine - 1);
-  // The second group's statistics and sums join the first group's, which divides, rounds once and stores.  Every MMA of the unit
-  // has finished once both groups are here: Q, P and the tiles' stages may be written over.
+  // The groups' statistics and sums meet: each finishes half of the columns (divides, rounds once, stores) and leaves the other
+  // half to the other.  Every MMA of the unit has finished once both are here: Q, P and the tiles' stages may be written over.
+  constexpr int kHalf = HD / 2, kShare = (kHalf + 2) * 128;
   float* const exchange = reinterpret_cast<float*>(smem) + row;
   named_bar_sync(1, 256);
-  if (g == 1) {
-    exchange[0] = m;
-    exchange[128] = l;
+  {
+    float* const to = exchange + g * kShare;
+    to[0] = m;
+    to[128] = l;
+    if (g == 0) {
 #pragma unroll
-    for (int d = 0; d < HD; ++d) exchange[(2 + d) * 128] = o[d];
+      for (int d = 0; d < kHalf; ++d) to[(2 + d) * 128] = o[kHalf + d];
+    } else {
+#pragma unroll
+      for (int d = 0; d < kHalf; ++d) {
+        to[(2 + d) * 128] = o[d];
+        o[d] = o[kHalf + d];
+      }
+    }
   }
   named_bar_sync(1, 256);
-  if (g == 0 && *reinterpret_cast<volatile int*>(&misc->abort) != 0) {
-    attn_store_nan<HD>(A, u, row);
-  } else if (g == 0 && r < A.sq) {
-    const float om = exchange[0], ol = exchange[128], n = fmaxf(m, om);
-    const float a = m > -INFINITY ? expf(m - n) : 0.f, b = om > -INFINITY ? expf(om - n) : 0.f;
-    const float total = l * a + ol * b, d = total > 0.f ? total : 1.f;  // a row that sees no key: zeros
-    const float inverse = 1.f / d;
+  if (*reinterpret_cast<volatile int*>(&misc->abort) != 0) {
+    if (g == 0) attn_store_nan<HD>(A, u, row);
+  } else if (r < A.sq) {
+    const float* const from = exchange + (1 - g) * kShare;
+    const float m0 = g == 0 ? m : from[0], m1 = g == 0 ? from[0] : m, l0 = g == 0 ? l : from[128], l1 = g == 0 ? from[128] : l, n = fmaxf(m0, m1);
+    const float a = m0 > -INFINITY ? expf(m0 - n) : 0.f, b = m1 > -INFINITY ? expf(m1 - n) : 0.f;
+    const float total = l0 * a + l1 * b, d = total > 0.f ? total : 1.f;  // a row that sees no key: zeros
+    const float inverse = 1.f / d, own = g == 0 ? a : b, other = g == 0 ? b : a;
     // a quotient by the reciprocal, corrected by its remainder (Markstein, 1990); what is no finite number stays what it is
-    auto quotient = [&](float first, float second) -> float {
-      const float v = first * a + second * b, by = v * inverse;
+    auto quotient = [&](float mine, float theirs) -> float {
+      const float v = mine * own + theirs * other, by = v * inverse;
       return fabsf(by) < INFINITY ? fmaf(fmaf(-by, d, v), inverse, by) : by;
     };
-    bf16* const out = A.out + u.b * A.out_bstride + static_cast<long long>(r) * A.out_tstride + u.h * A.out_hstride;
+    bf16* const out = A.out + u.b * A.out_bstride + static_cast<long long>(r) * A.out_tstride + u.h * A.out_hstride + g * kHalf;
     const bool vectors = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
 #pragma unroll
-    for (int d0 = 0; d0 < HD; d0 += 8) {
+    for (int d0 = 0; d0 < kHalf; d0 += 8) {
       uint32_t x[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        x[e] = pack2(quotient(o[d0 + 2 * e], exchange[(2 + d0 + 2 * e) * 128]), quotient(o[d0 + 2 * e + 1], exchange[(3 + d0 + 2 * e) * 128]));
+        x[e] = pack2(quotient(o[d0 + 2 * e], from[(2 + d0 + 2 * e) * 128]), quotient(o[d0 + 2 * e + 1], from[(3 + d0 + 2 * e) * 128]));
       if (vectors) {
         *reinterpret_cast<uint4*>(out + d0) = make_uint4(x[0], x[1], x[2], x[3]);
       } else {
@@ -393,11 +428,11 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
   }
 }
 
-template <int HD>
+template <int HD, bool MT>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ AttnTcMaps maps, const __grid_constant__ PromptGuard guard, int q_heads,
                     int kv_heads, int batch, int units) {
-  using T = AttnTc<HD>;
+  using T = AttnTc<HD, MT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ AttnTcMisc misc;
@@ -420,6 +455,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
     tma_prefetch_desc(&maps.q);
     tma_prefetch_desc(&maps.k);
     tma_prefetch_desc(&maps.v);
+    if constexpr (MT) tma_prefetch_desc(&maps.mask);
   }
   if (warp == 10) {
     tmem_alloc(smem_u32(&misc.tmem_base), T::kColumns);
@@ -455,13 +491,13 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
       walk([&](const AttnTcUnit& u) {
         if (!maps.q_ok) named_bar_sync(2, 288);  // the queries are there
         else if (!__all_sync(0xffffffffu, attn_wait(w, &misc.qfull, done & 1))) return;
-        attn_mma<HD>(w, &misc, u, q, p, stages, tmem, base, uses);
+        attn_mma<HD, MT>(w, &misc, u, q, p, stages, tmem, base, uses);
       });
     } else {
       walk([&](const AttnTcUnit& u) {
         if (warp == 8 && lane == 0) {
           fence_proxy_async_all();  // the operands, and (a later unit) the exchange's plain accesses, before the copies
-          attn_load<HD>(maps, w, &misc, u, q, stages, base);
+          attn_load<HD, MT>(maps, w, &misc, u, q, stages, base);
         }
         __syncwarp();
       });
@@ -482,7 +518,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
         fence_proxy_async_smem();
         named_bar_sync(2, 288);
       }
-      attn_softmax<HD>(A, w, &misc, u, smem, p, tmem, uses, warp, lane);
+      attn_softmax<HD, MT>(A, w, &misc, u, smem, p, stages, tmem, base, uses, warp, lane);
       fence_proxy_async_smem();
     });
     if (tid < kAttnQueries && *reinterpret_cast<volatile int*>(&misc.abort))  // the units behind the one that was given up

@@ -456,3 +456,22 @@ def test_streaming_decode_with_tiles_that_end_early(device, batch):
     epilogue has tokens, rows or copies that are not there."""
     config = tiny_config(hidden=320, q_heads=5, kv_heads=5, head_dim=64, intermediate=4992, vocab=5003)
     oracle_decode_compare(config, device, batch=batch, capacity=40, prefill=21, steps=3)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (8, 2, 128)])
+@pytest.mark.parametrize("queries,keys", [(70, 72), (129, 128), (257, 200), (128, 456), (300, 704)])
+@pytest.mark.parametrize("offset", [0, 4, 1])
+def test_prompt_attention_op_with_masks_that_come_in_tiles(device, heads, kv_heads, head_dim, queries, keys, offset):
+    """Mask rows on 16-byte boundaries come by tiled copies, whose boxes end beyond the last position, query or sequence; the
+    same mask elsewhere in memory comes row by row, with the same bits."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value = _tensors(device, 3, queries, keys, heads, kv_heads, head_dim)
+    generator = torch.Generator(device=device).manual_seed(keys + queries)
+    mask = torch.randn((3, 1, queries, keys), device=device, generator=generator).to(torch.bfloat16)
+    mask[:, 0, :, 1:].masked_fill_(torch.rand((3, queries, keys - 1), device=device, generator=generator) < 0.4, torch.finfo(torch.bfloat16).min)
+    moved = torch.empty(mask.numel() + offset, dtype=torch.bfloat16, device=device)[offset:].view(mask.shape)
+    moved.copy_(mask)
+    out = torch.ops.megabake.attention(query, key, value, moved, head_dim ** -0.5)
+    assert_parity(out, oracle.attention(query, key, value, mask, head_dim ** -0.5), f"attention {queries} x {keys}")
+    assert torch.equal(out, torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5))
