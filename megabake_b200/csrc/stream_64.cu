@@ -3,8 +3,7 @@
 
 namespace mk {
 const void* stream_kernel_64(int token_class) {
-  const void* kernels[] = {reinterpret_cast<const void*>(&decode_stream<1, 64>), reinterpret_cast<const void*>(&decode_stream<4, 64>),
-                           reinterpret_cast<const void*>(&decode_stream<8, 64>), reinterpret_cast<const void*>(&decode_stream<16, 64>),
+  const void* kernels[] = {reinterpret_cast<const void*>(&decode_stream<1, 64>), reinterpret_cast<const void*>(&decode_stream<8, 64>), reinterpret_cast<const void*>(&decode_stream<16, 64>),
                            reinterpret_cast<const void*>(&decode_stream<32, 64>)};
   return kernels[token_class];
 }

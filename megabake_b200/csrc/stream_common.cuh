@@ -37,13 +37,13 @@ constexpr uint32_t kUnset = 0xFFFFFFFFu;
 
 enum { SP_QKV = 0, SP_O = 1, SP_GU = 2, SP_DOWN = 3, SP_HEAD = 4, kStreamPhases = 5 };
 
-// Token classes: a kernel is compiled for at most 1, 4, 8, 16 or 32 tokens.
+// Token classes: a kernel is compiled for at most 1, 8, 16 or 32 tokens.
 __host__ __device__ constexpr int stream_token_tiles(int tm) { return tm <= 8 ? 1 : tm / 8; }
 // Copies of a slice whose operand a warp's registers hold.
 __host__ __device__ constexpr int stream_fit(int nt) { return nt == 4 ? 2 : 4; }
 // ... of a normalised operand, which is of the hidden size, at most 2048: two.  A phase's length in instructions is its time, so
-// its code holds no more (with four, us a step: 1.7B shape, 3 sequences 957 against 888, 16 sequences 1638 against 1583; 135M, 4
-// sequences 760 against 715) - but for one token, where the shorter code came out 1 to 2 % slower (831 against 848).
+// its code holds no more (with four, us a step: 1.7B shape, 16 sequences 1638 against 1583) - but for one token, where the shorter
+// code came out 1 to 2 % slower (831 against 848).
 __host__ __device__ constexpr int stream_fit_normalised(int tm) { return tm == 1 ? 4 : 2; }
 
 // Every CTA reads the whole residual stream, and while it waits it reads the same few lines again and again: with few tokens
@@ -51,7 +51,7 @@ __host__ __device__ constexpr int stream_fit_normalised(int tm) { return tm == 1
 // several copies, and a CTA reads one of them: the one of its place on the chip, so that a copy is read from few places (SMs with
 // adjacent numbers are neighbours; 135M shape, 16 steps 8094 -> 7875 us against dealing the copies round robin, 0.5B 520 -> 509,
 // 1.7B no difference).
-__host__ __device__ constexpr int stream_copies(int tm) { return tm == 1 ? 8 : (tm <= 4 ? 4 : (tm <= 8 ? 2 : 1)); }
+__host__ __device__ constexpr int stream_copies(int tm) { return tm == 1 ? 8 : (tm <= 8 ? 2 : 1); }
 
 __device__ __forceinline__ int stream_copy_of_sm(int copies) {
   uint32_t id, count;

@@ -70,7 +70,7 @@ __device__ __forceinline__ void stream_operand(StreamMisc* sm, const bf16* src, 
       frag[i][n][0] = frag[i][n][1] = frag[i][n][2] = frag[i][n][3] = init;
     }
   const bf16* const base = src + (kbase >> 5) * TM * 32 + grp * 32 + t * 8;
-  if constexpr (TM >= 8) {
+  if constexpr (TM > 1) {
     // Much data, and every CTA wants it: one word per warp is watched until it is there (all of it at once, again and
     // again, would hold up the stores it is waiting for).
     if (live > 0) {
@@ -162,76 +162,60 @@ __device__ __forceinline__ void stream_normalise(const bf16* normw, int ncopy, i
     }
 }
 
-// The normalised operand of up to TM = 1 or 4 tokens.  In fragment order only the four lanes of a token would have work,
-// so a warp deals its vectors to all lanes, normalises them there and passes them to the fragment's lanes through
-// shared memory of its own.
-template <int TM, int NC>
-__device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16* src, const bf16* normw, int k, int T, int ncopy, int live,
-                                                      int wtid, uint32_t (&frag)[NC * kStreamWpc][1][4]) {
-  constexpr int IT = NC * kStreamWpc * 4 / 32;  // vectors per lane and token; a second one only where a warp has more than eight windows
+// The normalised operand of one token.  In fragment order only four lanes would have work, so a warp deals its vectors to all
+// lanes, normalises them there and passes them to the fragment's lanes through shared memory of its own.
+template <int NC>
+__device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16* src, const bf16* normw, int k, int ncopy, int live, int wtid,
+                                                      uint32_t (&frag)[NC * kStreamWpc][1][4]) {
+  constexpr int IT = NC * kStreamWpc * 4 / 32;  // vectors per lane; a second one only where a warp has more than eight windows
   const int warp = wtid >> 5, lane = wtid & 31;
   const int first = (lane >> 2) * 8 + warp;  // this lane's first window; the next one is 64 on
   const int left = live - (lane >> 2);       // this lane has vector i if 8 i < left
   const bool more = live > 8;
   const float fk = static_cast<float>(k), eps = sm->p->eps;
-  uint4 w[IT], x[TM][IT];
+  uint4 w[IT], x[IT];
 #pragma unroll
   for (int i = 0; i < IT; ++i) {
-    w[i] = make_uint4(0u, 0u, 0u, 0u);
+    w[i] = x[i] = make_uint4(0u, 0u, 0u, 0u);
     if ((i == 0 || more) && 8 * i < left) w[i] = stream_plain_vec(normw + (first + i * 64) * 32, lane & 3);
-#pragma unroll
-    for (int tok = 0; tok < TM; ++tok) x[tok][i] = make_uint4(0u, 0u, 0u, 0u);
   }
-  const bf16* base = src + first * TM * 32 + (lane & 3) * 8;
+  const bf16* base = src + first * 32 + (lane & 3) * 8;
   uint32_t top;
   do {
     top = 0u;
 #pragma unroll
     for (int i = 0; i < IT; ++i)
-      if (i == 0 || more) {
+      if ((i == 0 || more) && 8 * i < left) x[i] = ld_relaxed_v4(base + i * 64 * 32);
 #pragma unroll
-        for (int tok = 0; tok < TM; ++tok)
-          if (tok < T && 8 * i < left) x[tok][i] = ld_relaxed_v4(base + (i * 64 * TM + tok) * 32);
-      }
-#pragma unroll
-    for (int tok = 0; tok < TM; ++tok)
-#pragma unroll
-      for (int i = 0; i < IT; ++i) top = stream_top(top, x[tok][i]);
+    for (int i = 0; i < IT; ++i) top = stream_top(top, x[i]);
   } while (top == kUnset && !stream_aborted(sm));
+  float sum = stream_square4(x[0], 0.f);
+  if (IT > 1 && more) {
 #pragma unroll
-  for (int tok = 0; tok < TM; ++tok) {
-    float sum = stream_square4(x[tok][0], 0.f);
-    if (IT > 1 && more) {
-#pragma unroll
-      for (int i = 1; i < IT; ++i) sum = stream_square4(x[tok][i], sum);
-    }
-    sum = warp_sum(sum);
-    if (lane == 0) sm->ss[warp][tok] = sum;
+    for (int i = 1; i < IT; ++i) sum = stream_square4(x[i], sum);
   }
+  sum = warp_sum(sum);
+  if (lane == 0) sm->ss[warp][0] = sum;
   stream_sync();
-  uint4* mine = reinterpret_cast<uint4*>(stream_scratch(sm)) + warp * TM * NC * kStreamWpc * 4;
+  uint4* mine = reinterpret_cast<uint4*>(stream_scratch(sm)) + warp * NC * kStreamWpc * 4;
+  float v[kStreamWarps];
 #pragma unroll
-  for (int tok = 0; tok < TM; ++tok) {
-    float v[kStreamWarps];
+  for (int s = 0; s < kStreamWarps; ++s) v[s] = sm->ss[s][0];
+  const float r = rsqrtf((((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) / fk + eps);
 #pragma unroll
-    for (int s = 0; s < kStreamWarps; ++s) v[s] = sm->ss[s][tok];
-    const float r = rsqrtf((((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) / fk + eps);
-#pragma unroll
-    for (int i = 0; i < IT; ++i)
-      if (i == 0 || more)
-        mine[(i * 32 + (lane & ~3)) * TM + tok * 4 + (lane & 3)] =
-            make_uint4(stream_norm_pair(x[tok][i].x, w[i].x, r), stream_norm_pair(x[tok][i].y, w[i].y, r),
-                       stream_norm_pair(x[tok][i].z, w[i].z, r), stream_norm_pair(x[tok][i].w, w[i].w, r));
-  }
+  for (int i = 0; i < IT; ++i)
+    if (i == 0 || more)
+      mine[i * 32 + lane] = make_uint4(stream_norm_pair(x[i].x, w[i].x, r), stream_norm_pair(x[i].y, w[i].y, r),
+                                       stream_norm_pair(x[i].z, w[i].z, r), stream_norm_pair(x[i].w, w[i].w, r));
   __syncwarp();
-  const uint4* from = mine + lane;  // window i: TM x 4 vectors, token lane / 4
+  const uint4* from = mine + lane;  // window i: four vectors
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int jj = 0; jj < kStreamWpc; ++jj) {
       const int i = c * kStreamWpc + jj;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (c < ncopy && (lane >> 2) < TM) v = from[i * TM * 4];
+      if (c < ncopy && lane < 4) v = from[i * 4];
       frag[i][0][0] = v.x; frag[i][0][1] = v.y; frag[i][0][2] = v.z; frag[i][0][3] = v.w;
     }
 }
@@ -316,8 +300,8 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
     };
     if constexpr (!NORM) {
       fetch(0);
-    } else if constexpr (TM <= 4) {
-      stream_operand_spread<TM, NC>(sm, src, normw, k, T, ncopy, live, wtid, frag);
+    } else if constexpr (TM == 1) {
+      stream_operand_spread<NC>(sm, src, normw, k, ncopy, live, wtid, frag);
     } else {
       const int kbase = slice * cs * kChunkK + warp * 32;
       uint4 ahead[kStreamWeightsAhead<NT> ? NC * WPC : 1];
@@ -425,14 +409,14 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
             const int ptok = n * 8 + (lane & 3) * 2 + (e & 1), prow = (lane >> 2) + (e >> 1) * 8;
             float v = acc[a][n][0][e];
             if constexpr (SETS == 2) v += acc[a][n][1][e];
-            if (TM >= 8 || ptok < TM) psum[((warp * NACC + a) * TM + ptok) * kStreamPartPitch + prow] = v;
+            if (TM > 1 || ptok < TM) psum[((warp * NACC + a) * TM + ptok) * kStreamPartPitch + prow] = v;
           }
       stream_sync();
       float2 sum[NACC];
 #pragma unroll
       for (int a = 0; a < NACC; ++a) {
         sum[a] = make_float2(0.f, 0.f);
-        if (TM >= 8 || tok < TM) {
+        if (TM > 1 || tok < TM) {
 #pragma unroll
           for (int w = 0; w < kStreamWarps / LPT; ++w) {
             const float2 v = *reinterpret_cast<const float2*>(

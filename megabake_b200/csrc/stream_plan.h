@@ -16,12 +16,14 @@ constexpr int kStreamSmemLimit = 232448;  // 227 KiB
 inline int stream_plan_of(int tokens) { return tokens <= 8 ? 0 : (tokens <= 16 ? 1 : 2); }
 inline bool stream_plan_used(const mk_config& c, int plan) { return plan == 0 || c.max_tokens > (4 << plan); }
 
-// The kernel for a token class (up to 1, 4, 8, 16, 32 tokens); one translation unit per head size.
-constexpr int kStreamClasses = 5;
-constexpr int kStreamClassTokens[kStreamClasses] = {1, 4, 8, 16, 32};
+// The kernel for a token class (up to 1, 8, 16, 32 tokens); one translation unit per head size.  A class for two to four tokens, with
+// the operand spread over all lanes as one token's is, was the slower one: its warps poll half lines of four tokens without a rest
+// (us a step, two sequences 1.7B 835 -> 786, three at 777 positions 886 -> 839, four at 1500 977 -> 915; 0.5B 633 -> 520; 135M 640 -> 476).
+constexpr int kStreamClasses = 4;
+constexpr int kStreamClassTokens[kStreamClasses] = {1, 8, 16, 32};
 const void* stream_kernel_64(int token_class);
 const void* stream_kernel_128(int token_class);
-inline int stream_class_of(int tokens) { return tokens <= 1 ? 0 : (tokens <= 4 ? 1 : (tokens <= 8 ? 2 : (tokens <= 16 ? 3 : 4))); }
+inline int stream_class_of(int tokens) { return tokens <= 1 ? 0 : (tokens <= 8 ? 1 : (tokens <= 16 ? 2 : 3)); }
 inline const void* stream_kernel(int token_class, int head_dim) {
   return head_dim == 64 ? stream_kernel_64(token_class) : stream_kernel_128(token_class);
 }
@@ -128,9 +130,9 @@ inline int stream_heads_per_tile(const mk_config& c, int batch) {
 }
 
 // Attention: one row per warp and query head of its KV head (and 64 pairs of statistics per KV head of a tile).
-// Up to four tokens: the normalised operand on its way to the fragments (16 windows of 64 bytes per warp and token).
+// One token: the normalised operand on its way to the fragments (16 windows of 64 bytes per warp).
 inline int stream_scratch_bytes(const mk_config& c, int batch) {
-  return std::max(batch <= 4 ? kStreamClassTokens[stream_class_of(batch)] * 8192 : 4096, (8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 15) / 16 * 16);
+  return std::max(batch == 1 ? 8192 : 4096, (8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 15) / 16 * 16);
 }
 inline int stream_psum_bytes(int batch) {
   return std::max(1024, (batch <= 16 ? 2 : 1) * kStreamWarps * 2 * kStreamClassTokens[stream_class_of(batch)] * kStreamPartPitch * 4);
