@@ -54,6 +54,15 @@ __device__ __forceinline__ float stream_square4(const uint4& x, float sum) {
 // Largest word of a fragment set: kUnset if any word is unset.
 __device__ __forceinline__ uint32_t stream_top(uint32_t top, const uint4& v) { return max(max(top, max(v.x, v.y)), max(v.z, v.w)); }
 
+// Every CTA wants the operand: one word per warp is watched until it is there.  (All of it at once, again and again, would hold up
+// the stores it is waiting for.  For one token it is the normalised operands: 135M shape, 16 steps 7763 -> 7346 us, 0.5B 503 -> 481, 1.7B
+// 739 -> 733; the others' few lines too: 0.5B 490, 1.7B 741; and a rest between two looks makes the 1.7B shape 0.7 % slower there.)
+template <int TM>
+__device__ __forceinline__ void stream_watch_word(StreamMisc* sm, const bf16* at) {
+  while (ld_relaxed_u32(reinterpret_cast<const uint32_t*>(at)) == kUnset && !stream_aborted(sm))
+    if constexpr (TM > 1) __nanosleep(40);
+}
+
 // Token operand of one K slice in fragment order: frag[i][n] is this lane's vector of window i * 8 + warp for token
 // n * 8 + lane / 4.  All addresses are one base plus constants.
 template <int TM, int NC>
@@ -70,14 +79,7 @@ __device__ __forceinline__ void stream_operand(StreamMisc* sm, const bf16* src, 
       frag[i][n][0] = frag[i][n][1] = frag[i][n][2] = frag[i][n][3] = init;
     }
   const bf16* const base = src + (kbase >> 5) * TM * 32 + grp * 32 + t * 8;
-  if constexpr (TM > 1) {
-    // Much data, and every CTA wants it: one word per warp is watched until it is there (all of it at once, again and
-    // again, would hold up the stores it is waiting for).
-    if (live > 0) {
-      const uint32_t* const last = reinterpret_cast<const uint32_t*>(src + ((kbase >> 5) + (live - 1) * 8) * TM * 32);
-      while (ld_relaxed_u32(last) == kUnset && !stream_aborted(sm)) __nanosleep(40);
-    }
-  }
+  if (TM > 1 && live > 0) stream_watch_word<TM>(sm, src + ((kbase >> 5) + (live - 1) * 8) * TM * 32);
   uint32_t top;
   do {  // every load of a pass is issued before any is looked at; what was there is mostly not read again
     top = 0u;
@@ -180,6 +182,7 @@ __device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16
     if ((i == 0 || more) && 8 * i < left) w[i] = stream_plain_vec(normw + (first + i * 64) * 32, lane & 3);
   }
   const bf16* base = src + first * 32 + (lane & 3) * 8;
+  if (live > 0) stream_watch_word<1>(sm, src + (warp + (live - 1) * 8) * 32);
   uint32_t top;
   do {
     top = 0u;
