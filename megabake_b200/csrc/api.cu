@@ -99,7 +99,7 @@ Carve carve(const mk_config& c, int grid) {
     size_t part[2] = {0, 0};
     for (int i = 0; i < kStreamPlans && stream_plan_used(c, i); ++i) {
       StreamPhase ph[kStreamPhases];
-      stream_phases(c, i, grid, ph);
+      stream_phases(c, i, stream_grid(c, i, grid), ph);
       const size_t t = std::min<size_t>(tokens, 8u << i);
       for (int k = 0; k < kStreamPhases; ++k) {
         const size_t sums = static_cast<size_t>(ph[k].ntiles) * t * kStreamRows * sizeof(float);
@@ -339,6 +339,7 @@ struct mk_handle_s {
   bool kv_maps_refused; // tests: the first encoding counts as refused by the driver
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
+  int stream_grid[kStreamPlans];  // CTAs of each plan's launches
   PromptPhase prompt[kPromptClasses][kPromptPhases];
   bool use3d;           // weight descriptors of the tensor engine are three-dimensional (several K chunks per copy)
   uint32_t tp_epoch;    // all-reduces launched so far (tensor parallel)
@@ -498,13 +499,14 @@ int prepare_kernels(int device, int head_dim) {
 
 int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
   void* args[] = {&p};
+  const int grid = p.splan ? h->stream_grid[stream_plan_of(p.m)] : h->grid;
   if (p.splan)
-    MK_CUDA(cudaLaunchCooperativeKernel(stream_kernel(stream_class_of(p.m), p.head_dim), dim3(h->grid), dim3(kStreamThreads), args,
+    MK_CUDA(cudaLaunchCooperativeKernel(stream_kernel(stream_class_of(p.m), p.head_dim), dim3(grid), dim3(kStreamThreads), args,
                                         stream_smem_bytes(p), static_cast<cudaStream_t>(stream)));
   else
-    MK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&megakernel), dim3(h->grid), dim3(kThreads), args,
+    MK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&megakernel), dim3(grid), dim3(kThreads), args,
                                         kSmemBytes, static_cast<cudaStream_t>(stream)));
-  h->epoch += static_cast<uint32_t>(p.nbar) * static_cast<uint32_t>(h->grid);
+  h->epoch += static_cast<uint32_t>(p.nbar) * static_cast<uint32_t>(grid);
   h->att_epoch += static_cast<uint32_t>(attention_phases);
   h->launches += 1;
   return MK_OK;
@@ -609,7 +611,8 @@ int bind_stream(mk_handle h, const mk_weights& w, std::vector<CUtensorMap>& maps
     h->stream_ok[i] = false;
     if (!stream_plan_used(c, i)) continue;
     StreamPlan& plan = plans[i];
-    stream_phases(c, i, h->grid, plan.ph);
+    h->stream_grid[i] = stream_grid(c, i, h->grid);
+    stream_phases(c, i, h->stream_grid[i], plan.ph);
     for (int l = 0; l < L; ++l) {
       const mk_layer_weights& lw = w.layers[l];
       const void* mats[7] = {lw.q, lw.k, lw.v, lw.o, lw.gate, lw.up, lw.down};
@@ -620,7 +623,7 @@ int bind_stream(mk_handle h, const mk_weights& w, std::vector<CUtensorMap>& maps
     }
     if (int e = encode_weight_map3(&maps[i * nmaps + 7 * L], w.lm_head, c.vocab, c.hidden, plan.ph[SP_HEAD].rows, kStreamKb)) return e;
     int* table = units.data() + static_cast<size_t>(i) * kStreamPhases * (kStreamMaxGrid + 1);
-    stream_deal_units(plan.ph, h->grid, table);
+    stream_deal_units(plan.ph, h->stream_grid[i], table);
     plan.maps = at<CUtensorMap>(h, h->cv.smaps) + i * nmaps;
     plan.layers = at<StreamLayer>(h, h->cv.slayers);
     plan.final_norm = static_cast<const bf16*>(w.final_norm);

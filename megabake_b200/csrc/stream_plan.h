@@ -86,6 +86,25 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
   return ok;
 }
 
+// CTAs of a plan's launches.  Every CTA polls for every hand-over and is in the way of the stores; where three quarters of the SMs
+// go through the phases of a layer in no more rounds of tiles than all of them, they are enough: at 60 GB/s each they still take
+// in what HBM delivers.  (us per pass, 148 and 112 CTAs: 135M shape, 16 steps 7345 -> 7185, one sequence at 1000 positions 472 -> 449,
+// eight at 1900 528 -> 515; 0.5B, one at 99 481 -> 466, eight at 1900 588 -> 554.)  Up to eight sequences: with more, long contexts are a
+// round of cache tiles longer (0.5B, 32 at 1900 904 -> 955; 135M, sixteen at 1900 715 -> 739) though short ones gain (135M, 32 at 300
+// 795 -> 770).  A handle with a limit on its SMs uses what it was given.
+inline int stream_grid(const mk_config& c, int plan, int sms) {
+  const int fewer = (3 * sms / 4 + 7) / 8 * 8;
+  if (plan > 0 || c.sm_limit > 0 || fewer >= sms) return sms;
+  auto rounds = [&](int grid) {
+    StreamPhase ph[kStreamPhases];
+    stream_phases(c, plan, grid, ph);
+    int sum = 0;
+    for (int i = 0; i < SP_HEAD; ++i) sum += (ph[i].ntiles * ph[i].nslice + grid - 1) / grid;
+    return sum;
+  };
+  return rounds(fewer) <= rounds(sms) ? fewer : sms;
+}
+
 // Hidden sizes up to 2048: an operand of 2048 columns fits a warp's registers at 32 tokens (two copies of a slice), and only
 // such shapes have been measured and tested here.  Wider ones would fit up to 16 tokens and are left on the tensor engine;
 // that is not a limit of the hardware.  What to expect of a change: on the 8B shape's 32 layers this kernel, the tensor

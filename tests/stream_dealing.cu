@@ -6,6 +6,35 @@
 
 using namespace mk;
 
+// CTAs of the launches of up to eight sequences, and the rounds of tiles of a layer's projections with `grid` CTAs.
+static mk_config shape(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int sm_limit) {
+  mk_config c{};
+  c.hidden = hidden;
+  c.q_heads = q_heads;
+  c.kv_heads = kv_heads;
+  c.head_dim = head_dim;
+  c.intermediate = intermediate;
+  c.vocab = 1000;
+  c.sm_limit = sm_limit;
+  return c;
+}
+extern "C" int grid_of(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int sm_limit, int plan, int sms) {
+  return stream_grid(shape(hidden, q_heads, kv_heads, head_dim, intermediate, sm_limit), plan, sms);
+}
+extern "C" int rounds_of(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int plan, int grid) {
+  StreamPhase ph[kStreamPhases];
+  stream_phases(shape(hidden, q_heads, kv_heads, head_dim, intermediate, 0), plan, grid, ph);
+  std::vector<int> table(kStreamPhases * (grid + 1));
+  stream_deal_units(ph, grid, table.data());
+  int sum = 0;
+  for (int kind = 0; kind < SP_HEAD; ++kind) {
+    int most = 0;
+    for (int i = 0; i < grid; ++i) most = std::max(most, table[kind * (grid + 1) + i + 1] - table[kind * (grid + 1) + i]);
+    sum += most;
+  }
+  return sum;
+}
+
 // Returns 0, or the number of the first rule that is broken; `longest` and `lists`: the most parts and lists of a CTA.
 extern "C" int check_dealing(int grid, int batch, int q_heads, int kv_heads, int head_dim, int ragged, const int* len, int* longest, int* lists) {
   mk_config c{};

@@ -27,6 +27,7 @@ def deal(tmp_path_factory):
         assert broken == 0, f"rule {broken} broken: lengths {lengths}, heads {heads}/{kv_heads} of {head_dim}, {grid} CTAs"
         return longest.value, lists.value
 
+    run.lib = lib
     return run
 
 
@@ -54,3 +55,14 @@ def test_every_position_is_dealt_exactly_once(deal):
         several += deal(lengths, heads, kv_heads, head_dim, grid=grid)[1] > 1
         deal(lengths[:1], heads, kv_heads, head_dim, batch=batch, grid=grid, ragged=False)
     assert several > 100
+
+
+@pytest.mark.parametrize("shape,fewer", [((576, 9, 3, 64, 1536), True), ((896, 14, 2, 64, 4864), True), ((2048, 32, 32, 64, 8192), False),
+                                         ((320, 5, 5, 64, 4992), True)])
+def test_fewer_ctas_only_where_no_phase_gets_longer(deal, shape, fewer):
+    """135M, 0.5B and 1.7B shapes: three quarters of the SMs where that is no round of tiles more, for up to eight sequences."""
+    grid = deal.lib.grid_of(*shape, 0, 0, 148)
+    assert grid == (112 if fewer else 148)
+    assert deal.lib.rounds_of(*shape, 0, grid) <= deal.lib.rounds_of(*shape, 0, 148)
+    assert deal.lib.grid_of(*shape, 0, 1, 148) == deal.lib.grid_of(*shape, 0, 2, 148) == 148
+    assert deal.lib.grid_of(*shape, 30, 0, 30) == 30 and deal.lib.grid_of(*shape, 0, 0, 7) == 7
