@@ -54,9 +54,10 @@ __device__ __forceinline__ float stream_square4(const uint4& x, float sum) {
 // Largest word of a fragment set: kUnset if any word is unset.
 __device__ __forceinline__ uint32_t stream_top(uint32_t top, const uint4& v) { return max(max(top, max(v.x, v.y)), max(v.z, v.w)); }
 
-// Every CTA wants the operand: one word per warp is watched until it is there.  (All of it at once, again and again, would hold up
-// the stores it is waiting for.  For one token it is the normalised operands: 135M shape, 16 steps 7763 -> 7346 us, 0.5B 503 -> 481, 1.7B
-// 739 -> 733; the others' few lines too: 0.5B 490, 1.7B 741; and a rest between two looks makes the 1.7B shape 0.7 % slower there.)
+// Every CTA wants a normalised operand, and its results come from all of them: one word per warp is watched until it is there.  (All
+// of it at once, again and again, would hold up the stores it is waiting for: one token, 135M shape, 16 steps 7763 -> 7346 us, 0.5B
+// 503 -> 481, 1.7B 739 -> 733.)  The operands of o_proj and down_proj are read at once, a round trip less: with a watch 0.5B at one
+// 490, 1.7B, eight sequences 3536 against 3494, sixteen 1464 against 1451.  A rest between two looks, one token: 1.7B 0.7 % slower.
 template <int TM>
 __device__ __forceinline__ void stream_watch_word(StreamMisc* sm, const bf16* at) {
   while (ld_relaxed_u32(reinterpret_cast<const uint32_t*>(at)) == kUnset && !stream_aborted(sm))
@@ -65,7 +66,7 @@ __device__ __forceinline__ void stream_watch_word(StreamMisc* sm, const bf16* at
 
 // Token operand of one K slice in fragment order: frag[i][n] is this lane's vector of window i * 8 + warp for token
 // n * 8 + lane / 4.  All addresses are one base plus constants.
-template <int TM, int NC>
+template <int TM, int NC, bool NORM>
 __device__ __forceinline__ void stream_operand(StreamMisc* sm, const bf16* src, int T, int ncopy, int live, int kbase, int wtid,
                                                uint32_t (&frag)[NC * kStreamWpc][stream_token_tiles(TM)][4]) {
   constexpr int NT = stream_token_tiles(TM);
@@ -79,7 +80,7 @@ __device__ __forceinline__ void stream_operand(StreamMisc* sm, const bf16* src, 
       frag[i][n][0] = frag[i][n][1] = frag[i][n][2] = frag[i][n][3] = init;
     }
   const bf16* const base = src + (kbase >> 5) * TM * 32 + grp * 32 + t * 8;
-  if (TM > 1 && live > 0) stream_watch_word<TM>(sm, src + ((kbase >> 5) + (live - 1) * 8) * TM * 32);
+  if (NORM && live > 0) stream_watch_word<TM>(sm, src + ((kbase >> 5) + (live - 1) * 8) * TM * 32);
   uint32_t top;
   do {  // every load of a pass is issued before any is looked at; what was there is mostly not read again
     top = 0u;
@@ -298,7 +299,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
     auto fetch = [&](int part) {
       const int at = part * NC * kStreamKb;  // first chunk
       const int chunks = min(cs - at, NC * kStreamKb);
-      stream_operand<TM, NC>(sm, src, T, (chunks + kStreamKb - 1) / kStreamKb, (2 * chunks - warp + 7) >> 3, (slice * cs + at) * kChunkK + warp * 32,
+      stream_operand<TM, NC, NORM>(sm, src, T, (chunks + kStreamKb - 1) / kStreamKb, (2 * chunks - warp + 7) >> 3, (slice * cs + at) * kChunkK + warp * 32,
                              wtid, frag);
     };
     if constexpr (!NORM) {
