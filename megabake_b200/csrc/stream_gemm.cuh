@@ -459,7 +459,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
           }
         }
       }
-      if (TM <= 16) th.pbuf ^= 1;  // two buffers: the next tile's sums go to the other one
+      if (TM <= 8) th.pbuf ^= 1;  // two buffers: the next tile's sums go to the other one
       else stream_sync();          // one buffer: everybody has read it
     }
     ++slice;

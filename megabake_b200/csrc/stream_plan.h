@@ -153,8 +153,11 @@ inline int stream_heads_per_tile(const mk_config& c, int batch) {
 inline int stream_scratch_bytes(const mk_config& c, int batch) {
   return std::max(batch == 1 ? 8192 : 4096, (8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 15) / 16 * 16);
 }
+// Two buffers of partial sums up to eight tokens.  With 16, one and a block barrier more per tile leave room for a sixth slot (1.7B shape,
+// sixteen sequences at 200 positions 1088 -> 1068 us, at 1024 1441 -> 1431, fourteen of different lengths 1389 -> 1344); with 32
+// there is no room for it either way.
 inline int stream_psum_bytes(int batch) {
-  return std::max(1024, (batch <= 16 ? 2 : 1) * kStreamWarps * 2 * kStreamClassTokens[stream_class_of(batch)] * kStreamPartPitch * 4);
+  return std::max(1024, (batch <= 8 ? 2 : 1) * kStreamWarps * 2 * kStreamClassTokens[stream_class_of(batch)] * kStreamPartPitch * 4);
 }
 // The ring takes as many slots as fit.
 inline void stream_divide(KParams& p, int scratch, int batch) {
