@@ -404,10 +404,12 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
     const float m0 = g == 0 ? m : from[0], m1 = g == 0 ? from[0] : m, l0 = g == 0 ? l : from[128], l1 = g == 0 ? from[128] : l, n = fmaxf(m0, m1);
     const float a = m0 > -INFINITY ? expf(m0 - n) : 0.f, b = m1 > -INFINITY ? expf(m1 - n) : 0.f;
     const float total = l0 * a + l1 * b, d = total > 0.f ? total : 1.f;  // a row that sees no key: zeros
-    const float inverse = 1.f / d, own = g == 0 ? a : b, other = g == 0 ? b : a;
-    // a quotient by the reciprocal, corrected by its remainder (Markstein, 1990); what is no finite number stays what it is
+    const float inverse = 1.f / d;
+    // The first group's share is the one that the fused step adds, whichever group is at it, so that a column's result does not hang on
+    // the half it lies in; a quotient by the reciprocal, corrected by its remainder (Markstein, 1990); what is no finite number stays
+    // what it is.  (Selects: a copy of the code for each group was no faster.)
     auto quotient = [&](float mine, float theirs) -> float {
-      const float v = mine * own + theirs * other, by = v * inverse;
+      const float v = fmaf(g == 0 ? mine : theirs, a, (g == 0 ? theirs : mine) * b), by = v * inverse;
       return fabsf(by) < INFINITY ? fmaf(fmaf(-by, d, v), inverse, by) : by;
     };
     bf16* const out = A.out + u.b * A.out_bstride + static_cast<long long>(r) * A.out_tstride + u.h * A.out_hstride + g * kHalf;

@@ -475,3 +475,15 @@ def test_prompt_attention_op_with_masks_that_come_in_tiles(device, heads, kv_hea
     out = torch.ops.megabake.attention(query, key, value, moved, head_dim ** -0.5)
     assert_parity(out, oracle.attention(query, key, value, mask, head_dim ** -0.5), f"attention {queries} x {keys}")
     assert torch.equal(out, torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5))
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (8, 2, 128)])
+@pytest.mark.parametrize("queries,keys,masked", [(128, 512, True), (200, 449, False), (257, 200, True)])
+def test_prompt_attention_op_gives_a_column_the_same_bits_in_either_half(device, heads, kv_heads, head_dim, queries, keys, masked):
+    """Two groups of warps finish half of the columns each: with the halves of the values exchanged, those of the results are, bit
+    by bit."""
+    query, key, value = _tensors(device, 2, queries, keys, heads, kv_heads, head_dim)
+    mask = torch.randn((2, 1, queries, keys), device=device, generator=torch.Generator(device=device).manual_seed(3)).to(torch.bfloat16) if masked else None
+    out = torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5)
+    moved = torch.ops.megabake.attention(query, key, value.roll(head_dim // 2, -1), mask, head_dim ** -0.5)
+    assert torch.equal(moved, out.roll(head_dim // 2, -1))
