@@ -3,7 +3,8 @@
 
 namespace mk {
 const void* stream_kernel_128(int token_class) {
-  const void* kernels[] = {reinterpret_cast<const void*>(&decode_stream<1, 128>), reinterpret_cast<const void*>(&decode_stream<8, 128>), reinterpret_cast<const void*>(&decode_stream<16, 128>),
+  const void* kernels[] = {reinterpret_cast<const void*>(&decode_stream<1, 128>), reinterpret_cast<const void*>(&decode_stream<8, 128, true>),
+                           reinterpret_cast<const void*>(&decode_stream<8, 128>), reinterpret_cast<const void*>(&decode_stream<16, 128>),
                            reinterpret_cast<const void*>(&decode_stream<32, 128>)};
   return kernels[token_class];
 }

@@ -37,7 +37,7 @@ constexpr uint32_t kUnset = 0xFFFFFFFFu;
 
 enum { SP_QKV = 0, SP_O = 1, SP_GU = 2, SP_DOWN = 3, SP_HEAD = 4, kStreamPhases = 5 };
 
-// Token classes: a kernel is compiled for at most 1, 8, 16 or 32 tokens.
+// Token classes: a kernel is compiled for at most 1, 4, 8, 16 or 32 tokens (4 in the layout of 8).
 __host__ __device__ constexpr int stream_token_tiles(int tm) { return tm <= 8 ? 1 : tm / 8; }
 // Copies of a slice whose operand a warp's registers hold.
 __host__ __device__ constexpr int stream_fit(int nt) { return nt == 4 ? 2 : 4; }

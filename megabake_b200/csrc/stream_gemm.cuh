@@ -133,6 +133,25 @@ __device__ __forceinline__ void stream_gram(int ncopy, const uint32_t (&frag)[NC
           }
     }
 }
+// The same of two to four tokens: a fused multiply-add an element in fp32, added up as the spread operand of one token is, so that a
+// sequence gets the bits it gets alone.  Products on the tensor cores are added up there by rules of their own.
+template <int NC>
+__device__ __forceinline__ float stream_squares(int ncopy, const uint32_t (&frag)[NC * kStreamWpc][1][4]) {
+  static_assert(NC == 2 && kStreamWpc == 4, "eight windows to a warp");
+  float s[kStreamWpc];
+#pragma unroll
+  for (int i = 0; i < kStreamWpc; ++i) s[i] = stream_square4(make_uint4(frag[i][0][0], frag[i][0][1], frag[i][0][2], frag[i][0][3]), 0.f);
+  if (ncopy > 1) {
+#pragma unroll
+    for (int i = 0; i < kStreamWpc; ++i) {
+      const uint32_t(&f)[4] = frag[kStreamWpc + i][0];
+      s[i] += stream_square4(make_uint4(f[0], f[1], f[2], f[3]), 0.f);
+    }
+  }
+  float sum = (s[0] + s[2]) + (s[1] + s[3]);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  return sum + __shfl_xor_sync(0xffffffffu, sum, 1);
+}
 // x * rinv and the product with the norm weight, on bf16 pairs: the two roundings of the Hugging Face RMSNorm.
 __device__ __forceinline__ uint32_t stream_norm_pair(uint32_t x, uint32_t w, float r) {
   return mul_bf16x2(w, pack2(__uint_as_float(x << 16) * r, __uint_as_float(x & 0xFFFF0000u) * r));
@@ -225,8 +244,8 @@ __device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16
 }
 
 // One projection phase for this CTA's units.  TM: token class; NACC: weight matrices per tile (gate and up: two); NC:
-// copies of a slice whose operand fits the registers; GROUP: what happens to operand and result.
-template <int TM, int NACC, int NC, int GROUP>
+// copies of a slice whose operand fits the registers; GROUP: what happens to operand and result; FEW: at most four tokens.
+template <int TM, int NACC, int NC, int GROUP, bool FEW>
 __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pipe, int kind, int layer) {
   constexpr int NT = stream_token_tiles(TM), WPC = kStreamWpc;
   constexpr int SETS = NT <= 2 ? 2 : 1;  // accumulator sets: consecutive MMAs of a tile do not wait for one another
@@ -317,14 +336,19 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
         }
       }
       fetch(0);
-      float gram[NT][4];
+      if constexpr (FEW) {
+        const float sum = stream_squares<NC>(ncopy, frag);
+        if ((lane & 3) == 0) sm->ss[warp][lane >> 2] = sum;
+      } else {
+        float gram[NT][4];
 #pragma unroll
-      for (int n = 0; n < NT; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
-      stream_gram<NT, NC>(ncopy, frag, gram);
-      if (((lane >> 2) >> 1) == (lane & 3)) {  // this lane has the diagonal element of token lane / 4
+        for (int n = 0; n < NT; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
+        stream_gram<NT, NC>(ncopy, frag, gram);
+        if (((lane >> 2) >> 1) == (lane & 3)) {  // this lane has the diagonal element of token lane / 4
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
-          sm->ss[warp][n * 8 + (lane >> 2)] = (n & 1) ? (((lane >> 2) & 1) ? gram[n][3] : gram[n][2]) : (((lane >> 2) & 1) ? gram[n][1] : gram[n][0]);
+          for (int n = 0; n < NT; ++n)
+            sm->ss[warp][n * 8 + (lane >> 2)] = (n & 1) ? (((lane >> 2) & 1) ? gram[n][3] : gram[n][2]) : (((lane >> 2) & 1) ? gram[n][1] : gram[n][0]);
+        }
       }
       stream_sync();
       const float fk = static_cast<float>(k), eps = sm->p->eps;

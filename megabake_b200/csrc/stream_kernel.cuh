@@ -1,5 +1,6 @@
 // The streaming decode kernel: one cooperative launch per step, up to 32 sequences.
-// See stream_common.cuh for the scheme.  One instantiation per token class (at most TM tokens) and head size.
+// See stream_common.cuh for the scheme.  One instantiation per token class (at most TM tokens; FEW: at
+// most four of TM = 8) and head size.
 #pragma once
 #include "stream_attention.cuh"
 #include "stream_gemm.cuh"
@@ -125,7 +126,7 @@ __device__ __forceinline__ void stream_reset(bf16* buffer, long long elems, int 
   for (long long i = at; i < elems / 8; i += step) __stcg(v + i, make_uint4(kUnset, kUnset, kUnset, kUnset));
 }
 
-template <int TM, int HD>
+template <int TM, int HD, bool FEW>
 __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe, int wtid) {
   const KParams& p = *sm->p;
   constexpr int NT = stream_token_tiles(TM);
@@ -151,15 +152,15 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     // the next layer's vectors: requested here, passed on through shared memory at the end of the layer
     uint32_t word = 0u;
     if (wtid < kLayerWords && layer + 1 < layers) word = __ldg(reinterpret_cast<const uint32_t*>(sm->plan.layers + layer + 1) + wtid);
-    stream_project<TM, 1, CNORM, SG_NORM>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
+    stream_project<TM, 1, CNORM, SG_NORM, FEW>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
     if (head) break;
     stream_attention<HD>(th, pipe, layer);                           // RoPE, append, attention
     th.trace(EV_ATTENTION_DONE);
 #pragma unroll 1
     for (int kind = SP_O;; kind = SP_DOWN) {  // one copy of the code for both (1.7B shape, 16 sequences 1551 -> 1465 us, 32 2334 -> 2268)
-      stream_project<TM, 1, CPLAIN, SG_PLAIN>(th, pipe, kind, layer);  // o_proj, down_proj + residual
+      stream_project<TM, 1, CPLAIN, SG_PLAIN, FEW>(th, pipe, kind, layer);  // o_proj, down_proj + residual
       if (kind == SP_DOWN) break;
-      stream_project<TM, 2, CNORM, SG_MLP>(th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
+      stream_project<TM, 2, CNORM, SG_MLP, FEW>(th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
       if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
       __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
     }
@@ -209,7 +210,7 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
   }
 }
 
-template <int TM, int HD>
+template <int TM, int HD, bool FEW = false>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_constant__ KParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
     else if (tid == 96) stream_plan_parts(sm);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    stream_consumers<TM, HD>(sm, pipe, tid - 128);
+    stream_consumers<TM, HD, FEW>(sm, pipe, tid - 128);
   }
 }
 

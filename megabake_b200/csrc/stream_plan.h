@@ -16,14 +16,15 @@ constexpr int kStreamSmemLimit = 232448;  // 227 KiB
 inline int stream_plan_of(int tokens) { return tokens <= 8 ? 0 : (tokens <= 16 ? 1 : 2); }
 inline bool stream_plan_used(const mk_config& c, int plan) { return plan == 0 || c.max_tokens > (4 << plan); }
 
-// The kernel for a token class (up to 1, 8, 16, 32 tokens); one translation unit per head size.  A class for two to four tokens, with
-// the operand spread over all lanes as one token's is, was the slower one: its warps poll half lines of four tokens without a rest
-// (us a step, two sequences 1.7B 835 -> 786, three at 777 positions 886 -> 839, four at 1500 977 -> 915; 0.5B 633 -> 520; 135M 640 -> 476).
-constexpr int kStreamClasses = 4;
-constexpr int kStreamClassTokens[kStreamClasses] = {1, 8, 16, 32};
+// The kernel for a token class (up to 1, 4, 8, 16, 32 tokens); one translation unit per head size.  Two to four tokens are laid out as up
+// to eight are, and only the squares of a norm are summed as one token's (see stream_squares).  With the operand spread over all lanes
+// they were slower: a warp polls half lines of four tokens without a rest (us a step, two sequences 1.7B 835 -> 786, three at 777
+// positions 886 -> 839, four at 1500 977 -> 915; 0.5B 633 -> 520; 135M 640 -> 476).
+constexpr int kStreamClasses = 5;
+constexpr int kStreamClassTokens[kStreamClasses] = {1, 8, 8, 16, 32};  // the layout's
 const void* stream_kernel_64(int token_class);
 const void* stream_kernel_128(int token_class);
-inline int stream_class_of(int tokens) { return tokens <= 1 ? 0 : (tokens <= 8 ? 1 : (tokens <= 16 ? 2 : 3)); }
+inline int stream_class_of(int tokens) { return tokens <= 1 ? 0 : (tokens <= 4 ? 1 : (tokens <= 8 ? 2 : (tokens <= 16 ? 3 : 4))); }
 inline const void* stream_kernel(int token_class, int head_dim) {
   return head_dim == 64 ? stream_kernel_64(token_class) : stream_kernel_128(token_class);
 }

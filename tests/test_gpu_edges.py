@@ -487,3 +487,23 @@ def test_prompt_attention_op_gives_a_column_the_same_bits_in_either_half(device,
     out = torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5)
     moved = torch.ops.megabake.attention(query, key, value.roll(head_dim // 2, -1), mask, head_dim ** -0.5)
     assert torch.equal(moved, out.roll(head_dim // 2, -1))
+
+
+@pytest.mark.parametrize("batch", [2, 3, 4])
+@pytest.mark.parametrize("hidden", [320, 1088, 2048])
+def test_streaming_decode_of_a_few_sequences_gives_each_the_bits_it_gets_alone(device, batch, hidden):
+    """Up to four sequences every sum is made in the same order, the squares of the norms among them: contexts of one tile are in
+    one part, whatever the batch."""
+    config = tiny_config(hidden=hidden, q_heads=8, kv_heads=4, head_dim=64, intermediate=1024, vocab=1000, layers=6)
+    weights = synth_weights(config, seed=21, norm_std=0.1, device=device)
+    together, alone = (make_kernel(config, weights, device, max_tokens=n, max_positions=12) for n in (batch, 1))
+    states = [new_kv_state(config, n, 12, device) for n in (batch, *[1] * batch)]
+    ids = synth_ids(batch * 12, config.vocab, seed=21).view(batch, 12).to(device)
+    for position in range(12):
+        positions = torch.full((batch, 1), position, dtype=torch.int64, device=device)
+        step = ids[:, position:position + 1].contiguous()
+        logits = together.decode(step, positions, *states[0])
+        for row in range(batch):
+            assert torch.equal(logits[row:row + 1], alone.decode(step[row:row + 1].contiguous(), positions[:1], *states[1 + row])), f"{row} at {position}"
+    together.check()
+    alone.check()
