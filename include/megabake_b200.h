@@ -138,7 +138,7 @@ int mk_bind_weights(mk_handle handle, const mk_weights* weights, void* stream);
  * config.layers device pointers, each bf16 [batch, capacity, kv_heads,
  * head_dim] contiguous.  valid_lengths: host array of config.layers device
  * pointers to int32 [1]; read, used as the append row, and advanced by one.
- * logits: bf16 [batch, vocab].
+ * logits: bf16 [batch, vocab], beginning at any element (here and below).
  * Reference: the bound callable's warm call, src/megabake/compiler.py:964-1081,
  * running the decode graph of tests/fixtures.py:247-312 whose attention is
  * megabake::kv_attention (src/megabake/lowering.py:211-247). */

@@ -170,7 +170,7 @@ __device__ __noinline__ void greedy_sample(const Ctx& cx, int wtid, float* scrat
     const bf16* row = p.logits + static_cast<size_t>(t) * p.vocab;
     float best = -INFINITY;
     int idx = 0x7fffffff;
-    if ((p.vocab & 7) == 0) {
+    if ((p.vocab & 7) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {  // (logits may begin at any element)
       // Eight vectors in flight: with one, a vocabulary of 49152 was 24 round trips to L2.
       constexpr int kAhead = 8;
       const uint4* vrow = reinterpret_cast<const uint4*>(row);

@@ -325,6 +325,38 @@ def test_logits_may_begin_at_any_element(batch):
     assert float(buffer[0]) == -3.0 and float(buffer[-1]) == -3.0
 
 
+@pytest.mark.parametrize("batch,engine", [(1, "auto"), (5, "auto"), (17, "auto"), (3, "tcgen05")])
+@pytest.mark.parametrize("offset", [1, 4])
+def test_the_sampler_reads_logits_that_begin_at_any_element(batch, engine, offset):
+    """Steps sampled on the device into a C caller's logits buffer off a 16-byte boundary, with a vocabulary in whole vectors: the
+    tokens and logits of an aligned buffer, and nothing beside it is written."""
+    config = tiny_config(q_heads=4, kv_heads=2, hidden=256)
+    assert config.vocab % 8 == 0
+    kernel = make_kernel(config, synth_weights(config, seed=6, norm_std=0.1, device=DEVICE), max_tokens=batch, max_positions=16, engine=engine)
+    first = synth_ids(batch, config.vocab, seed=6).view(batch, 1).to(DEVICE)
+    expected, logits = kernel.decode_steps(first.clone(), torch.zeros_like(first), *new_kv_state(config, batch, 16, DEVICE), steps=3,
+                                           return_logits=True)
+    buffer = torch.full((batch * config.vocab + 2 * offset,), -3.0, dtype=torch.bfloat16, device=DEVICE)
+    at = buffer.data_ptr() + 2 * offset
+    stream = torch.cuda.current_stream(DEVICE).cuda_stream
+
+    def state():
+        return [(ctypes.c_void_p * config.layers)(*[t.data_ptr() for t in tensors]) for tensors in caches]
+
+    caches = new_kv_state(config, batch, 16, DEVICE)
+    ids, positions, tokens = first.clone(), torch.zeros_like(first), torch.empty((3, batch), dtype=torch.int64, device=DEVICE)
+    _native.check("mk_decode_steps", kernel.lib.mk_decode_steps(kernel._handle, ids.data_ptr(), positions.data_ptr(), batch, *state(), 16, 3,
+                                                                tokens.data_ptr(), at, stream))
+    kernel.check()
+    assert torch.equal(tokens.t(), expected) and torch.equal(buffer[offset:-offset].view(logits.shape), logits)
+    caches = new_kv_state(config, batch, 16, DEVICE)
+    host = [first.cpu(), torch.zeros((batch, 1), dtype=torch.int64), torch.empty((batch, 1), dtype=torch.int64)]
+    _native.check("mk_decode_step_host", kernel.lib.mk_decode_step_host(kernel._handle, host[0].data_ptr(), host[1].data_ptr(), batch, *state(),
+                                                                        16, at, host[2].data_ptr(), stream))
+    assert torch.equal(host[2][:, 0], expected[:, 0].cpu())
+    assert (buffer[:offset] == -3.0).all() and (buffer[-offset:] == -3.0).all()
+
+
 def test_silu_of_the_epilogues_has_the_bits_of_the_division(tmp_path):
     """``silu_inner`` over every bf16 below 80 (the sign of zero aside), built as the library is."""
     import subprocess
