@@ -70,7 +70,7 @@ typedef struct mk_config {
   int32_t max_tokens;    /* largest batch (decode) or batch*sequence (prefill) per launch */
   int32_t max_positions; /* rows of the cos/sin tables */
   int32_t engine;        /* MK_ENGINE_* */
-  int32_t sm_limit;      /* 0: one CTA per SM on the whole GPU; >0: use this many CTAs */
+  int32_t sm_limit;      /* 0: at most one CTA per SM on the whole GPU; >0: use this many CTAs */
   /* Tensor parallel (0 or 1: off).  With tp_size > 1 this handle is one rank of a group on one
    * node: q_heads, kv_heads and intermediate are the rank's shard (q/k/v and gate/up sharded by
    * output rows, o and down by input columns), hidden is whole, vocab is the rows of this rank's
@@ -279,7 +279,7 @@ int mk_ipc_close(void* base);
  * (mk_linear) is timed against it by `python -m megabake_b200.bench_linear`. */
 int mk_baseline_mma_gemm(const void* x, const void* weight, void* y, int m, int n, int k, void* stream);
 
-/* Plain-text summary of what the handle will launch (CTAs, the form of the weight copies, tile height /
+/* Plain-text summary of what the handle will launch (CTAs, and those of streaming decode of up to eight sequences, the form of the weight copies, tile height /
  * K split / chunks per copy / unit count of each projection phase per table, and of a prompt pass per launch class).  Synchronous (reads the
  * phase tables back).  Reference: the plan report, src/megabake/plan.py:342-395. */
 int mk_describe(mk_handle handle, char* buffer, size_t bytes);
@@ -297,7 +297,8 @@ int mk_debug_skew_barrier(mk_handle handle, uint32_t delta);
  * ctas * events_per_cta * 8 bytes (NULL turns tracing off).  Worker thread 0 of
  * every CTA appends (event code << 56) | globaltimer-ns at phase entry, operand
  * staged, first accumulator ready, phase done, barrier passed, attention done;
- * a launch restarts each CTA's list at 0.  A prompt pass of one GPU writes the same list for every CTA:
+ * a launch or prompt pass clears the buffer and starts each CTA's list at 0 (a launch of fewer CTAs leaves
+ * the other lists empty).  A prompt pass of one GPU writes the same list for every CTA:
  * phase entry at its beginning, then per layer phase done, phase done, attention done and four times
  * phase done, as norm, QKV, attention, O, norm, gate/up and down end, then the same of the last norm
  * and the output head.  The attention ops write none.
@@ -305,7 +306,7 @@ int mk_debug_skew_barrier(mk_handle handle, uint32_t delta);
  * src/megabake/codegen.py:1723-1751. */
 int mk_set_trace(mk_handle handle, void* buffer, int events_per_cta);
 
-/* Number of CTAs each launch uses, bytes of dynamic shared memory, kernels launched so far. */
+/* Largest number of CTAs of a launch (decode of a few sequences may use fewer: mk_describe), bytes of dynamic shared memory, kernels launched so far. */
 int mk_launch_info(mk_handle handle, int32_t* ctas, int32_t* smem_bytes, int64_t* launches);
 
 /* mk_kv_attention without a handle and without any device allocation, for callers

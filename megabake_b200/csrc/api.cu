@@ -500,6 +500,8 @@ int prepare_kernels(int device, int head_dim) {
 int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
   void* args[] = {&p};
   const int grid = p.splan ? h->stream_grid[stream_plan_of(p.m)] : h->grid;
+  // The launch before may have had more CTAs or longer lists: nothing of it stays.
+  if (p.trace) MK_CUDA(cudaMemsetAsync(p.trace, 0, sizeof(*p.trace) * p.trace_cap * h->grid, static_cast<cudaStream_t>(stream)));
   if (p.splan)
     MK_CUDA(cudaLaunchCooperativeKernel(stream_kernel(stream_class_of(p.m), p.head_dim), dim3(grid), dim3(kStreamThreads), args,
                                         stream_smem_bytes(p), static_cast<cudaStream_t>(stream)));
@@ -1397,8 +1399,10 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
     va_end(ap);
     if (n > 0) used += static_cast<size_t>(n);
   };
+  char streamed[64] = "no";
+  if (h->stream_ok[0]) snprintf(streamed, sizeof streamed, "yes (%d ctas up to 8 sequences)", h->stream_grid[0]);
   add("ctas %d, weight copies %s, streaming decode %s, tp %d/%d\n", h->grid,
-      h->use3d ? "3-D (several K chunks per copy)" : "2-D (one K chunk per copy)", h->stream_ok[0] ? "yes" : "no",
+      h->use3d ? "3-D (several K chunks per copy)" : "2-D (one K chunk per copy)", streamed,
       h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
       h->cfg.tp_size > 1 ? h->cfg.tp_size : 1);
   if (h->bound) {

@@ -540,3 +540,28 @@ def test_event_trace_reports_every_phase(device, engine):
     stamps = times[0][codes[0] > 0][:barriers]
     assert bool((stamps[1:] >= stamps[:-1]).all())
     kernel.set_trace(0)
+
+
+def test_event_trace_holds_the_last_launch_only(device):
+    """Up to eight sequences this shape decodes on fewer CTAs than there are: the lists of the others are empty, also behind a
+    launch that filled them."""
+    import re
+
+    from megabake_b200.runtime import decode_trace
+
+    config = tiny_config(hidden=576, q_heads=9, kv_heads=3, head_dim=64, intermediate=1536)
+    kernel = make_kernel(config, synth_weights(config, device=device), device, max_tokens=16, max_positions=8)
+    ctas = kernel.launch_info()["ctas"]
+    few = int(re.search(r"streaming decode yes \((\d+) ctas", kernel.describe()).group(1))
+    assert few < ctas
+    buffer = kernel.set_trace(64)
+    assert buffer.shape[0] == ctas
+    counts = []
+    for batch in (16, 1, 16):
+        ids = torch.arange(batch, device=device).view(batch, 1)
+        kernel.decode(ids, torch.zeros_like(ids), *new_kv_state(config, batch, 8, device))
+        kernel.check()
+        counts.append((decode_trace(buffer)[0] > 0).sum(1))
+    assert counts[0].min() > 0 and torch.equal(counts[0], counts[2])
+    assert counts[1][:few].min() > 0 and counts[1][few:].max() == 0
+    kernel.set_trace(0)
