@@ -279,7 +279,7 @@ int mk_ipc_close(void* base);
  * (mk_linear) is timed against it by `python -m megabake_b200.bench_linear`. */
 int mk_baseline_mma_gemm(const void* x, const void* weight, void* y, int m, int n, int k, void* stream);
 
-/* Plain-text summary of what the handle will launch (CTAs, and those of streaming decode of up to eight sequences, the form of the weight copies, tile height /
+/* Plain-text summary of what the handle will launch (CTAs, and those of streaming decode of few sequences, the form of the weight copies, tile height /
  * K split / chunks per copy / unit count of each projection phase per table, and of a prompt pass per launch class).  Synchronous (reads the
  * phase tables back).  Reference: the plan report, src/megabake/plan.py:342-395. */
 int mk_describe(mk_handle handle, char* buffer, size_t bytes);
@@ -306,7 +306,7 @@ int mk_debug_skew_barrier(mk_handle handle, uint32_t delta);
  * src/megabake/codegen.py:1723-1751. */
 int mk_set_trace(mk_handle handle, void* buffer, int events_per_cta);
 
-/* Largest number of CTAs of a launch (decode of a few sequences may use fewer: mk_describe), bytes of dynamic shared memory, kernels launched so far. */
+/* Largest number of CTAs of a launch (decode of few sequences may use fewer: mk_describe), bytes of dynamic shared memory, kernels launched so far. */
 int mk_launch_info(mk_handle handle, int32_t* ctas, int32_t* smem_bytes, int64_t* launches);
 
 /* mk_kv_attention without a handle and without any device allocation, for callers

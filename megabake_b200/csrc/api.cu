@@ -97,10 +97,12 @@ Carve carve(const mk_config& c, int grid) {
     v.sunits = take(sizeof(int) * kStreamPlans * kStreamPhases * (kStreamMaxGrid + 1));
     v.srec = take(tokens * c.q_heads * kStreamMaxSegments * (c.head_dim + 2) * 8);
     size_t part[2] = {0, 0};
-    for (int i = 0; i < kStreamPlans && stream_plan_used(c, i); ++i) {
+    for (int i = 0; i < kStreamPlans; ++i) {
       StreamPhase ph[kStreamPhases];
-      stream_phases(c, i, stream_grid(c, i, grid), ph);
-      const size_t t = std::min<size_t>(tokens, 8u << i);
+      const int ctas = stream_grid(c, i, grid);
+      if (ctas == 0) continue;
+      stream_phases(c, i, ctas, ph);
+      const size_t t = std::min<size_t>(tokens, 8u * stream_plan_tiles(i));
       for (int k = 0; k < kStreamPhases; ++k) {
         const size_t sums = static_cast<size_t>(ph[k].ntiles) * t * kStreamRows * sizeof(float);
         if (ph[k].nslice > 1) part[k == SP_O ? 0 : 1] = std::max(part[k == SP_O ? 0 : 1], sums * ph[k].nslice);
@@ -339,7 +341,7 @@ struct mk_handle_s {
   bool kv_maps_refused; // tests: the first encoding counts as refused by the driver
   bool kv_maps_ok;      // the driver takes the four-dimensional view of a cache
   bool stream_ok[kStreamPlans];  // the streaming decode kernel's plan for this many token tiles is bound
-  int stream_grid[kStreamPlans];  // CTAs of each plan's launches
+  int stream_grid[kStreamPlans];  // CTAs of each plan's launches, 0: the plan is not used
   PromptPhase prompt[kPromptClasses][kPromptPhases];
   bool use3d;           // weight descriptors of the tensor engine are three-dimensional (several K chunks per copy)
   uint32_t tp_epoch;    // all-reduces launched so far (tensor parallel)
@@ -499,7 +501,7 @@ int prepare_kernels(int device, int head_dim) {
 
 int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
   void* args[] = {&p};
-  const int grid = p.splan ? h->stream_grid[stream_plan_of(p.m)] : h->grid;
+  const int grid = p.splan ? h->stream_grid[stream_plan_of(h->cfg, p.m, h->stream_grid[kStreamFew])] : h->grid;
   // The launch before may have had more CTAs or longer lists: nothing of it stays.
   if (p.trace) MK_CUDA(cudaMemsetAsync(p.trace, 0, sizeof(*p.trace) * p.trace_cap * h->grid, static_cast<cudaStream_t>(stream)));
   if (p.splan)
@@ -516,7 +518,7 @@ int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
 
 // The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.
 bool stream_usable(mk_handle h, int batch, bool ragged) {
-  return batch <= kStreamTokens && h->stream_ok[stream_plan_of(batch)] &&
+  return batch <= kStreamTokens && h->stream_ok[stream_plan_of(h->cfg, batch, h->stream_grid[kStreamFew])] &&
          h->kv_maps_ok && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
 }
 
@@ -611,9 +613,9 @@ int bind_stream(mk_handle h, const mk_weights& w, std::vector<CUtensorMap>& maps
   }
   for (int i = 0; i < kStreamPlans; ++i) {
     h->stream_ok[i] = false;
-    if (!stream_plan_used(c, i)) continue;
-    StreamPlan& plan = plans[i];
     h->stream_grid[i] = stream_grid(c, i, h->grid);
+    if (h->stream_grid[i] == 0) continue;
+    StreamPlan& plan = plans[i];
     stream_phases(c, i, h->stream_grid[i], plan.ph);
     for (int l = 0; l < L; ++l) {
       const mk_layer_weights& lw = w.layers[l];
@@ -696,7 +698,7 @@ int mk_create(const mk_config* config, void* workspace, size_t workspace_bytes, 
     h->use3d = getenv("MEGABAKE_NO_3D_MAPS") == nullptr &&
                encode_weight_map3(&probe, workspace, 128, 256, 64, 2) == MK_OK;
   }
-  for (int i = 0; i < kStreamPlans; ++i) h->stream_ok[i] = false;
+  for (int i = 0; i < kStreamPlans; ++i) h->stream_ok[i] = false, h->stream_grid[i] = 0;
   h->kv_maps_ok = getenv("MEGABAKE_NO_CACHE_MAPS") == nullptr;
   h->kv_maps_refused = getenv("MEGABAKE_REFUSE_CACHE_MAPS") != nullptr;
   h->tp_epoch = 0;
@@ -1077,7 +1079,7 @@ int decode_once(mk_handle h, const int64_t* ids, const int64_t* positions, int b
   p.nbar = 7 * L + 1;  // tensor engine: five per layer and one behind each norm phase (two per layer, one for the lm_head)
   if (streamed) {
     const mk_config& c = h->cfg;
-    const int plan = stream_plan_of(batch);
+    const int plan = stream_plan_of(c, batch, h->stream_grid[kStreamFew]);
     p.splan = at<StreamPlan>(h, h->cv.splan) + plan;
     p.nbar = 1;
     p.stream_hpu = stream_heads_per_tile(c, batch);
@@ -1400,7 +1402,10 @@ int mk_describe(mk_handle h, char* buffer, size_t bytes) {
     if (n > 0) used += static_cast<size_t>(n);
   };
   char streamed[64] = "no";
-  if (h->stream_ok[0]) snprintf(streamed, sizeof streamed, "yes (%d ctas up to 8 sequences)", h->stream_grid[0]);
+  if (h->stream_ok[0]) snprintf(streamed, sizeof streamed, "yes");
+  int most = 0;  // sequences of the largest launch on fewer CTAs
+  while (h->stream_ok[kStreamFew] && most < h->cfg.max_tokens && stream_few_fits(h->cfg, most + 1, h->stream_grid[kStreamFew])) ++most;
+  if (most > 0) snprintf(streamed, sizeof streamed, "yes (%d ctas up to batch %d)", h->stream_grid[kStreamFew], most);
   add("ctas %d, weight copies %s, streaming decode %s, tp %d/%d\n", h->grid,
       h->use3d ? "3-D (several K chunks per copy)" : "2-D (one K chunk per copy)", streamed,
       h->cfg.tp_size > 1 ? h->cfg.tp_rank : 0,
@@ -1603,7 +1608,7 @@ int mk_kv_attention_static(int q_heads, int kv_heads, int head_dim, const void* 
   view.epoch = slot.epoch; view.att_epoch = slot.att_epoch; view.launches = slot.launches;
   view.timeout_cycles = slot.timeout_cycles;
   view.att_scale = static_cast<float>(std::pow(static_cast<double>(head_dim), -0.5));
-  for (int i = 0; i < kStreamPlans; ++i) view.stream_ok[i] = false;
+  for (int i = 0; i < kStreamPlans; ++i) view.stream_ok[i] = false, view.stream_grid[i] = 0;
   view.trace = nullptr; view.trace_cap = 0;
   view.mirror = nullptr; view.use3d = false; view.kv_done = nullptr;
   view.tp_epoch = 0; view.tp_bound = false;

@@ -9,12 +9,12 @@
 
 namespace mk {
 
-constexpr int kStreamPlans = 3;           // 8, 16 and 32 tokens (one, two and four MMA tiles)
+constexpr int kStreamPlans = 4;           // 8, 16 and 32 tokens (one, two and four MMA tiles), 8 tokens on fewer CTAs
+constexpr int kStreamFew = 3;
 constexpr int kStreamMaxGrid = 512;
 constexpr int kStreamSmemLimit = 232448;  // 227 KiB
 
-inline int stream_plan_of(int tokens) { return tokens <= 8 ? 0 : (tokens <= 16 ? 1 : 2); }
-inline bool stream_plan_used(const mk_config& c, int plan) { return plan == 0 || c.max_tokens > (4 << plan); }
+inline int stream_plan_tiles(int plan) { return plan == kStreamFew ? 1 : 1 << plan; }
 
 // The kernel for a token class (up to 1, 4, 8, 16, 32 tokens); one translation unit per head size.  Two to four tokens are laid out as up
 // to eight are, and only the squares of a norm are summed as one token's (see stream_squares).  With the operand spread over all lanes
@@ -61,7 +61,7 @@ inline void stream_rows(StreamPhase& ph, const int* matrices, int count, int gri
 }
 
 inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* ph) {
-  const int nt = 1 << plan, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const int nt = stream_plan_tiles(plan), q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
   const int ks[kStreamPhases] = {c.hidden, q_size, c.hidden, c.intermediate, c.hidden};
   const int ns[kStreamPhases] = {q_size + 2 * kv_size, c.hidden, c.intermediate, c.hidden, c.vocab};
   bool ok = true;
@@ -87,23 +87,42 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
   return ok;
 }
 
-// CTAs of a plan's launches.  Every CTA polls for every hand-over and is in the way of the stores; where three quarters of the SMs
-// go through the phases of a layer in no more rounds of tiles than all of them, they are enough: at 60 GB/s each they still take
-// in what HBM delivers.  (us per pass, 148 and 112 CTAs: 135M shape, 16 steps 7345 -> 7185, one sequence at 1000 positions 472 -> 449,
-// eight at 1900 528 -> 515; 0.5B, one at 99 481 -> 466, eight at 1900 588 -> 554.)  Up to eight sequences: with more, long contexts are a
-// round of cache tiles longer (0.5B, 32 at 1900 904 -> 955; 135M, sixteen at 1900 715 -> 739) though short ones gain (135M, 32 at 300
-// 795 -> 770).  A handle with a limit on its SMs uses what it was given.
+// Fewer CTAs for up to eight sequences.  Every CTA polls for every hand-over and is in the way of the stores, so three quarters of the
+// SMs go through a short layer faster than all of them, though a CTA's tiles get taller and a phase of few rounds longer: at
+// 60 GB/s each they still take in what HBM delivers.  Where they lose is a round of tiles or of cache runs more:
+//  - the projections of a layer take no more rounds of tiles, summed over the four, and the output head no more than a round per layer
+//    of the model more (rounds of a layer, us a step of 16 layers at 60 positions on 148 and 112 CTAs, one / eight sequences: 135M shape
+//    4 -> 4, 255 / 283 -> 249 / 264; hidden 1408 with 22 heads 9 -> 9, 402 / 440 -> 397 / 434; hidden 768 5 -> 6, 280 / 302 -> 281 / 315;
+//    hidden 1152 6 -> 7, 333 / 359 -> 352 / 381; 1.7B 9 -> 13, 495 / 546 -> 544 / 591; two layers of the 135M shape, head 21 -> 28,
+//    53 / 58 -> 55 / 60);
+//  - there are four CTAs to every KV head of every sequence of the launch, else a long context is cut into too few runs (1000 to 16000
+//    positions, KV heads x sequences: 15 442 -> 431, 341 -> 332, 24 518 -> 489, 298 -> 279; 32 365 -> 376, 594 -> 645; 48 753 -> 878;
+//    128 363 -> 394).
+// With more than eight sequences long contexts are a round of cache tiles longer (0.5B, 32 at 1900 904 -> 955).  A handle with a limit
+// on its SMs uses what it was given.  Returns the number of CTAs, 0 where the shape has all of them in any case.
+inline int stream_few_ctas(const mk_config& c, int sms) {
+  const int few = (3 * sms / 4 + 7) / 8 * 8;
+  if (c.sm_limit > 0 || few >= sms) return 0;
+  StreamPhase less[kStreamPhases], all[kStreamPhases];
+  stream_phases(c, kStreamFew, few, less);
+  stream_phases(c, 0, sms, all);
+  auto rounds = [](const StreamPhase& p, int grid) { return (p.ntiles * p.nslice + grid - 1) / grid; };
+  int more = 0;
+  for (int i = 0; i < SP_HEAD; ++i) more += rounds(less[i], few) - rounds(all[i], sms);
+  return more <= 0 && rounds(less[SP_HEAD], few) - rounds(all[SP_HEAD], sms) <= c.layers ? few : 0;
+}
+inline bool stream_few_fits(const mk_config& c, int batch, int few) { return batch <= 8 && 4 * batch * c.kv_heads <= few; }
+// CTAs of a plan's launches, 0: no launch uses the plan.
 inline int stream_grid(const mk_config& c, int plan, int sms) {
-  const int fewer = (3 * sms / 4 + 7) / 8 * 8;
-  if (plan > 0 || c.sm_limit > 0 || fewer >= sms) return sms;
-  auto rounds = [&](int grid) {
-    StreamPhase ph[kStreamPhases];
-    stream_phases(c, plan, grid, ph);
-    int sum = 0;
-    for (int i = 0; i < SP_HEAD; ++i) sum += (ph[i].ntiles * ph[i].nslice + grid - 1) / grid;
-    return sum;
-  };
-  return rounds(fewer) <= rounds(sms) ? fewer : sms;
+  if (plan == 0) return sms;
+  if (plan < kStreamFew) return c.max_tokens > (4 << plan) ? sms : 0;
+  const int few = stream_few_ctas(c, sms);
+  return stream_few_fits(c, 1, few) ? few : 0;
+}
+// The plan of a launch.
+inline int stream_plan_of(const mk_config& c, int tokens, int few) {
+  if (few > 0 && stream_few_fits(c, tokens, few)) return kStreamFew;
+  return tokens <= 8 ? 0 : (tokens <= 16 ? 1 : 2);
 }
 
 // Hidden sizes up to 2048: an operand of 2048 columns fits a warp's registers at 32 tokens (two copies of a slice), and only
@@ -113,8 +132,8 @@ inline int stream_grid(const mk_config& c, int plan, int sms) {
 inline bool stream_shape_ok(const mk_config& c) {
   if (c.tp_size > 1 || c.hidden > 2048) return false;
   StreamPhase ph[kStreamPhases];
-  for (int i = 0; i < kStreamPlans; ++i)
-    if (stream_plan_used(c, i) && !stream_phases(c, i, 148, ph)) return false;
+  for (int i = 0; i < kStreamFew; ++i)  // (the other plan's reductions are cut as the first one's)
+    if (stream_grid(c, i, 148) > 0 && !stream_phases(c, i, 148, ph)) return false;
   return true;
 }
 

@@ -6,33 +6,34 @@
 
 using namespace mk;
 
-// CTAs of the launches of up to eight sequences, and the rounds of tiles of a layer's projections with `grid` CTAs.
-static mk_config shape(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int sm_limit) {
+static mk_config shape(const int* s) {  // hidden, query heads, KV heads, head size, intermediate, vocabulary, layers, SM limit
   mk_config c{};
-  c.hidden = hidden;
-  c.q_heads = q_heads;
-  c.kv_heads = kv_heads;
-  c.head_dim = head_dim;
-  c.intermediate = intermediate;
-  c.vocab = 1000;
-  c.sm_limit = sm_limit;
+  c.hidden = s[0];
+  c.q_heads = s[1];
+  c.kv_heads = s[2];
+  c.head_dim = s[3];
+  c.intermediate = s[4];
+  c.vocab = s[5];
+  c.layers = s[6];
+  c.sm_limit = s[7];
+  c.max_tokens = 32;
   return c;
 }
-extern "C" int grid_of(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int sm_limit, int plan, int sms) {
-  return stream_grid(shape(hidden, q_heads, kv_heads, head_dim, intermediate, sm_limit), plan, sms);
+// CTAs of a launch of `batch` sequences.
+extern "C" int grid_of(const int* s, int batch, int sms) {
+  const mk_config c = shape(s);
+  const int few = stream_grid(c, kStreamFew, sms);
+  return stream_grid(c, stream_plan_of(c, batch, few), sms);
 }
-extern "C" int rounds_of(int hidden, int q_heads, int kv_heads, int head_dim, int intermediate, int plan, int grid) {
+// Units of a phase's busiest CTA.
+extern "C" int rounds_of(const int* s, int kind, int grid) {
   StreamPhase ph[kStreamPhases];
-  stream_phases(shape(hidden, q_heads, kv_heads, head_dim, intermediate, 0), plan, grid, ph);
+  stream_phases(shape(s), 0, grid, ph);
   std::vector<int> table(kStreamPhases * (grid + 1));
   stream_deal_units(ph, grid, table.data());
-  int sum = 0;
-  for (int kind = 0; kind < SP_HEAD; ++kind) {
-    int most = 0;
-    for (int i = 0; i < grid; ++i) most = std::max(most, table[kind * (grid + 1) + i + 1] - table[kind * (grid + 1) + i]);
-    sum += most;
-  }
-  return sum;
+  int most = 0;
+  for (int i = 0; i < grid; ++i) most = std::max(most, table[kind * (grid + 1) + i + 1] - table[kind * (grid + 1) + i]);
+  return most;
 }
 
 // Returns 0, or the number of the first rule that is broken; `longest` and `lists`: the most parts and lists of a CTA.
