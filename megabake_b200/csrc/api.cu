@@ -302,7 +302,7 @@ int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, const mk_config& 
   if (int e = encode_attention_map(&maps->k, A.k, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
   if (int e = encode_attention_map(&maps->v, A.v, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
   // The mask's tiles come by TMA where its rows begin on 16-byte boundaries (a tiled copy's strides are multiples of that).
-  maps->mask_ok = A.mask != nullptr && (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
+  maps->mask_ok = A.mask != nullptr && attention_mask_in_tiles(head_dim, A.sq, A.klen) && (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
   if (maps->mask_ok) {
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(A.klen), static_cast<cuuint64_t>(A.sq), static_cast<cuuint64_t>(batch)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(A.klen) * 2, static_cast<cuuint64_t>(A.sq) * A.klen * 2};

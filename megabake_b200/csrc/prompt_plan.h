@@ -125,6 +125,16 @@ inline bool attention_on_tcgen05(int head_dim, int q_len, int k_len, long long h
   return first <= second;
 }
 
+// Whether a mask's tiles, 64 positions of 128 queries, come by TMA (where its rows allow it) or each row to its thread with plain loads.
+// A copy costs its whole box, also the rows past the last query; the plain loads of a full block are 32 lines a request.  So few queries
+// take the loads, unless there are many tiles to hide behind; with head size 128, three stages deep, four tiles have to pay for the
+// longer prologue.  us, loads / tiles: head size 64, 32 heads x 4 sequences, 1 x 512 13.6 / 20.6, 24 x 128 7.5 / 8.9, 65 x 200 9.8 / 10.8,
+// 96 x 128 7.8 / 7.7, 128 x 512 14.2 / 13.2, 16 x 1024 20.6 / 19.6; head size 128, 32 heads, 64 x 1400 33.4 / 34.4, 200 x 72 9.4 / 9.9,
+// 200 x 200 12.6 / 12.6, 96 x 256 12.1 / 11.6, 512 x 512 20.3 / 18.1.
+inline bool attention_mask_in_tiles(int head_dim, int q_len, int k_len) {
+  return head_dim == 128 ? q_len >= 96 && k_len > 192 : q_len >= 96 || (q_len >= 16 && k_len >= 1024);
+}
+
 // What a CTA still waits for before it leaves: that the last use of every pipeline slot has been consumed, so that no commit
 // is on its way to a barrier of shared memory that is somebody else's by then.  The uses count up over the launch, use u lies in
 // slot u % stages, and a slot's barrier has the parity of its use; wait(slot, parity) returns false to give up.

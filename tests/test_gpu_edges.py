@@ -459,10 +459,10 @@ def test_streaming_decode_with_tiles_that_end_early(device, batch):
 
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (8, 2, 128)])
-@pytest.mark.parametrize("queries,keys", [(70, 72), (129, 128), (257, 200), (128, 456), (300, 704)])
+@pytest.mark.parametrize("queries,keys", [(70, 72), (129, 128), (257, 200), (128, 456), (300, 704), (96, 200), (95, 1024), (15, 1032), (16, 1024)])
 @pytest.mark.parametrize("offset", [0, 4, 1])
 def test_prompt_attention_op_with_masks_that_come_in_tiles(device, heads, kv_heads, head_dim, queries, keys, offset):
-    """Mask rows on 16-byte boundaries come by tiled copies, whose boxes end beyond the last position, query or sequence; the
+    """Mask rows on 16-byte boundaries come by tiled copies where there are queries or positions enough, whose boxes end beyond the last position, query or sequence; the
     same mask elsewhere in memory comes row by row, with the same bits."""
     from oracle import decoder_oracle as oracle
 
