@@ -104,8 +104,9 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
 // Whether a call of the attention op (not causal; heads: of all sequences) goes to the tcgen05 kernel, with blocks of 128 queries,
 // or to the one on mma.sync, with blocks of 64.  Times in us of a round of blocks as fitted to both kernels over heads 9 to 1024, 1 to
 // 320 queries and 64 to 1400 keys: the first has one block to an SM and half the time per tile of 64 keys; the second has two with head size
-// 64, and half the idle rows where the queries are few.  32 heads of 64 x 32 sequences, one query and 128 keys: 52.6 us on tcgen05, 28.7
-// on mma.sync; 64 x 128 54.8 and 37.4 with a mask; 128 x 512 100 and 146.
+// 64, and half the idle rows where the queries are few.  32 heads of 64 x 32 sequences with a mask, one query and 128 keys: 48 us on
+// tcgen05, 27 on mma.sync; 64 x 128 50 and 33; 128 x 512 91 and 145.  The fit is of times from before masks came in tiles; over 423
+// shapes timed since, the kernel taken is within a tenth of the other but for seven, which are within 17 %.
 inline bool attention_on_tcgen05(int head_dim, int q_len, int k_len, long long heads, bool masked, int sms, bool limited) {
   if (k_len < 65) return false;  // one tile: 9.3 us against 10.0 for 32 heads of 64 x 64 with a mask
   const double tiles = (k_len + 63) / 64;
