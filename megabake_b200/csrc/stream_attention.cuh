@@ -60,7 +60,7 @@ __device__ __forceinline__ void stream_head_words(StreamMisc* sm, const bf16* he
 // a / b from 1 / b and one correction by the remainder (Markstein, 1990): the quotient rounded to nearest wherever that and the
 // remainder are normal numbers.  A division takes a branch of its own for a = 0, and a short context has many: positions
 // behind it weigh nothing (a context of one tile: 135M shape, 16 steps 8644 -> 8094 us, 0.5B 546 -> 520).
-__device__ __forceinline__ float stream_divide(float a, float b, float inverse) {
+__host__ __device__ __forceinline__ float stream_quotient(float a, float b, float inverse) {
   const float q = a * inverse;
   return fmaf(fmaf(-q, b, a), inverse, q);
 }
@@ -257,8 +257,8 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
           const float inverse = 1.f / total;
 #pragma unroll
           for (int bi = 0; bi < BPW; ++bi) {
-            s[bi][h] = bf16_round(stream_divide(ex2(s[bi][h] - top), total, inverse));
-            s[bi][h + 2] = bf16_round(stream_divide(ex2(s[bi][h + 2] - top), total, inverse));
+            s[bi][h] = bf16_round(stream_quotient(ex2(s[bi][h] - top), total, inverse));
+            s[bi][h + 2] = bf16_round(stream_quotient(ex2(s[bi][h + 2] - top), total, inverse));
           }
         }
         if (nsplit > 1) stream_sync();  // the statistics have been read: the area is free for the sums

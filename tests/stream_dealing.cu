@@ -1,7 +1,10 @@
 // Host build of the streaming decode kernel's dealing of cached positions, for test_stream_dealing.py: walks one layer the
-// way the kernel's producer and its helper thread do and checks what the consumers rely on.
+// way the kernel's producer and its helper thread do and checks what the consumers rely on.  Beside it its quotient.
+#include <cmath>
+#include <cstring>
 #include <vector>
 
+#include "../megabake_b200/csrc/stream_attention.cuh"
 #include "../megabake_b200/csrc/stream_plan.h"
 
 using namespace mk;
@@ -98,3 +101,20 @@ extern "C" int check_dealing(int grid, int batch, int q_heads, int kv_heads, int
     }
   return 0;
 }
+
+// Numerators of `count` random mantissas with exponents low to high over denominators 1 to 2^14: quotients that are not the
+// division's, and those that are not after the rounding to bf16.
+extern "C" void quotients(int low, int high, int count, long long* differ, long long* differ_rounded) {
+  unsigned long long state = 88172645463325252ull;
+  *differ = *differ_rounded = 0;
+  for (int i = 0; i < count; ++i) {
+    state ^= state << 13, state ^= state >> 7, state ^= state << 17;
+    const float a = std::ldexp(1.f + static_cast<float>((state >> 20) & 0x7FFFFF) / 8388608.f, low + static_cast<int>(state % (high - low + 1)));
+    const float b = i % 2 ? 1.f + static_cast<float>((state >> 43) % 65536) * 0.25f
+                          : std::ldexp(1.f + static_cast<float>((state >> 41) & 0x7FFFFF) / 8388608.f, static_cast<int>((state >> 8) % 14));
+    const float mine = stream_quotient(a, b, 1.f / b), exact = a / b;
+    *differ += mine != exact;
+    *differ_rounded += __bfloat162float(__float2bfloat16_rn(mine)) != __bfloat162float(__float2bfloat16_rn(exact));
+  }
+}
+extern "C" float quotient(float a, float b) { return stream_quotient(a, b, 1.f / b); }

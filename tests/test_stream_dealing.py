@@ -120,3 +120,18 @@ def test_fewer_ctas_take_no_more_rounds_of_tiles(deal):
     small = (576, 9, 3, 64, 1536, 30)
     assert deal.lib.grid_of(_shape(small, sm_limit=30), 1, 30) == 30 and deal.lib.grid_of(_shape(small), 1, 7) == 7
     assert deal.lib.grid_of(_shape(small), 9, 148) == deal.lib.grid_of(_shape(small), 17, 148) == 148
+
+
+def test_quotients_of_the_probabilities_are_the_divisions(deal):
+    """Every quotient is the division's while it and its remainder are normal numbers, and below that, of the smallest
+    probabilities, after the rounding to bf16."""
+    differ, rounded = ctypes.c_longlong(), ctypes.c_longlong()
+    deal.lib.quotients(-80, 0, 4000000, ctypes.byref(differ), ctypes.byref(rounded))
+    assert differ.value == 0 and rounded.value == 0
+    deal.lib.quotients(-126, -81, 4000000, ctypes.byref(differ), ctypes.byref(rounded))
+    assert rounded.value == 0
+    deal.lib.quotient.restype = ctypes.c_float
+    deal.lib.quotient.argtypes = [ctypes.c_float, ctypes.c_float]
+    assert deal.lib.quotient(0.0, 3.0) == 0.0 and deal.lib.quotient(1.0, 1.0) == 1.0
+    for a, b in ((float("nan"), 2.0), (1.0, float("nan")), (float("nan"), float("nan"))):
+        assert deal.lib.quotient(a, b) != deal.lib.quotient(a, b)
