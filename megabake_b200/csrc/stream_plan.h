@@ -98,11 +98,13 @@ inline bool stream_phases(const mk_config& c, int plan, int grid, StreamPhase* p
 //  - there are four CTAs to every KV head of every sequence of the launch, else a long context is cut into too few runs (1000 to 16000
 //    positions, KV heads x sequences: 15 442 -> 431, 341 -> 332, 24 518 -> 489, 298 -> 279; 32 365 -> 376, 594 -> 645; 48 753 -> 878;
 //    128 363 -> 394).
+//  - the hidden size is 512 at least: below it there is less to gain than a tile of the cache more costs (hidden 256, 8 layers, one
+//    sequence at 1000 134 -> 138, four at 4000 153 -> 163).
 // With more than eight sequences long contexts are a round of cache tiles longer (0.5B, 32 at 1900 904 -> 955).  A handle with a limit
 // on its SMs uses what it was given.  Returns the number of CTAs, 0 where the shape has all of them in any case.
 inline int stream_few_ctas(const mk_config& c, int sms) {
   const int few = (3 * sms / 4 + 7) / 8 * 8;
-  if (c.sm_limit > 0 || few >= sms) return 0;
+  if (c.sm_limit > 0 || c.hidden < 512 || few >= sms) return 0;
   StreamPhase less[kStreamPhases], all[kStreamPhases];
   stream_phases(c, kStreamFew, few, less);
   stream_phases(c, 0, sms, all);

@@ -73,6 +73,7 @@ TIMES = {
     (768, 12, 12, 64, 3072, 16): {(1, 60): (281, 280), (4, 4000): (399, 368), (8, 60): (315, 302)},
     (512, 8, 8, 64, 1536, 16): {(1, 4000): (288, 312), (3, 1000): (271, 276), (4, 4000): (338, 332), (8, 60): (274, 286), (8, 4000): (439, 408)},
     (640, 10, 2, 64, 2560, 16): {(1, 60): (274, 282), (8, 60): (297, 312), (8, 4000): (339, 353)},
+    (256, 4, 4, 64, 512, 8): {(1, 1000): (138, 134), (4, 1000): (142, 142), (4, 4000): (163, 153), (8, 4000): (179, 171)},
     (320, 5, 5, 64, 4992, 16): {(1, 300): (296, 301), (1, 16000): (390, 387), (4, 4000): (350, 353), (8, 4000): (408, 388)},
     (1536, 12, 2, 128, 8960, 16): {(1, 60): (491, 488), (8, 60): (537, 529)},
     (2048, 32, 32, 64, 8192, 16): {(1, 60): (544, 495), (4, 1000): (664, 585), (8, 4000): (1208, 1174)},
@@ -106,13 +107,13 @@ def test_fewer_ctas_take_no_more_rounds_of_tiles(deal):
         head_dim = rng.choice((64, 128))
         kv_heads = rng.randint(1, 16)
         heads = kv_heads * rng.randint(1, 8)
-        sizes = (64 * rng.randint(2, 32), heads, kv_heads, head_dim, 64 * rng.randint(4, 140), rng.randint(1, 32))
+        sizes = (64 * rng.randint(6, 32), heads, kv_heads, head_dim, 64 * rng.randint(4, 140), rng.randint(1, 32))
         batch, sms = rng.randint(1, 32), rng.choice((148, 148, 132, 20))
         grid = deal.lib.grid_of(_shape(sizes), batch, sms)
         if grid == sms:
             continue
         fewer += 1
-        assert batch <= 8 and grid >= 3 * sms // 4 and 4 * batch * kv_heads <= grid
+        assert batch <= 8 and sizes[0] >= 512 and grid >= 3 * sms // 4 and 4 * batch * kv_heads <= grid
         less, every = ([deal.lib.rounds_of(_shape(sizes), kind, n) for kind in range(5)] for n in (grid, sms))
         assert sum(less[:4]) <= sum(every[:4]) and less[4] <= every[4] + sizes[5]
         a_phase_more += any(a > b for a, b in zip(less[:4], every[:4]))
