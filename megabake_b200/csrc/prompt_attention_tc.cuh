@@ -13,11 +13,11 @@
 // What bounds it: the chain of a group's tile, one block of eight such warps to an SM (32 heads of 64 x 512 with a mask 12.9 us on
 // the device).  From the first look at memory: scores after 1.9 us, then 1.75 a tile of a group (0.45 scores and mask, 0.65
 // exponentials, of which 0.27 are the unit's rate, 0.3 sums, 0.35 P and waits), 1.2 exchange, 1.3 quotients and stores.
-// A mask with rows on 16-byte boundaries comes by TMA beside the keys and values: a thread reading its own row touched 32 lines a
-// request, 2000 cycles of the load unit for a pair of tiles (512: 13.7 -> 12.9 us, 1024 41.5 -> 38.2, head size 128 20.5 -> 17.7,
-// a third of it the columns that both groups now finish).  Others keep those loads: fetched a row at a time through shared memory
-// they were faster with an even number of positions (500: 17.7 -> 15.8) and slower with an odd one (501: 17.7 -> 20.4); by two warps of
-// their own 27.8.
+// A mask with rows on 16-byte boundaries and queries enough (attention_mask_in_tiles) comes by TMA beside the keys and values: a
+// thread reading its own row touched 32 lines a request, 2000 cycles of the load unit for a pair of tiles (512: 13.7 -> 12.9 us, 1024
+// 41.5 -> 38.2, head size 128 20.5 -> 17.7, a third of it the columns that both groups now finish).  Others keep those loads: fetched a
+// row at a time through shared memory they were faster with an even number of positions (500: 17.7 -> 15.8) and slower with an odd one
+// (501: 17.7 -> 20.4); by two warps of their own 27.8.
 #pragma once
 #include <type_traits>
 
@@ -55,7 +55,7 @@ struct AttnTcMisc {
 struct AttnTcMaps {
   CUtensorMap q, k, v, mask;  // (mask: (positions, queries, sequences))
   int q_ok;     // the queries begin on a 16-byte boundary; otherwise their rows are fetched with plain loads
-  int mask_ok;  // there is a mask, and its rows begin on 16-byte boundaries
+  int mask_ok;  // there is a mask that comes in tiles: its rows begin on 16-byte boundaries
 };
 
 // B operand stored with its N dimension contiguous: 64-element chunks [8 rows of K][128 B], 128-byte swizzle.  Rows of K in
