@@ -10,6 +10,13 @@
 //   values: D[16 dims][heads]           += V tile^T (ldmatrix.trans) x p[positions][heads]
 // where p's B fragment is the transpose of the score fragment (movmatrix).  The new position is not in the cache
 // yet: the warp whose block holds it writes its rows into the tile (and into the caches) before it reads them.
+//
+// What comes behind the last tile is a chain of dependent instructions that every CTA's o_proj waits for, as is all of a context of
+// one tile, so its length counts: no value sums for blocks that hold no position, one exchange of statistics instead of two, the
+// warps' sums weighed in every lane instead of passed along, as many stores as there are copies and no loop.  Of the 2.9 us from
+// the first score to the last result of a context of 49 positions (135M shape, by clock) 1.4 are left; a step, us: 135M, one
+// sequence at 48 447 -> 407, 18 at 55 790 -> 702; 0.5B, one at 99 467 -> 447; 1.7B, one at 1024 745 -> 731, three at 777 827 -> 812, six of up
+// to 1500 975 -> 927, sixteen at 1024 1425 -> 1404, 32 at 500 1728 -> 1705.  The same bits.
 #pragma once
 #include "stream_common.cuh"
 
@@ -65,7 +72,7 @@ __host__ __device__ __forceinline__ float stream_quotient(float a, float b, floa
   return fmaf(fmaf(-q, b, a), inverse, q);
 }
 
-template <int HD>
+template <int TM, int HD>
 __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& pipe, int layer) {
   StreamMisc* const sm = stream_opaque(th.sm);
   const int wtid = stream_opaque(th.wtid);
@@ -85,6 +92,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
   const float scale = p.att_scale * 1.4426950408889634f;  // scores in units of log2
   const int style = p.rope_style;
   constexpr int kRow = HD + 2;
+  float4* const stats = reinterpret_cast<float4*>(scratch + kStreamWarps * gs * kRow);  // behind the sums: [KV head][split][pair of query heads]
 
   // Lists of parts, mostly one (every layer has at least one, if empty).
   int count = stream_next_list(sm, th.list);
@@ -98,6 +106,10 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
       count = stream_next_list(sm, th.list);
       part = -1;
       continue;
+    }
+    if (TM > 8 && part > 0) {  // the scratch has been read
+      if (nsplit == 1) __syncwarp();
+      else stream_sync();
     }
     const StreamSegment sg = sm->seg[th.list & 1][part];
     const int len = sg.len;  // the new position
@@ -118,7 +130,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
     // The part that ends the context has the new position in its last tile: the warp of its block fetches the new key
     // and value, a word and its rotation partner per lane.
     const int new_block = (len % tk) >> 4;  // block of the tile
-    const bool owner = sg.t1 == sg.nt && new_block % nsplit == split && lane < HD / 4;
+    const bool own_warp = sg.t1 == sg.nt && new_block % nsplit == split, owner = own_warp && lane < HD / 4;
     uint32_t kn[2] = {0u, 0u}, vn[2] = {0u, 0u}, kc = 0u, ks = 0u;
     const uint32_t* const kw = reinterpret_cast<const uint32_t*>(row + q_size + kvh * HD) + lane;
     if (owner) {
@@ -170,12 +182,15 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
 #pragma unroll 1
     for (int tl = sg.t0; tl < sg.t1; ++tl) {
       const int key0 = tl * tk;
+      const bool patched = own_warp && tl == sg.nt - 1;
+      // Blocks behind the new position's meet no values: of a short context's only tile that is most of them.
+      const int blocks = ((len - key0) >> 4) - split;  // of this warp's: block bi is live if bi * nsplit <= blocks
       // --- scores of this warp's blocks of the tile (two at most)
       float s[BPW][4];
       stream_wait(sm, pipe.full(), pipe.parity);
       {
         const uint32_t base = pipe.addr() + static_cast<uint32_t>(hh) * (HD / 64) * chunk_bytes;
-        if (tl == sg.nt - 1) patch(base, kn);
+        if (patched) patch(base, kn);
 #pragma unroll
         for (int bi = 0; bi < BPW; ++bi) {
           s[bi][0] = s[bi][1] = s[bi][2] = s[bi][3] = 0.f;
@@ -189,7 +204,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
           }
         }
       }
-      if (tl == sg.nt - 1) fence_proxy_async_smem();  // the next copy into this slot comes after the stores above
+      if (patched) fence_proxy_async_smem();  // the next copy into this slot comes after the stores above
       stream_release(pipe, lane);
       float mt[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -208,7 +223,6 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
         mt[0] = fmaxf(mt[0], __shfl_xor_sync(0xffffffffu, mt[0], x));
         mt[1] = fmaxf(mt[1], __shfl_xor_sync(0xffffffffu, mt[1], x));
       }
-      float alpha[2];
       if (sg.nt == 1) {
         // The whole context is this tile: the warps exchange maximum and sum first, and the probabilities are
         // normalised before they are rounded, as the reference's are.
@@ -225,44 +239,44 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
           own[0] += __shfl_xor_sync(0xffffffffu, own[0], x);
           own[1] += __shfl_xor_sync(0xffffffffu, own[1], x);
         }
-        // A warp that holds its heads' whole context alone has nothing to exchange: the others, which it does not wait for,
-        // may have their value sums in the scratch already.
-        float2* const stat = reinterpret_cast<float2*>(scratch) + hh * 64;  // [split][query head]
+        // A warp that holds its heads' whole context alone has nothing to exchange.
+        float4* const stat = stats + hh * nsplit * 4 + lt;
         if (nsplit > 1) {
-          if (lg == 0) {
-            stat[split * 8 + 2 * lt] = make_float2(mt[0], own[0]);
-            stat[split * 8 + 2 * lt + 1] = make_float2(mt[1], own[1]);
-          }
+          if (lg == 0) stat[split * 4] = make_float4(mt[0], own[0], mt[1], own[1]);
           stream_sync();
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float2 all[8];
-          float top = -INFINITY, total = 0.f;
+        if (blocks >= 0) {
+          float4 all[8];
 #pragma unroll
           for (int s8 = 0; s8 < 8; ++s8) {
-            all[s8] = make_float2(-INFINITY, 0.f);
+            all[s8] = make_float4(-INFINITY, 0.f, -INFINITY, 0.f);
             if (nsplit == 1) {
-              if (s8 == 0) all[s8] = make_float2(mt[h], own[h]);
+              if (s8 == 0) all[s8] = make_float4(mt[0], own[0], mt[1], own[1]);
             } else if (s8 < nsplit) {
-              all[s8] = stat[s8 * 8 + 2 * lt + h];
+              all[s8] = stat[s8 * 4];
             }
-            top = fmaxf(top, all[s8].x);
           }
 #pragma unroll
-          for (int s8 = 0; s8 < 8; ++s8) total = fmaf(all[s8].y, ex2(all[s8].x - top), total);
-          alpha[h] = 0.f;
-          m[h] = top;
-          l[h] = (split == 0 && lg == 0) ? 1.f : 0.f;  // the parts are only to be added
-          const float inverse = 1.f / total;
+          for (int h = 0; h < 2; ++h) {
+            if (h == 1 && gs == 1) continue;  // nobody's head
+            float top = -INFINITY, total = 0.f;
 #pragma unroll
-          for (int bi = 0; bi < BPW; ++bi) {
-            s[bi][h] = bf16_round(stream_quotient(ex2(s[bi][h] - top), total, inverse));
-            s[bi][h + 2] = bf16_round(stream_quotient(ex2(s[bi][h + 2] - top), total, inverse));
+            for (int s8 = 0; s8 < 8; ++s8) top = fmaxf(top, h == 0 ? all[s8].x : all[s8].z);
+#pragma unroll
+            for (int s8 = 0; s8 < 8; ++s8) total = fmaf(h == 0 ? all[s8].y : all[s8].w, ex2((h == 0 ? all[s8].x : all[s8].z) - top), total);
+            m[h] = top;
+            l[h] = (split == 0 && lg == 0) ? 1.f : 0.f;  // the parts are only to be added
+            const float inverse = 1.f / total;
+#pragma unroll
+            for (int bi = 0; bi < BPW; ++bi) {
+              if (bi * nsplit > blocks) continue;
+              s[bi][h] = bf16_round(stream_quotient(ex2(s[bi][h] - top), total, inverse));
+              s[bi][h + 2] = bf16_round(stream_quotient(ex2(s[bi][h + 2] - top), total, inverse));
+            }
           }
         }
-        if (nsplit > 1) stream_sync();  // the statistics have been read: the area is free for the sums
-      } else {
+      } else if (blocks >= 0) {
+        float alpha[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float mn = fmaxf(m[h], mt[h]);
@@ -277,34 +291,32 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
             l[h] += s[bi][h] + s[bi][h + 2];
           }
         }
-      }
 #pragma unroll
-      for (int d = 0; d < KS; ++d) {
-        o[d][0] *= alpha[0];
-        o[d][1] *= alpha[1];
-        o[d][2] *= alpha[0];
-        o[d][3] *= alpha[1];
+        for (int d = 0; d < KS; ++d) {
+          o[d][0] *= alpha[0];
+          o[d][1] *= alpha[1];
+          o[d][2] *= alpha[0];
+          o[d][3] *= alpha[1];
+        }
       }
       // --- value sums
       stream_wait(sm, pipe.full(), pipe.parity);
-      {
+      if (blocks >= 0) {
         const uint32_t base = pipe.addr() + static_cast<uint32_t>(hh) * (HD / 64) * chunk_bytes;
-        if (tl == sg.nt - 1) {
+        if (patched) {
           // positions past the context meet zero probabilities, but what the cache holds there must be finite for
-          // the product to be zero: clear those rows of this warp's blocks
-#pragma unroll
-          for (int bi = 0; bi < BPW; ++bi) {
+          // the product to be zero: clear those rows of the new position's block
+          const int piece = lane % (HD / 8), block0 = (len - key0) & ~15;
 #pragma unroll 1
-            for (int it = lane; it < 16 * (HD / 8); it += 32) {
-              const int key = (split + bi * nsplit) * 16 + it / (HD / 8), piece = it % (HD / 8);
-              if (key0 + key > len)
-                asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(base + (piece >> 3) * chunk_bytes + key * 128 + ((piece & 7) << 4)), "r"(0u) : "memory");
-            }
+          for (int r = (len & 15) + 1 + lane / (HD / 8); r < 16; r += 32 / (HD / 8)) {
+            const int key = block0 + r;
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(base + (piece >> 3) * chunk_bytes + key * 128 + ((piece & 7) << 4)), "r"(0u) : "memory");
           }
           patch(base, vn);
         }
 #pragma unroll
         for (int bi = 0; bi < BPW; ++bi) {
+          if (bi * nsplit > blocks) continue;
           // probabilities as a bf16 and the bf16 of what it leaves out: they are not normalised yet, so one rounding here
           // would not be the reference's, and the tensor cores have time for both
           const uint32_t w0 = pack2(s[bi][0], s[bi][1]), w1 = pack2(s[bi][2], s[bi][3]);
@@ -321,7 +333,7 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
             mma_bf16_16816(o[d], af, c0, c1);
           }
         }
-        if (tl == sg.nt - 1) fence_proxy_async_smem();
+        if (patched) fence_proxy_async_smem();
       }
       stream_release(pipe, lane);
     }
@@ -351,36 +363,40 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
     }
     if (nsplit == 1) __syncwarp();
     else stream_sync();
+    bf16* const attn = sm->plan.attn[th.turn];
+    bf16* const clear = sm->plan.attn[th.last_turn];
     const int h0 = nsplit == 1 ? hh * gs : warp, h1 = nsplit == 1 ? h0 + gs : min(warp + 1, heads);
 #pragma unroll 1
     for (int hl = h0; hl < h1; ++hl) {
-      // lane s weighs warp s's sums (a warp that saw no position has -inf: weight zero)
+      // Every lane weighs all warps' sums itself (a warp that saw no position has -inf: weight zero): the block waits for this
+      // warp, and a maximum and a sum passed from lane to lane are a chain of eight exchanges.
       const float* const mine = scratch + hl * kRow;
       const int split_row = heads * kRow;
-      float mm = -INFINITY, ll = 0.f, acc[DPL];
-      if (lane < nsplit) {
-        mm = mine[lane * split_row + HD];
-        ll = mine[lane * split_row + HD + 1];
+      float2 st[8];
+#pragma unroll
+      for (int s8 = 0; s8 < 8; ++s8) {
+        st[s8] = make_float2(-INFINITY, 0.f);
+        if (s8 < nsplit) st[s8] = *reinterpret_cast<const float2*>(mine + s8 * split_row + HD);
       }
-      float weight = mm;
-#pragma unroll
-      for (int x = 1; x < 8; x <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, x));
-      mm = __shfl_sync(0xffffffffu, mm, 0);
-      weight = ex2(weight - (mm > -INFINITY ? mm : 0.f));  // (a part may hold nothing but scores of -inf: its weights are zero)
-      ll *= weight;
-#pragma unroll
-      for (int x = 1; x < 8; x <<= 1) ll += __shfl_xor_sync(0xffffffffu, ll, x);
-      ll = __shfl_sync(0xffffffffu, ll, 0);
+      float mm = fmaxf(fmaxf(fmaxf(st[0].x, st[1].x), fmaxf(st[2].x, st[3].x)), fmaxf(fmaxf(st[4].x, st[5].x), fmaxf(st[6].x, st[7].x)));
+      const float safe = mm > -INFINITY ? mm : 0.f;  // (a part may hold nothing but scores of -inf: its weights are zero)
+      float acc[DPL];
 #pragma unroll
       for (int i = 0; i < DPL; ++i) acc[i] = 0.f;
 #pragma unroll
       for (int s8 = 0; s8 < 8; ++s8) {
+        const float w = ex2(st[s8].x - safe);
+        st[s8].y = __fmul_rn(st[s8].y, w);  // (rounded before it is added)
         if (s8 < nsplit) {
-          const float w = __shfl_sync(0xffffffffu, weight, s8);
 #pragma unroll
-          for (int i = 0; i < DPL; ++i) acc[i] = fmaf(w, mine[s8 * split_row + lane * DPL + i], acc[i]);
+          for (int i = 0; i < DPL / 2; ++i) {
+            const float2 v = *reinterpret_cast<const float2*>(mine + s8 * split_row + lane * DPL + 2 * i);
+            acc[2 * i] = fmaf(w, v.x, acc[2 * i]);
+            acc[2 * i + 1] = fmaf(w, v.y, acc[2 * i + 1]);
+          }
         }
       }
+      float ll = ((st[0].y + st[1].y) + (st[2].y + st[3].y)) + ((st[4].y + st[5].y) + (st[6].y + st[7].y));
       const int head = sg.group * heads + hl;
       unsigned long long* rec = sm->plan.rec + (static_cast<size_t>(sg.b) * p.q_heads + head) * kStreamMaxSegments * kRow;
       const unsigned long long tag = static_cast<unsigned long long>(stamp) << 32;
@@ -432,18 +448,29 @@ __device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& p
             for (int i = 0; i < DPL; ++i) acc[i] = acc[i] * wa + __uint_as_float(static_cast<uint32_t>(w[s4][i])) * wb;
           }
       }
-      const int tm = sm->token_class;
+      constexpr int copies = stream_copies(TM);
+      bf16* const out = attn + stream_place(TM, sg.b, head * HD + lane * DPL);
+      bf16* const reset = clear + stream_place(TM, sg.b, head * HD + lane * DPL);
+      // A word is two adjacent columns; the next two of a lane, of the same group of eight, lie 8 elements on.
 #pragma unroll
-      for (int i = 0; i < DPL; i += 2) {
-        const int to = stream_place(tm, sg.b, head * HD + lane * DPL + i);
-        const uint32_t word = pack2(acc[i] / ll, acc[i + 1] / ll);
-        const int copies = sm->copies, elems = tm * q_size;
-        for (int c = 0; c < copies; ++c) st_relaxed_u32(reinterpret_cast<uint32_t*>(sm->plan.attn[th.turn] + to + c * elems), word);
-        for (int c = 0; c < copies; ++c) st_relaxed_u32(reinterpret_cast<uint32_t*>(sm->plan.attn[th.last_turn] + to + c * elems), kUnset);
+      for (int i = 0; i < DPL / 2; ++i) {
+        const uint32_t word = pack2(acc[2 * i] / ll, acc[2 * i + 1] / ll);
+#pragma unroll
+        for (int c = 0; c < copies; ++c) st_relaxed_u32(reinterpret_cast<uint32_t*>(out + static_cast<size_t>(c) * TM * q_size + 8 * i), word);
       }
+#pragma unroll
+      for (int i = 0; i < DPL / 2; ++i)
+#pragma unroll
+        for (int c = 0; c < copies; ++c) st_relaxed_u32(reinterpret_cast<uint32_t*>(reset + static_cast<size_t>(c) * TM * q_size + 8 * i), kUnset);
     }
-    if (nsplit == 1) __syncwarp();
-    else stream_sync();  // the scratch has been read
+    // The next part's sums come when these have been read.  Behind the last part that is so without a barrier, and the warps that add
+    // nothing up could go on; but up to eight tokens they would look for o_proj's operand the whole time, in the way of those who
+    // write it (us with the barrier and without: 1.7B shape, one sequence 738 and 742, three 819 and 823, eight 875 and 878, twelve 1056 and
+    // 1048, sixteen 1403 and 1399; 135M 411 and 414).
+    if (TM <= 8) {
+      if (nsplit == 1) __syncwarp();
+      else stream_sync();
+    }
   }
 }
 

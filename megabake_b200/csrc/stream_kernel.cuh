@@ -154,7 +154,7 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     if (wtid < kLayerWords && layer + 1 < layers) word = __ldg(reinterpret_cast<const uint32_t*>(sm->plan.layers + layer + 1) + wtid);
     stream_project<TM, 1, CNORM, SG_NORM, FEW>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
     if (head) break;
-    stream_attention<HD>(th, pipe, layer);                           // RoPE, append, attention
+    stream_attention<TM, HD>(th, pipe, layer);                       // RoPE, append, attention
     th.trace(EV_ATTENTION_DONE);
 #pragma unroll 1
     for (int kind = SP_O;; kind = SP_DOWN) {  // one copy of the code for both (1.7B shape, 16 sequences 1551 -> 1465 us, 32 2334 -> 2268)

@@ -170,10 +170,10 @@ inline int stream_heads_per_tile(const mk_config& c, int batch) {
   return hpu;
 }
 
-// Attention: one row per warp and query head of its KV head (and 64 pairs of statistics per KV head of a tile).
+// Attention: one row per warp and query head of its KV head, and behind them eight warps' statistics of eight query heads.
 // One token: the normalised operand on its way to the fragments (16 windows of 64 bytes per warp).
 inline int stream_scratch_bytes(const mk_config& c, int batch) {
-  return std::max(batch == 1 ? 8192 : 4096, (8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 15) / 16 * 16);
+  return std::max(batch == 1 ? 8192 : 4096, 8 * (c.q_heads / c.kv_heads) * (c.head_dim + 2) * 4 + 512);
 }
 // Two buffers of partial sums up to eight tokens.  With 16, one and a block barrier more per tile leave room for a sixth slot (1.7B shape,
 // sixteen sequences at 200 positions 1088 -> 1068 us, at 1024 1441 -> 1431, fourteen of different lengths 1389 -> 1344); with 32

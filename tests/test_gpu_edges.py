@@ -39,6 +39,30 @@ def test_streaming_decode_with_a_context_of_one_tile_to_a_warp(device, batch, co
     oracle_decode_compare(config, device, batch=batch, capacity=context + 3, prefill=context, steps=3)
 
 
+@pytest.mark.parametrize("batch,heads,kv_heads,head_dim", [(1, 9, 3, 64), (1, 4, 4, 64), (3, 14, 2, 64), (8, 8, 8, 64), (2, 8, 2, 128), (16, 32, 32, 64)])
+@pytest.mark.parametrize("context", [0, 14, 15, 16, 31, 47, 48, 127, 128, 240, 256, 271])
+def test_streaming_decode_reads_nothing_behind_the_new_position(device, batch, heads, kv_heads, head_dim, context):
+    """Blocks of 16 positions behind the new one are left out, its own block is cleared behind it: whatever the caches hold there, not
+    numbers included, the result is the one beside zeros, in every bit."""
+    config = tiny_config(hidden=512, q_heads=heads, kv_heads=kv_heads, head_dim=head_dim, intermediate=768)
+    capacity = context + 300
+    kernel = make_kernel(config, synth_weights(config, seed=21, norm_std=0.1, device=device), device, max_tokens=batch, max_positions=capacity)
+    ids = synth_ids(batch, config.vocab, seed=21).view(batch, 1).to(device)
+    positions = torch.full((batch, 1), context, dtype=torch.int64, device=device)
+    results = []
+    for behind in (0.0, float("nan"), float("inf")):
+        keys, values, lengths = new_kv_state(config, batch, capacity, device)
+        for layer in range(config.layers):
+            for name, caches in (("k", keys), ("v", values)):
+                caches[layer].copy_(synth_normal(tuple(caches[layer].shape), seed=21, name=f"{name}{layer}", std=0.5, device=device))
+                caches[layer][:, context:] = behind
+            lengths[layer].fill_(context)
+        results.append(kernel.decode(ids, positions, keys, values, lengths))
+        kernel.check()
+    assert bool(torch.isfinite(results[0]).all())
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+
+
 @pytest.mark.parametrize("lengths_now,sm_limit", [
     ([1000] * 28 + [10] * 4, 0), ([10] * 7 + [4000] * 9, 0), ([8000] * 6 + [10] * 6, 0),  # 17, 22 and 42 parts in one CTA
     ([40] * 32, 4),                                                                       # 32 of equal lengths: few CTAs
