@@ -73,10 +73,9 @@ __host__ __device__ __forceinline__ float stream_quotient(float a, float b, floa
 }
 
 template <int TM, int HD>
-__device__ __forceinline__ void stream_attention(StreamThread& th, StreamPipe& pipe, int layer) {
+__device__ __forceinline__ void stream_attention(const KParams& p, StreamThread& th, StreamPipe& pipe, int layer) {
   StreamMisc* const sm = stream_opaque(th.sm);
   const int wtid = stream_opaque(th.wtid);
-  const KParams& p = *sm->p;
   const bf16* const qkv = sm->plan.dst[SP_QKV][th.turn];  // [sequence][q | k | v], plain order
   const uint32_t stamp = p.att_epoch + static_cast<uint32_t>(layer) + 1u;
   float* const scratch = reinterpret_cast<float*>(stream_scratch(sm));  // [slot of a (warp, head)][HD + 2]

@@ -30,8 +30,7 @@ __device__ __forceinline__ uint4 stream_plain_vec(const bf16* window, int t) {
 // Layer 0's residual stream is the embedding rows of the token ids: dealt to the CTAs and written like any result, so that
 // its readers need not know.
 template <int TM>
-__device__ __forceinline__ void stream_embed(StreamMisc* sm, int wtid) {
-  const KParams& p = *sm->p;
+__device__ __forceinline__ void stream_embed(const KParams& p, StreamMisc* sm, int wtid) {
   const int pairs = p.hidden / 2, items = p.m * pairs;
   uint32_t* const dst = reinterpret_cast<uint32_t*>(const_cast<bf16*>(sm->plan.src[SP_QKV][0]));
   for (int i = sm->cta * kStreamConsumers + wtid; i < items; i += sm->grid * kStreamConsumers) {
@@ -187,14 +186,14 @@ __device__ __forceinline__ void stream_normalise(const bf16* normw, int ncopy, i
 // The normalised operand of one token.  In fragment order only four lanes would have work, so a warp deals its vectors to all
 // lanes, normalises them there and passes them to the fragment's lanes through shared memory of its own.
 template <int NC>
-__device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16* src, const bf16* normw, int k, int ncopy, int live, int wtid,
+__device__ __forceinline__ void stream_operand_spread(const KParams& p, StreamMisc* sm, const bf16* src, const bf16* normw, int k, int ncopy, int live, int wtid,
                                                       uint32_t (&frag)[NC * kStreamWpc][1][4]) {
   constexpr int IT = NC * kStreamWpc * 4 / 32;  // vectors per lane; a second one only where a warp has more than eight windows
   const int warp = wtid >> 5, lane = wtid & 31;
   const int first = (lane >> 2) * 8 + warp;  // this lane's first window; the next one is 64 on
   const int left = live - (lane >> 2);       // this lane has vector i if 8 i < left
   const bool more = live > 8;
-  const float fk = static_cast<float>(k), eps = sm->p->eps;
+  const float fk = static_cast<float>(k), eps = p.eps;
   uint4 w[IT], x[IT];
 #pragma unroll
   for (int i = 0; i < IT; ++i) {
@@ -246,7 +245,7 @@ __device__ __forceinline__ void stream_operand_spread(StreamMisc* sm, const bf16
 // One projection phase for this CTA's units.  TM: token class; NACC: weight matrices per tile (gate and up: two); NC:
 // copies of a slice whose operand fits the registers; GROUP: what happens to operand and result; FEW: at most four tokens.
 template <int TM, int NACC, int NC, int GROUP, bool FEW>
-__device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pipe, int kind, int layer) {
+__device__ __forceinline__ void stream_project(const KParams& p, StreamThread& th, StreamPipe& pipe, int kind, int layer) {
   constexpr int NT = stream_token_tiles(TM), WPC = kStreamWpc;
   constexpr int SETS = NT <= 2 ? 2 : 1;  // accumulator sets: consecutive MMAs of a tile do not wait for one another
   constexpr int LPT = 4 / NT;            // lanes per token in the epilogue
@@ -324,7 +323,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
     if constexpr (!NORM) {
       fetch(0);
     } else if constexpr (TM == 1) {
-      stream_operand_spread<NC>(sm, src, normw, k, ncopy, live, wtid, frag);
+      stream_operand_spread<NC>(p, sm, src, normw, k, ncopy, live, wtid, frag);
     } else {
       const int kbase = slice * cs * kChunkK + warp * 32;
       uint4 ahead[kStreamWeightsAhead<NT> ? NC * WPC : 1];
@@ -351,7 +350,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
         }
       }
       stream_sync();
-      const float fk = static_cast<float>(k), eps = sm->p->eps;
+      const float fk = static_cast<float>(k), eps = p.eps;
       float r[NT];
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
@@ -474,7 +473,7 @@ __device__ __forceinline__ void stream_project(StreamThread& th, StreamPipe& pip
         } else if (kind == SP_QKV) {
           store(col, pack2(sum[0].x + b0, sum[0].y + b1));
         } else if (q == 0) {
-          bf16* out = sm->p->logits + static_cast<size_t>(tok) * n_cols + col;
+          bf16* out = p.logits + static_cast<size_t>(tok) * n_cols + col;
           if ((n_cols & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0) {  // logits may begin at any element
             *reinterpret_cast<uint32_t*>(out) = pack2(sum[0].x, sum[0].y);
           } else {

@@ -8,8 +8,7 @@
 namespace mk {
 
 // warp 0, one thread: every copy of this CTA in the order of use.
-__device__ __forceinline__ void stream_producer(StreamMisc* sm, StreamPipe pipe) {
-  const KParams& p = *sm->p;
+__device__ __forceinline__ void stream_producer(const KParams& p, StreamMisc* sm, StreamPipe pipe) {
   const CUtensorMap* const maps = sm->plan.maps;
   const CUtensorMap* const kv_maps = p.kv_maps;
   const uint64_t policy = l2_policy_evict_first();
@@ -106,8 +105,7 @@ __device__ __forceinline__ void stream_producer(StreamMisc* sm, StreamPipe pipe)
 
 // Ask L2 for the small vectors that no copy brings (norm weights, biases): all layers, once, by a warp that has nothing
 // else to do.
-__device__ __forceinline__ void stream_prefetch_vectors(StreamMisc* sm, int lane) {
-  const KParams& p = *sm->p;
+__device__ __forceinline__ void stream_prefetch_vectors(const KParams& p, StreamMisc* sm, int lane) {
   for (int layer = 0; layer < p.layers; ++layer) {
     const StreamLayer* lw = sm->plan.layers + layer;
     for (int i = lane; i < p.hidden / 64; i += 32) {
@@ -127,8 +125,7 @@ __device__ __forceinline__ void stream_reset(bf16* buffer, long long elems, int 
 }
 
 template <int TM, int HD, bool FEW>
-__device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe, int wtid) {
-  const KParams& p = *sm->p;
+__device__ __forceinline__ void stream_consumers(const KParams& p, StreamMisc* sm, StreamPipe pipe, int wtid) {
   constexpr int NT = stream_token_tiles(TM);
   constexpr int CNORM = stream_fit_normalised(TM), CPLAIN = stream_fit(NT);
   constexpr int kLayerWords = sizeof(StreamLayer) / 4;
@@ -141,7 +138,7 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
   th.last_turn = 2;
   th.list = 0;
   th.tracing = wtid == 0 && sm->trace_on != 0;
-  stream_embed<TM>(sm, wtid);
+  stream_embed<TM>(p, sm, wtid);
 #pragma unroll 1
   for (int layer = 0;; ++layer) {  // the last round is the output head
     const bool head = layer == layers;
@@ -152,15 +149,15 @@ __device__ __forceinline__ void stream_consumers(StreamMisc* sm, StreamPipe pipe
     // the next layer's vectors: requested here, passed on through shared memory at the end of the layer
     uint32_t word = 0u;
     if (wtid < kLayerWords && layer + 1 < layers) word = __ldg(reinterpret_cast<const uint32_t*>(sm->plan.layers + layer + 1) + wtid);
-    stream_project<TM, 1, CNORM, SG_NORM, FEW>(th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
+    stream_project<TM, 1, CNORM, SG_NORM, FEW>(p, th, pipe, head ? SP_HEAD : SP_QKV, layer);  // RMSNorm; q, k, v (+ bias) or the output head
     if (head) break;
-    stream_attention<TM, HD>(th, pipe, layer);                       // RoPE, append, attention
+    stream_attention<TM, HD>(p, th, pipe, layer);                       // RoPE, append, attention
     th.trace(EV_ATTENTION_DONE);
 #pragma unroll 1
     for (int kind = SP_O;; kind = SP_DOWN) {  // one copy of the code for both (1.7B shape, 16 sequences 1551 -> 1465 us, 32 2334 -> 2268)
-      stream_project<TM, 1, CPLAIN, SG_PLAIN, FEW>(th, pipe, kind, layer);  // o_proj, down_proj + residual
+      stream_project<TM, 1, CPLAIN, SG_PLAIN, FEW>(p, th, pipe, kind, layer);  // o_proj, down_proj + residual
       if (kind == SP_DOWN) break;
-      stream_project<TM, 2, CNORM, SG_MLP, FEW>(th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
+      stream_project<TM, 2, CNORM, SG_MLP, FEW>(p, th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
       if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
       __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
     }
@@ -293,13 +290,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
   // 384 threads x 168 registers at launch = 128 x 56 + 256 x 224: the token operand of a slice is up to 128 registers
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (tid == 0) stream_producer(sm, pipe);
-    else if (warp == 1 && blockIdx.x == 0) stream_prefetch_vectors(sm, tid - 32);
+    if (tid == 0) stream_producer(p, sm, pipe);
+    else if (warp == 1 && blockIdx.x == 0) stream_prefetch_vectors(p, sm, tid - 32);
     else if (tid == 64) stream_watch(sm);
-    else if (tid == 96) stream_plan_parts(sm);
+    else if (tid == 96) stream_plan_parts(p, sm);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    stream_consumers<TM, HD, FEW>(sm, pipe, tid - 128);
+    stream_consumers<TM, HD, FEW>(p, sm, pipe, tid - 128);
   }
 }
 
