@@ -253,6 +253,10 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, uint32_t addr) {
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+// Arrive on it without waiting.
+__device__ __forceinline__ void named_bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 // The same barrier, and whether any of the threads brought `value`: the same answer for all of them.
 __device__ __forceinline__ bool named_bar_any(int id, int threads, bool value) {
   uint32_t any;

@@ -14,8 +14,8 @@
 // one load: no flag, no fence, no barrier.  Every buffer exists three times, used in turn by the layers; whoever writes a
 // word in layer l resets the same word of layer l - 1's copy, whose readers are done: to write in layer l a CTA has
 // read data that depends on every result of layer l - 1.  That copy is written again in layer l + 2; one fence per layer
-// and thread comes between the reset and the thread's results of layer l + 1, which every reader of layer l + 2 has
-// seen.  The launch ends with a grid barrier, behind which the last layer's words are reset.
+// (of each thread, or of a warp for its CTA: stream_fence) comes between the reset and the thread's results of layer l + 1,
+// which every reader of layer l + 2 has seen.  The launch ends with a grid barrier, behind which the last layer's words are reset.
 #pragma once
 #include "device_common.cuh"
 
@@ -34,6 +34,8 @@ constexpr int kStreamPartPitch = 20;     // floats per token of a tile's partial
 constexpr int kStreamMaxSegments = 24;   // parts a (sequence, head group)'s context may be cut into
 constexpr int kStreamLengths = 1024;     // valid lengths kept in shared memory (layers x sequences when they differ per sequence)
 constexpr uint32_t kUnset = 0xFFFFFFFFu;
+constexpr int kStreamStoredBarrier = 2, kStreamFencedBarrier = 3;  // named barriers of the consumers and the fencing warp (stream_fence)
+constexpr int kStreamFenceThreads = kStreamConsumers + 32;
 
 enum { SP_QKV = 0, SP_O = 1, SP_GU = 2, SP_DOWN = 3, SP_HEAD = 4, kStreamPhases = 5 };
 
@@ -124,6 +126,7 @@ struct StreamMisc {
   int bad;       // prologue verdict
   int complete;  // the grid barrier was reached: one thread's verdict, so that all threads end the launch the same way
   int trace_n, trace_on;
+  int fence_aside;  // stream_fence
   int copies;       // hand-over buffers exist this often
   int psum_offset;  // bytes from the end of this block to the partial sums (the attention area comes first)
   int first_tile[kStreamPhases], first_slice[kStreamPhases], units[kStreamPhases];  // where this CTA's units start, how many
@@ -162,6 +165,30 @@ __device__ __forceinline__ V stream_opaque(V v) {
   if constexpr (sizeof(V) == 4) asm volatile("" : "+r"(v));
   else asm volatile("" : "+l"(v));
   return v;
+}
+
+// The fence of a layer, by a warp of the producer's group: the consumers tell it that their results and resets of the layer up to gate
+// and up are stored, go on, and look whether it has come through before the layer ends.  A fence orders what its thread knows of, so
+// what went before the barrier comes, for everybody on the GPU, before what follows the second one.  (1400 cycles a layer of the 135M
+// shape by clock stamps, ahead of down_proj.)
+// Two to eight tokens only where the ring holds the gate and up matrices of a layer: elsewhere the CTAs end that phase one by one as HBM
+// brings them their weights, and those that are through and have no fence to wait for look for the others' results all the longer.
+// With 32 tokens there is no difference.  A step, fence on the way -> aside (mean of 60 to 1900 positions): 135M shape, one sequence -2.1 %,
+// ten -4.5, sixteen -2.9; 0.5B, one -5.2, eight -3.4, ten -4.4, sixteen -3.6; 1.7B, one 0, two to six +1.0 to 1.3, ten -0.3, sixteen +0.5.
+// The first look comes late, too, with few tokens: 135M, one sequence -2.1 % without and -3.7 to -4.7 with 300 ns; two to six +0.3 to +2.9 and, with
+// 500 ns, -0.8 to -2.0; sixteen -2.9 and -2.0.
+__host__ __device__ constexpr int stream_look_late(int tm) { return tm == 1 ? 300 : (tm <= 8 ? 500 : 0); }  // ns
+template <int TM>
+__device__ __forceinline__ bool stream_fence_aside(const KParams& p, int grid) {
+  if (TM != 8) return TM < 32;
+  return 4ll * p.inter * p.hidden <= static_cast<long long>(p.stream_slots) * kStreamSlotBytes * grid;
+}
+__device__ __forceinline__ void stream_fence(int layers) {
+  for (int layer = 0; layer < layers; ++layer) {
+    named_bar_sync(kStreamStoredBarrier, kStreamFenceThreads);
+    __threadfence();
+    named_bar_arrive(kStreamFencedBarrier, kStreamFenceThreads);
+  }
 }
 
 __device__ __forceinline__ void stream_sync() { named_bar_sync(1, kStreamConsumers); }

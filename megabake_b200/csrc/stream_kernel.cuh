@@ -105,18 +105,18 @@ __device__ __forceinline__ void stream_producer(const KParams& p, StreamMisc* sm
 
 // Ask L2 for the small vectors that no copy brings (norm weights, biases): all layers, once, by a warp that has nothing
 // else to do.
-__device__ __forceinline__ void stream_prefetch_vectors(const KParams& p, StreamMisc* sm, int lane) {
+__device__ __forceinline__ void stream_prefetch_vectors(const KParams& p, StreamMisc* sm, int at, int step) {
   for (int layer = 0; layer < p.layers; ++layer) {
     const StreamLayer* lw = sm->plan.layers + layer;
-    for (int i = lane; i < p.hidden / 64; i += 32) {
+    for (int i = at; i < p.hidden / 64; i += step) {
       prefetch_l2(lw->input_norm + i * 64);
       prefetch_l2(lw->post_norm + i * 64);
     }
     for (int seg = 0; seg < 3; ++seg)
       if (lw->bias[seg] != nullptr)
-        for (int i = lane; i < (seg == 0 ? p.q_heads : p.kv_heads) * p.head_dim / 64; i += 32) prefetch_l2(lw->bias[seg] + i * 64);
+        for (int i = at; i < (seg == 0 ? p.q_heads : p.kv_heads) * p.head_dim / 64; i += step) prefetch_l2(lw->bias[seg] + i * 64);
   }
-  for (int i = lane; i < p.hidden / 64; i += 32) prefetch_l2(sm->plan.final_norm + i * 64);
+  for (int i = at; i < p.hidden / 64; i += step) prefetch_l2(sm->plan.final_norm + i * 64);
 }
 
 __device__ __forceinline__ void stream_reset(bf16* buffer, long long elems, int at, int step) {
@@ -159,9 +159,13 @@ __device__ __forceinline__ void stream_consumers(const KParams& p, StreamMisc* s
       if (kind == SP_DOWN) break;
       stream_project<TM, 2, CNORM, SG_MLP, FEW>(p, th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
       if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
-      __threadfence();  // this layer's resets come before the next layer's results (see stream_common.cuh)
+      // this layer's resets come before the next layer's results (see stream_common.cuh)
+      if (TM == 8 ? sm->fence_aside != 0 : TM < 32) named_bar_arrive(kStreamStoredBarrier, kStreamFenceThreads);
+      else __threadfence();
     }
-    stream_sync();    // the next layer's vectors are in place
+    // the next layer's vectors are in place
+    if (TM == 8 ? sm->fence_aside != 0 : TM < 32) named_bar_sync(kStreamFencedBarrier, kStreamFenceThreads);
+    else stream_sync();
     th.last_turn = th.turn;
     th.turn = th.turn == 2 ? 0 : th.turn + 1;
   }
@@ -233,6 +237,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
     sm->copies = stream_copies(TM);
     sm->bad = 0;
     sm->trace_n = 0;
+    sm->fence_aside = stream_fence_aside<TM>(p, gridDim.x);
     sm->trace_on = p.trace_cap != 0;
     sm->psum_offset = p.stream_scratch_bytes;
     mbar_fence_init();
@@ -291,8 +296,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream(const __grid_
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (tid == 0) stream_producer(p, sm, pipe);
-    else if (warp == 1 && blockIdx.x == 0) stream_prefetch_vectors(p, sm, tid - 32);
+    else if (warp == 1) stream_fence(sm->fence_aside ? p.layers : 0);
     else if (tid == 64) stream_watch(sm);
+    else if (warp == 2 && blockIdx.x == 0) stream_prefetch_vectors(p, sm, tid - 65, 31);
     else if (tid == 96) stream_plan_parts(p, sm);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
