@@ -125,6 +125,25 @@ def test_prompts_at_token_tile_edges(device, tokens, head_dim):
     assert_parity(logits, expected, f"prompt of {tokens}")
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,intermediate", [(9, 3, 64, 832), (3, 1, 64, 64), (5, 5, 128, 448), (2, 1, 128, 1088)])
+@pytest.mark.parametrize("tokens", [1, 2, 31, 33, 63, 66, 127])
+def test_short_prompts_whose_tiles_end_in_either_half(device, heads, kv_heads, head_dim, intermediate, tokens):
+    """Up to 128 tokens, projections on pairs: half of the tokens and half of a tile's weight rows to each CTA.  Odd numbers of heads and
+    narrow matrices end in the first half or in the second; one token leaves the second CTA without any."""
+    from oracle import decoder_oracle as oracle
+
+    config = tiny_config(hidden=320, q_heads=heads, kv_heads=kv_heads, head_dim=head_dim, intermediate=intermediate, vocab=1003, qkv_bias=True)
+    weights = synth_weights(config, seed=31, norm_std=0.1, device=device)
+    kernel = make_kernel(config, weights, device, max_tokens=tokens, max_positions=max(tokens, 16))
+    ids = synth_ids(tokens, config.vocab, seed=31).view(1, tokens).to(device)
+    positions = torch.arange(tokens, device=device).view(1, tokens)
+    with torch.no_grad():
+        expected = oracle.prefill(config, weights, rope_tables(config, max(tokens, 16), device=device), ids, positions,
+                                  oracle.causal_mask(1, tokens).to(device))
+    assert_parity(kernel.prefill(ids), expected, f"prompt of {tokens}")
+    kernel.check()
+
+
 @pytest.mark.parametrize("batch,sequence", [(1, 1), (3, 7), (2, 33), (5, 25), (3, 61), (4, 129)])
 @pytest.mark.parametrize("head_dim", [64, 128])
 def test_prompts_with_biases_masks_and_buffers_on_any_element(device, batch, sequence, head_dim):
