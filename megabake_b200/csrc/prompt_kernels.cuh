@@ -422,19 +422,8 @@ __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t ac
               if (c + 16 <= live) st_global_v8(out + 8, r + 8);
             }
           } else if constexpr (EPI == PE_SILU) {
-            bool inner = true;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              v[e] = bf16_round(v[e]);
-              inner = inner && fabsf(v[e]) < 80.f;
-            }
-            if (inner) {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) v[e] = silu_inner(v[e]);
-            } else {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) v[e] = silu(v[e]);
-            }
+            for (int e = 0; e < 16; ++e) v[e] = silu_to_bf16(bf16_round(v[e]));
             uint32_t o[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e)  // the product of two bf16 values is exact in fp32: one rounding, packed

@@ -371,6 +371,8 @@ def test_silu_of_the_epilogues_has_the_bits_of_the_division(tmp_path):
     assert ctypes.CDLL(str(library)).silu_sweep(counts) == 0
     below = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float().abs() < 80
     assert list(counts) == [int(below.sum()), 0]
+    assert ctypes.CDLL(str(library)).silu_rounded_sweep(counts) == 0  # rounded to bf16: every pattern there is
+    assert list(counts) == [1 << 16, 0]
 
 
 def test_static_scratch_status_recovers_from_a_refused_launch():
