@@ -469,7 +469,10 @@ __device__ __forceinline__ void stream_project(const KParams& p, StreamThread& t
         } else if constexpr (GROUP == SG_PLAIN) {
           finish_residual(col, old, sum[0].x, sum[0].y);
         } else if constexpr (GROUP == SG_MLP) {
-          const float s0 = bf16_round(silu(bf16_round(sum[0].x))), s1 = bf16_round(silu(bf16_round(sum[0].y)));
+          // (the same bits either way; the shorter one with two to eight tokens, 0.5B shape 1 to 1.8 % of a step, others 0 to 0.5: with one
+          // and with sixteen the 1.7B shape is 0.3 and 0.5 % slower)
+          auto gate = [](float x) { return bf16_round(TM == 8 ? silu_to_bf16(x) : silu(x)); };
+          const float s0 = gate(bf16_round(sum[0].x)), s1 = gate(bf16_round(sum[0].y));
           store(col, pack2(s0 * bf16_round(sum[NACC - 1].x), s1 * bf16_round(sum[NACC - 1].y)));
         } else if (kind == SP_QKV) {
           store(col, pack2(sum[0].x + b0, sum[0].y + b1));
