@@ -301,15 +301,31 @@ int encode_attention_maps(AttnTcMaps* maps, const AttnArgs& A, const mk_config& 
   maps->q_ok = (reinterpret_cast<uintptr_t>(A.q) & 15) == 0;
   if (int e = encode_attention_map(&maps->k, A.k, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
   if (int e = encode_attention_map(&maps->v, A.v, batch, A.klen, kv_heads, head_dim, A.kv_ld, A.kv_bstride, kAttnKeys)) return e;
-  // The mask's tiles come by TMA where its rows begin on 16-byte boundaries (a tiled copy's strides are multiples of that).
-  maps->mask_ok = A.mask != nullptr && attention_mask_in_tiles(head_dim, A.sq, A.klen) && (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
-  if (maps->mask_ok) {
+  // The mask comes by TMA: in tiles where its rows begin on 16-byte boundaries (a tiled copy's strides are multiples of that), else the
+  // rows of each residue modulo eight as a matrix of their own.
+  maps->mask_by = AM_LOADS;
+  if (A.mask != nullptr && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0) {
+    if ((A.klen & 7) != 0) maps->mask_by = attention_mask_in_eights(head_dim, A.sq, A.klen) ? AM_EIGHTS : AM_LOADS;
+    else maps->mask_by = attention_mask_in_tiles(head_dim, A.sq, A.klen) ? AM_TILES : AM_LOADS;
+  }
+  if (maps->mask_by == AM_TILES) {
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(A.klen), static_cast<cuuint64_t>(A.sq), static_cast<cuuint64_t>(batch)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(A.klen) * 2, static_cast<cuuint64_t>(A.sq) * A.klen * 2};
     const cuuint32_t box[3] = {kAttnKeys, kAttnQueries, 1}, elem[3] = {1, 1, 1};
-    const CUresult r = encode_fn()(&maps->mask, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(A.mask), dims, strides, box, elem,
+    const CUresult r = encode_fn()(&maps->mask[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(A.mask), dims, strides, box, elem,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) maps->mask_ok = 0;  // plain loads
+    if (r != CUDA_SUCCESS) maps->mask_by = AM_LOADS;
+  }
+  const long long rows = static_cast<long long>(batch) * A.sq;
+  for (int j = 0; j < 8 && maps->mask_by == AM_EIGHTS; ++j) {
+    const int lead = static_cast<int>((static_cast<long long>(j) * A.klen) & 7);  // elements between the boundary and row j's first
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(A.klen) + lead, static_cast<cuuint64_t>((rows - j + 7) / 8)};  // ends with the last row
+    const cuuint64_t stride[1] = {static_cast<cuuint64_t>(A.klen) * 16};
+    const cuuint32_t box[2] = {kMaskBox, kMaskRows}, elem[2] = {1, 1};
+    const CUresult r = encode_fn()(&maps->mask[j], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(A.mask + static_cast<long long>(j) * A.klen - lead), dims,
+                                   stride, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) maps->mask_by = AM_LOADS;
   }
   return maps->q_ok ? encode_attention_map(&maps->q, A.q, batch, A.sq, q_heads, head_dim, A.q_ld, A.q_bstride, kAttnQueries) : MK_OK;
 }

@@ -78,10 +78,14 @@ cudaError_t prompt_prepare() {
   const auto attention = [&](auto kernel, int smem) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   };
-  attention(prompt_attention_tc<64, false>, AttnTc<64, false>::kSmem);
-  attention(prompt_attention_tc<64, true>, AttnTc<64, true>::kSmem);
-  attention(prompt_attention_tc<128, false>, AttnTc<128, false>::kSmem);
-  attention(prompt_attention_tc<128, true>, AttnTc<128, true>::kSmem);
+  const auto attention_tc = [&](auto by) {
+    constexpr int kBy = decltype(by)::value;
+    attention(prompt_attention_tc<64, kBy>, AttnTc<64, kBy>::kSmem);
+    attention(prompt_attention_tc<128, kBy>, AttnTc<128, kBy>::kSmem);
+  };
+  attention_tc(std::integral_constant<int, AM_LOADS>());
+  attention_tc(std::integral_constant<int, AM_TILES>());
+  attention_tc(std::integral_constant<int, AM_EIGHTS>());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<64>::kSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptLaunch<128>::kSmem);
   return e;
@@ -109,8 +113,14 @@ cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps
     const auto go = [&](auto kernel, int smem) {
       return launch(kernel, blocks, kAttnThreads, smem, 1, true, stream, args, maps, guard, q_heads, kv_heads, batch, units);
     };
-    if (head_dim == 64) return maps.mask_ok ? go(prompt_attention_tc<64, true>, AttnTc<64, true>::kSmem) : go(prompt_attention_tc<64, false>, AttnTc<64, false>::kSmem);
-    return maps.mask_ok ? go(prompt_attention_tc<128, true>, AttnTc<128, true>::kSmem) : go(prompt_attention_tc<128, false>, AttnTc<128, false>::kSmem);
+    const auto by_mask = [&](auto by) {
+      constexpr int kBy = decltype(by)::value;
+      if (head_dim == 64) return go(prompt_attention_tc<64, kBy>, AttnTc<64, kBy>::kSmem);
+      return go(prompt_attention_tc<128, kBy>, AttnTc<128, kBy>::kSmem);
+    };
+    if (maps.mask_by == AM_EIGHTS) return by_mask(std::integral_constant<int, AM_EIGHTS>());
+    if (maps.mask_by == AM_TILES) return by_mask(std::integral_constant<int, AM_TILES>());
+    return by_mask(std::integral_constant<int, AM_LOADS>());
   }
   if (head_dim == 64)
     return launch(prompt_attention<64>, blocks, kWorkers, PromptLaunch<64>::kSmem, 1, true, stream, args, q_heads, kv_heads, batch, units);

@@ -15,9 +15,10 @@
 // exponentials, of which 0.27 are the unit's rate, 0.3 sums, 0.35 P and waits), 1.2 exchange, 1.3 quotients and stores.
 // A mask with rows on 16-byte boundaries and queries enough (attention_mask_in_tiles) comes by TMA beside the keys and values: a
 // thread reading its own row touched 32 lines a request, 2000 cycles of the load unit for a pair of tiles (512: 13.7 -> 12.9 us, 1024
-// 41.5 -> 38.2, head size 128 20.5 -> 17.7, a third of it the columns that both groups now finish).  Others keep those loads: fetched a
-// row at a time through shared memory they were faster with an even number of positions (500: 17.7 -> 15.8) and slower with an odd one
-// (501: 17.7 -> 20.4); by two warps of their own 27.8.
+// 41.5 -> 38.2, head size 128 20.5 -> 17.7, a third of it the columns that both groups now finish).  With rows off those boundaries eight
+// copies of a residue of the rows each (AM_EIGHTS, attention_mask_in_eights): 500 positions 17.6 -> 13.8, 501 17.6 -> 13.6, 4 x 250 21.9
+// -> 19.3, head size 128, 500 21.4 -> 19.4.  (Fetched a row at a time through shared memory 500 came to 15.8 and 501 to 20.4; by two
+// warps of their own 27.8.)  What is left keeps the loads.
 #pragma once
 #include <type_traits>
 
@@ -29,13 +30,21 @@ namespace mk {
 constexpr int kAttnQueries = 128, kAttnKeys = 64;
 constexpr int kAttnThreads = 384;  // two groups of four warps; of the third the loader and the MMA warp
 
-// MT: the mask's tiles come by TMA beside the keys' and values'.
-template <int HD, bool MT = false>
+// How a mask comes.  In tiles: by TMA beside the keys and values, where its rows begin on 16-byte boundaries.  In eights: rows that lie
+// eight apart begin at the same place within 16 bytes, however long they are, so each of the eight residues is a matrix of its own
+// whose rows are 16 klen bytes apart, and a copy that begins on the boundary before a row's first element is wide enough to hold 64 of
+// them from any element on.  Otherwise with loads of each thread's row.
+enum { AM_LOADS = 0, AM_TILES = 1, AM_EIGHTS = 2 };
+constexpr int kMaskBox = kAttnKeys + 8, kMaskRows = kAttnQueries / 8 + 1;  // elements and rows of a copy of one residue
+constexpr int kMaskRegion = (kMaskRows * kMaskBox * 2 + 127) / 128 * 128;
+
+template <int HD, int MASK = AM_LOADS>
 struct AttnTc {
   static constexpr int kChunks = HD / 64;                         // 64-dimension chunks of a row
-  static constexpr int kStages = HD == 64 ? (MT ? 5 : 6) : 3;
+  static constexpr int kStages = HD == 64 ? (MASK == AM_EIGHTS ? 4 : (MASK == AM_TILES ? 5 : 6)) : 3;
   static constexpr int kKeys = 2 * kChunks * kAttnKeys * 128;     // a K and a V tile
-  static constexpr int kTile = kKeys + (MT ? kAttnQueries * 128 : 0);
+  static constexpr int kTile = kKeys + (MASK == AM_EIGHTS ? 8 * kMaskRegion : (MASK == AM_TILES ? kAttnQueries * 128 : 0));
+  static constexpr int kArrives = kKeys + (MASK == AM_EIGHTS ? 8 * kMaskRows * kMaskBox * 2 : (MASK == AM_TILES ? kAttnQueries * 128 : 0));  // bytes
   static constexpr int kQ = kChunks * kAttnQueries * 128, kP = kAttnQueries * 128;
   static constexpr int kSmem = 1024 + kQ + 2 * kP + kStages * kTile;
   static constexpr int kColumns = HD == 64 ? 256 : 512;           // 2 x 64 of scores, 2 x head_dim of values
@@ -53,9 +62,9 @@ struct AttnTcMisc {
 // Descriptors of a launch's operands, rows of 64-element chunks: (64, rows, chunks of all heads, sequences).  Rows past the last
 // one read as zeros.
 struct AttnTcMaps {
-  CUtensorMap q, k, v, mask;  // (mask: (positions, queries, sequences))
+  CUtensorMap q, k, v, mask[8];  // mask: (positions, queries, sequences), or of each residue (positions, every eighth row)
   int q_ok;     // the queries begin on a 16-byte boundary; otherwise their rows are fetched with plain loads
-  int mask_ok;  // there is a mask that comes in tiles: its rows begin on 16-byte boundaries
+  int mask_by;  // AM_*
 };
 
 // B operand stored with its N dimension contiguous: 64-element chunks [8 rows of K][128 B], 128-byte swizzle.  Rows of K in
@@ -133,10 +142,10 @@ __device__ __forceinline__ AttnTcUnit attn_unit(const AttnArgs& A, int q_heads, 
 }
 
 // One thread of warp 8: the queries, then tile t into stage t % kStages (t counts over the launch).
-template <int HD, bool MT>
-__device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t stages,
+template <int HD, int MASK>
+__device__ __forceinline__ void attn_load(const AttnTcMaps& maps, int sq, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t stages,
                                           int base) {
-  using T = AttnTc<HD, MT>;
+  using T = AttnTc<HD, MASK>;
   const uint64_t policy = l2_policy_evict_normal();
   if (maps.q_ok) {
     mbar_expect_tx(smem_u32(&misc->qfull), T::kQ);
@@ -146,18 +155,20 @@ __device__ __forceinline__ void attn_load(const AttnTcMaps& maps, const AttnTcWa
     const int at = base + t, s = at % T::kStages, use = at / T::kStages;
     if (use > 0 && !attn_wait(w, &misc->kvempty[s], (use - 1) & 1)) return;
     const uint32_t bar = smem_u32(&misc->kvfull[s]), dst = stages + s * T::kTile;
-    mbar_expect_tx(bar, T::kTile);
+    mbar_expect_tx(bar, T::kArrives);
     tma_load_4d(dst, &maps.k, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
     tma_load_4d(dst + T::kKeys / 2, &maps.v, 0, t * kAttnKeys, u.kvh * T::kChunks, u.b, bar, policy);
-    if constexpr (MT) tma_load_3d(dst + T::kKeys, &maps.mask, t * kAttnKeys, u.q0, u.b, bar, policy);
+    if constexpr (MASK == AM_TILES) tma_load_3d(dst + T::kKeys, &maps.mask[0], t * kAttnKeys, u.q0, u.b, bar, policy);
+    if constexpr (MASK == AM_EIGHTS)
+      for (int j = 0; j < 8; ++j) tma_load_2d(dst + T::kKeys + j * kMaskRegion, &maps.mask[j], t * kAttnKeys, (u.b * sq + u.q0) >> 3, bar, policy);
   }
 }
 
 // Warp 10.  `base` and `uses`: tiles of earlier units, all and of each group (uses of the barriers).
-template <int HD, bool MT>
+template <int HD, int MASK>
 __device__ __forceinline__ void attn_mma(const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint32_t q, uint32_t p, uint32_t stages, uint32_t tmem,
                                          int base, const int* uses) {
-  using T = AttnTc<HD, MT>;
+  using T = AttnTc<HD, MASK>;
   constexpr uint32_t kScores = umma_idesc_bf16(kAttnQueries, kAttnKeys), kValues = umma_idesc_bf16(kAttnQueries, HD) | kIdescBMajorN;
   auto scores = [&](int t) -> bool {
     const int at = base + t, s = at % T::kStages;
@@ -236,10 +247,10 @@ __device__ __forceinline__ void attn_store_nan(const AttnArgs& A, const AttnTcUn
 }
 
 // Warps 0 to 7.  A wait that was given up ends the loop; the block barriers behind it are passed all the same.
-template <int HD, bool MT>
+template <int HD, int MASK>
 __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait& w, AttnTcMisc* misc, const AttnTcUnit& u, uint8_t* smem, uint32_t p,
                                              uint32_t stages, uint32_t tmem, int base, const int* uses, int warp, int lane) {
-  using T = AttnTc<HD, MT>;
+  using T = AttnTc<HD, MASK>;
   const int g = warp >> 2, quad = warp & 3, row = quad * 32 + lane, r = u.q0 + row;
   const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
   const uint32_t s_at = tmem + lanes + g * kAttnKeys, v_at = tmem + lanes + 2 * kAttnKeys + g * HD;
@@ -248,6 +259,7 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
   const uint32_t scale2 = pack2(A.scale, A.scale);
   const bf16* const mrow = A.mask + (static_cast<long long>(u.b) * A.sq + min(r, A.sq - 1)) * A.klen;
   const bool wide = (A.klen & 7) == 0 && (reinterpret_cast<uintptr_t>(A.mask) & 15) == 0;
+  constexpr bool MT = MASK != AM_LOADS;
   const bool fetched = !MT && A.mask;  // the mask comes with plain loads
   bool ok = true, unseen = false;  // unseen: this warp saw nothing of the tile whose sums come next
   float m = -INFINITY, l = 0.f, alpha = 1.f, o[HD];
@@ -266,6 +278,10 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
       for (int d = 0; d < 32; ++d) o[c + d] = fmaf(o[c + d], alpha, __uint_as_float(v[d]));
     }
   };
+  // This row's place in its residue's copy, from the word of the tile's first element on, and whether that is the word's second element.
+  const int at_row = u.b * A.sq + u.q0 + row, residue = at_row & 7, first_element = (residue * A.klen) & 7;
+  const uint32_t eighth = static_cast<uint32_t>(residue * kMaskRegion + ((at_row >> 3) - ((at_row - row) >> 3)) * kMaskBox * 2 + (first_element >> 1) * 4);
+  const uint32_t halfword = (first_element & 1) * 16;
   uint32_t x[32];  // the mask of a tile's row, its scores, its probabilities
   if (fetched && g < u.ntiles) attn_mask(mrow, g * kAttnKeys, A.klen, wide, x);
 #pragma unroll 1
@@ -284,7 +300,7 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
       if constexpr (MT) {  // (the scores came behind the same copies; this thread's own look makes them visible to it)
         const int at = base + t, s = at % T::kStages;
         ok = __all_sync(0xffffffffu, attn_wait(w, &misc->kvfull[s], (at / T::kStages) & 1));
-        mask_at = stages + s * T::kTile + T::kKeys + row * 128;
+        mask_at = stages + s * T::kTile + T::kKeys + (MASK == AM_EIGHTS ? eighth : row * 128);
       }
       // What a pair of scores goes through depends on the launch and the tile: straight lines, not three tests a pair.
       auto take = [&](auto exact, auto masked) {
@@ -292,7 +308,14 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
         for (int c = 0; c < 2; ++c) {
           uint32_t s[32];
           tmem_ld32_async(s_at + c * 32, s);
-          if constexpr (MT) {
+          if constexpr (MASK == AM_EIGHTS) {
+            uint32_t words[17];
+#pragma unroll
+            for (int i = 0; i < 17; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(words[i]) : "r"(mask_at + (c * 16 + i) * 4) : "memory");
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[c * 16 + i] = __funnelshift_r(words[i], words[i + 1], halfword);
+          }
+          if constexpr (MASK == AM_TILES) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x[c * 16 + 4 * i]), "=r"(x[c * 16 + 4 * i + 1]), "=r"(x[c * 16 + 4 * i + 2]),
@@ -430,11 +453,11 @@ __device__ __forceinline__ void attn_softmax(const AttnArgs& A, const AttnTcWait
   }
 }
 
-template <int HD, bool MT>
+template <int HD, int MASK>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ AttnTcMaps maps, const __grid_constant__ PromptGuard guard, int q_heads,
                     int kv_heads, int batch, int units) {
-  using T = AttnTc<HD, MT>;
+  using T = AttnTc<HD, MASK>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ AttnTcMisc misc;
@@ -457,7 +480,8 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
     tma_prefetch_desc(&maps.q);
     tma_prefetch_desc(&maps.k);
     tma_prefetch_desc(&maps.v);
-    if constexpr (MT) tma_prefetch_desc(&maps.mask);
+    if constexpr (MASK != AM_LOADS)
+      for (int j = 0; j < (MASK == AM_EIGHTS ? 8 : 1); ++j) tma_prefetch_desc(&maps.mask[j]);
   }
   if (warp == 10) {
     tmem_alloc(smem_u32(&misc.tmem_base), T::kColumns);
@@ -493,7 +517,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
       walk([&](const AttnTcUnit& u) {
         if (!maps.q_ok) named_bar_sync(2, 288);  // the queries are there
         else if (!__all_sync(0xffffffffu, attn_wait(w, &misc.qfull, done & 1))) return;
-        attn_mma<HD, MT>(w, &misc, u, q, p, stages, tmem, base, uses);
+        attn_mma<HD, MASK>(w, &misc, u, q, p, stages, tmem, base, uses);
       });
     } else {
       walk([&](const AttnTcUnit& u) {
@@ -501,7 +525,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
           // The exchange's plain accesses come before a later unit's copies.  (The operands are complete and visible behind
           // griddepcontrol.wait, to copies too: without a fence for them 128 positions 6.97 -> 6.59 us, 512 12.8 -> 12.6.)
           if (done > 0) fence_proxy_async_smem();
-          attn_load<HD, MT>(maps, w, &misc, u, q, stages, base);
+          attn_load<HD, MASK>(maps, A.sq, w, &misc, u, q, stages, base);
         }
         __syncwarp();
       });
@@ -522,7 +546,7 @@ prompt_attention_tc(const __grid_constant__ AttnArgs A, const __grid_constant__ 
         fence_proxy_async_smem();
         named_bar_sync(2, 288);
       }
-      attn_softmax<HD, MT>(A, w, &misc, u, smem, p, stages, tmem, base, uses, warp, lane);
+      attn_softmax<HD, MASK>(A, w, &misc, u, smem, p, stages, tmem, base, uses, warp, lane);
       fence_proxy_async_smem();
     });
     if (tid < kAttnQueries && *reinterpret_cast<volatile int*>(&misc.abort))  // the units behind the one that was given up

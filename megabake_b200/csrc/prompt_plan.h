@@ -152,6 +152,17 @@ inline bool attention_mask_in_tiles(int head_dim, int q_len, int k_len) {
   return head_dim == 128 ? q_len >= 96 && k_len > 192 : q_len >= 96 || (q_len >= 16 && k_len >= 1024);
 }
 
+// The same of a mask whose rows begin off 16-byte boundaries: eight copies a tile, one of each residue of the rows modulo eight, or loads,
+// a word of a row at a time or two.  The copies are worth it from fewer positions on, where the last block of queries is not mostly
+// empty.  us, loads / copies: head size 64, 32 heads, 96 x 130 8.7 / 8.1, 500 x 500 17.6 / 13.8, 130 x 205 11.2 / 12.1, 130 x 650 23.4 / 15.7,
+// 64 x 330 12.4 / 10.7, x 4 sequences 13.0 / 11.9, 32 x 650 18.3 / 16.6, 32 x 330 12.1 / 16.4, 16 x 650 17.6 / 24.7; head size 128, 32 heads,
+// 96 x 205 12.4 / 11.6, 500 x 500 21.4 / 19.4, 130 x 205 13.4 / 13.9, 200 x 330 18.4 / 15.4, 64 x 205 x 4 12.5 / 13.3.
+inline bool attention_mask_in_eights(int head_dim, int q_len, int k_len) {
+  const bool full = (q_len - 1) % 128 >= 63;  // the last block
+  if (q_len >= 96) return k_len > (full ? (head_dim == 128 ? 192 : 128) : 256);
+  return head_dim == 64 && k_len >= (q_len >= 64 ? 320 : 640) && q_len >= 32;
+}
+
 // What a CTA still waits for before it leaves: that the last use of every pipeline slot has been consumed, so that no commit
 // is on its way to a barrier of shared memory that is somebody else's by then.  The uses count up over the launch, use u lies in
 // slot u % stages, and a slot's barrier has the parity of its use; wait(slot, parity) returns false to give up.

@@ -89,3 +89,20 @@ def test_a_mask_comes_the_faster_way_or_close(rule, head_dim, heads, batch, quer
     """Or within 6 %, where the rule's lines cross what was measured."""
     taken, other = (tiles, loads) if rule.library.mask_in_tiles(head_dim, queries, keys) else (loads, tiles)
     assert taken <= 1.06 * other
+
+
+# The same of masks whose rows begin off 16-byte boundaries, and copies of every eighth row
+EIGHTHS = [
+    (64, 32, 1, 96, 130, 8.7, 8.1), (64, 32, 1, 130, 75, 7.8, 8.4), (64, 32, 1, 130, 205, 11.2, 12.1), (64, 32, 1, 130, 330, 15.2, 14.5),
+    (64, 32, 1, 200, 75, 7.8, 8.0), (64, 32, 1, 200, 205, 11.2, 9.5), (64, 32, 1, 500, 130, 9.8, 9.3), (64, 32, 1, 500, 1030, 30.5, 22.0),
+    (64, 32, 4, 16, 650, 17.6, 24.7), (64, 32, 4, 16, 1030, 24.1, 26.8), (64, 32, 4, 32, 330, 12.1, 16.4), (64, 32, 4, 32, 650, 18.3, 16.6),
+    (64, 32, 4, 64, 205, 10.3, 11.2), (64, 32, 4, 64, 330, 13.0, 11.9), (64, 32, 4, 96, 130, 9.4, 9.4), (64, 9, 1, 500, 650, 23.1, 15.1),
+    (64, 9, 4, 32, 75, 6.7, 7.5), (64, 9, 4, 200, 330, 15.2, 10.9), (128, 32, 1, 16, 1030, 27.5, 30.4), (128, 32, 1, 96, 205, 12.4, 11.6),
+    (128, 32, 1, 130, 205, 13.4, 13.9), (128, 32, 1, 200, 330, 18.4, 15.4), (128, 32, 1, 500, 75, 9.9, 10.7), (128, 32, 1, 500, 650, 29.2, 23.8),
+    (128, 32, 4, 32, 650, 22.1, 23.8), (128, 32, 4, 64, 205, 12.5, 13.3), (128, 32, 4, 130, 330, 32.7, 31.0), (128, 32, 4, 200, 1030, 68.4, 66.0)]
+
+
+@pytest.mark.parametrize("head_dim,heads,batch,queries,keys,loads,copies", EIGHTHS)
+def test_a_mask_off_16_bytes_comes_the_faster_way_or_close(rule, head_dim, heads, batch, queries, keys, loads, copies):
+    taken, other = (copies, loads) if rule.library.mask_in_eights(head_dim, queries, keys) else (loads, copies)
+    assert taken <= 1.06 * other

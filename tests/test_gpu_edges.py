@@ -521,11 +521,29 @@ def test_prompt_attention_op_with_masks_that_come_in_tiles(device, heads, kv_hea
         assert torch.equal(out, torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5))
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(9, 3, 64), (8, 2, 128)])
+@pytest.mark.parametrize("queries,keys", [(96, 257), (128, 259), (129, 321), (200, 194), (257, 262), (300, 327), (64, 323), (33, 641), (256, 1020)])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_prompt_attention_op_with_masks_whose_rows_begin_anywhere(device, heads, kv_heads, head_dim, queries, keys, batch):
+    """Every residue of the row length modulo eight: copies of every eighth row, whose boxes begin before a row's first element and end beyond
+    the last position, query or sequence.  The same mask at an odd element comes with loads, and with the same bits."""
+    from oracle import decoder_oracle as oracle
+
+    query, key, value = _tensors(device, batch, queries, keys, heads, kv_heads, head_dim)
+    generator = torch.Generator(device=device).manual_seed(keys + queries)
+    mask = torch.randn((batch, 1, queries, keys), device=device, generator=generator).to(torch.bfloat16)
+    mask[:, 0, :, 1:].masked_fill_(torch.rand((batch, queries, keys - 1), device=device, generator=generator) < 0.4, float("-inf"))
+    out = torch.ops.megabake.attention(query, key, value, mask, head_dim ** -0.5)
+    assert_parity(out, oracle.attention(query, key, value, mask, head_dim ** -0.5), f"attention {queries} x {keys}")
+    moved = torch.empty(mask.numel() + 1, dtype=torch.bfloat16, device=device)[1:].view(mask.shape).copy_(mask)
+    assert torch.equal(out, torch.ops.megabake.attention(query, key, value, moved, head_dim ** -0.5))
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(6, 2, 64), (6, 2, 128)])
 @pytest.mark.parametrize("keys", [456, 704, 701])
 def test_prompt_attention_with_a_mask_and_several_units_to_a_block(device, heads, kv_heads, head_dim, keys):
     """On five SMs a block goes on from unit to unit: the ring of tiles carries over, and the exchange at a unit's end lies where the
-    next one's queries, probabilities and (head size 128) first tile come.  701: masks off 16 bytes, by plain loads."""
+    next one's queries, probabilities and (head size 128) first tile come.  701: masks off 16 bytes, copies of every eighth row."""
     from oracle import decoder_oracle as oracle
 
     query, key, value = _tensors(device, 2, 700, keys, heads, kv_heads, head_dim)
