@@ -11,20 +11,13 @@ struct AttnArgs {
   const bf16* q; long long q_bstride; int q_ld;
   // key/value of (b, position j, kv head g): k + b*kv_bstride + j*kv_ld + g*head_dim
   bf16* k; bf16* v; long long kv_bstride; int kv_ld;
-  // decode only: the new token's key/value at knew + b*new_ld + g*head_dim
-  const bf16* knew; const bf16* vnew; int new_ld;
   // output of (b, qi, h): out + b*out_bstride + qi*out_tstride + h*out_hstride
   bf16* out; long long out_bstride; int out_tstride; int out_hstride;
   const bf16* mask;   // additive bf16 [batch, 1, sq, klen] or null
-  int sq;             // query tokens per sequence (1 in decode)
-  int klen;           // keys per sequence (prefill); decode attends len + 1
-  int len;            // decode: filled positions before this call (the longest sequence's when lengths are per sequence)
-  const int* lens;    // decode with per-sequence valid lengths: filled positions of each sequence; null = `len` for all
-  int decode;         // 1: append the new key/value at `len` and attend over [0, len]
-  int causal;         // prefill without a mask tensor: key j <= query qi
-  uint32_t stamp;     // value the chunks of this phase publish with their softmax statistics
+  int sq;             // query tokens per sequence
+  int klen;           // keys per sequence
+  int causal;         // without a mask tensor: key j <= query qi
   float scale;
-  const CUtensorMap *kmap, *vmap;  // decode: tiled descriptors of the two caches (see attention_decode), or null
 };
 
 // A unit is (sequence, query head, block of 64 query tokens).  The eight worker warps are four row

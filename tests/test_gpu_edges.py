@@ -106,6 +106,15 @@ def test_tensor_engine_attention_with_two_units_to_a_block(device, kv_heads, hea
     oracle_decode_compare(config, device, batch=32, capacity=context + 2, prefill=context, steps=2, engine="tcgen05")
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (3, 3, 64), (8, 2, 128), (16, 8, 64)])
+@pytest.mark.parametrize("context", [0, 63, 130, 300, 700, 1023])
+def test_tensor_engine_attention_with_any_number_of_chunks(device, heads, kv_heads, head_dim, context):
+    """A context in 1 to 16 chunks of up to 64 positions: their statistics and sums come four chunks and four columns at a time, whatever is
+    there of them."""
+    config = tiny_config(hidden=256, q_heads=heads, kv_heads=kv_heads, head_dim=head_dim)
+    oracle_decode_compare(config, device, batch=1, capacity=context + 3, prefill=context, steps=2, engine="tcgen05")
+
+
 @pytest.mark.parametrize("tokens", [16, 17, 64, 65, 128, 129, 256, 257, 385, 513])
 @pytest.mark.parametrize("head_dim", [64, 128])
 def test_prompts_at_token_tile_edges(device, tokens, head_dim):
