@@ -176,9 +176,8 @@ __device__ __forceinline__ void stream_consumers(const KParams& p, StreamMisc* s
     *reinterpret_cast<volatile int*>(&sm->progress) = layers + 1;
     red_release_add_u32(&sm->ctrl->barrier, 1u);
     const uint32_t target = p.epoch + static_cast<uint32_t>(sm->grid);
-    while (static_cast<int32_t>(ld_relaxed_u32(&sm->ctrl->barrier) - target) < 0 && !stream_aborted(sm)) {
+    while (static_cast<int32_t>(ld_acquire_u32(&sm->ctrl->barrier) - target) < 0 && !stream_aborted(sm)) {
     }
-    __threadfence();
     sm->complete = !stream_aborted(sm);
     *reinterpret_cast<volatile int*>(&sm->progress) = -1;
   }
