@@ -116,6 +116,17 @@ __device__ __forceinline__ float silu_to_bf16(float x) {
   return x * y;
 }
 
+// exp(score - max) over the sum of a softmax, for weights that are zero or at least kQuotientLeast: without a branch, so that
+// several overlap.  `reciprocal` is 1 / sum, rounded; a quotient that two remainders have corrected has the bits of the division
+// (Markstein, 1990), and within these limits no remainder is lost to underflow.
+constexpr float kQuotientLeast = 0x1p-60f;
+__device__ __forceinline__ bool quotient_fits(float weight) { return !(weight > 0.f && weight < kQuotientLeast); }
+__device__ __forceinline__ float quotient(float weight, float sum, float reciprocal) {
+  float q = weight * reciprocal;
+  q = fmaf(fmaf(-q, sum, weight), reciprocal, q);
+  return fmaf(fmaf(-q, sum, weight), reciprocal, q);
+}
+
 __device__ __forceinline__ float ldcg_bf16(const bf16* ptr) {
   return __bfloat162float(__ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short*>(ptr))));
 }

@@ -115,6 +115,14 @@ def test_tensor_engine_attention_with_any_number_of_chunks(device, heads, kv_hea
     oracle_decode_compare(config, device, batch=1, capacity=context + 3, prefill=context, steps=2, engine="tcgen05")
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,batch,context", [(16, 4, 64, 80, 1300), (8, 2, 128, 120, 1290), (8, 1, 64, 120, 2600)])
+def test_tensor_engine_attention_of_more_units_than_ctas(device, heads, kv_heads, head_dim, batch, context):
+    """Chunks that have to be cut for their scores' room, two or three to a CTA one behind the other: a sequence's chunks are summed
+    at the end of the phase by the CTA that had the first of them, some CTAs for several sequences and some for none."""
+    config = tiny_config(hidden=256, q_heads=heads, kv_heads=kv_heads, head_dim=head_dim)
+    oracle_decode_compare(config, device, batch=batch, capacity=context + 3, prefill=context, steps=2, engine="tcgen05")
+
+
 @pytest.mark.parametrize("tokens", [16, 17, 64, 65, 128, 129, 256, 257, 385, 513])
 @pytest.mark.parametrize("head_dim", [64, 128])
 def test_prompts_at_token_tile_edges(device, tokens, head_dim):

@@ -375,6 +375,22 @@ def test_silu_of_the_epilogues_has_the_bits_of_the_division(tmp_path):
     assert list(counts) == [1 << 16, 0]
 
 
+def test_quotients_of_the_softmax_have_the_bits_of_the_division(tmp_path):
+    """``quotient`` over 2^26 weights and sums, built as the library is; weights below 2^-60 are left to the division."""
+    import subprocess
+    from pathlib import Path
+
+    from megabake_b200.build import NVCC_FLAGS, find_nvcc
+
+    library = tmp_path / "quotient_sweep.so"
+    subprocess.run([find_nvcc(), *NVCC_FLAGS, "-o", str(library), str(Path(__file__).resolve().parent / "quotient_sweep.cu"), "-lcudart"],
+                   check=True, capture_output=True, text=True)
+    counts = (ctypes.c_uint32 * 3)()
+    assert ctypes.CDLL(str(library)).quotient_sweep(counts) == 0
+    equal, different, left = counts
+    assert different == 0 and equal > (1 << 26) // 32 * 2 // 5 and left > (1 << 26) * 2 // 5
+
+
 def test_static_scratch_status_recovers_from_a_refused_launch():
     """The allocation-free attention entry point has no handle: its status word lives in the static
     array and is read and cleared through mk_kv_attention_static_status."""
