@@ -88,7 +88,8 @@ def measured_peaks():
 
 
 class ClockSampler(threading.Thread):
-    """Samples SM clock and throttle reasons of one GPU through NVML while the timed region runs."""
+    """Samples SM clock and throttle reasons of one GPU through NVML from ``begin`` to ``stop_flag``: a timed region can be shorter
+    than NVML takes to start, so the thread is ready before the region begins."""
 
     REASONS = {
         0x8: "hw_slowdown", 0x40: "hw_thermal_slowdown", 0x20: "sw_thermal_slowdown", 0x4: "sw_power_cap",
@@ -101,8 +102,13 @@ class ClockSampler(threading.Thread):
         self.samples: list[int] = []
         self.max_mhz = None
         self.reason_bits = 0
-        self.stop_flag = threading.Event()
+        self.ready, self.go, self.stop_flag = threading.Event(), threading.Event(), threading.Event()
         self.error = None
+
+    def begin(self):
+        self.start()
+        self.ready.wait(timeout=10)
+        self.go.set()
 
     def run(self):
         try:
@@ -111,15 +117,18 @@ class ClockSampler(threading.Thread):
             pynvml.nvmlInit()
             handle = pynvml.nvmlDeviceGetHandleByIndex(self.index)
             self.max_mhz = pynvml.nvmlDeviceGetMaxClockInfo(handle, pynvml.NVML_CLOCK_SM)
+            self.ready.set()
+            self.go.wait()
             while not self.stop_flag.is_set():
                 self.samples.append(pynvml.nvmlDeviceGetClockInfo(handle, pynvml.NVML_CLOCK_SM))
                 try:
                     self.reason_bits |= pynvml.nvmlDeviceGetCurrentClocksEventReasons(handle)
                 except Exception:
                     self.reason_bits |= pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(handle)
-                time.sleep(0.01)
+                time.sleep(0.002)
         except Exception as error:  # NVML missing: report that instead of clocks
             self.error = repr(error)
+            self.ready.set()
 
     def summary(self) -> dict:
         if self.error or not self.samples:
@@ -420,7 +429,7 @@ def main():
     kernel.check()
     group.sync()
     sampler = ClockSampler(local_rank)
-    sampler.start()
+    sampler.begin()
     events = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps + 1)]
     launches_before = kernel.launch_info()["launches"]
     events[0].record()
