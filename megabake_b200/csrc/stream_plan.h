@@ -114,10 +114,24 @@ inline int stream_few_ctas(const mk_config& c, int sms) {
   return more <= 0 && rounds(less[SP_HEAD], few) - rounds(all[SP_HEAD], sms) <= c.layers ? few : 0;
 }
 inline bool stream_few_fits(const mk_config& c, int batch, int few) { return batch <= 8 && 4 * batch * c.kv_heads <= few; }
+// The most CTAs, up to `ctas`, of which each has a unit of a layer's projections.  One that has none, of the output head alone, would
+// wait for no layer, and takes what the first layers leave in the head's operand for the last one's.  (Left-over units go to the CTAs
+// that have the least so far, see stream_deal_units: as many units as CTAs are enough.  Shapes of a hidden size of 128 and about; the
+// 135M shape has 392.)
+inline int stream_busy_ctas(const mk_config& c, int plan, int ctas) {
+  StreamPhase ph[kStreamPhases];
+  for (;;) {
+    stream_phases(c, plan, ctas, ph);
+    int units = 0;
+    for (int i = 0; i < SP_HEAD; ++i) units += ph[i].ntiles * ph[i].nslice;
+    if (units >= ctas) return ctas;
+    ctas = units;
+  }
+}
 // CTAs of a plan's launches, 0: no launch uses the plan.
 inline int stream_grid(const mk_config& c, int plan, int sms) {
-  if (plan == 0) return sms;
-  if (plan < kStreamFew) return c.max_tokens > (4 << plan) ? sms : 0;
+  if (plan == 0) return stream_busy_ctas(c, plan, sms);
+  if (plan < kStreamFew) return c.max_tokens > (4 << plan) ? stream_busy_ctas(c, plan, sms) : 0;
   const int few = stream_few_ctas(c, sms);
   return stream_few_fits(c, 1, few) ? few : 0;
 }
