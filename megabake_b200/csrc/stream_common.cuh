@@ -13,9 +13,11 @@
 // produce); a reader loads the data itself and reads again what is still unset.  A hand-over is one store and
 // one load: no flag, no fence, no barrier.  Every buffer exists three times, used in turn by the layers; whoever writes a
 // word in layer l resets the same word of layer l - 1's copy, whose readers are done: to write in layer l a CTA has
-// read data that depends on every result of layer l - 1.  That copy is written again in layer l + 2; one fence per layer
-// (of each thread, or of a warp for its CTA: stream_fence) comes between the reset and the thread's results of layer l + 1,
-// which every reader of layer l + 2 has seen.  The launch ends with a grid barrier, behind which the last layer's words are reset.
+// read data that depends on every result of layer l - 1.  That copy is written again in layer l + 2.  A CTA that looks for it there has
+// read something of layer l + 1 (each has a unit of every layer, see stream_busy_ctas), and what it has read depends on a result that the
+// resetting CTA stored behind a fence behind the reset.  The fence of layer l lies between gate/up and the first result of down_proj
+// (kStreamFenceMet): behind the resets of layer l up to gate and up and of down_proj in layer l - 1.  The launch ends with a grid
+// barrier, behind which the last layer's words are reset.
 #pragma once
 #include "device_common.cuh"
 
@@ -38,6 +40,7 @@ constexpr int kStreamStoredBarrier = 2, kStreamFencedBarrier = 3;  // named barr
 constexpr int kStreamFenceThreads = kStreamConsumers + 32;
 
 enum { SP_QKV = 0, SP_O = 1, SP_GU = 2, SP_DOWN = 3, SP_HEAD = 4, kStreamPhases = 5 };
+constexpr int kStreamFenceMet = SP_DOWN;  // no result of this projection, or of one behind it, is stored ahead of its layer's fence
 
 // Token classes: a kernel is compiled for at most 1, 4, 8, 16 or 32 tokens (4 in the layout of 8).
 __host__ __device__ constexpr int stream_token_tiles(int tm) { return tm <= 8 ? 1 : tm / 8; }
@@ -168,9 +171,11 @@ __device__ __forceinline__ V stream_opaque(V v) {
 }
 
 // The fence of a layer, by a warp of the producer's group: the consumers tell it that their results and resets of the layer up to gate
-// and up are stored, go on, and look whether it has come through before the layer ends.  A fence orders what its thread knows of, so
-// what went before the barrier comes, for everybody on the GPU, before what follows the second one.  (1400 cycles a layer of the 135M
-// shape by clock stamps, ahead of down_proj.)
+// and up are stored, go on, and meet it again ahead of the first result of down_proj, in the block barrier that is there anyway.  A
+// fence orders what its thread knows of, and the first barrier has made the consumers' stores known to it; it has come through when those
+// are performed for the whole GPU, and no consumer stores a result of down_proj before the second barrier.  (A reader needs none: it
+// looks for a word when the loop that waited for an earlier one has ended.)  (1400 cycles a layer of the
+// 135M shape by clock stamps, ahead of down_proj.)
 // Two to eight tokens only where the ring holds the gate and up matrices of a layer: elsewhere the CTAs end that phase one by one as HBM
 // brings them their weights, and those that are through and have no fence to wait for look for the others' results all the longer.
 // With 32 tokens there is no difference.  A step, fence on the way -> aside (mean of 60 to 1900 positions): 135M shape, one sequence -2.1 %,
@@ -182,6 +187,11 @@ template <int TM>
 __device__ __forceinline__ bool stream_fence_aside(const KParams& p, int grid) {
   if (TM != 8) return TM < 32;
   return 4ll * p.inter * p.hidden <= static_cast<long long>(p.stream_slots) * kStreamSlotBytes * grid;
+}
+// Whether it is in a launch of this token class.
+template <int TM>
+__device__ __forceinline__ bool stream_is_aside(const StreamMisc* sm) {
+  return TM == 8 ? sm->fence_aside != 0 : TM < 32;
 }
 __device__ __forceinline__ void stream_fence(int layers) {
   for (int layer = 0; layer < layers; ++layer) {

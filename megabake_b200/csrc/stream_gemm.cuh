@@ -309,6 +309,7 @@ __device__ __forceinline__ void stream_project(const KParams& p, StreamThread& t
     const int at = lane * 256 + warp * 32;
     if (count > 0 && at < k) asm volatile("prefetch.global.L1 [%0];" ::"l"(normw + at));
   }
+  bool fence = GROUP == SG_PLAIN && kind == kStreamFenceMet && stream_is_aside<TM>(sm);  // the layer's fence has not been met yet
   int tile = sm->first_tile[kind];
 #pragma unroll 1
   for (int left = count; left > 0;) {  // runs of units of one slice
@@ -439,7 +440,9 @@ __device__ __forceinline__ void stream_project(const KParams& p, StreamThread& t
             if constexpr (SETS == 2) v += acc[a][n][1][e];
             if (TM > 1 || ptok < TM) psum[((warp * NACC + a) * TM + ptok) * kStreamPartPitch + prow] = v;
           }
-      stream_sync();
+      if (GROUP == SG_PLAIN && fence) named_bar_sync(kStreamFencedBarrier, kStreamFenceThreads);
+      else stream_sync();
+      fence = false;
       float2 sum[NACC];
 #pragma unroll
       for (int a = 0; a < NACC; ++a) {
@@ -493,6 +496,7 @@ __device__ __forceinline__ void stream_project(const KParams& p, StreamThread& t
     tile = 0;
   }
 
+  if (GROUP == SG_PLAIN && fence) named_bar_sync(kStreamFencedBarrier, kStreamFenceThreads);  // a CTA without a unit of down_proj
   if constexpr (CUT) {
     if (cut) {  // this CTA's share of the tiles is summed over the slices
       const int j0 = static_cast<int>(static_cast<long long>(ntiles) * sm->cta / sm->grid);

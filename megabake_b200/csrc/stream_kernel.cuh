@@ -160,12 +160,10 @@ __device__ __forceinline__ void stream_consumers(const KParams& p, StreamMisc* s
       stream_project<TM, 2, CNORM, SG_MLP, FEW>(p, th, pipe, SP_GU, layer);    // RMSNorm, SiLU(gate) * up
       if (wtid < kLayerWords) reinterpret_cast<uint32_t*>(&sm->lw[(layer + 1) & 1])[wtid] = word;
       // this layer's resets come before the next layer's results (see stream_common.cuh)
-      if (TM == 8 ? sm->fence_aside != 0 : TM < 32) named_bar_arrive(kStreamStoredBarrier, kStreamFenceThreads);
+      if (stream_is_aside<TM>(sm)) named_bar_arrive(kStreamStoredBarrier, kStreamFenceThreads);
       else __threadfence();
     }
-    // the next layer's vectors are in place
-    if (TM == 8 ? sm->fence_aside != 0 : TM < 32) named_bar_sync(kStreamFencedBarrier, kStreamFenceThreads);
-    else stream_sync();
+    stream_sync();  // the next layer's vectors are in place
     th.last_turn = th.turn;
     th.turn = th.turn == 2 ? 0 : th.turn + 1;
   }

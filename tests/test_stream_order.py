@@ -49,3 +49,36 @@ def test_every_cta_of_the_output_head_has_a_unit_of_each_layer(lib):
     for sizes in ((576, 9, 3, 64, 1536), (896, 14, 2, 64, 4864), (2048, 32, 32, 64, 8192)):
         lib.ctas_without_a_layer(_shape(*sizes), 16, 148, ctypes.byref(ctas))
         assert ctas.value == 148
+
+
+DOWN, HEAD = 3, 4
+MODELS = ((576, 9, 3, 64, 1536), (896, 14, 2, 64, 4864), (2048, 32, 32, 64, 8192))
+
+
+def _early(lib, sizes, batch, sms, lengths, met):
+    where = (ctypes.c_int * 4)(-1, -1, -1, -1)
+    found = lib.looks_too_early(_shape(*sizes), batch, sms, int(len(lengths) > 1), (ctypes.c_int * len(lengths))(*lengths), met, where)
+    return found, f"{sizes}, {batch} sequences, {sms} SMs, {lengths}: {found}, CTA {where[0]} of {where[1]} in layer {where[2]}, step {where[3]}"
+
+
+def test_no_cta_looks_for_a_word_before_it_knows_of_its_reset(lib):
+    """Buffers are used in turn by three layers.  Whoever looks for a word must depend on something its last writer stored behind a fence
+    behind the reset of what was there, or it may take that."""
+    assert lib.fence_met() == DOWN
+    cases = [(sizes, batch, 148, [length]) for sizes in MODELS for batch in (1, 3, 8, 16, 32) for length in (0, 1000)]
+    cases += [((256, 4, 2, 64, 512), 1, 148, [5]), ((256, 4, 4, 64, 512), 16, 148, [300])]
+    rng = random.Random(7)
+    for sizes, batch, sms in _shapes(60, 5):
+        cases += [(sizes, batch, sms, [rng.randint(0, 600)]), (sizes, batch, sms, [rng.randint(0, 3000) if rng.random() < 0.3 else 9 for _ in range(batch)])]
+    for sizes, batch, sms, lengths in cases:
+        if lib.has_plan(_shape(*sizes)):
+            found, what = _early(lib, sizes, batch, sms, lengths, lib.fence_met())
+            assert found == 0, what
+
+
+def test_a_fence_behind_down_proj_would_be_too_late(lib):
+    """The same walk sees it in small shapes; in the models' every CTA has other work that comes behind the fence."""
+    assert _early(lib, (256, 4, 2, 64, 512), 1, 148, [5], HEAD)[0] > 0
+    for sizes in MODELS:
+        for batch in (1, 3, 8, 12, 16, 32):
+            assert _early(lib, sizes, batch, 148, [1000], HEAD)[0] == 0
