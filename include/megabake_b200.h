@@ -99,7 +99,7 @@ typedef struct mk_weights {
   const void* embed;       /* bf16 [vocab, hidden] */
   const void* final_norm;  /* bf16 [hidden] */
   const void* lm_head;     /* bf16 [vocab, hidden]; equals embed when tied */
-  const void* rope_cos;    /* bf16 [max_positions, head_dim] */
+  const void* rope_cos;    /* bf16 [max_positions, head_dim]; 16-byte aligned for mk_prefill, from any element on for decode */
   const void* rope_sin;
   const mk_layer_weights* layers; /* host array of config.layers entries */
 } mk_weights;

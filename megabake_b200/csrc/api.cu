@@ -532,9 +532,15 @@ int launch(mk_handle h, KParams& p, void* stream, int attention_phases = 0) {
   return MK_OK;
 }
 
-// The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.
+// Whether the RoPE tables begin on boundaries of `bytes`.
+bool tables_aligned(mk_handle h, uintptr_t bytes) {
+  return ((reinterpret_cast<uintptr_t>(h->weights.rope_cos) | reinterpret_cast<uintptr_t>(h->weights.rope_sin)) & (bytes - 1)) == 0;
+}
+
+// The streaming kernel takes decode launches of up to 32 sequences, unless the tensor engine is asked for.  (It reads the RoPE tables in
+// words; the tensor engine takes them from any element on.)
 bool stream_usable(mk_handle h, int batch, bool ragged) {
-  return batch <= kStreamTokens && h->stream_ok[stream_plan_of(h->cfg, batch, h->stream_grid[kStreamFew])] &&
+  return tables_aligned(h, 4) && batch <= kStreamTokens && h->stream_ok[stream_plan_of(h->cfg, batch, h->stream_grid[kStreamFew])] &&
          h->kv_maps_ok && (ragged ? h->cfg.layers * batch : h->cfg.layers) <= kStreamLengths;
 }
 
@@ -1131,6 +1137,7 @@ int mk_prefill(mk_handle h, const int64_t* ids, const int64_t* positions, const 
   if (batch < 1 || sequence < 1 || m > h->cfg.max_tokens)
     return fail(MK_ERR_INVALID, "mk_prefill: %d x %d tokens outside [1, %d]", batch, sequence, h->cfg.max_tokens);
   if (int e = attention_fits(h, sequence, "mk_prefill")) return e;
+  if (!tables_aligned(h, 16)) return fail(MK_ERR_ALIGNMENT, "mk_prefill: the rope tables must be 16-byte aligned");
   if (sequence > prompt_keys(h)) return fail(MK_ERR_UNSUPPORTED, "mk_prefill: sequence %d exceeds %d keys", sequence, prompt_keys(h));
   const int L = h->cfg.layers;
   if (h->cfg.tp_size <= 1 && h->use3d) {
