@@ -88,8 +88,9 @@ def measured_peaks():
 
 
 class ClockSampler(threading.Thread):
-    """Samples SM clock and throttle reasons of one GPU through NVML from ``begin`` to ``stop_flag``: a timed region can be shorter
-    than NVML takes to start, so the thread is ready before the region begins."""
+    """Samples SM clock and throttle reasons of one GPU through NVML from ``begin`` to ``stop_flag``, every 2 ms: a timed region can be
+    shorter than NVML takes to start and to answer for the first time (4 ms for the clock, 2 for the reasons, more beside other
+    readers), so both have been asked once before the region begins."""
 
     REASONS = {
         0x8: "hw_slowdown", 0x40: "hw_thermal_slowdown", 0x20: "sw_thermal_slowdown", 0x4: "sw_power_cap",
@@ -117,14 +118,21 @@ class ClockSampler(threading.Thread):
             pynvml.nvmlInit()
             handle = pynvml.nvmlDeviceGetHandleByIndex(self.index)
             self.max_mhz = pynvml.nvmlDeviceGetMaxClockInfo(handle, pynvml.NVML_CLOCK_SM)
+
+            def query():
+                clock = pynvml.nvmlDeviceGetClockInfo(handle, pynvml.NVML_CLOCK_SM)
+                try:
+                    return clock, pynvml.nvmlDeviceGetCurrentClocksEventReasons(handle)
+                except Exception:
+                    return clock, pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(handle)
+
+            query()
             self.ready.set()
             self.go.wait()
             while not self.stop_flag.is_set():
-                self.samples.append(pynvml.nvmlDeviceGetClockInfo(handle, pynvml.NVML_CLOCK_SM))
-                try:
-                    self.reason_bits |= pynvml.nvmlDeviceGetCurrentClocksEventReasons(handle)
-                except Exception:
-                    self.reason_bits |= pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(handle)
+                clock, reasons = query()
+                self.samples.append(clock)
+                self.reason_bits |= reasons
                 time.sleep(0.002)
         except Exception as error:  # NVML missing: report that instead of clocks
             self.error = repr(error)
