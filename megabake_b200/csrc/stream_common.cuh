@@ -177,12 +177,15 @@ __device__ __forceinline__ V stream_opaque(V v) {
 // looks for a word when the loop that waited for an earlier one has ended.)  (1400 cycles a layer of the
 // 135M shape by clock stamps, ahead of down_proj.)
 // Two to eight tokens only where the ring holds the gate and up matrices of a layer: elsewhere the CTAs end that phase one by one as HBM
-// brings them their weights, and those that are through and have no fence to wait for look for the others' results all the longer.
-// With 32 tokens there is no difference.  A step, fence on the way -> aside (mean of 60 to 1900 positions): 135M shape, one sequence -2.1 %,
-// ten -4.5, sixteen -2.9; 0.5B, one -5.2, eight -3.4, ten -4.4, sixteen -3.6; 1.7B, one 0, two to six +1.0 to 1.3, ten -0.3, sixteen +0.5.
-// The first look comes late, too, with few tokens: 135M, one sequence -2.1 % without and -3.7 to -4.7 with 300 ns; two to six +0.3 to +2.9 and, with
-// 500 ns, -0.8 to -2.0; sixteen -2.9 and -2.0.
-__host__ __device__ constexpr int stream_look_late(int tm) { return tm == 1 ? 300 : (tm <= 8 ? 500 : 0); }  // ns
+// brings them their weights, and those that are through and have no fence to wait for look for the others' results all the longer.  With nine
+// to sixteen, who wait for more anyway, it is as well there.  With 32 tokens there is no difference.  A step, fence on the way -> aside (60
+// to 1900 positions): 135M shape, one sequence -2.1 %, ten -4.5, sixteen -2.9; 0.5B, one -5.2, eight -3.4, ten -4.4, sixteen -3.6; 1.7B, whose
+// gate and up the ring does not hold, one 0, two to six +1.0 to 1.3, nine -1.5 to -2.4, twelve and fourteen -1.3 to -1.7, sixteen -1.7 to -2.7.
+// With one token the first look at down_proj's operand comes late, too: it is not there at once, and a look that comes too early is in
+// the way of the stores.  Without the 300 ns: 135M +1.5 to 3.8 %, 0.5B +0.3 to 0.7, 1.7B +0.4 to 0.5.  (Two to eight tokens gain nothing in the
+// mean, 500 ns: 135M -0.2, 0.5B +0.5.  One look first and a rest only where the operand is unset, one token: 135M +3.8 to 6.5, 0.5B +1.4
+// to 2.2, 1.7B +1.2.)
+constexpr int kStreamLookLate = 300;  // ns
 template <int TM>
 __device__ __forceinline__ bool stream_fence_aside(const KParams& p, int grid) {
   if (TM != 8) return TM < 32;

@@ -322,7 +322,7 @@ __device__ __forceinline__ void stream_project(const KParams& p, StreamThread& t
                              wtid, frag);
     };
     if constexpr (!NORM) {
-      if (stream_look_late(TM) > 0 && kind == SP_DOWN && (TM == 1 || sm->fence_aside)) __nanosleep(stream_look_late(TM));
+      if (TM == 1 && kind == SP_DOWN && left == count) __nanosleep(kStreamLookLate);
       fetch(0);
     } else if constexpr (TM == 1) {
       stream_operand_spread<NC>(p, sm, src, normw, k, ncopy, live, wtid, frag);
