@@ -9,7 +9,7 @@
 // Projections: D[tokens, rows] = X[tokens, K] . W[rows, K]^T on tcgen05 with the tokens on the MMA's M side, so that a thread
 // of the epilogue has one token's row: contiguous outputs (32-byte stores), the two halves of a RoPE pair, gate and up.
 // A CTA pair works on up to 256 tokens x up to 256 rows (cta_group::2): each CTA brings its own half of the tokens and half of the
-// weight rows, which is half of the bytes per product of two CTAs on their own, and L2 is what bounds them.  With 65 to 128 tokens
+// weight rows, which is half of the bytes per product of two CTAs on their own, and L2 is what bounds them.  Up to 128 tokens
 // the pair's MMA has 128 rows, 64 to a CTA, and its columns lie in two halves: lanes 0-63 of tensor memory have the columns of
 // the first CTA's weight rows, lanes 64-127 those of the second's.
 #pragma once
@@ -188,7 +188,7 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
     p.b0 = seg == 0 ? g.b[0] : (seg == 1 ? g.b[1] : g.b[2]);
     p.b1 = g.b[1];
     p.b_row = (u.tile - (seg == 0 ? 0 : (seg == 1 ? g.tile_start[1] : g.tile_start[2]))) * g.rows + (CTAS == 2 ? rank * (g.rows / 2) : 0);
-    p.a_row = u.tt * CTAS * TM + rank * TM;
+    p.a_row = u.tt * CTAS * TM + rank * g.cta_tokens;
     p.chunk0 = u.slice * g.kslice;
     return p;
   };
@@ -334,6 +334,7 @@ __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t ac
   // the first half of the tile's columns and lane 64 + r the second.
   const int warp_row = kNarrow ? (quad & 1) * 32 : (TM == 64 ? quad * 16 : quad * 32);
   const int row = CTAS == 1 && TM == 64 ? (lane < 16 ? warp_row + lane : TM) : warp_row + lane;
+  const int cta_rows = kNarrow ? g.cta_tokens : TM;
   const int rows = kNarrow ? g.rows / 2 : g.rows, half = kNarrow ? (quad >> 1) * rows : 0;  // weight rows of the warp, and where they begin
   grid_dependency_wait();
   const PromptWait w{&g.guard, clock64() + g.guard.timeout_cycles};
@@ -347,10 +348,10 @@ __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t ac
     if (EPI == PE_QKV) seg = u.tile >= g.tile_start[2] ? 2 : (u.tile >= g.tile_start[1] ? 1 : 0);
     const int n0 = (u.tile - g.tile_start[seg]) * g.rows + half;  // the warp's first row in its matrix
     const int live = min(rows, g.n[seg] - n0);                    // how many it has (none, if the matrix ends before)
-    const int token0 = u.tt * CTAS * TM + rank * TM;
+    const int token0 = u.tt * CTAS * TM + rank * cta_rows;
     const int token = token0 + row;
-    const bool mine = row < TM && token < g.m;
-    const bool any = warp_row < TM && token0 + warp_row < g.m;  // the warp has a token
+    const bool mine = row < cta_rows && token < g.m;
+    const bool any = warp_row < cta_rows && token0 + warp_row < g.m;  // the warp has a token
     const uint32_t acc = tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * 256;
     const bool ok = __all_sync(0xffffffffu, prompt_wait(w, accfull0 + buf * 8u, use & 1u, SITE_EPI_ACC));
     if (!ok) return;

@@ -15,17 +15,11 @@ enum { PP_QKV = 0, PP_O = 1, PP_GU = 2, PP_DOWN = 3, PP_HEAD = 4, kPromptPhases 
 // the tokens and half of the weight tile), and tiles chosen for one, two, or three and more of those (beyond three the cut of three:
 // 1.7B shape, 1024 tokens 4422 us, 2048 8316).  Up to 128 tokens it is bound by reading the weights, and by what the SMs take out of
 // L2, weights and tokens: a CTA on its own brings every token beside its weights, one of a pair half of them, a quarter to half of
-// all it takes in.  So from 65 tokens on q/k/v, gate/up and the output head run on narrow pairs (an MMA of 128 rows, 64 to a CTA); o_proj
-// and down_proj do not: their slices take fewer tokens, and 64 pairs, which is what their tiles come to, leave SMs idle that the blocks
-// of the norm behind them, one to a row, then crowd on.  Up to 64 tokens CTAs on their own, whose MMAs have 64 rows then, are level
-// with pairs, and ahead with very few.  us, on their own / narrow pairs (135M, 0.5B, 1.7B shape and eight layers of the 8B shape):
-//   tokens      1            16            64            65            100            128
-//   135M     870 /  878    897 /  918    954 /  958   1081 / 1020   1061 / 1027    1037 / 1030
-//   0.5B     969 /  978    980 /  977   1015 /  993   1207 / 1094   1070 / 1027    1090 / 1044
-//   1.7B    1226 / 1269   1236 / 1239   1249 / 1241   1494 / 1383   1435 / 1371    1447 / 1392
-//   8B       988 /  982    986 /  976   1025 / 1011   1099 / 1069   1141 / 1107    1174 / 1135
-constexpr int kPromptClasses = 5;
-constexpr int kPromptShort = 64;  // tokens of the MMA rows of a CTA on its own, up to which there are no pairs
+// all it takes in.  So q/k/v, gate/up and the output head run on narrow pairs (an MMA of 128 rows, 64 to a CTA; us against single CTAs,
+// 1.7B shape, 64 tokens 1283 -> 1284, 100 1479 -> 1422, 128 1476 -> 1419; 135M, 64 1058 -> 996; 0.5B, 128 1120 -> 1074).  o_proj and down_proj
+// do not: their slices take fewer tokens, and 64 pairs, which is what their tiles come to, leave SMs idle that the blocks of the norm
+// behind them, one to a row, then crowd on (1.7B shape, 64 tokens, us of a layer: the two projections -1.7, the two norms +3.2).
+constexpr int kPromptClasses = 4;
 constexpr int kPromptRow = 128;   // token rows per CTA (64 rows are used for up to 64 tokens)
 constexpr int kPromptStages = 16; // most stages of a pipeline
 // Shared memory of a projection's CTA: one per SM, whose first stages travel while the kernels before it end.  (With two to an
@@ -38,12 +32,9 @@ constexpr int kPromptSmem = 225 * 1024;
 constexpr int kOperandTiles = 4, kOperandChunks = 4, kOperandKinds = 3;
 enum { kOperandXnorm = 0, kOperandAttn = 1, kOperandAct = 2 };
 
-// CTAs on their own, narrow pairs, then one, two, three and more pairs' rows of tokens.
 inline int prompt_class(int tokens, int grid) {
-  if (tokens <= kPromptShort || grid < 2) return 0;
-  return tokens <= kPromptRow ? 1 : std::min(4, 1 + (tokens + 2 * kPromptRow - 1) / (2 * kPromptRow));
+  return tokens <= kPromptRow || grid < 2 ? 0 : std::min(3, (tokens + 2 * kPromptRow - 1) / (2 * kPromptRow));
 }
-inline bool prompt_wide(int cls) { return cls > 1; }
 
 // One projection, the same for every layer of a class.
 struct PromptPhase {
@@ -56,8 +47,8 @@ struct PromptPhase {
 };
 
 // Whether a projection runs on pairs with 64 MMA rows to a CTA, and on pairs at all.
-inline bool prompt_narrow(int kind, int cls) { return cls == 1 && kind != PP_O && kind != PP_DOWN; }
-inline bool prompt_pairs(int kind, int cls) { return prompt_wide(cls) || prompt_narrow(kind, cls); }
+inline bool prompt_narrow(int kind, int cls, int grid) { return cls == 0 && grid >= 2 && kind != PP_O && kind != PP_DOWN; }
+inline bool prompt_pairs(int kind, int cls, int grid) { return cls > 0 || prompt_narrow(kind, cls, grid); }
 
 inline void prompt_tiles(PromptPhase& p, int rows) {
   p.rows = rows;
@@ -82,7 +73,7 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
     p.nmat = i == PP_GU ? 2 : 1;
     p.n[0] = ns[i];
     if (i == PP_QKV) p.n[1] = p.n[2] = kv_size;
-    const bool wide = prompt_wide(cls), narrow = prompt_narrow(i, cls), may_split = i == PP_O || i == PP_DOWN;
+    const bool wide = cls > 0, narrow = prompt_narrow(i, cls, grid), may_split = i == PP_O || i == PP_DOWN;
     // A tile of q or k rows is whole heads: its epilogue rotates pairs half a head apart (a narrow pair's halves lie in different
     // lanes of tensor memory: whole heads each).  Elsewhere the MMA's N decides for a pair (multiples of 32), the logits' 32-byte
     // stores, the swizzle's eight rows otherwise.
@@ -101,7 +92,7 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
         if (wide) {
           // per chunk: the MMAs (an N = 256 one of a pair takes 128 cycles) or the operands out of L2 at 44 bytes per cycle
           // and SM; plus what a unit costs besides, its epilogue included
-          const long long units = static_cast<long long>(t.tile_start[3]) * split * (cls - 1), pairs = std::max(1, grid / 2);
+          const long long units = static_cast<long long>(t.tile_start[3]) * split * cls, pairs = std::max(1, grid / 2);
           const long long chunk = std::max<long long>(2 * p.nmat * rows, (kPromptRow + p.nmat * rows / 2) * 128 / 44);
           cost = (units + pairs - 1) / pairs * (t.kslice * chunk + 2000 + 8 * rows) + split * 600;
         } else if (narrow) {
@@ -183,7 +174,7 @@ __host__ __device__ inline bool prompt_drain(int uses, int stages, Wait wait) {
 }
 
 // Rows of the weight descriptors' boxes: a CTA of a pair brings half a tile.
-inline int prompt_box_rows(const PromptPhase& p, int kind, int cls) { return prompt_pairs(kind, cls) ? p.rows / 2 : p.rows; }
+inline int prompt_box_rows(const PromptPhase& p, int kind, int cls, int grid) { return prompt_pairs(kind, cls, grid) ? p.rows / 2 : p.rows; }
 
 // ---------------------------------------------------------------------------
 // kernel parameters
@@ -213,6 +204,7 @@ struct PromptGemm {
   const long long* pos;
   int n[3], tile_start[4], out_col[3];
   int m, ld, rows, nmat;
+  int cta_tokens;           // tokens of a CTA of a pair (narrow: 16, 32 or 64 of the MMA's 64 rows)
   int ksplit, kslice;
   int token_tiles, units;
   int kb;                                     // K chunks per stage
