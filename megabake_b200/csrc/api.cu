@@ -921,9 +921,9 @@ int mk_bind_weights(mk_handle h, const mk_weights* w, void* stream) {
         const int rows[7] = {q_size, kv_size, kv_size, c.hidden, c.intermediate, c.intermediate, c.hidden};
         const int which[7] = {PP_QKV, PP_QKV, PP_QKV, PP_O, PP_GU, PP_GU, PP_DOWN};
         for (int i = 0; i < 7; ++i)
-          if (int e = encode_weight_map3(&to[7 * l + i], mats[i], rows[i], pp[which[i]].k, prompt_box_rows(pp[which[i]], which[i], cls, h->grid), 1)) return e;
+          if (int e = encode_weight_map3(&to[7 * l + i], mats[i], rows[i], pp[which[i]].k, prompt_box_rows(pp[which[i]], cls), 1)) return e;
       }
-      if (int e = encode_weight_map3(&to[7 * L], w->lm_head, c.vocab, c.hidden, prompt_box_rows(pp[PP_HEAD], PP_HEAD, cls, h->grid), 1)) return e;
+      if (int e = encode_weight_map3(&to[7 * L], w->lm_head, c.vocab, c.hidden, prompt_box_rows(pp[PP_HEAD], cls), 1)) return e;
     }
     MK_CUDA(cudaMemcpyAsync(at<CUtensorMap>(h, h->cv.pmaps), prompt_maps.data(), prompt_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s));
   }

@@ -42,22 +42,19 @@ __global__ void __launch_bounds__(256) prompt_stamp(const __grid_constant__ Prom
 }
 
 template <int EPI>
-cudaError_t launch_gemm(const PromptGemm& g, int kind, int cls, int grid, cudaStream_t stream) {
-  const int blocks = std::min(g.units, grid), pairs = 2 * std::min(g.units, grid / 2);
-  if (cls > 0) return launch(prompt_gemm<2, kPromptRow, EPI>, pairs, kPromptThreads, kPromptSmem, 2, true, stream, g);
-  if constexpr (EPI != PE_PARTIAL)
-    if (prompt_narrow(kind, cls, grid)) return launch(prompt_gemm<2, 64, EPI>, pairs, kPromptThreads, kPromptSmem, 2, true, stream, g);
-  if constexpr (EPI == PE_PARTIAL)
-    if (g.m <= 64) return launch(prompt_gemm<1, 64, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);
-  return launch(prompt_gemm<1, kPromptRow, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);  // (but for o and down: a handle with one SM)
+cudaError_t launch_gemm(const PromptGemm& g, int cls, int grid, cudaStream_t stream) {
+  if (cls > 0)
+    return launch(prompt_gemm<2, kPromptRow, EPI>, 2 * std::min(g.units, grid / 2), kPromptThreads, kPromptSmem, 2, true, stream, g);
+  const int blocks = std::min(g.units, grid);
+  if (g.m <= 64) return launch(prompt_gemm<1, 64, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);
+  return launch(prompt_gemm<1, kPromptRow, EPI>, blocks, kPromptThreads, kPromptSmem, 1, true, stream, g);
 }
 
 template <int EPI>
 cudaError_t prepare_gemm() {
   cudaError_t e = cudaFuncSetAttribute(prompt_gemm<2, kPromptRow, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_gemm<1, kPromptRow, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
-  constexpr int ctas = EPI == PE_PARTIAL ? 1 : 2;
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_gemm<ctas, 64, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(prompt_gemm<1, 64, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPromptSmem);
   return e;
 }
 
@@ -130,15 +127,11 @@ cudaError_t prompt_attention_launch(const AttnArgs& args, const AttnTcMaps& maps
 cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
   const mk_config& c = *pass.config;
   const int cls = pass.cls, m = pass.m, q_size = c.q_heads * c.head_dim, kv_size = c.kv_heads * c.head_dim;
+  const int per_tile = cls > 0 ? 2 * kPromptRow : (m <= 64 ? 64 : kPromptRow), rows_per_cta = cls > 0 ? kPromptRow : per_tile;
+  // the token operand's box: the smallest that holds the launch, a CTA's rows otherwise
+  const int box = m <= 16 ? 0 : (m <= 32 ? 1 : (m <= 64 ? 2 : 3)), box_rows = 16 << box;
   auto gemm = [&](int kind, int operand) {
     const PromptPhase& p = pass.phases[kind];
-    const bool narrow = prompt_narrow(kind, cls, pass.grid);
-    // (o and down of up to 64 tokens: MMAs of 64 rows)
-    const int rows_per_cta = narrow || (cls == 0 && m <= 64 && (kind == PP_O || kind == PP_DOWN)) ? 64 : kPromptRow;
-    const int per_tile = cls > 0 || narrow ? 2 * rows_per_cta : rows_per_cta;
-    // the token operand's box: the smallest that holds the launch, or a CTA's share of it
-    const int share = narrow ? (m + 1) / 2 : m;
-    const int box = share <= 16 ? 0 : (share <= 32 ? 1 : (share <= 64 ? 2 : 3)), box_rows = 16 << box;
     PromptGemm g{};
     g.guard = pass.guard;
     // Without pairs a chunk's MMAs take less than a step of the pipeline: two chunks to a stage (1.7B shape, 70 tokens 1536 ->
@@ -149,21 +142,20 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     for (int s = 0; s < 4; ++s) g.tile_start[s] = p.tile_start[s];
     g.m = m;
     g.rows = p.rows;
-    g.cta_tokens = narrow ? box_rows : kPromptRow;
     g.nmat = p.nmat;
     g.ksplit = p.ksplit;
     g.kslice = p.kslice;
     g.token_tiles = (m + per_tile - 1) / per_tile;
     g.units = p.tile_start[3] * p.ksplit * g.token_tiles;
     g.a_bytes = box_rows * 128;
-    g.b_bytes = prompt_box_rows(p, kind, cls, pass.grid) * 128;
+    g.b_bytes = prompt_box_rows(p, cls) * 128;
     g.stage_bytes = g.kb * (g.a_bytes + p.nmat * g.b_bytes);
     // an MMA reads a CTA's full rows of tokens, past a smaller box whatever lies there: room for that behind the last stage
     const int room = kPromptSmem - 1024 - rows_per_cta * 128;
     g.stages = std::min(kPromptStages, room / g.stage_bytes);  // (at least two: a stage is 64 KB at most)
     const bool joined = p.nmat == 2 && cls == 0;  // gate and up as one MMA of twice the rows
     g.instr_n = ((joined ? 2 * p.rows : p.rows) + 15) / 16 * 16;  // (a tile may end within an MMA's N: columns nobody reads)
-    g.up_column = joined ? prompt_box_rows(p, kind, cls, pass.grid) : 256;
+    g.up_column = joined ? p.rows : 256;
     g.buffers = p.nmat == 2 && !joined ? 1 : 2;
     g.head_dim = c.head_dim;
     g.max_positions = c.max_positions;
@@ -207,7 +199,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
       g.b[0] = maps;
       g.dst = pass.logits;
       g.ld = c.vocab;
-      return stamp(launch_gemm<PE_LOGITS>(g, PP_HEAD, cls, pass.grid, stream), EV_PHASE_DONE);
+      return stamp(launch_gemm<PE_LOGITS>(g, cls, pass.grid, stream), EV_PHASE_DONE);
     }
     const mk_layer_weights& lw = w.layers[l];
     PromptGemm g = gemm(PP_QKV, kOperandXnorm);
@@ -223,7 +215,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     g.cos_t = static_cast<const bf16*>(w.rope_cos);
     g.sin_t = static_cast<const bf16*>(w.rope_sin);
     g.pos = pass.pos;
-    e = stamp(launch_gemm<PE_QKV>(g, PP_QKV, cls, pass.grid, stream), EV_PHASE_DONE);
+    e = stamp(launch_gemm<PE_QKV>(g, cls, pass.grid, stream), EV_PHASE_DONE);
     if (e == cudaSuccess)
       e = stamp(prompt_attention_launch(*pass.attention, *pass.attention_maps, pass.guard, c.head_dim, c.q_heads, c.kv_heads, pass.batch, pass.grid,
                                         c.sm_limit > 0, true, stream), EV_ATTENTION_DONE);
@@ -231,7 +223,7 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     g = gemm(PP_O, kOperandAttn);
     g.b[0] = maps + 3;
     g.partial = pass.partial;
-    e = stamp(launch_gemm<PE_PARTIAL>(g, PP_O, cls, pass.grid, stream), EV_PHASE_DONE);
+    e = stamp(launch_gemm<PE_PARTIAL>(g, cls, pass.grid, stream), EV_PHASE_DONE);
     if (e != cudaSuccess) return e;
     norm.src = pass.hidden_b;
     norm.parts = pass.phases[PP_O].ksplit;
@@ -244,12 +236,12 @@ cudaError_t prompt_forward(const PromptPass& pass, cudaStream_t stream) {
     g.b[1] = maps + 5;
     g.dst = pass.act;
     g.ld = c.intermediate;
-    e = stamp(launch_gemm<PE_SILU>(g, PP_GU, cls, pass.grid, stream), EV_PHASE_DONE);
+    e = stamp(launch_gemm<PE_SILU>(g, cls, pass.grid, stream), EV_PHASE_DONE);
     if (e != cudaSuccess) return e;
     g = gemm(PP_DOWN, kOperandAct);
     g.b[0] = maps + 6;
     g.partial = pass.partial;
-    e = stamp(launch_gemm<PE_PARTIAL>(g, PP_DOWN, cls, pass.grid, stream), EV_PHASE_DONE);
+    e = stamp(launch_gemm<PE_PARTIAL>(g, cls, pass.grid, stream), EV_PHASE_DONE);
   }
   return e;
 }

@@ -8,10 +8,8 @@
 //
 // Projections: D[tokens, rows] = X[tokens, K] . W[rows, K]^T on tcgen05 with the tokens on the MMA's M side, so that a thread
 // of the epilogue has one token's row: contiguous outputs (32-byte stores), the two halves of a RoPE pair, gate and up.
-// A CTA pair works on up to 256 tokens x up to 256 rows (cta_group::2): each CTA brings its own half of the tokens and half of the
-// weight rows, which is half of the bytes per product of two CTAs on their own, and L2 is what bounds them.  Up to 128 tokens
-// the pair's MMA has 128 rows, 64 to a CTA, and its columns lie in two halves: lanes 0-63 of tensor memory have the columns of
-// the first CTA's weight rows, lanes 64-127 those of the second's.
+// Beyond 128 tokens a CTA pair works on 256 tokens x up to 256 rows (cta_group::2): each CTA brings its own 128 tokens and
+// half of the weight rows, which is half of the bytes per product of two CTAs on their own, and L2 is what bounds them.
 #pragma once
 #include "device_common.cuh"
 #include "prompt_attention.cuh"
@@ -169,7 +167,7 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
                                                 int producer) {
   const uint64_t weight_policy = g.stream_weights ? l2_policy_evict_first() : l2_policy_evict_normal();
   const uint64_t token_policy = l2_policy_evict_normal();
-  const int kb = TM == 128 && CTAS == 2 ? 1 : g.kb, groups = g.kslice / kb, nmat = g.nmat, stages = g.stages, units = g.units;
+  const int kb = CTAS == 1 ? g.kb : 1, groups = g.kslice / kb, nmat = g.nmat, stages = g.stages, units = g.units;
   const uint32_t base = smem_u32(smem), stage_bytes = g.stage_bytes, a_bytes = kb * g.a_bytes, b_bytes = g.b_bytes;
   const uint32_t tx = CTAS * stage_bytes;
   const uint32_t count0 = CTAS == 2 ? leader_address(full0) : full0;  // where copies are counted
@@ -188,7 +186,7 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
     p.b0 = seg == 0 ? g.b[0] : (seg == 1 ? g.b[1] : g.b[2]);
     p.b1 = g.b[1];
     p.b_row = (u.tile - (seg == 0 ? 0 : (seg == 1 ? g.tile_start[1] : g.tile_start[2]))) * g.rows + (CTAS == 2 ? rank * (g.rows / 2) : 0);
-    p.a_row = u.tt * CTAS * TM + rank * g.cta_tokens;
+    p.a_row = u.tt * CTAS * TM + rank * TM;
     p.chunk0 = u.slice * g.kslice;
     return p;
   };
@@ -327,15 +325,11 @@ template <int CTAS, int TM, int EPI>
 __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t accfull0, uint32_t accempty0, uint32_t tmem, int rank, int first,
                                                 int step, int ewarp, int lane) {
   constexpr int kParts = kPromptEpilogueWarps / 4;
-  constexpr bool kNarrow = CTAS == 2 && TM == 64;
   const int quad = (ewarp + kPromptFirstEpilogue) & 3;  // tensor-memory lanes a warp may read: 32 * (warp index % 4)
   const int part = ewarp >> 2;                          // the warps of a quadrant take items in turn
-  // M = 128 (or 256 of a pair): token row r is lane r.  M = 64: row r is lane 32 * (r / 16) + r % 16.  A narrow pair's: of row r, lane r has
-  // the first half of the tile's columns and lane 64 + r the second.
-  const int warp_row = kNarrow ? (quad & 1) * 32 : (TM == 64 ? quad * 16 : quad * 32);
-  const int row = CTAS == 1 && TM == 64 ? (lane < 16 ? warp_row + lane : TM) : warp_row + lane;
-  const int cta_rows = kNarrow ? g.cta_tokens : TM;
-  const int rows = kNarrow ? g.rows / 2 : g.rows, half = kNarrow ? (quad >> 1) * rows : 0;  // weight rows of the warp, and where they begin
+  // M = 128 (or 256 of a pair): token row r is lane r.  M = 64: row r is lane 32 * (r / 16) + r % 16.
+  const int row = TM == 64 ? (lane < 16 ? quad * 16 + lane : TM) : quad * 32 + lane;
+  const int warp_row = TM == 64 ? quad * 16 : quad * 32;
   grid_dependency_wait();
   const PromptWait w{&g.guard, clock64() + g.guard.timeout_cycles};
   const int refused = EPI == PE_LOGITS ? *reinterpret_cast<volatile int*>(&g.guard.ctrl->prompt_refused) : 0;
@@ -346,12 +340,12 @@ __device__ __forceinline__ void prompt_epilogue(const PromptGemm& g, uint32_t ac
     const uint32_t use = g.buffers == 2 ? (q >> 1) : q;
     int seg = 0;
     if (EPI == PE_QKV) seg = u.tile >= g.tile_start[2] ? 2 : (u.tile >= g.tile_start[1] ? 1 : 0);
-    const int n0 = (u.tile - g.tile_start[seg]) * g.rows + half;  // the warp's first row in its matrix
-    const int live = min(rows, g.n[seg] - n0);                    // how many it has (none, if the matrix ends before)
-    const int token0 = u.tt * CTAS * TM + rank * cta_rows;
+    const int n0 = (u.tile - g.tile_start[seg]) * g.rows;        // first row of the tile in its matrix
+    const int live = min(g.rows, g.n[seg] - n0);                 // rows of the tile
+    const int token0 = u.tt * CTAS * TM + rank * TM;
     const int token = token0 + row;
-    const bool mine = row < cta_rows && token < g.m;
-    const bool any = warp_row < cta_rows && token0 + warp_row < g.m;  // the warp has a token
+    const bool mine = row < TM && token < g.m;
+    const bool any = token0 + warp_row < g.m;                    // the warp has a token
     const uint32_t acc = tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * 256;
     const bool ok = __all_sync(0xffffffffu, prompt_wait(w, accfull0 + buf * 8u, use & 1u, SITE_EPI_ACC));
     if (!ok) return;
@@ -509,13 +503,9 @@ __global__ void __launch_bounds__(kPromptThreads, 1) prompt_gemm(const __grid_co
     if (lane == 0) prompt_producer<CTAS, TM>(g, smem, full0, empty0, rank, first, step, warp);
   } else if (warp == kPromptMmaWarp) {
     grid_dependency_wait();
-    constexpr int kBlocks = CTAS == 2 && TM == 128 && EPI == PE_SILU ? 2 : 1;
-    constexpr bool kDouble = CTAS == 1 || TM == 64;  // stages of two chunks
-    if (kDouble && g.kb == 2) {
-      if (rank == 0) prompt_mma_loop<CTAS, TM, kDouble ? 2 : 1, 1>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
-    } else if (rank == 0) {
-      prompt_mma_loop<CTAS, TM, 1, kBlocks>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
-    }
+    constexpr int kBlocks = CTAS == 2 && EPI == PE_SILU ? 2 : 1;
+    if (CTAS == 1 && g.kb == 2) prompt_mma_loop<1, TM, 2, 1>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
+    else if (rank == 0) prompt_mma_loop<CTAS, TM, 1, kBlocks>(g, smem_u32(smem), full0, empty0, accfull0, accempty0, tmem, first, step);
   } else {
     prompt_epilogue<CTAS, TM, EPI>(g, accfull0, accempty0, tmem, rank, first, step, warp - kPromptFirstEpilogue, lane);
   }

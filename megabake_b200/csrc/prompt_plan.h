@@ -11,14 +11,12 @@ namespace mk {
 
 enum { PP_QKV = 0, PP_O = 1, PP_GU = 2, PP_DOWN = 3, PP_HEAD = 4, kPromptPhases = 5 };
 
-// Launch classes.  Beyond 128 tokens a prompt is bound by tensor cores and L2: CTA pairs with 256 tokens each (each CTA brings half of
-// the tokens and half of the weight tile), and tiles chosen for one, two, or three and more of those (beyond three the cut of three:
-// 1.7B shape, 1024 tokens 4422 us, 2048 8316).  Up to 128 tokens it is bound by reading the weights, and by what the SMs take out of
-// L2, weights and tokens: a CTA on its own brings every token beside its weights, one of a pair half of them, a quarter to half of
-// all it takes in.  So q/k/v, gate/up and the output head run on narrow pairs (an MMA of 128 rows, 64 to a CTA; us against single CTAs,
-// 1.7B shape, 64 tokens 1283 -> 1284, 100 1479 -> 1422, 128 1476 -> 1419; 135M, 64 1058 -> 996; 0.5B, 128 1120 -> 1074).  o_proj and down_proj
-// do not: their slices take fewer tokens, and 64 pairs, which is what their tiles come to, leave SMs idle that the blocks of the norm
-// behind them, one to a row, then crowd on (1.7B shape, 64 tokens, us of a layer: the two projections -1.7, the two norms +3.2).
+// Launch classes.  Up to 128 tokens a prompt is bound by reading the weights: one CTA per tile, and tiles that give every SM
+// some.  (Pairs with 64 MMA rows to a CTA for q/k/v, gate/up and the head are level up to 64 tokens and faster from 65 on, 1.7B shape, us,
+// one CTA / a pair: 1 token 1226 / 1269, 64 1249 / 1241, 65 1494 / 1383, 100 1435 / 1371, 128 1447 / 1392; 0.5B, 128 1090 / 1044.  But a
+// unit's walk along K begins at a place that the number of CTAs decides, so they add the same products up in another order: 2.5 % at the
+// logits after 24 layers, no further from 64-bit results, and further than results may move.)  Beyond, by tensor cores and L2: CTA pairs (256 tokens each), and tiles chosen for one, two, or three and more of
+// those (beyond three the cut of three: 1.7B shape, 1024 tokens 4422 us, 2048 8316).
 constexpr int kPromptClasses = 4;
 constexpr int kPromptRow = 128;   // token rows per CTA (64 rows are used for up to 64 tokens)
 constexpr int kPromptStages = 16; // most stages of a pipeline
@@ -46,10 +44,6 @@ struct PromptPhase {
   int ksplit, kslice;    // K slices, and chunks per slice
 };
 
-// Whether a projection runs on pairs with 64 MMA rows to a CTA, and on pairs at all.
-inline bool prompt_narrow(int kind, int cls, int grid) { return cls == 0 && grid >= 2 && kind != PP_O && kind != PP_DOWN; }
-inline bool prompt_pairs(int kind, int cls, int grid) { return cls > 0 || prompt_narrow(kind, cls, grid); }
-
 inline void prompt_tiles(PromptPhase& p, int rows) {
   p.rows = rows;
   int tiles = 0;
@@ -73,12 +67,11 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
     p.nmat = i == PP_GU ? 2 : 1;
     p.n[0] = ns[i];
     if (i == PP_QKV) p.n[1] = p.n[2] = kv_size;
-    const bool wide = cls > 0, narrow = prompt_narrow(i, cls, grid), may_split = i == PP_O || i == PP_DOWN;
-    // A tile of q or k rows is whole heads: its epilogue rotates pairs half a head apart (a narrow pair's halves lie in different
-    // lanes of tensor memory: whole heads each).  Elsewhere the MMA's N decides for a pair (multiples of 32), the logits' 32-byte
-    // stores, the swizzle's eight rows otherwise.
-    const int step = i == PP_QKV ? c.head_dim * (narrow ? 2 : 1) : (wide ? 32 : (narrow ? 32 / p.nmat : (i == PP_HEAD ? 16 : 8)));
-    const int most = wide ? 256 : (narrow ? 256 : 128) / p.nmat;
+    const bool wide = cls > 0, may_split = i == PP_O || i == PP_DOWN;
+    // A tile of q or k rows is whole heads: its epilogue rotates pairs half a head apart.  Elsewhere the MMA's N decides for a
+    // pair (multiples of 32), the logits' 32-byte stores, the swizzle's eight rows otherwise.
+    const int step = i == PP_QKV ? c.head_dim : (wide ? 32 : (i == PP_HEAD ? 16 : 8));
+    const int most = wide ? 256 : 128 / p.nmat;
     long long best = -1;
     PromptPhase chosen = p;
     for (int split = 1; split <= (may_split ? kMaxSplit : 1); ++split) {
@@ -95,12 +88,6 @@ inline void prompt_phases(const mk_config& c, int cls, int grid, PromptPhase* ou
           const long long units = static_cast<long long>(t.tile_start[3]) * split * cls, pairs = std::max(1, grid / 2);
           const long long chunk = std::max<long long>(2 * p.nmat * rows, (kPromptRow + p.nmat * rows / 2) * 128 / 44);
           cost = (units + pairs - 1) / pairs * (t.kslice * chunk + 2000 + 8 * rows) + split * 600;
-        } else if (narrow) {
-          // per chunk of the busiest SM: its weights out of HBM at 30 bytes per cycle, weights and (32) tokens out of L2 at 42, or the
-          // MMAs
-          const long long units = static_cast<long long>(t.tile_start[3]) * split, pairs = grid / 2;
-          const long long chunk = std::max({p.nmat * rows * 128 / 60, (32 + p.nmat * rows / 2) * 128 / 42, 2 * p.nmat * rows, 256});
-          cost = (units + pairs - 1) / pairs * (t.kslice * chunk + 2500) + split * 300;
         } else {
           // per chunk of the busiest SM: its weights at 30 bytes per cycle, weights and (64) tokens at 42, or the pipeline's step
           const long long units = static_cast<long long>(t.tile_start[3]) * split;
@@ -174,7 +161,7 @@ __host__ __device__ inline bool prompt_drain(int uses, int stages, Wait wait) {
 }
 
 // Rows of the weight descriptors' boxes: a CTA of a pair brings half a tile.
-inline int prompt_box_rows(const PromptPhase& p, int kind, int cls, int grid) { return prompt_pairs(kind, cls, grid) ? p.rows / 2 : p.rows; }
+inline int prompt_box_rows(const PromptPhase& p, int cls) { return cls > 0 ? p.rows / 2 : p.rows; }
 
 // ---------------------------------------------------------------------------
 // kernel parameters
@@ -204,7 +191,6 @@ struct PromptGemm {
   const long long* pos;
   int n[3], tile_start[4], out_col[3];
   int m, ld, rows, nmat;
-  int cta_tokens;           // tokens of a CTA of a pair (narrow: 16, 32 or 64 of the MMA's 64 rows)
   int ksplit, kslice;
   int token_tiles, units;
   int kb;                                     // K chunks per stage
