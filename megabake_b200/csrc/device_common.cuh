@@ -109,7 +109,7 @@ __device__ __forceinline__ float silu_inner(float x) {
 
 // A value that rounds to the bf16 of the division's result, from two approximations and no branch: for each of the 65536 bf16 x,
 // infinities and not-numbers included.  (The reciprocal must not flush: 2^-127 times x = -88 is a normal bf16.)  In the prompts' gate/up, whose
-// epilogue follows its unit, 1.7B shape, 64 tokens 1284 -> 1267 us, 128 1419 -> 1403, 300 2282 -> 2225, 512 2598 -> 2515.
+// epilogue follows its unit, 1.7B shape, 64 tokens 1264 -> 1252 us, 128 1437 -> 1426, 300 2261 -> 2226, 512 2432 -> 2409.
 __device__ __forceinline__ float silu_to_bf16(float x) {
   float y;
   asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(1.0f + ex2(x * -kLog2e)));

@@ -219,8 +219,8 @@ __device__ __forceinline__ void prompt_producer(const PromptGemm& g, uint8_t* sm
     load_b(p, chunk_of(p, n - unit * groups), n);
   }
   // What the kernels before have written is complete and visible when this wait ends, to copies as to loads, as at any end of a kernel: a
-  // proxy fence here is for nothing and takes 0.3 us of every projection (64 tokens of the 1.7B shape 1272 -> 1252 us, 128 1406 -> 1386;
-  // 135M, 128 tokens 1057 -> 1017).
+  // proxy fence here is for nothing and takes 0.3 us of every projection (64 tokens of the 1.7B shape 1267 -> 1252 us, 128 1452 -> 1426;
+  // 135M, 128 tokens 1077 -> 1034).
   grid_dependency_wait();
   grid_dependents_go();
   const PromptWait w{&g.guard, clock64() + g.guard.timeout_cycles};
